@@ -24,7 +24,7 @@
 // CTA finds its group and row tile from the run starts on the device; boxes that reach into the next run are multiplied along and
 // not stored. The activation of an expert is folded into the epilogue, which then writes the bf16 operand of the next product.
 //
-// Kernel. One CTA = 128 tokens x 128 outputs over a slice of k (split-k fills the GPU when there are few
+// Kernels. Up to 64 rows given as a pair of planes: linear_few_kernel, below. More rows, or one plane: one CTA = 128 tokens x 128 outputs over a slice of k (split-k fills the GPU when there are few
 // output tiles; slices go to a scratch and are summed in slice order, by a small kernel or by the kernel
 // that consumes the product, so results are reproducible). 6 warps: warp 0 streams [128 rows][64 k] boxes of hi, lo and W (128-byte swizzle, 48 KB per
 // stage, 4 stages) with TMA; warp 1 issues tcgen05.mma (kind::f16, M = N = 128, K = 16; all lanes walk the
@@ -378,6 +378,286 @@ linear_sm100_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_con
     }
 }
 
+// ---- few rows ----------------------------------------------------------------------------------------------------------
+//
+// Products of up to kFewRows rows whose activations are a pair of planes: decoded tokens, short prompts, experts with a few rows each.
+// What bounds them is reading the weights once. The tiles above give a stage of 16 KB of weights 32 KB for activation rows that are
+// mostly padding, so that 64 KB of weights are on their way per SM, and every output tile starts and drains a pipeline of its own.
+// Here the weights are the M side of the MMA (128 outputs) and the rows its N side, hi and lo planes side by side (N = 2 x rows padded to
+// 8; both halves of the accumulator are added on the way out): a stage is 16 KB of weights and 256 bytes per padded row, two
+// CTAs share an SM, and a CTA goes through its share of the items (output tile, k slice, group) with one ring and two accumulators,
+// so loads run on across items and into the kernel before (its weights do not depend on it).
+// Measured (B200, inside a decoding step, against the 128-row tiles): 16384 x 2048 by 8 rows 13.2 us (17.3 before; 5.1 TB/s), 32768 x 2048
+// by 8 rows 22.7 us (35.3; 5.9 TB/s), about 30 experts of 2816 x 2048 with a row each 45 us (84), their 2048 x 1408 down products 27 us (56).
+constexpr int kFewRows = 64;  // as many as two CTAs per SM have tensor memory for: 2 accumulators x 2 planes x 64 rows = 256 columns
+constexpr int kFewStages = 6, kFewGroups = 512;
+constexpr int kFewSmem = 115712;  // half of what an SM has, less what is reserved per CTA
+struct FewParams {
+    GemmParams g;
+    int rows;            // padded rows: of an activation box
+    int n_stages, items; // items: the most there can be
+    int tmem_cols;       // of one accumulator: a power of two, at least 2 x rows
+    uint32_t idesc;
+    int off_swap, off_groups, off_bar;  // shared memory behind the ring: up halves on their way to the gate halves, groups with rows
+};
+struct FewBars {
+    uint64_t full[kFewStages], empty[kFewStages], acc_full[2], acc_empty[2];
+    uint32_t tmem_base, abort_flag;
+    int n_groups;
+};
+
+// Barrier of two warps that says whether all their threads passed true.
+__device__ __forceinline__ bool pair_all(int barrier, bool v) {
+    uint32_t r;
+    asm volatile("{\n.reg .pred p, q;\nsetp.ne.u32 q, %2, 0;\nbar.red.and.pred p, %1, 64, q;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(r) : "r"(barrier), "r"((uint32_t)v) : "memory");
+    return r != 0;
+}
+
+template <bool kGrouped>
+__global__ void __launch_bounds__(kThreads, 2)
+linear_few_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_constant__ CUtensorMap map_lo,
+                  const __grid_constant__ CUtensorMap map_w0, const __grid_constant__ CUtensorMap map_w1,
+                  const __grid_constant__ CUtensorMap map_w2, const FewParams fp) {
+    const GemmParams& p = fp.g;
+    extern __shared__ unsigned char smem_dyn[];
+    const uint32_t smem_base = (smem_u32(smem_dyn) + 1023u) & ~1023u;
+    unsigned char* smem_al = smem_dyn + (smem_base - smem_u32(smem_dyn));
+    FewBars* bars = reinterpret_cast<FewBars*>(smem_al + fp.off_bar);
+    int* group_list = reinterpret_cast<int*>(smem_al + fp.off_groups);  // {group, first row, end} of the groups that have rows
+    volatile uint32_t* abort_flag = &bars->abort_flag;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp_u = __shfl_sync(0xffffffffu, warp, 0);
+    const int n_stages = fp.n_stages, plane_bytes = fp.rows * kBK * 2, stage_bytes = kBoxBytes + 2 * plane_bytes;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < n_stages; s++) { mbar_init(smem_u32(&bars->full[s]), 1); mbar_init(smem_u32(&bars->empty[s]), 1); }
+        for (int b = 0; b < 2; b++) { mbar_init(smem_u32(&bars->acc_full[b]), 1); mbar_init(smem_u32(&bars->acc_empty[b]), 4); }
+        bars->abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&bars->tmem_base)), "r"(2u * fp.tmem_cols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if (kGrouped) {
+        LINEAR_PDL_WAIT();  // the runs come from a kernel before
+        if (warp == 0) {
+            int count = 0;
+            for (int g0 = 0; g0 < p.n_groups; g0 += 32) {
+                const int mine = g0 + lane;
+                const int a = mine < p.n_groups ? p.group_start[mine] : 0, b = mine < p.n_groups ? p.group_start[mine + 1] : 0;
+                const unsigned some = __ballot_sync(0xffffffffu, b > a);
+                if (b > a) {
+                    int* e = group_list + 3 * (count + __popc(some & ((1u << lane) - 1)));
+                    e[0] = mine; e[1] = a; e[2] = b;
+                }
+                count += __popc(some);
+            }
+            if (lane == 0) bars->n_groups = count;
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    // Only now: a kernel that starts early and shares the SM must find its predecessor's tensor memory taken already.
+    LINEAR_PDL_TRIGGER();
+    const uint32_t tmem = bars->tmem_base;
+    const int n_items = kGrouped ? bars->n_groups * p.tiles_n : fp.items;
+
+    struct Item { int mat, n0, col_end, a_k0, m0, row_end, w_row0, k_begin, n_it, blk, split; };
+    auto item_at = [&](int index) {
+        Item t;
+        const int tile_n = index % p.tiles_n, rest = index / p.tiles_n;  // the k slice, or the group
+        t.split = kGrouped ? 0 : rest;
+        t.mat = (tile_n >= p.tile_end[0]) + (tile_n >= p.tile_end[1]);
+        const int n_out = t.mat == 0 ? p.n_out[0] : t.mat == 1 ? p.n_out[1] : p.n_out[2];
+        t.blk = p.tiles_per_block > 0 ? tile_n / p.tiles_per_block : 0;
+        t.col_end = p.tiles_per_block > 0 ? (t.blk + 1) * p.rows_per_block : n_out;
+        t.a_k0 = t.blk * p.k_block;
+        t.n0 = p.tiles_per_block > 0 ? t.blk * p.rows_per_block + (tile_n - t.blk * p.tiles_per_block) * 128
+                                     : (tile_n - (t.mat == 0 ? 0 : t.mat == 1 ? p.tile_end[0] : p.tile_end[1])) * 128;
+        t.m0 = kGrouped ? group_list[3 * rest + 1] : 0;
+        t.row_end = kGrouped ? group_list[3 * rest + 2] : p.n_tok;
+        t.w_row0 = kGrouped ? group_list[3 * rest] * n_out + t.n0 : t.n0;
+        t.k_begin = (int)((long long)p.k_steps * t.split / p.n_split);
+        t.n_it = (int)((long long)p.k_steps * (t.split + 1) / p.n_split) - t.k_begin;
+        return t;
+    };
+    auto map_of_mat = [&](int mat) { return mat == 0 ? &map_w0 : mat == 1 ? &map_w1 : &map_w2; };
+
+    // The weights of the first item that fit the ring are requested before the wait for the kernel before.
+    const bool any = (int)blockIdx.x < n_items;
+    int n_pre = 0;
+    if (warp_u == 0 && any) {
+        const Item t = item_at(blockIdx.x);
+        n_pre = min(t.n_it, n_stages);
+        if (lane == 0)
+            for (int it = 0; it < n_pre; it++) {
+                const uint32_t full = smem_u32(&bars->full[it]);
+                mbar_expect_tx(full, stage_bytes);
+                tma_load_2d(smem_base + it * stage_bytes, map_of_mat(t.mat), (t.k_begin + it) * kBK, t.w_row0, full);
+            }
+    }
+    if (!kGrouped) LINEAR_PDL_WAIT();
+
+    if (warp_u == 0) {
+        // ---------------- TMA producer ----------------
+        int done = 0, s = 0;  // k-steps requested, ring slot
+        uint32_t round = 0;
+        bool ok = true;
+        for (int index = blockIdx.x; index < n_items && ok; index += gridDim.x) {
+            const Item t = item_at(index);
+            for (int it = 0; it < t.n_it && ok; it++) {
+                if (lane == 0) {
+                    const uint32_t full = smem_u32(&bars->full[s]), dst = smem_base + s * stage_bytes;
+                    const int k = (t.k_begin + it) * kBK;
+                    if (done >= n_pre) {
+                        ok = mbar_wait(smem_u32(&bars->empty[s]), (round & 1) ^ 1, abort_flag, kWaitLimitNs);
+                        if (ok) {
+                            mbar_expect_tx(full, stage_bytes);
+                            tma_load_2d(dst, map_of_mat(t.mat), k, t.w_row0, full);
+                        }
+                    }
+                    if (ok) {
+                        tma_load_2d(dst + kBoxBytes, &map_hi, t.a_k0 + k, t.m0, full);
+                        tma_load_2d(dst + kBoxBytes + plane_bytes, &map_lo, t.a_k0 + k, t.m0, full);
+                    }
+                }
+                ok = __shfl_sync(0xffffffffu, ok, 0);
+                if (ok) {
+                    done++;
+                    if (++s == n_stages) { s = 0; round++; }
+                }
+            }
+        }
+        if (!ok && lane == 0) {
+            // copies already issued must land before the CTA's shared memory is released
+            for (int it = max(0, done - n_stages); it < done; it++) {
+                const uint64_t t0 = globaltimer_ns();
+                while (!mbar_try_wait(smem_u32(&bars->full[it % n_stages]), (uint32_t)((it / n_stages) & 1)) && globaltimer_ns() - t0 < 100000000ull) {}
+            }
+        }
+    } else if (warp_u == 1) {
+        // ---------------- MMA issuer ----------------
+        int s = 0, j = 0;
+        uint32_t round = 0;
+        bool ok = true;
+        for (int index = blockIdx.x; index < n_items && ok; index += gridDim.x, j++) {
+            const Item t = item_at(index);
+            const uint32_t acc = tmem + (uint32_t)((j & 1) * fp.tmem_cols);
+            ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars->acc_empty[j & 1]), (uint32_t)((j >> 1) & 1) ^ 1, abort_flag, kWaitLimitNs)) != 0;
+            for (int it = 0; it < t.n_it && ok; it++) {
+                ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars->full[s]), round & 1, abort_flag, kWaitLimitNs)) != 0;
+                if (!ok) break;
+                tc_fence_after();
+                if (elect_one()) {
+                    const uint32_t a = smem_base + s * stage_bytes, b = a + kBoxBytes;
+#pragma unroll
+                    for (int ks = 0; ks < kBK / 16; ks++)
+                        tc_mma_ss(acc, make_desc(a + ks * 32, 16, 1024), make_desc(b + ks * 32, 16, 1024), fp.idesc, (it > 0 || ks > 0) ? 1u : 0u);
+                    tc_commit(smem_u32(&bars->empty[s]));
+                    if (it == t.n_it - 1) tc_commit(smem_u32(&bars->acc_full[j & 1]));
+                }
+                __syncwarp();
+                if (++s == n_stages) { s = 0; round++; }
+            }
+        }
+    } else {
+        // ---------------- epilogue: one thread per output, eight rows at a time ----------------
+        const int lg = warp & 3;  // the tensor-memory lane group this warp may read
+        float* const swap = reinterpret_cast<float*>(smem_al + fp.off_swap) + (lg >> 1) * fp.rows * 32;  // [row][32] of a gate / up pair of warps
+        const bool split_k = p.n_split > 1 || p.to_partial;
+        int j = 0;
+        bool ok = true;
+        for (int index = blockIdx.x; index < n_items && ok; index += gridDim.x, j++) {
+            const Item t = item_at(index);
+            ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars->acc_full[j & 1]), (uint32_t)((j >> 1) & 1), abort_flag, kWaitLimitNs)) != 0;
+            if (kGrouped && p.act == 2) ok = pair_all(1 + (lg >> 1), ok);  // they go on, or leave, together
+            if (!ok) break;
+            tc_fence_after();
+            const uint32_t acc = tmem + (uint32_t)((j & 1) * fp.tmem_cols) + ((uint32_t)(lg * 32) << 16);
+            const int n_out = t.mat == 0 ? p.n_out[0] : t.mat == 1 ? p.n_out[1] : p.n_out[2];
+            const int col = t.n0 + lg * 32 + lane, n_rows = t.row_end - t.m0;
+            auto read = [&](int c, float (&v)[8]) {  // rows c .. c + 7 of this thread's output
+                float lo[8];
+                tmem_ld8(acc + c, v);
+                tmem_ld8(acc + fp.rows + c, lo);
+                tmem_wait_ld();
+#pragma unroll
+                for (int i = 0; i < 8; i++) v[i] += lo[i];
+            };
+            auto put_pair = [&](size_t at, float x) {
+                const __nv_bfloat16 h = __float2bfloat16_rn(x);
+                p.out_hi[at] = h;
+                if (p.out_lo) p.out_lo[at] = __float2bfloat16_rn(x - __bfloat162float(h));
+            };
+            if (kGrouped && p.act == 2) {
+                // runs of 32 gate outputs, each followed by the 32 up outputs that go with them: one warp's lanes and the next one's
+                if (lg & 1)
+                    for (int c = 0; c < n_rows; c += 8) {
+                        float v[8];
+                        read(c, v);
+#pragma unroll
+                        for (int i = 0; i < 8; i++)
+                            if (c + i < n_rows) swap[(c + i) * 32 + lane] = v[i];
+                    }
+                asm volatile("bar.sync %0, 64;" ::"r"(1 + (lg >> 1)) : "memory");
+                if (!(lg & 1) && col < t.col_end) {
+                    const int half_out = n_out / 2, out_col = t.n0 / 2 + (lg >> 1) * 32 + lane;
+                    for (int c = 0; c < n_rows; c += 8) {
+                        float v[8];
+                        read(c, v);
+#pragma unroll
+                        for (int i = 0; i < 8; i++)
+                            if (c + i < n_rows) {
+                                const int row = t.m0 + c + i;
+                                put_pair((size_t)row * half_out + out_col, v[i] / (1.0f + expf(-v[i])) * swap[(c + i) * 32 + lane] * (p.row_scale ? p.row_scale[row] : 1.0f));
+                            }
+                    }
+                }
+                asm volatile("bar.sync %0, 64;" ::"r"(1 + (lg >> 1)) : "memory");
+            } else {
+                float* const part = t.mat == 0 ? p.partial[0] : t.mat == 1 ? p.partial[1] : p.partial[2];
+                float* const dst = (split_k ? part + (size_t)t.split * p.n_tok * n_out : p.out) + col;
+                for (int c = 0; c < n_rows; c += 8) {
+                    float v[8];
+                    read(c, v);
+                    if (col >= t.col_end) continue;
+#pragma unroll
+                    for (int i = 0; i < 8; i++) {
+                        if (c + i >= n_rows) break;
+                        const int row = t.m0 + c + i;
+                        float x = v[i];
+                        if (kGrouped) {
+                            if (p.row_scale) x *= p.row_scale[row];
+                            if (p.act == 1) x = x > 0.f ? x * x : 0.f;
+                        }
+                        if (kGrouped && p.out_hi) {
+                            put_pair((size_t)row * n_out + col, x);
+                        } else if (!kGrouped && p.out_half) {
+                            p.out_half[(size_t)row * p.half_ld + t.blk * p.half_block + (col - t.blk * p.rows_per_block)] = __float2half_rn(fminf(fmaxf(x, -65504.f), 65504.f));
+                        } else {
+                            float* const d = dst + (size_t)row * n_out;
+                            *d = !split_k && p.accumulate ? *d + x : x;
+                        }
+                    }
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&bars->acc_empty[j & 1]));
+        }
+    }
+
+    tc_fence_before();
+    __syncthreads();
+    if (threadIdx.x == 0 && *abort_flag) atomicOr(p.status, 1);
+    if (warp == 1) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2u * fp.tmem_cols) : "memory");
+    }
+}
+
 // out (+)= sum over the k slices, in slice order
 __global__ void splitk_reduce_kernel(float* out, const float* partial, int n_split, size_t n, int accumulate) {
     LINEAR_PDL_TRIGGER();
@@ -613,6 +893,25 @@ bool make_map(CUtensorMap* map, const void* base, int rows, int cols, int box_ro
               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// The launch of linear_few_kernel: `rows` padded rows per activation box, `items` at most.
+template <bool kGrouped>
+cudaError_t launch_few(const GemmParams& g, int rows, int items, int num_sms, const CUtensorMap& hi, const CUtensorMap& lo, const CUtensorMap* const* w, cudaStream_t s) {
+    FewParams p = {};
+    p.g = g;
+    p.rows = rows;
+    p.items = items;
+    p.tmem_cols = 16;  // two of them: at least 32 columns, a power of two
+    while (p.tmem_cols < 2 * rows) p.tmem_cols *= 2;
+    p.idesc = (g.idesc & ~(0x3Fu << 17)) | ((uint32_t)(2 * rows >> 3) << 17);
+    const int stage = kBoxBytes + 2 * rows * kBK * 2, swap = kGrouped && g.act == 2 ? 2 * rows * 32 * 4 : 0, list = kGrouped ? 3 * 4 * std::min(g.n_groups, g.n_tok) : 0;
+    const int fixed = 1024 + swap + (list + 15) / 16 * 16 + (int)sizeof(FewBars);
+    p.n_stages = std::min(kFewStages, (kFewSmem - fixed) / stage);
+    p.off_swap = p.n_stages * stage;
+    p.off_groups = p.off_swap + swap;
+    p.off_bar = p.off_groups + (list + 15) / 16 * 16;
+    return launch_pdl(linear_few_kernel<kGrouped>, dim3(std::min(items, 2 * num_sms)), dim3(kThreads), (size_t)kFewSmem, s, hi, lo, *w[0], *w[1], *w[2], p);
+}
+
 }  // namespace
 
 struct ingot_linear_ws {
@@ -671,7 +970,9 @@ static cudaError_t ws_create(ingot_linear_ws** out, size_t act_elems, size_t par
         (e = cudaFuncSetAttribute(linear_sm100_kernel<1, 256, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, Ring<1, 256>::kSmemBytes)) != cudaSuccess ||
         (e = cudaFuncSetAttribute(linear_sm100_kernel<2, 128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, Ring<2, 128>::kSmemBytes)) != cudaSuccess ||
         (e = cudaFuncSetAttribute(linear_sm100_kernel<1, 128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, Ring<1, 128>::kSmemBytes)) != cudaSuccess ||
-        (e = cudaFuncSetAttribute(linear_sm100_kernel<1, 256, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, Ring<1, 256>::kSmemBytes)) != cudaSuccess) {
+        (e = cudaFuncSetAttribute(linear_sm100_kernel<1, 256, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, Ring<1, 256>::kSmemBytes)) != cudaSuccess ||
+        (e = cudaFuncSetAttribute(linear_few_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFewSmem)) != cudaSuccess ||
+        (e = cudaFuncSetAttribute(linear_few_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFewSmem)) != cudaSuccess) {
         cudaFree(ws->hi); cudaFree(ws->lo); cudaFree(ws->partial); cudaFree(ws->status);
         delete ws;
         return e;
@@ -779,6 +1080,7 @@ static cudaError_t launch_gemm(ingot_linear_ws* ws, float* out, const void* cons
     const CUtensorMap* maps[3] = {nullptr, nullptr, nullptr};
     GemmParams p = {};
     const int tiles_m = (n_tok + kBM - 1) / kBM;
+    const bool few = ws->planes > 1 && n_tok <= kFewRows;  // linear_few_kernel
     // 256 outputs per CTA where the operand traffic bounds the kernel (one plane, whole waves of tiles): a 256-wide tile takes
     // about 1.5 times as long as a 128-wide one
     int kBN = 128;
@@ -824,12 +1126,14 @@ static cudaError_t launch_gemm(ingot_linear_ws* ws, float* out, const void* cons
     p.k_block = rows_per_block > 0 ? n_in : 0;
     p.tiles_per_block = rows_per_block > 0 ? (rows_per_block + kBN - 1) / kBN : 0;
     dim3 grid(tiles, 1, n_split);
+    cudaError_t le;
     auto run = [&](auto kernel, int smem) {
         return launch_pdl(kernel, grid, dim3(kThreads), (size_t)smem, s, ws->map_hi, ws->map_lo, *maps[0], *maps[1], *maps[2], p);
     };
-    cudaError_t le = ws->planes > 1 ? run(linear_sm100_kernel<2, 128, false>, Ring<2, 128>::kSmemBytes)
-                   : kBN == 256     ? run(linear_sm100_kernel<1, 256, false>, Ring<1, 256>::kSmemBytes)
-                                    : run(linear_sm100_kernel<1, 128, false>, Ring<1, 128>::kSmemBytes);
+    le = few              ? launch_few<false>(p, ws->box_rows, tiles * n_split, ws->num_sms, ws->map_hi, ws->map_lo, maps, s)
+         : ws->planes > 1 ? run(linear_sm100_kernel<2, 128, false>, Ring<2, 128>::kSmemBytes)
+         : kBN == 256     ? run(linear_sm100_kernel<1, 256, false>, Ring<1, 256>::kSmemBytes)
+                          : run(linear_sm100_kernel<1, 128, false>, Ring<1, 128>::kSmemBytes);
     if (le != cudaSuccess) return le;
     for (int m = 0; m < count; m++) {
         ws->slot_split[first_slot + m] = held + n_split;
@@ -936,6 +1240,11 @@ cudaError_t ingot_grouped_tc_run(ingot_linear_ws* ws, const ingot_grouped_gemm* 
     p.act = g->act;
     p.out_hi = static_cast<__nv_bfloat16*>(g->out_hi);
     p.out_lo = static_cast<__nv_bfloat16*>(g->out_lo);
+    // experts with a few rows each (one row tile per group that has rows)
+    if (planes > 1 && g->rows_per_group <= kFewRows && std::min(g->n_groups, g->n_rows) <= kFewGroups) {
+        const CUtensorMap* const ww[3] = {w, w, w};
+        return launch_few<true>(p, box_rows, std::min(g->n_groups, g->n_rows) * p.tiles_n, ws->num_sms, *hi, *lo, ww, s);
+    }
     auto run = [&](auto kernel, int smem) {
         return launch_pdl(kernel, dim3(p.tiles_n * p.tiles_m), dim3(kThreads), (size_t)smem, s, *hi, *lo, *w, *w, *w, p);
     };

@@ -109,7 +109,6 @@ __global__ void __launch_bounds__(kThreads, 1)
 latent_decode_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ AttendParams p) {
     constexpr int kHeadsPerWarp = kN / 4;
     extern __shared__ unsigned char smem_dyn[];
-    INGOT_PDL_TRIGGER();
     const Layout<kN> L(p.dim);
     const uint32_t smem_base = (smem_u32(smem_dyn) + 1023u) & ~1023u;
     unsigned char* smem_al = smem_dyn + (smem_base - smem_u32(smem_dyn));
@@ -146,6 +145,7 @@ latent_decode_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    INGOT_PDL_TRIGGER();  // tensor memory is held: of a successor that starts on the same SM only what it leaves is taken
     const uint32_t tmem = bars->tmem_base;  // S0 S1 | O, one column per head each
 
     if (warp_u == 0) {
