@@ -168,6 +168,7 @@ public:
     }
 
     const float* forward_step(const StepEntry* entries, int n, int n_vocab) override {
+        float* const into = std::exchange(into_, nullptr);
         if (n_vocab != n_vocab_) throw std::runtime_error("engine: vocabulary size mismatch");
         Step step = check(entries, n);
         reserve_pages(entries, n);
@@ -198,11 +199,12 @@ public:
         }
         cuda_check(cudaEventRecord(ev1_, ops_.stream), "cudaEventRecord");
         const int ld = head_.n_out;
-        if (step.n_want)
-            cuda_check(cudaMemcpy2DAsync(logits_, size_t(n_vocab_) * 4, logits_dev_, size_t(ld) * 4, size_t(n_vocab_) * 4, size_t(step.n_want),
+        float* const logits = into ? into : logits_;
+        const int by_kernel = step.n_want <= kDeliveredRows ? step.n_want : 0;
+        if (step.n_want > by_kernel)
+            cuda_check(cudaMemcpy2DAsync(logits, size_t(n_vocab_) * 4, logits_dev_, size_t(ld) * 4, size_t(n_vocab_) * 4, size_t(step.n_want),
                                          cudaMemcpyDeviceToHost, ops_.stream), "D2H logits");
-        for (size_t i = 0; i < status_words_.size(); i++)
-            cuda_check(cudaMemcpyAsync(status_host_ + i, status_words_[i], sizeof(int), cudaMemcpyDeviceToHost, ops_.stream), "D2H status");
+        cuda_check(ingot_support_deliver(logits, logits_dev_, ld, n_vocab_, by_kernel, status_host_, status_words_.data(), int(status_words_.size()), ops_.stream), "logits and status");
         cuda_check(cudaStreamSynchronize(ops_.stream), "step");
         cudaEventElapsedTime(&last_ms_, ev0_, ev1_);
         for (size_t i = 0; i < status_words_.size(); i++)
@@ -219,7 +221,11 @@ public:
             for (auto& g : ops_.caches)
                 if (g->forgets() && next < max_ctx_) g->pool.release(seq, 0, g->page(g->first_visible(next)));
         }
-        return step.n_want ? logits_ : nullptr;
+        return step.n_want ? logits : nullptr;
+    }
+    bool step_into(float* rows) override {
+        into_ = rows;
+        return true;
     }
 
     void release_sequence(int seq_id) override {
@@ -271,6 +277,7 @@ private:
         cudaGraphExec_t exec = nullptr;
     };
     static constexpr size_t kMaxStatus = 64;
+    static constexpr int kDeliveredRows = 64;  // more rows leave by the copy engine: megabytes, whatever the start costs
 
     bool in_loop(size_t i) const { return loop_times_ > 0 && i >= loop_start_ && i < loop_stop_; }
 
@@ -628,7 +635,7 @@ private:
     std::vector<int32_t> lens_sorted_, rows_asked_;  // of the current step: portions in the order they run; row of each token as asked
     int32_t *meta_dev_ = nullptr, *meta_host_ = nullptr;
     size_t meta_cap_ = 0;
-    float *logits_dev_ = nullptr, *logits_ = nullptr;
+    float *logits_dev_ = nullptr, *logits_ = nullptr, *into_ = nullptr;
     int logit_rows_ = 0;
     std::vector<int*> status_words_;
     int* status_host_ = nullptr;

@@ -34,6 +34,7 @@ cudaError_t ingot_support_embed_rows_bf16(float* out, const void* table, int n_i
 cudaError_t ingot_support_embed_sum_bf16(float* out, float* copy, const void* table, int n_rows_table, const int32_t* rows_dev, const void* table2,
                                          int n_rows_table2, const int32_t* rows2_dev, int n_in, int n_rows, float scale, int* status_dev, cudaStream_t s);
 cudaError_t ingot_support_concat_rows(float* f32, void* hi, void* lo, const float* a, const float* b, int n, int n_rows, cudaStream_t s);
+cudaError_t ingot_support_deliver(float* dst, const float* src, int src_ld, int n, int rows, int* status, int* const* words, int n_words, cudaStream_t s);
 cudaError_t ingot_support_softcap(float* x, size_t n, float cap, cudaStream_t s);
 cudaError_t ingot_support_rmsnorm_rows(float* out, const float* x, const float* w, const int32_t* rows_dev, int n_rows, int n, int n_mean,
                                        float eps, cudaStream_t s);

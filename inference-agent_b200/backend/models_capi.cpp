@@ -1,5 +1,7 @@
 // C interface over the model registry, the step function and the scheduler, for the tests, bench.py and other languages.
 // Every call returns 0 (or a handle / a count) and leaves its message in ingot_models_last_error() otherwise.
+#include <cuda_runtime.h>
+
 #include <cstdint>
 #include <memory>
 #include <string>
@@ -52,7 +54,7 @@ long long ingot_model_weight_bytes(const ingot_model* m) { return (long long)m->
 float ingot_model_last_step_ms(const ingot_model* m) { return m->backend->last_step_ms(); }
 
 // One step: n portions; tokens and want hold the portions' tokens and wanted places back to back. logits_out (may be null)
-// receives the wanted rows [total wanted][vocab].
+// receives the wanted rows [total wanted][vocab]; into pinned host memory (ingot_model_host_alloc) the device writes them itself.
 int ingot_model_step(ingot_model* m, int n, const int32_t* seq_ids, const int32_t* pos0, const int32_t* n_tokens, const int32_t* tokens,
                      const int32_t* n_want, const int32_t* want, float* logits_out) {
     return guarded([&] {
@@ -64,10 +66,24 @@ int ingot_model_step(ingot_model* m, int n, const int32_t* seq_ids, const int32_
             want += n_want[i];
             rows += size_t(n_want[i]);
         }
+        cudaPointerAttributes at = {};
+        const bool pinned = logits_out && cudaPointerGetAttributes(&at, logits_out) == cudaSuccess && at.type == cudaMemoryTypeHost && at.devicePointer == logits_out;
+        if (logits_out && !pinned) cudaGetLastError();
+        if (pinned) m->backend->step_into(logits_out);
         const float* logits = m->backend->forward_step(e.data(), n, m->backend->n_vocab());
-        if (logits_out && logits) std::copy(logits, logits + rows * size_t(m->backend->n_vocab()), logits_out);
+        if (logits_out && logits && logits != logits_out) std::copy(logits, logits + rows * size_t(m->backend->n_vocab()), logits_out);
     });
 }
+// Pinned host memory for results; null if there is none to be had.
+void* ingot_model_host_alloc(size_t bytes) {
+    void* p = nullptr;
+    if (cudaHostAlloc(&p, bytes, cudaHostAllocPortable) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    return p;
+}
+void ingot_model_host_free(void* p) { cudaFreeHost(p); }
 int ingot_model_release(ingot_model* m, int seq_id) {
     return guarded([&] { m->backend->release_sequence(seq_id); });
 }

@@ -4,6 +4,7 @@ Build it with `make -C inference-agent_b200/backend models`. Tokens are ids; log
 """
 import ctypes as C
 import os
+import threading
 
 import numpy as np
 
@@ -28,7 +29,10 @@ def lib():
         l.ingot_model_weight_bytes.restype = C.c_longlong
         l.ingot_model_last_step_ms.argtypes = [C.c_void_p]
         l.ingot_model_last_step_ms.restype = C.c_float
-        l.ingot_model_step.argtypes = [C.c_void_p, C.c_int, _i32, _i32, _i32, _i32, _i32, _i32, C.c_void_p]
+        l.ingot_model_step.argtypes = [C.c_void_p, C.c_int] + [C.c_void_p] * 7
+        l.ingot_model_host_alloc.argtypes = [C.c_size_t]
+        l.ingot_model_host_alloc.restype = C.c_void_p
+        l.ingot_model_host_free.argtypes = [C.c_void_p]
         l.ingot_model_release.argtypes = [C.c_void_p, C.c_int]
         l.ingot_model_tap.argtypes = [C.c_void_p, C.c_int]
         l.ingot_model_residuals.argtypes = [C.c_void_p, C.c_void_p, C.c_longlong]
@@ -47,6 +51,58 @@ def _a(x):
     return np.ascontiguousarray(np.asarray(x, dtype=np.int32).reshape(-1))
 
 
+class _Results:
+    """Pinned host memory for the rows that steps return: the device writes them there, so that nothing is copied or faulted in on the way
+    to the caller. A block serves the arrays of one result at a time and comes back when the last of them is gone; at most BLOCKS blocks and
+    BYTES bytes are in use or kept (past that, or without a device, results are ordinary arrays). Freed with the last array and the model."""
+    BLOCKS, BYTES = 64, 128 << 20
+
+    def __init__(self):
+        self.free = {}  # bytes -> addresses
+        self.blocks = self.bytes = 0
+        self.lock = threading.RLock()  # a result may be collected, and given back, while its thread is in here
+        self.release = lib().ingot_model_host_free
+
+    def empty(self, rows, columns):
+        size = 4 * columns * (1 << (rows - 1).bit_length())
+        with self.lock:
+            kept = self.free.get(size)
+            at = kept.pop() if kept else None
+            for other, idle in list(self.free.items()) if at is None else ():
+                while idle and (self.blocks >= self.BLOCKS or self.bytes + size > self.BYTES):  # idle blocks of other sizes make room
+                    self.release(idle.pop())
+                    self.blocks -= 1
+                    self.bytes -= other
+            new = at is None and self.blocks < self.BLOCKS and self.bytes + size <= self.BYTES
+            if new:
+                self.blocks += 1
+                self.bytes += size
+        if new:
+            at = lib().ingot_model_host_alloc(size)
+            if not at:
+                with self.lock:
+                    self.blocks -= 1
+                    self.bytes -= size
+        if not at:
+            return np.empty((rows, columns), dtype=np.float32)
+        return np.asarray(_Lease(self, at, size, (rows, columns)))
+
+    def __del__(self):
+        for kept in self.free.values():
+            for at in kept:
+                self.release(at)
+
+
+class _Lease:
+    def __init__(self, results, at, size, shape):
+        self.results, self.at, self.size = results, at, size
+        self.__array_interface__ = {"shape": shape, "typestr": "<f4", "data": (at, False), "version": 3}
+
+    def __del__(self):
+        with self.results.lock:
+            self.results.free.setdefault(self.size, []).append(self.at)
+
+
 class Model:
     """An opened model folder. max_tokens: tokens the live sequences hold together; max_seqs: sequences alive at a time."""
 
@@ -55,6 +111,7 @@ class Model:
         if not self.handle:
             raise ModelError(lib().ingot_models_last_error().decode())
         self.n_vocab = lib().ingot_model_vocab(self.handle)
+        self._results = _Results()
 
     def close(self):
         if self.handle:
@@ -73,12 +130,15 @@ class Model:
 
     def step(self, portions):
         """portions: [(seq_id, pos0, tokens, want)]: one batch. Returns the wanted logits rows, in order, [n, vocab]."""
-        n_want = sum(len(p[3]) for p in portions)
-        out = np.empty((n_want, self.n_vocab), dtype=np.float32)
-        cat = lambda k: _a(np.concatenate([np.asarray(p[k], dtype=np.int32).reshape(-1) for p in portions]))
-        self._check(lib().ingot_model_step(self.handle, len(portions), _a([p[0] for p in portions]), _a([p[1] for p in portions]),
-                                           _a([len(p[2]) for p in portions]), cat(2), _a([len(p[3]) for p in portions]), cat(3),
-                                           out.ctypes.data if n_want else None))
+        n = len(portions)
+        tokens = [np.asarray(p[2], dtype=np.int32).reshape(-1) for p in portions]
+        want = [np.asarray(p[3], dtype=np.int32).reshape(-1) for p in portions]
+        heads = _a([[p[0] for p in portions], [p[1] for p in portions], [len(p[2]) for p in portions], [len(p[3]) for p in portions]])
+        tokens, want = np.concatenate(tokens), np.concatenate(want)
+        out = self._results.empty(len(want), self.n_vocab) if len(want) else np.empty((0, self.n_vocab), dtype=np.float32)
+        at = heads.ctypes.data
+        self._check(lib().ingot_model_step(self.handle, n, at, at + 4 * n, at + 8 * n, tokens.ctypes.data, at + 12 * n, want.ctypes.data,
+                                           out.ctypes.data if len(want) else None))
         return out
 
     def release(self, seq_id):
