@@ -19,17 +19,17 @@
 // by TMA), and a matrix may be block-diagonal: output tiles of block b then read the k_block activation columns that
 // start at b * k_block.
 //
-// Grouped products (ingot_grouped_tc_run). One matrix per group of rows - the experts of a mixture - in one launch: the rows are
-// sorted by group, group g's rows are a run of the activation matrix that starts anywhere, and its matrix is the g-th of a stack. A
-// CTA finds its group and row tile from the run starts on the device; boxes that reach into the next run are multiplied along and
+// Grouped products (ingot_grouped_tc_run). One matrix per group of rows - the experts of a mixture - in one launch (up to 512 groups): the
+// rows are sorted by group, group g's rows are a run of the activation matrix that starts anywhere, and its matrix is the g-th of a stack.
+// CTAs list the groups that have rows from the run starts on the device; boxes that reach into the next run are multiplied along and
 // not stored. The activation of an expert is folded into the epilogue, which then writes the bf16 operand of the next product.
 //
-// Kernels. Up to 64 rows given as a pair of planes: linear_few_kernel, below. More rows, or one plane: one CTA = 128 tokens x 128 outputs over a slice of k (split-k fills the GPU when there are few
-// output tiles; slices go to a scratch and are summed in slice order, by a small kernel or by the kernel
-// that consumes the product, so results are reproducible). 6 warps: warp 0 streams [128 rows][64 k] boxes of hi, lo and W (128-byte swizzle, 48 KB per
-// stage, 4 stages) with TMA; warp 1 issues tcgen05.mma (kind::f16, M = N = 128, K = 16; all lanes walk the
-// loop, one elected lane issues); warps 2-5 read the 128x128 f32 accumulator out of tensor memory, one
-// thread per token row. Rows past n_tok and outputs past n_out are zero-filled by TMA and not stored.
+// Kernels. Up to 64 rows given as a pair of planes: linear_few_kernel; everything else: linear_pair_kernel. Both put the weights on the M
+// side of tcgen05.mma (kind::f16) and the rows on its N side, go through their items (output tile, row tile, k slice) persistently, and
+// have 6 warps: warp 0 requests [rows][64 k] boxes of weights and planes (128-byte swizzle) with TMA, warp 1 issues the MMAs (all
+// lanes walk the loop, one elected lane issues), warps 2-5 read the f32 accumulators out of tensor memory while the next item is
+// multiplied. Split-k fills the GPU when there are few tiles; slices go to a scratch and are summed in slice order, by a small kernel or by the
+// kernel that consumes the product, so results are reproducible. Rows past n_tok and outputs past n_out are zero-filled by TMA and not stored.
 // Every mbarrier wait is bounded; on expiry the CTA raises the workspace's status word and leaves.
 #include "grouped_linear.h"
 #include "../csrc/sm100_ptx.cuh"
@@ -46,21 +46,11 @@ namespace {
 
 using namespace ingot_sm100;
 
-constexpr int kBM = 128, kBK = 64;  // outputs per CTA (kBN): 128, or 256 (a quarter less L2 traffic per output with one plane)
-constexpr int kGroupM = 16;         // token tiles that sweep the weight matrix together (see the tile order in the kernel)
-constexpr int kMaxStages = 6;
+constexpr int kBK = 64;
+constexpr int kSweepRows = 2048;  // rows that sweep the weight matrix together (see the tile order of linear_pair_kernel)
 constexpr int kBoxBytes = 128 * kBK * 2;        // 16 KB: 128 rows x 64 f16
 constexpr int kThreads = 192;
-template <int kPlanes, int kBN>
-struct Ring {
-    static constexpr int kWBytes = kBN * kBK * 2;                      // the W box: kBN rows
-    static constexpr int kStageBytes = kPlanes * kBoxBytes + kWBytes;  // hi(, lo), W
-    static constexpr int kStages = 196608 / kStageBytes;               // 192 KB ring: 4 stages of 48 KB or 6 of 32 KB
-    static constexpr int kOffBar = kStages * kStageBytes;
-    static constexpr int kSmemBytes = kOffBar + 256 + 1024;            // barriers + alignment slack
-    static_assert(kStages <= kMaxStages, "barrier arrays");
-};
-constexpr uint32_t idesc_f16(int kBN) { return (1u << 4) | ((uint32_t)(kBN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24); }  // f16 x f16 -> f32, both K-major
+constexpr uint32_t kIdescF16 = 1u << 4;                  // f16 x f16 -> f32, both K-major; M and N are filled in
 constexpr uint32_t kIdescBF16 = (1u << 7) | (1u << 10);  // bf16 x bf16 -> f32
 constexpr unsigned long long kWaitLimitNs = 2000000000ull;
 
@@ -87,14 +77,6 @@ static cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
     return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 
-struct Bars {
-    uint64_t full[kMaxStages];
-    uint64_t empty[kMaxStages];
-    uint64_t done;
-    uint32_t tmem_base;
-    uint32_t abort_flag;
-};
-
 // One launch covers up to three weight matrices that read the same activations (q/k/v, gate/up): grid.x runs over
 // the token tiles and the output tiles of all of them, tile_end[m] being the running total of tiles up to and including matrix m.
 struct GemmParams {
@@ -103,9 +85,8 @@ struct GemmParams {
     int* status;
     int n_tok, k_steps, n_split, accumulate;
     int n_out[3], tile_end[3];
-    int tiles_n, tiles_m;
-    int a_bytes;  // of one activation box: 128 rows, or fewer for a single short token tile
-    uint32_t idesc;
+    int tiles_n;
+    uint32_t idesc;  // without M and N
     int rows_per_block, k_block, tiles_per_block;  // block-diagonal matrix (rows_per_block > 0, count == 1)
     // grouped: run starts [n_groups + 1] of the rows; out rows are the sorted rows
     const int32_t* group_start;
@@ -117,266 +98,6 @@ struct GemmParams {
     int half_ld, half_block;
     int to_partial;  // write the slice(s) to `partial` even when there is only one (a consumer kernel sums them)
 };
-
-template <int kPlanes, int kBN, bool kGrouped>
-__global__ void __launch_bounds__(kThreads, 1)
-linear_sm100_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_constant__ CUtensorMap map_lo,
-                    const __grid_constant__ CUtensorMap map_w0, const __grid_constant__ CUtensorMap map_w1,
-                    const __grid_constant__ CUtensorMap map_w2, const GemmParams p) {
-    using R = Ring<kPlanes, kBN>;
-    constexpr int kStages = R::kStages, kStageBytes = R::kStageBytes, kOffBar = R::kOffBar;
-    constexpr uint32_t kTmemCols = kBN;
-    constexpr int kOffW = kPlanes * kBoxBytes;
-    extern __shared__ unsigned char smem_dyn[];
-    LINEAR_PDL_TRIGGER();
-    const uint32_t smem_base = (smem_u32(smem_dyn) + 1023u) & ~1023u;
-    unsigned char* smem_al = smem_dyn + (smem_base - smem_u32(smem_dyn));
-    Bars* bars = reinterpret_cast<Bars*>(smem_al + kOffBar);
-    volatile uint32_t* abort_flag = &bars->abort_flag;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int warp_u = __shfl_sync(0xffffffffu, warp, 0);
-    // Tile order: kGroupM token tiles walk the output tiles together, so that CTAs that run at the same time share weight
-    // boxes and the weight matrix comes out of HBM once per kGroupM * 128 tokens instead of once per 128.
-    const int group_tiles = kGroupM * p.tiles_n, grp = (int)blockIdx.x / group_tiles, in_grp = (int)blockIdx.x - grp * group_tiles;
-    const int group_m = min(kGroupM, p.tiles_m - grp * kGroupM);
-    const int tile_n = in_grp / group_m, tile_m = grp * kGroupM + in_grp - tile_n * group_m;
-    const int mat = (tile_n >= p.tile_end[0]) + (tile_n >= p.tile_end[1]);  // warp-uniform
-    const CUtensorMap* const map_w_p = mat == 0 ? &map_w0 : mat == 1 ? &map_w1 : &map_w2;
-    const int mat_n_out = mat == 0 ? p.n_out[0] : mat == 1 ? p.n_out[1] : p.n_out[2];
-    // grouped: which group's which row tile this is, 32 groups at a time
-    int group = 0, group_m0 = 0, group_end = 0;
-    if (kGrouped) {
-        LINEAR_PDL_WAIT();  // the runs come from a kernel before
-        int tile = tile_m;
-        bool found = false;
-        for (int g0 = 0; g0 < p.n_groups && !found; g0 += 32) {
-            const int mine = g0 + lane;
-            const int a = mine < p.n_groups ? p.group_start[mine] : 0, b = mine < p.n_groups ? p.group_start[mine + 1] : 0;
-            const int n = (b - a + kBM - 1) / kBM;
-            int upto = n;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int v = __shfl_up_sync(0xffffffffu, upto, o);
-                if (lane >= o) upto += v;
-            }
-            const unsigned hit = __ballot_sync(0xffffffffu, tile < upto);
-            if (hit) {
-                const int src = __ffs(hit) - 1;
-                const int local = tile - (__shfl_sync(0xffffffffu, upto, src) - __shfl_sync(0xffffffffu, n, src));
-                group = g0 + src;
-                group_m0 = __shfl_sync(0xffffffffu, a, src) + local * kBM;
-                group_end = __shfl_sync(0xffffffffu, b, src);
-                found = true;
-            } else {
-                tile -= __shfl_sync(0xffffffffu, upto, 31);
-            }
-        }
-        if (!found) return;  // the grid covers the most row tiles there can be
-    }
-    const int row_end = kGrouped ? group_end : p.n_tok;
-    const int blk = p.tiles_per_block > 0 ? tile_n / p.tiles_per_block : 0;
-    const int col_end = p.tiles_per_block > 0 ? (blk + 1) * p.rows_per_block : mat_n_out;
-    const int a_k0 = blk * p.k_block;  // first activation column of this tile's products
-    float* const mat_partial = mat == 0 ? p.partial[0] : mat == 1 ? p.partial[1] : p.partial[2];
-    const int n0 = p.tiles_per_block > 0 ? blk * p.rows_per_block + (tile_n - blk * p.tiles_per_block) * kBN
-                                         : (tile_n - (mat == 0 ? 0 : mat == 1 ? p.tile_end[0] : p.tile_end[1])) * kBN;
-    const int m0 = kGrouped ? group_m0 : tile_m * kBM, split = blockIdx.z;
-    const int w_row0 = kGrouped ? group * mat_n_out + n0 : n0;  // row of the weight matrix, or of the stack of matrices
-    const int ks_begin = (int)((long long)p.k_steps * split / p.n_split);
-    const int ks_end = (int)((long long)p.k_steps * (split + 1) / p.n_split);
-    const int n_it = ks_end - ks_begin;
-
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < kStages; s++) { mbar_init(smem_u32(&bars->full[s]), 1); mbar_init(smem_u32(&bars->empty[s]), 1); }
-        mbar_init(smem_u32(&bars->done), 1);
-        bars->abort_flag = 0;
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&bars->tmem_base)), "r"(kTmemCols) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem = bars->tmem_base;
-    // Barriers and tensor memory are this CTA's own and the weights never depend on the kernel before: the W boxes of
-    // the first ring stages are requested now, the activation boxes (and, under accumulate, the output) only after the
-    // wait for the predecessor. A stage's barrier is armed once for all three boxes.
-    const uint32_t stage_tx = kPlanes * p.a_bytes + R::kWBytes;
-    const int n_pre = min(n_it, kStages);
-    if (warp_u == 0 && lane == 0) {
-        for (int it = 0; it < n_pre; it++) {
-            const uint32_t full = smem_u32(&bars->full[it]);
-            mbar_expect_tx(full, stage_tx);
-            tma_load_2d(smem_base + it * kStageBytes + kOffW, map_w_p, (ks_begin + it) * kBK, w_row0, full);
-        }
-    }
-    if (!kGrouped) LINEAR_PDL_WAIT();
-
-    if (warp_u == 0) {
-        // ---------------- TMA producer ----------------
-        int armed = 0;
-        bool ok = true;
-        for (int it = 0; it < n_it && ok; it++) {
-            const int s = it % kStages;
-            const uint32_t full = smem_u32(&bars->full[s]);
-            if (lane == 0) {
-                const uint32_t dst = smem_base + s * kStageBytes;
-                const int k = (ks_begin + it) * kBK;
-                if (it < n_pre) {  // first use of the slot: armed and its W box requested before the wait above
-                    tma_load_2d(dst, &map_hi, a_k0 + k, m0, full);
-                    if (kPlanes > 1) tma_load_2d(dst + kBoxBytes, &map_lo, a_k0 + k, m0, full);
-                } else {
-                    ok = mbar_wait(smem_u32(&bars->empty[s]), (uint32_t)(((it / kStages) & 1) ^ 1), abort_flag, kWaitLimitNs);
-                    if (ok) {
-                        mbar_expect_tx(full, stage_tx);
-                        tma_load_2d(dst, &map_hi, a_k0 + k, m0, full);
-                        if (kPlanes > 1) tma_load_2d(dst + kBoxBytes, &map_lo, a_k0 + k, m0, full);
-                        tma_load_2d(dst + kOffW, map_w_p, k, w_row0, full);
-                    }
-                }
-            }
-            ok = __shfl_sync(0xffffffffu, ok, 0);
-            if (ok) armed = it + 1;
-        }
-        if (!ok && lane == 0) {
-            // copies already issued must land before the CTA's shared memory is released
-            for (int it = max(0, armed - kStages); it < armed; it++) {
-                const uint64_t t0 = globaltimer_ns();
-                while (!mbar_try_wait(smem_u32(&bars->full[it % kStages]), (uint32_t)((it / kStages) & 1)) &&
-                       globaltimer_ns() - t0 < 100000000ull) {}
-            }
-        }
-    } else if (warp_u == 1) {
-        // ---------------- MMA issuer ----------------
-        bool ok = true;
-        for (int it = 0; it < n_it && ok; it++) {
-            const int s = it % kStages;
-            ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars->full[s]), (uint32_t)((it / kStages) & 1), abort_flag, kWaitLimitNs)) != 0;
-            if (!ok) break;
-            tc_fence_after();
-            if (elect_one()) {
-                const uint32_t a_hi = smem_base + s * kStageBytes, a_lo = a_hi + kBoxBytes, b = a_hi + kOffW;
-#pragma unroll
-                for (int ks = 0; ks < kBK / 16; ks++)
-                    tc_mma_ss(tmem, make_desc(a_hi + ks * 32, 16, 1024), make_desc(b + ks * 32, 16, 1024), p.idesc, (it > 0 || ks > 0) ? 1u : 0u);
-                if (kPlanes > 1) {
-#pragma unroll
-                    for (int ks = 0; ks < kBK / 16; ks++)
-                        tc_mma_ss(tmem, make_desc(a_lo + ks * 32, 16, 1024), make_desc(b + ks * 32, 16, 1024), p.idesc, 1u);
-                }
-                tc_commit(smem_u32(&bars->empty[s]));
-                if (it == n_it - 1) tc_commit(smem_u32(&bars->done));
-            }
-            __syncwarp();
-        }
-    } else {
-        // ---------------- epilogue: accumulator -> global, one thread per token row ----------------
-        const int lg = warp & 3;  // the tensor-memory lane group this warp may read
-        const int row = m0 + lg * 32 + lane;
-        bool ok = n_it > 0 && mbar_wait(smem_u32(&bars->done), 0, abort_flag, kWaitLimitNs);
-        ok = __all_sync(0xffffffffu, ok) != 0;
-        const bool split_k = p.n_split > 1 || p.to_partial;
-        if (ok) {
-            tc_fence_after();
-            float* dst = (split_k ? mat_partial + (size_t)split * p.n_tok * mat_n_out : p.out) + (size_t)row * mat_n_out + n0;
-            const bool add = !split_k && p.accumulate;
-            const float scale = p.row_scale && row < row_end ? p.row_scale[row] : 1.0f;
-            if (kGrouped && p.act == 2) {
-                // Runs of 32 gate columns, each followed by the 32 up columns of the same outputs: scale * silu(gate) * up, half as wide.
-                const int half_out = mat_n_out / 2;
-#pragma unroll
-                for (int c = 0; c < kBN / 64; c++) {
-                    float g[32], u[32];
-                    tmem_ld32(tmem + ((uint32_t)(lg * 32) << 16) + c * 64, g);
-                    tmem_ld32(tmem + ((uint32_t)(lg * 32) << 16) + c * 64 + 32, u);
-                    tmem_wait_ld();
-                    if (row >= row_end || n0 + c * 64 >= mat_n_out) continue;
-                    const size_t at = (size_t)row * half_out + n0 / 2 + c * 32;
-#pragma unroll
-                    for (int i = 0; i < 32; i += 8) {
-                        __nv_bfloat162 h[4], l[4];
-#pragma unroll
-                        for (int e = 0; e < 4; e++) {
-                            const float a = g[i + 2 * e], b = g[i + 2 * e + 1];
-                            const float x = a / (1.0f + expf(-a)) * u[i + 2 * e] * scale, y = b / (1.0f + expf(-b)) * u[i + 2 * e + 1] * scale;
-                            h[e] = __floats2bfloat162_rn(x, y);
-                            l[e] = __floats2bfloat162_rn(x - __low2float(h[e]), y - __high2float(h[e]));
-                        }
-                        *reinterpret_cast<uint4*>(p.out_hi + at + i) = *reinterpret_cast<const uint4*>(h);
-                        if (p.out_lo) *reinterpret_cast<uint4*>(p.out_lo + at + i) = *reinterpret_cast<const uint4*>(l);
-                    }
-                }
-            } else {
-#pragma unroll
-                for (int c = 0; c < kBN / 32; c++) {
-                    float v[32];
-                    tmem_ld32(tmem + ((uint32_t)(lg * 32) << 16) + c * 32, v);
-                    tmem_wait_ld();
-                    if (row < row_end) {
-                        if (kGrouped && (p.row_scale || p.act)) {
-#pragma unroll
-                            for (int i = 0; i < 32; i++) {
-                                v[i] *= scale;
-                                if (p.act == 1) v[i] = v[i] > 0.f ? v[i] * v[i] : 0.f;
-                            }
-                        }
-                        if (kGrouped && p.out_hi) {  // n_out is a multiple of 8
-#pragma unroll
-                            for (int i = 0; i < 32; i += 8) {
-                                const int col = n0 + c * 32 + i;
-                                if (col >= col_end) break;
-                                const size_t at = (size_t)row * mat_n_out + col;
-                                __nv_bfloat162 h[4], l[4];
-#pragma unroll
-                                for (int e = 0; e < 4; e++) {
-                                    h[e] = __floats2bfloat162_rn(v[i + 2 * e], v[i + 2 * e + 1]);
-                                    l[e] = __floats2bfloat162_rn(v[i + 2 * e] - __low2float(h[e]), v[i + 2 * e + 1] - __high2float(h[e]));
-                                }
-                                *reinterpret_cast<uint4*>(p.out_hi + at) = *reinterpret_cast<const uint4*>(h);
-                                if (p.out_lo) *reinterpret_cast<uint4*>(p.out_lo + at) = *reinterpret_cast<const uint4*>(l);
-                            }
-                        } else if (!kGrouped && p.out_half) {  // n_out and the blocks are multiples of 8
-#pragma unroll
-                            for (int i = 0; i < 32; i += 8) {
-                                const int col = n0 + c * 32 + i;
-                                if (col >= col_end) break;
-                                __half2 h[4];
-#pragma unroll
-                                for (int e = 0; e < 4; e++)
-                                    h[e] = __floats2half2_rn(fminf(fmaxf(v[i + 2 * e], -65504.f), 65504.f), fminf(fmaxf(v[i + 2 * e + 1], -65504.f), 65504.f));
-                                *reinterpret_cast<uint4*>(p.out_half + (size_t)row * p.half_ld + blk * p.half_block + (col - blk * p.rows_per_block)) = *reinterpret_cast<const uint4*>(h);
-                            }
-                        } else {
-#pragma unroll
-                            for (int i = 0; i < 32; i += 4) {
-                                const int col = n0 + c * 32 + i;
-                                if (col + 3 < col_end) {
-                                    float4* d4 = reinterpret_cast<float4*>(dst + c * 32 + i);
-                                    float4 o = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
-                                    if (add) { const float4 old = *d4; o.x += old.x; o.y += old.y; o.z += old.z; o.w += old.w; }
-                                    *d4 = o;
-                                } else {
-                                    for (int e = 0; e < 4; e++)
-                                        if (col + e < col_end) dst[c * 32 + i + e] = add ? dst[c * 32 + i + e] + v[i + e] : v[i + e];
-                                }
-                            }
-                        }
-                    }
-                }
-            }
-        }
-    }
-
-    tc_fence_before();
-    __syncthreads();
-    if (threadIdx.x == 0 && *abort_flag) atomicOr(p.status, 1);
-    if (warp == 1) {
-        tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
-    }
-}
 
 // ---- few rows ----------------------------------------------------------------------------------------------------------
 //
@@ -658,6 +379,308 @@ linear_few_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_const
     }
 }
 
+// ---- many rows ---------------------------------------------------------------------------------------------------------
+//
+// Products of more rows (or of one plane). Bound by the tensor cores, once tiles are loaded often enough from L2 and the accumulators are
+// emptied while the next tile is multiplied. Two CTAs of a cluster form a tile of 256 outputs (the M side: 128 of each CTA) by up to
+// 256 rows (the N side: each CTA fetches half of them, both multiply with all), so 32 KB per SM and k-step feed 512 cycles of
+// MMA, two thirds of what a 128 x 256 tile of one CTA takes. The pair goes through its share of the items (output tile, row tile, k slice) with a
+// 6-stage ring and two accumulators. Rows per tile are the launch's choice (any multiple of 32; a group's rows are spread evenly over its tiles),
+// so that little is multiplied for padding. A lane holds an output, so that a warp writes whole lines of a row.
+// Measured (B200, inside a prompt's step, against one-CTA tiles of 128 x 256 that each start, drain and write on their own): 4096 rows by
+// 28672 x 4096 603 us (807 before; 1595 TFLOP/s), by 4096 x 14336 322 us (376), by 10240 x 4096 210 us (312).
+constexpr int kPairStages = 6, kPairRows = 256, kPairGroups = 512;
+constexpr int kPairStageBytes = 2 * kBoxBytes;                       // W, and the activation rows of all planes
+constexpr int kPairSwapBytes = 2 * 2 * 2 * 16 * 32 * 4;              // halves of gate / up columns on their way: [buffer][warp pair][from][16 rows][32 outputs]
+struct PairParams {
+    GemmParams g;
+    int rows, planes;     // rows of a tile at most (grouped: 256 / planes)
+    int row_tiles, items; // plain products
+    int box_bytes;        // of one plane's activation box
+    uint32_t idesc;       // without N
+};
+struct PairBars {
+    uint64_t full[kPairStages], empty[kPairStages], acc_full[2], acc_empty[2];
+    uint32_t tmem_base, abort_flag;
+    int n_groups, n_items;
+};
+constexpr int kPairOffSwap = kPairStages * kPairStageBytes, kPairOffBar = kPairOffSwap + kPairSwapBytes, kPairOffGroups = kPairOffBar + 256;
+constexpr int kPairSmem = kPairOffGroups + kPairGroups * 16 + 1024;  // groups: {group, first row, end, first item}
+static_assert(sizeof(PairBars) <= 256 && kPairSmem <= 227 * 1024, "shared memory");
+
+template <bool kGrouped>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
+linear_pair_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_constant__ CUtensorMap map_lo,
+                   const __grid_constant__ CUtensorMap map_w0, const __grid_constant__ CUtensorMap map_w1,
+                   const __grid_constant__ CUtensorMap map_w2, const PairParams pp) {
+    const GemmParams& p = pp.g;
+    extern __shared__ unsigned char smem_dyn[];
+    const uint32_t smem_base = (smem_u32(smem_dyn) + 1023u) & ~1023u;
+    unsigned char* smem_al = smem_dyn + (smem_base - smem_u32(smem_dyn));
+    PairBars* bars = reinterpret_cast<PairBars*>(smem_al + kPairOffBar);
+    int4* groups = reinterpret_cast<int4*>(smem_al + kPairOffGroups);
+    volatile uint32_t* abort_flag = &bars->abort_flag;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp_u = __shfl_sync(0xffffffffu, warp, 0);
+    const int rank = (int)cluster_rank(), pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < kPairStages; s++) { mbar_init(smem_u32(&bars->full[s]), 1); mbar_init(smem_u32(&bars->empty[s]), 1); }
+        for (int b = 0; b < 2; b++) { mbar_init(smem_u32(&bars->acc_full[b]), 1); mbar_init(smem_u32(&bars->acc_empty[b]), 8); }
+        bars->abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&bars->tmem_base)), "r"(512u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+    if (kGrouped) {
+        LINEAR_PDL_WAIT();  // the runs come from a kernel before
+        if (warp == 0) {
+            int count = 0, items = 0;
+            for (int g0 = 0; g0 < p.n_groups; g0 += 32) {
+                const int mine = g0 + lane;
+                const int a = mine < p.n_groups ? p.group_start[mine] : 0, b = mine < p.n_groups ? p.group_start[mine + 1] : 0;
+                const int n = (b - a + pp.rows - 1) / pp.rows * p.tiles_n;
+                const unsigned some = __ballot_sync(0xffffffffu, b > a);
+                int upto = n;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int v = __shfl_up_sync(0xffffffffu, upto, o);
+                    if (lane >= o) upto += v;
+                }
+                if (b > a) groups[count + __popc(some & ((1u << lane) - 1))] = make_int4(mine, a, b, items + upto - n);
+                count += __popc(some);
+                items += __shfl_sync(0xffffffffu, upto, 31);
+            }
+            if (lane == 0) { bars->n_groups = count; bars->n_items = items; }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync();  // the peer's barriers are there before anything is counted on them
+    tc_fence_after();
+    LINEAR_PDL_TRIGGER();  // tensor memory is held
+    const uint32_t tmem = bars->tmem_base;
+    const int n_items = kGrouped ? bars->n_items : pp.items;
+
+    struct Item { int mat, n0, col_end, a_k0, m0, n_rows, mma_rows, w_row0, k_begin, n_it, blk, split; };
+    auto item_at = [&](int index) {
+        Item t;
+        int tile_n, row_end;
+        t.split = 0;
+        if (kGrouped) {
+            int lo = 0, hi = bars->n_groups - 1;  // the last group whose first item is not behind this one
+            while (lo < hi) {
+                const int mid = (lo + hi + 1) >> 1;
+                if (groups[mid].w <= index) lo = mid; else hi = mid - 1;
+            }
+            const int4 e = groups[lo];
+            const int tiles = (e.z - e.y + pp.rows - 1) / pp.rows, per = ((e.z - e.y + tiles - 1) / tiles + 31) & ~31, local = index - e.w;
+            tile_n = local / tiles;  // row tiles of a group side by side: they share the weights
+            t.m0 = e.y + (local - tile_n * tiles) * per;
+            t.n_rows = min(per, e.z - t.m0);  // may be none: rows rounded up
+            t.w_row0 = e.x * p.n_out[0];
+        } else {
+            const int tiles = p.tiles_n * pp.row_tiles, per_group = max(1, kSweepRows / pp.rows);
+            t.split = index / tiles;
+            // row tiles of about 2048 rows sweep the outputs together: what runs at a time shares weights and rows in L2
+            const int local = index - t.split * tiles, grp = local / (per_group * p.tiles_n), in = local - grp * per_group * p.tiles_n;
+            const int n_m = min(per_group, pp.row_tiles - grp * per_group);
+            tile_n = in / n_m;
+            t.m0 = (grp * per_group + in - tile_n * n_m) * pp.rows;
+            row_end = p.n_tok;
+            t.n_rows = min(pp.rows, row_end - t.m0);
+            t.w_row0 = 0;
+        }
+        t.mma_rows = max(32, (t.n_rows + 31) & ~31);
+        t.mat = (tile_n >= p.tile_end[0]) + (tile_n >= p.tile_end[1]);
+        const int n_out = t.mat == 0 ? p.n_out[0] : t.mat == 1 ? p.n_out[1] : p.n_out[2];
+        t.blk = p.tiles_per_block > 0 ? tile_n / p.tiles_per_block : 0;
+        t.col_end = p.tiles_per_block > 0 ? (t.blk + 1) * p.rows_per_block : n_out;
+        t.a_k0 = t.blk * p.k_block;
+        t.n0 = (p.tiles_per_block > 0 ? t.blk * p.rows_per_block + (tile_n - t.blk * p.tiles_per_block) * 256
+                                      : (tile_n - (t.mat == 0 ? 0 : t.mat == 1 ? p.tile_end[0] : p.tile_end[1])) * 256) + rank * 128;  // of this CTA
+        t.w_row0 += t.n0;
+        t.k_begin = (int)((long long)p.k_steps * t.split / p.n_split);
+        t.n_it = (int)((long long)p.k_steps * (t.split + 1) / p.n_split) - t.k_begin;
+        return t;
+    };
+    auto map_of_mat = [&](int mat) { return mat == 0 ? &map_w0 : mat == 1 ? &map_w1 : &map_w2; };
+    const uint32_t stage_tx = 2 * (kBoxBytes + pp.planes * pp.box_bytes);  // of both CTAs, counted on the first one's barrier
+
+    int n_pre = 0;
+    if (warp_u == 0 && pair < n_items) {  // weights do not depend on the kernel before
+        const Item t = item_at(pair);
+        n_pre = min(t.n_it, kPairStages);
+        if (lane == 0)
+            for (int it = 0; it < n_pre; it++) {
+                if (rank == 0) mbar_expect_tx(smem_u32(&bars->full[it]), stage_tx);
+                tma_load_2d_pair(smem_base + it * kPairStageBytes, map_of_mat(t.mat), (t.k_begin + it) * kBK, t.w_row0, map_to_rank(smem_u32(&bars->full[it]), 0));
+            }
+    }
+    if (!kGrouped) LINEAR_PDL_WAIT();
+
+    if (warp_u == 0) {
+        // ---------------- TMA producer of this CTA's halves ----------------
+        int done = 0, s = 0;
+        uint32_t round = 0;
+        bool ok = true;
+        for (int index = pair; index < n_items && ok; index += n_pairs) {
+            const Item t = item_at(index);
+            const int row = t.m0 + rank * (t.mma_rows >> 1);
+            for (int it = 0; it < t.n_it && ok; it++) {
+                if (lane == 0) {
+                    const uint32_t full = map_to_rank(smem_u32(&bars->full[s]), 0), dst = smem_base + s * kPairStageBytes;
+                    const int k = (t.k_begin + it) * kBK;
+                    if (done >= n_pre) {
+                        ok = mbar_wait(smem_u32(&bars->empty[s]), (round & 1) ^ 1, abort_flag, kWaitLimitNs);
+                        if (ok) {
+                            if (rank == 0) mbar_expect_tx(smem_u32(&bars->full[s]), stage_tx);
+                            tma_load_2d_pair(dst, map_of_mat(t.mat), k, t.w_row0, full);
+                        }
+                    }
+                    if (ok) {
+                        tma_load_2d_pair(dst + kBoxBytes, &map_hi, t.a_k0 + k, row, full);
+                        if (pp.planes > 1) tma_load_2d_pair(dst + kBoxBytes + (kBoxBytes >> 1), &map_lo, t.a_k0 + k, row, full);
+                    }
+                }
+                ok = __shfl_sync(0xffffffffu, ok, 0);
+                if (ok) {
+                    done++;
+                    if (++s == kPairStages) { s = 0; round++; }
+                }
+            }
+        }
+        // the last arrivals on this CTA's barriers come from the first one's MMAs: they must be over before it leaves
+        for (int i = 0; i < kPairStages && ok && lane == 0; i++) {
+            ok = mbar_wait(smem_u32(&bars->empty[s]), (round & 1) ^ 1, abort_flag, kWaitLimitNs);
+            if (++s == kPairStages) { s = 0; round++; }
+        }
+        if (!ok && lane == 0) {  // copies already issued must land before the CTA's shared memory is released
+            const uint64_t t0 = globaltimer_ns();
+            while (globaltimer_ns() - t0 < 100000000ull) {}
+        }
+    } else if (warp_u == 1 && rank == 0) {
+        // ---------------- MMA issuer, for both ----------------
+        int s = 0, j = 0;
+        uint32_t round = 0;
+        bool ok = true;
+        for (int index = pair; index < n_items && ok; index += n_pairs, j++) {
+            const Item t = item_at(index);
+            const uint32_t acc = tmem + (uint32_t)((j & 1) * kPairRows), idesc = pp.idesc | ((uint32_t)(t.mma_rows >> 3) << 17);
+            ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars->acc_empty[j & 1]), (uint32_t)((j >> 1) & 1) ^ 1, abort_flag, kWaitLimitNs)) != 0;
+            tc_fence_after();
+            for (int it = 0; it < t.n_it && ok; it++) {
+                ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars->full[s]), round & 1, abort_flag, kWaitLimitNs)) != 0;
+                if (!ok) break;
+                tc_fence_after();
+                if (elect_one()) {
+                    const uint32_t a = smem_base + s * kPairStageBytes, b = a + kBoxBytes;
+#pragma unroll
+                    for (int ks = 0; ks < kBK / 16; ks++)
+                        tc_mma_pair(acc, make_desc(a + ks * 32, 16, 1024), make_desc(b + ks * 32, 16, 1024), idesc, (it > 0 || ks > 0) ? 1u : 0u);
+                    if (pp.planes > 1) {
+#pragma unroll
+                        for (int ks = 0; ks < kBK / 16; ks++)
+                            tc_mma_pair(acc, make_desc(a + ks * 32, 16, 1024), make_desc(b + (kBoxBytes >> 1) + ks * 32, 16, 1024), idesc, 1u);
+                    }
+                    tc_commit_pair(smem_u32(&bars->empty[s]));
+                    if (it == t.n_it - 1) tc_commit_pair(smem_u32(&bars->acc_full[j & 1]));
+                }
+                __syncwarp();
+                if (++s == kPairStages) { s = 0; round++; }
+            }
+        }
+    } else if (warp_u >= 2) {
+        // ---------------- epilogue: one thread per output, 32 rows at a time ----------------
+        const int lg = warp & 3;  // the tensor-memory lane group this warp may read
+        const bool split_k = p.n_split > 1 || p.to_partial;
+        int j = 0;
+        bool ok = true;
+        for (int index = pair; index < n_items && ok; index += n_pairs, j++) {
+            const Item t = item_at(index);
+            ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars->acc_full[j & 1]), (uint32_t)((j >> 1) & 1), abort_flag, kWaitLimitNs)) != 0;
+            if (kGrouped && p.act == 2) ok = pair_all(1 + (lg >> 1), ok);  // they go on, or leave, together
+            if (!ok) break;
+            tc_fence_after();
+            const uint32_t acc = tmem + (uint32_t)((j & 1) * kPairRows) + ((uint32_t)(lg * 32) << 16);
+            const int n_out = t.mat == 0 ? p.n_out[0] : t.mat == 1 ? p.n_out[1] : p.n_out[2];
+            const int col = t.n0 + lg * 32 + lane;
+            auto put_pair = [&](size_t at, float x) {
+                const __nv_bfloat16 h = __float2bfloat16_rn(x);
+                p.out_hi[at] = h;
+                if (p.out_lo) p.out_lo[at] = __float2bfloat16_rn(x - __bfloat162float(h));
+            };
+            if (kGrouped && p.act == 2) {
+                // Runs of 32 gate outputs, each followed by the 32 up outputs that go with them: one warp's lanes and the next one's. Of 32
+                // rows each warp finishes 16: it hands the other half of its own values over.
+                const bool is_up = lg & 1;
+                const int half_out = n_out / 2, out_col = t.n0 / 2 + (lg >> 1) * 32 + lane;
+                for (int c = 0, buffer = 0; c < t.n_rows; c += 32, buffer ^= 1) {
+                    float v[32];
+                    tmem_ld32(acc + c, v);
+                    tmem_wait_ld();
+                    float* const swap = reinterpret_cast<float*>(smem_al + kPairOffSwap) + ((buffer * 2 + (lg >> 1)) * 2) * 512;
+#pragma unroll
+                    for (int i = 0; i < 16; i++) swap[is_up * 512 + i * 32 + lane] = is_up ? v[i] : v[16 + i];
+                    asm volatile("bar.sync %0, 64;" ::"r"(1 + (lg >> 1)) : "memory");
+                    if (col >= t.col_end) continue;
+#pragma unroll
+                    for (int i = 0; i < 16; i++) {
+                        const int local = c + (is_up ? 16 : 0) + i;
+                        const float other = swap[!is_up * 512 + i * 32 + lane], gate = is_up ? other : v[i], up = is_up ? v[16 + i] : other;
+                        if (local < t.n_rows) {
+                            const int row = t.m0 + local;
+                            put_pair((size_t)row * half_out + out_col, gate / (1.0f + expf(-gate)) * up * (p.row_scale ? p.row_scale[row] : 1.0f));
+                        }
+                    }
+                }
+            } else {
+                float* const part = t.mat == 0 ? p.partial[0] : t.mat == 1 ? p.partial[1] : p.partial[2];
+                float* const dst = (split_k ? part + (size_t)t.split * p.n_tok * n_out : p.out) + col;
+                for (int c = 0; c < t.n_rows; c += 32) {
+                    float v[32];
+                    tmem_ld32(acc + c, v);
+                    tmem_wait_ld();
+                    if (col >= t.col_end) continue;
+                    const int n = t.n_rows - c;
+#pragma unroll
+                    for (int i = 0; i < 32; i++) {
+                        if (i >= n) break;
+                        const int row = t.m0 + c + i;
+                        float x = v[i];
+                        if (kGrouped) {
+                            if (p.row_scale) x *= p.row_scale[row];
+                            if (p.act == 1) x = x > 0.f ? x * x : 0.f;
+                        }
+                        if (kGrouped && p.out_hi) {
+                            put_pair((size_t)row * n_out + col, x);
+                        } else if (!kGrouped && p.out_half) {
+                            p.out_half[(size_t)row * p.half_ld + t.blk * p.half_block + (col - t.blk * p.rows_per_block)] = __float2half_rn(fminf(fmaxf(x, -65504.f), 65504.f));
+                        } else {
+                            float* const d = dst + (size_t)row * n_out;
+                            *d = !split_k && p.accumulate ? *d + x : x;
+                        }
+                    }
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(map_to_rank(smem_u32(&bars->acc_empty[j & 1]), 0));
+        }
+    }
+
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync();  // neither leaves while the other may still count on its barriers or multiply from its shared memory
+    if (threadIdx.x == 0 && *abort_flag) atomicOr(p.status, 1);
+    if (warp == 1) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+    }
+}
+
 // out (+)= sum over the k slices, in slice order
 __global__ void splitk_reduce_kernel(float* out, const float* partial, int n_split, size_t n, int accumulate) {
     LINEAR_PDL_TRIGGER();
@@ -902,7 +925,7 @@ cudaError_t launch_few(const GemmParams& g, int rows, int items, int num_sms, co
     p.items = items;
     p.tmem_cols = 16;  // two of them: at least 32 columns, a power of two
     while (p.tmem_cols < 2 * rows) p.tmem_cols *= 2;
-    p.idesc = (g.idesc & ~(0x3Fu << 17)) | ((uint32_t)(2 * rows >> 3) << 17);
+    p.idesc = g.idesc | ((uint32_t)(2 * rows >> 3) << 17) | ((128u >> 4) << 24);
     const int stage = kBoxBytes + 2 * rows * kBK * 2, swap = kGrouped && g.act == 2 ? 2 * rows * 32 * 4 : 0, list = kGrouped ? 3 * 4 * std::min(g.n_groups, g.n_tok) : 0;
     const int fixed = 1024 + swap + (list + 15) / 16 * 16 + (int)sizeof(FewBars);
     p.n_stages = std::min(kFewStages, (kFewSmem - fixed) / stage);
@@ -910,6 +933,41 @@ cudaError_t launch_few(const GemmParams& g, int rows, int items, int num_sms, co
     p.off_groups = p.off_swap + swap;
     p.off_bar = p.off_groups + (list + 15) / 16 * 16;
     return launch_pdl(linear_few_kernel<kGrouped>, dim3(std::min(items, 2 * num_sms)), dim3(kThreads), (size_t)kFewSmem, s, hi, lo, *w[0], *w[1], *w[2], p);
+}
+
+// The launch of linear_pair_kernel with tiles of up to `rows` rows; `items` at most.
+template <bool kGrouped>
+cudaError_t launch_pair(const GemmParams& g, int rows, int planes, int box_rows, int row_tiles, int items, int num_sms, const CUtensorMap& hi, const CUtensorMap& lo,
+                        const CUtensorMap* const* w, cudaStream_t s) {
+    PairParams p = {};
+    p.g = g;
+    p.rows = rows;
+    p.planes = planes;
+    p.row_tiles = row_tiles;
+    p.items = items;
+    p.box_bytes = box_rows * kBK * 2;
+    p.idesc = g.idesc | ((256u >> 4) << 24);
+    return launch_pdl(linear_pair_kernel<kGrouped>, dim3(2 * std::min(items, num_sms / 2)), dim3(kThreads), (size_t)kPairSmem, s, hi, lo, *w[0], *w[1], *w[2], p);
+}
+
+// Rows of a tile and k slices for n_tok rows against tiles_n tiles of 256 outputs: the least rounds of all pairs of CTAs times what one costs.
+// A k-step takes a pair as long as it takes to load it, about as 256 + rows (at 256 rows that is 512 cycles, what the MMAs take), and a
+// tile starts and ends for about four k-steps.
+struct PairTiles { int rows, row_tiles, n_split; };
+PairTiles pair_tiles(int n_tok, int tiles_n, int planes, int k_steps, int most_splits, int num_sms) {
+    const int pairs = num_sms / 2;
+    PairTiles best = {};
+    long long least = 0;
+    for (int rows = kPairRows / planes; rows >= 32; rows -= 32) {
+        PairTiles t;
+        t.rows = rows;
+        t.row_tiles = (n_tok + rows - 1) / rows;
+        const long long tiles = (long long)tiles_n * t.row_tiles;
+        t.n_split = (int)std::max(1ll, std::min({pairs / tiles, (long long)k_steps / 4, (long long)most_splits}));
+        const long long rounds = (tiles * t.n_split + pairs - 1) / pairs, cost = rounds * ((k_steps + t.n_split - 1) / t.n_split + 4) * (256 + rows * planes);
+        if (best.rows == 0 || cost < least) { best = t; least = cost; }
+    }
+    return best;
 }
 
 }  // namespace
@@ -926,23 +984,29 @@ struct ingot_linear_ws {
     bool bf16 = false;
     int n_slots = 3;
     int planes = 2;                            // of the prepared activations
-    int box_rows = 128;
     int prepared_tok = 0, prepared_in = 0;
-    CUtensorMap map_hi, map_lo;
-    std::map<std::tuple<const void*, int, int, int>, CUtensorMap> w_maps;  // one per weight matrix (and per row count of grouped activations)
+    std::map<std::tuple<const void*, int, int, int>, CUtensorMap> maps;  // of weight matrices and activations, by place, shape and box
 };
 
-// (Re)builds the activation tensor maps when the prepared shape changes.
-static cudaError_t set_prepared(ingot_linear_ws* ws, int n_in, int n_tok) {
-    if (ws->prepared_tok != n_tok || ws->prepared_in != n_in) {
-        // A batch of few tokens fetches only its own rows (whole 8-row swizzle groups) of the 128 a tile has. What the other rows of
-        // the tile hold is multiplied along and never stored: rows of a product do not mix.
-        ws->box_rows = n_tok >= 128 ? 128 : (n_tok + 7) / 8 * 8;
-        if (!make_map(&ws->map_hi, ws->hi, n_tok, n_in, ws->box_rows, ws->bf16) || !make_map(&ws->map_lo, ws->lo, n_tok, n_in, ws->box_rows, ws->bf16))
-            return cudaErrorUnknown;
-        ws->prepared_tok = n_tok;
-        ws->prepared_in = n_in;
+// The map of an activation or weight buffer, made once. At most kMaxMaps are kept: make_room() before a launch looks up its own.
+static constexpr size_t kMaxMaps = 65536;
+static void make_room(ingot_linear_ws* ws) {
+    if (ws->maps.size() > kMaxMaps) ws->maps.clear();
+}
+static const CUtensorMap* map_of(ingot_linear_ws* ws, const void* base, int rows, int cols, int box, bool bf16) {
+    const auto key = std::make_tuple(base, rows, cols, box);
+    auto it = ws->maps.find(key);
+    if (it == ws->maps.end()) {
+        CUtensorMap tm;
+        if (!make_map(&tm, base, rows, cols, box, bf16)) return nullptr;
+        it = ws->maps.emplace(key, tm).first;
     }
+    return &it->second;
+}
+
+static cudaError_t set_prepared(ingot_linear_ws* ws, int n_in, int n_tok) {
+    ws->prepared_tok = n_tok;
+    ws->prepared_in = n_in;
     return cudaGetLastError();
 }
 
@@ -965,12 +1029,8 @@ static cudaError_t ws_create(ingot_linear_ws** out, size_t act_elems, size_t par
         (e = cudaMemset(ws->hi, 0, ws->act_elems * 2)) != cudaSuccess || (e = cudaMemset(ws->lo, 0, ws->act_elems * 2)) != cudaSuccess ||
         (e = cudaMalloc(&ws->partial, n_slots * ws->partial_floats * 4)) != cudaSuccess || (e = cudaMalloc(&ws->status, sizeof(int))) != cudaSuccess ||
         (e = cudaMemset(ws->status, 0, sizeof(int))) != cudaSuccess ||
-        (e = cudaFuncSetAttribute(linear_sm100_kernel<2, 128, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, Ring<2, 128>::kSmemBytes)) != cudaSuccess ||
-        (e = cudaFuncSetAttribute(linear_sm100_kernel<1, 128, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, Ring<1, 128>::kSmemBytes)) != cudaSuccess ||
-        (e = cudaFuncSetAttribute(linear_sm100_kernel<1, 256, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, Ring<1, 256>::kSmemBytes)) != cudaSuccess ||
-        (e = cudaFuncSetAttribute(linear_sm100_kernel<2, 128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, Ring<2, 128>::kSmemBytes)) != cudaSuccess ||
-        (e = cudaFuncSetAttribute(linear_sm100_kernel<1, 128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, Ring<1, 128>::kSmemBytes)) != cudaSuccess ||
-        (e = cudaFuncSetAttribute(linear_sm100_kernel<1, 256, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, Ring<1, 256>::kSmemBytes)) != cudaSuccess ||
+        (e = cudaFuncSetAttribute(linear_pair_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem)) != cudaSuccess ||
+        (e = cudaFuncSetAttribute(linear_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem)) != cudaSuccess ||
         (e = cudaFuncSetAttribute(linear_few_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFewSmem)) != cudaSuccess ||
         (e = cudaFuncSetAttribute(linear_few_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFewSmem)) != cudaSuccess) {
         cudaFree(ws->hi); cudaFree(ws->lo); cudaFree(ws->partial); cudaFree(ws->status);
@@ -1077,63 +1137,44 @@ static cudaError_t launch_gemm(ingot_linear_ws* ws, float* out, const void* cons
     const int held = append ? ws->slot_split[first_slot] : 0;
     for (int m = 0; m < count && append; m++)
         if (ws->slot_split[first_slot + m] != held || ws->slot_out[first_slot + m] != n_out[m]) return cudaErrorInvalidValue;
+    make_room(ws);
     const CUtensorMap* maps[3] = {nullptr, nullptr, nullptr};
     GemmParams p = {};
-    const int tiles_m = (n_tok + kBM - 1) / kBM;
     const bool few = ws->planes > 1 && n_tok <= kFewRows;  // linear_few_kernel
-    // 256 outputs per CTA where the operand traffic bounds the kernel (one plane, whole waves of tiles): a 256-wide tile takes
-    // about 1.5 times as long as a 128-wide one
-    int kBN = 128;
-    if (ws->planes == 1 && count == 1 && rows_per_block == 0) {
-        const long long waves128 = ((long long)((n_out[0] + 127) / 128) * tiles_m + ws->num_sms - 1) / ws->num_sms;
-        const long long waves256 = ((long long)((n_out[0] + 255) / 256) * tiles_m + ws->num_sms - 1) / ws->num_sms;
-        if (waves128 > 1 && 3 * waves256 < 2 * waves128) kBN = 256;
-        if (const char* e = getenv("INGOT_GEMM_BN")) kBN = atoi(e) == 256 ? 256 : 128;
-    }
+    const int tile = few ? 128 : 256;
     int tiles_n = 0, fit = 1 << 30;
     for (int m = 0; m < count; m++) {
-        const auto key = std::make_tuple(w[m], n_out[m], n_in, kBN);
-        auto it = ws->w_maps.find(key);
-        if (it == ws->w_maps.end()) {
-            CUtensorMap tm;
-            if (!make_map(&tm, w[m], n_out[m], n_in, kBN, ws->bf16)) return cudaErrorUnknown;
-            it = ws->w_maps.emplace(key, tm).first;
-        }
-        maps[m] = &it->second;
-        tiles_n += rows_per_block > 0 ? n_out[m] / rows_per_block * ((rows_per_block + kBN - 1) / kBN) : (n_out[m] + kBN - 1) / kBN;
+        if (!(maps[m] = map_of(ws, w[m], n_out[m], n_in, 128, ws->bf16))) return cudaErrorUnknown;
+        tiles_n += rows_per_block > 0 ? n_out[m] / rows_per_block * ((rows_per_block + tile - 1) / tile) : (n_out[m] + tile - 1) / tile;
         p.tile_end[m] = tiles_n;
         p.n_out[m] = n_out[m];
         p.partial[m] = ws->partial + (size_t)(first_slot + m) * ws->partial_floats + (size_t)held * n_tok * n_out[m];
         fit = std::min(fit, (int)(ws->partial_floats / ((size_t)n_tok * n_out[m])) - held);
     }
     for (int m = count; m < 3; m++) { maps[m] = maps[count - 1]; p.tile_end[m] = tiles_n; p.n_out[m] = n_out[count - 1]; p.partial[m] = p.partial[count - 1]; }
-    const int tiles = tiles_n * tiles_m;
     p.tiles_n = tiles_n;
-    p.tiles_m = tiles_m;
-    p.a_bytes = ws->box_rows * kBK * 2;
     const int k_steps = (n_in + kBK - 1) / kBK;
     // enough k slices to give every SM a CTA, at least 4 k-steps each, and no more than the slots hold
     if (to_partial && fit < 1) return cudaErrorInvalidValue;
-    const int n_split = out_half ? 1 : std::max(1, std::min({ws->num_sms / tiles, k_steps / 4, fit}));
+    const int most = out_half ? 1 : std::max(fit, 1);
+    const PairTiles t = pair_tiles(n_tok, tiles_n, ws->planes, k_steps, most, ws->num_sms);
+    const int n_split = few ? std::max(1, std::min({ws->num_sms / tiles_n, k_steps / 4, most})) : t.n_split;
+    // A batch of few tokens fetches only its own rows (whole 8-row swizzle groups). What else the boxes hold is multiplied along and never stored.
+    const int box = few ? (n_tok + 7) / 8 * 8 : t.rows / 2;
+    const CUtensorMap *hi = map_of(ws, ws->hi, n_tok, act_in, box, ws->bf16), *lo = ws->planes > 1 ? map_of(ws, ws->lo, n_tok, act_in, box, ws->bf16) : hi;
+    if (!hi || !lo) return cudaErrorUnknown;
     p.out_half = out_half;
     p.half_ld = half_ld;
     p.half_block = half_block;
     p.out = out; p.status = ws->status;
     p.n_tok = n_tok; p.k_steps = k_steps; p.n_split = n_split; p.accumulate = accumulate;
     p.to_partial = to_partial ? 1 : 0;
-    p.idesc = idesc_f16(kBN) | (ws->bf16 ? kIdescBF16 : 0u);
+    p.idesc = kIdescF16 | (ws->bf16 ? kIdescBF16 : 0u);
     p.rows_per_block = rows_per_block;
     p.k_block = rows_per_block > 0 ? n_in : 0;
-    p.tiles_per_block = rows_per_block > 0 ? (rows_per_block + kBN - 1) / kBN : 0;
-    dim3 grid(tiles, 1, n_split);
-    cudaError_t le;
-    auto run = [&](auto kernel, int smem) {
-        return launch_pdl(kernel, grid, dim3(kThreads), (size_t)smem, s, ws->map_hi, ws->map_lo, *maps[0], *maps[1], *maps[2], p);
-    };
-    le = few              ? launch_few<false>(p, ws->box_rows, tiles * n_split, ws->num_sms, ws->map_hi, ws->map_lo, maps, s)
-         : ws->planes > 1 ? run(linear_sm100_kernel<2, 128, false>, Ring<2, 128>::kSmemBytes)
-         : kBN == 256     ? run(linear_sm100_kernel<1, 256, false>, Ring<1, 256>::kSmemBytes)
-                          : run(linear_sm100_kernel<1, 128, false>, Ring<1, 128>::kSmemBytes);
+    p.tiles_per_block = rows_per_block > 0 ? (rows_per_block + tile - 1) / tile : 0;
+    cudaError_t le = few ? launch_few<false>(p, box, tiles_n * n_split, ws->num_sms, *hi, *lo, maps, s)
+                         : launch_pair<false>(p, t.rows, ws->planes, box, t.row_tiles, tiles_n * t.row_tiles * n_split, ws->num_sms, *hi, *lo, maps, s);
     if (le != cudaSuccess) return le;
     for (int m = 0; m < count; m++) {
         ws->slot_split[first_slot + m] = held + n_split;
@@ -1167,90 +1208,63 @@ cudaError_t ingot_linear_tc_run_half(ingot_linear_ws* ws, void* out, int out_ld,
     return launch_gemm(ws, nullptr, &w, n_in, &n_out, 1, 0, 0, false, false, s, rows_per_block, static_cast<__half*>(out), out_ld, out_block);
 }
 
-// The map of an activation or weight buffer, made once.
-static const CUtensorMap* map_of(ingot_linear_ws* ws, const void* base, int rows, int cols, int box, bool bf16) {
-    const auto key = std::make_tuple(base, rows, cols, box);
-    auto it = ws->w_maps.find(key);
-    if (it == ws->w_maps.end()) {
-        CUtensorMap tm;
-        if (!make_map(&tm, base, rows, cols, box, bf16)) return nullptr;
-        it = ws->w_maps.emplace(key, tm).first;
-    }
-    return &it->second;
-}
-
 // out f16 [n_tok][out_ld] = a W^T, both operands f16: a [a_rows][n_in] with n_tok <= a_rows, W [n_out][n_in]. Lengths are multiples of 8.
 cudaError_t ingot_linear_tc_run_f16(ingot_linear_ws* ws, void* out, int out_ld, const void* a, int a_rows, int n_tok, const void* w, int n_in, int n_out, cudaStream_t s) {
     if (n_in % 8 != 0 || n_out % 8 != 0 || out_ld % 8 != 0 || n_tok < 1 || n_tok > a_rows) return cudaErrorInvalidValue;
     GemmParams p = {};
-    p.tiles_m = (n_tok + kBM - 1) / kBM;
-    const long long waves128 = ((long long)((n_out + 127) / 128) * p.tiles_m + ws->num_sms - 1) / ws->num_sms;
-    const long long waves256 = ((long long)((n_out + 255) / 256) * p.tiles_m + ws->num_sms - 1) / ws->num_sms;
-    const int kBN = waves128 > 1 && 3 * waves256 < 2 * waves128 ? 256 : 128;
-    if (ws->w_maps.size() > 65536) ws->w_maps.clear();
-    const CUtensorMap *ma = map_of(ws, a, a_rows, n_in, 128, false), *mw = map_of(ws, w, n_out, n_in, kBN, false);
+    p.tiles_n = (n_out + 255) / 256;
+    p.k_steps = (n_in + kBK - 1) / kBK;
+    const PairTiles t = pair_tiles(n_tok, p.tiles_n, 1, p.k_steps, 1, ws->num_sms);
+    make_room(ws);
+    const CUtensorMap *ma = map_of(ws, a, a_rows, n_in, t.rows / 2, false), *mw = map_of(ws, w, n_out, n_in, 128, false);
     if (!ma || !mw) return cudaErrorUnknown;
-    p.tiles_n = (n_out + kBN - 1) / kBN;
     for (int m = 0; m < 3; m++) { p.n_out[m] = n_out; p.tile_end[m] = p.tiles_n; }
     p.status = ws->status;
     p.n_tok = n_tok;
-    p.k_steps = (n_in + kBK - 1) / kBK;
     p.n_split = 1;
-    p.a_bytes = kBoxBytes;
-    p.idesc = idesc_f16(kBN);
+    p.idesc = kIdescF16;
     p.out_half = static_cast<__half*>(out);
     p.half_ld = out_ld;
-    auto run = [&](auto kernel, int smem) {
-        return launch_pdl(kernel, dim3(p.tiles_n * p.tiles_m), dim3(kThreads), (size_t)smem, s, *ma, *ma, *mw, *mw, *mw, p);
-    };
-    return kBN == 256 ? run(linear_sm100_kernel<1, 256, false>, Ring<1, 256>::kSmemBytes) : run(linear_sm100_kernel<1, 128, false>, Ring<1, 128>::kSmemBytes);
+    const CUtensorMap* const maps[3] = {mw, mw, mw};
+    return launch_pair<false>(p, t.rows, 1, t.rows / 2, t.row_tiles, p.tiles_n * t.row_tiles, ws->num_sms, *ma, *ma, maps, s);
 }
 
 cudaError_t ingot_grouped_tc_run(ingot_linear_ws* ws, const ingot_grouped_gemm* g, cudaStream_t s) {
     if (g->act == 2 && (g->n_out % 64 != 0 || !g->out_hi)) return cudaErrorInvalidValue;
     if (!ws->bf16 || g->n_in % 8 != 0 || g->n_out % 8 != 0 || g->n_rows < 1 || g->n_groups < 1 || g->rows_per_group < 1) return cudaErrorInvalidValue;
-    const int planes = g->a_lo ? 2 : 1, box_rows = g->rows_per_group >= 128 ? 128 : (g->rows_per_group + 7) / 8 * 8;
+    const int planes = g->a_lo ? 2 : 1;
+    const bool few = planes > 1 && g->rows_per_group <= kFewRows;  // as for plain products
+    const int tile = few ? 128 : 256, rows = few ? (g->rows_per_group + 7) / 8 * 8 : kPairRows / planes, box = few ? rows : rows / 2;
+    make_room(ws);
+    const CUtensorMap* hi = map_of(ws, g->a_hi, g->n_rows, g->n_in, box, true);
+    const CUtensorMap* lo = planes > 1 ? map_of(ws, g->a_lo, g->n_rows, g->n_in, box, true) : hi;
+    if (!hi || !lo) return cudaErrorUnknown;
     GemmParams p = {};
-    p.tiles_m = g->n_rows / kBM + std::min(g->n_rows, g->n_groups);  // at least as many as there can be
-    // as for plain products: 256 outputs per CTA if that saves waves, judged by the row tiles of evenly filled groups
-    const int likely = std::max(1, std::min(g->n_groups, g->n_rows) * ((g->n_rows / std::min(g->n_groups, g->n_rows) + kBM - 1) / kBM));
-    int kBN = 128;
-    if (planes == 1) {
-        const long long waves128 = ((long long)((g->n_out + 127) / 128) * likely + ws->num_sms - 1) / ws->num_sms;
-        const long long waves256 = ((long long)((g->n_out + 255) / 256) * likely + ws->num_sms - 1) / ws->num_sms;
-        if (waves128 > 1 && 3 * waves256 < 2 * waves128) kBN = 256;
-    }
-    if (ws->w_maps.size() > 65536) ws->w_maps.clear();
-    const CUtensorMap* hi = map_of(ws, g->a_hi, g->n_rows, g->n_in, box_rows, true);
-    const CUtensorMap* lo = planes > 1 ? map_of(ws, g->a_lo, g->n_rows, g->n_in, box_rows, true) : hi;
-    const CUtensorMap* w = map_of(ws, g->w, g->n_groups * g->n_out, g->n_in, kBN, true);
-    if (!hi || !lo || !w) return cudaErrorUnknown;
-    p.tiles_n = (g->n_out + kBN - 1) / kBN;
+    p.tiles_n = (g->n_out + tile - 1) / tile;
     for (int m = 0; m < 3; m++) { p.n_out[m] = g->n_out; p.tile_end[m] = p.tiles_n; }
     p.out = g->out;
     p.status = ws->status;
     p.n_tok = g->n_rows;
     p.k_steps = (g->n_in + kBK - 1) / kBK;
     p.n_split = 1;
-    p.a_bytes = box_rows * kBK * 2;
-    p.idesc = idesc_f16(kBN) | kIdescBF16;
-    p.group_start = g->group_start;
-    p.n_groups = g->n_groups;
+    p.idesc = kIdescF16 | kIdescBF16;
     p.row_scale = g->row_scale;
     p.act = g->act;
     p.out_hi = static_cast<__nv_bfloat16*>(g->out_hi);
     p.out_lo = static_cast<__nv_bfloat16*>(g->out_lo);
-    // experts with a few rows each (one row tile per group that has rows)
-    if (planes > 1 && g->rows_per_group <= kFewRows && std::min(g->n_groups, g->n_rows) <= kFewGroups) {
-        const CUtensorMap* const ww[3] = {w, w, w};
-        return launch_few<true>(p, box_rows, std::min(g->n_groups, g->n_rows) * p.tiles_n, ws->num_sms, *hi, *lo, ww, s);
+    static_assert(kFewGroups == kPairGroups, "groups of a launch");
+    for (int first = 0; first < g->n_groups; first += kPairGroups) {  // a CTA keeps a list of the groups
+        p.group_start = g->group_start + first;
+        p.n_groups = std::min(g->n_groups - first, kPairGroups);
+        const CUtensorMap* w = map_of(ws, static_cast<const char*>(g->w) + (size_t)first * g->n_out * g->n_in * 2, p.n_groups * g->n_out, g->n_in, 128, true);
+        if (!w) return cudaErrorUnknown;
+        const CUtensorMap* const maps[3] = {w, w, w};
+        const int some = std::min(p.n_groups, g->n_rows);  // groups that can have rows
+        const cudaError_t le = few ? launch_few<true>(p, rows, some * p.tiles_n, ws->num_sms, *hi, *lo, maps, s)
+                                   : launch_pair<true>(p, rows, planes, box, 0, (g->n_rows / rows + some) * p.tiles_n, ws->num_sms, *hi, *lo, maps, s);
+        if (le != cudaSuccess) return le;
     }
-    auto run = [&](auto kernel, int smem) {
-        return launch_pdl(kernel, dim3(p.tiles_n * p.tiles_m), dim3(kThreads), (size_t)smem, s, *hi, *lo, *w, *w, *w, p);
-    };
-    return planes > 1   ? run(linear_sm100_kernel<2, 128, true>, Ring<2, 128>::kSmemBytes)
-           : kBN == 256 ? run(linear_sm100_kernel<1, 256, true>, Ring<1, 256>::kSmemBytes)
-                        : run(linear_sm100_kernel<1, 128, true>, Ring<1, 128>::kSmemBytes);
+    return cudaSuccess;
 }
 
 // The same product left as k slices in scratch slot 0..2 for one of the ingot_linear_tc_finish_* calls below.

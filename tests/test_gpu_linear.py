@@ -266,18 +266,26 @@ def test_grouped_projection_launch_matches_float64():
         lib.ingot_linear_ws_destroy(ws)
 
 
-@pytest.mark.parametrize("n_tok,n_in,n_out,blocks", [
-    (2, 8, 8, 1),          # one k-step that is mostly zero fill, one tile that is mostly empty
-    (7, 2048, 16384, 1),   # a wave of tiles, no k slices
-    (8, 8192, 2048, 1),    # few tiles: k slices and their sum
-    (9, 1000, 40000, 1),   # more items than two CTAs per SM, ragged k and outputs
-    (33, 264, 1320, 1),
-    (64, 2048, 4104, 1),   # the most rows
-    (5, 136, 24 * 40, 40), # blocks shorter than a tile
-    (64, 64, 200 * 3, 3),  # and longer
+@pytest.mark.parametrize("n_tok,n_in,n_out,blocks,planes", [
+    (2, 8, 8, 1, 2),          # one k-step that is mostly zero fill, one tile that is mostly empty
+    (7, 2048, 16384, 1, 2),   # a wave of tiles, no k slices
+    (8, 8192, 2048, 1, 2),    # few tiles: k slices and their sum
+    (9, 1000, 40000, 1, 2),   # more items than two CTAs per SM, ragged k and outputs
+    (33, 264, 1320, 1, 2),
+    (64, 2048, 4104, 1, 2),   # the most rows
+    (5, 136, 24 * 40, 40, 2), # blocks shorter than a tile
+    (64, 64, 200 * 3, 3, 2),  # and longer
+    # more rows, or one plane: pairs of CTAs
+    (2, 8, 8, 1, 1),
+    (65, 72, 264, 1, 2),       # one tile more than half empty
+    (129, 2048, 4104, 1, 2),   # the next row tile has one row
+    (257, 1000, 520, 1, 1),    # k slices, ragged everywhere
+    (1000, 512, 9000, 1, 1),   # rows spread over their tiles, several items per pair
+    (300, 64, 24 * 40, 40, 2), # blocks much shorter than a tile
+    (2600, 264, 304 * 3, 3, 1),  # and a little longer; more rows than sweep the outputs together
 ])
-def test_products_of_few_rows(n_tok, n_in, n_out, blocks):
-    """bf16 weights, activations as a pair of bf16 planes, up to 64 rows: against float64 on the planes' values, f32 and f16 results."""
+def test_products_of_bf16_planes(n_tok, n_in, n_out, blocks, planes):
+    """bf16 weights, activations as one or two bf16 planes, few rows and many: against float64 on the planes' values, f32 and f16 results."""
     import torch
     lib = _lib()
     vp, ci = C.c_void_p, C.c_int
@@ -286,19 +294,19 @@ def test_products_of_few_rows(n_tok, n_in, n_out, blocks):
     lib.ingot_linear_tc_run_blocks.argtypes = [vp, vp, vp, ci, ci, ci, vp]
     lib.ingot_linear_tc_run_half.argtypes = [vp, vp, ci, ci, vp, ci, ci, ci, vp]
     ws = vp()
-    assert lib.ingot_linear_ws_create_bf16(C.byref(ws), 64, n_in * blocks, n_out) == 0
+    assert lib.ingot_linear_ws_create_bf16(C.byref(ws), n_tok, n_in * blocks, n_out) == 0
     try:
         g = torch.Generator(device="cuda").manual_seed(n_tok + n_in)
         x = torch.randn(n_tok, n_in * blocks, device="cuda", generator=g)
         w = (torch.randn(n_out, n_in, device="cuda", generator=g) / n_in ** 0.5).bfloat16()
         hi = x.bfloat16()
-        seen = hi.double() + (x - hi.float()).bfloat16().double()
+        seen = hi.double() + ((x - hi.float()).bfloat16().double() if planes > 1 else 0)
         want = torch.einsum("tbk,bok->tbo", seen.view(n_tok, blocks, n_in), w.double().view(blocks, n_out // blocks, n_in)).reshape(n_tok, n_out)
         rows = n_out // blocks if blocks > 1 else 0
         st = vp(torch.cuda.current_stream().cuda_stream)
         out = torch.full((n_tok, n_out), float("nan"), device="cuda")
         half = torch.full((n_tok, n_out + 8), float("nan"), device="cuda", dtype=torch.float16)
-        assert lib.ingot_linear_tc_prepare_bf16(ws, x.data_ptr(), n_in * blocks, n_in * blocks, n_tok, 2, st) == 0
+        assert lib.ingot_linear_tc_prepare_bf16(ws, x.data_ptr(), n_in * blocks, n_in * blocks, n_tok, planes, st) == 0
         if rows:
             assert lib.ingot_linear_tc_run_blocks(ws, out.data_ptr(), w.data_ptr(), n_in, n_out, rows, st) == 0
         else:

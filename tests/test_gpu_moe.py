@@ -184,6 +184,14 @@ def test_grouped_product(counts, n_in, n_out, planes):
         L.ingot_linear_ws_destroy(ws)
 
 
+@pytest.mark.parametrize("planes,every,most", [(1, 1, 3), (2, 1, 3), (2, 9, 70), (1, 9, 520)])
+def test_grouped_product_of_many_groups(planes, every, most):
+    """More groups than a launch lists, with few rows and with more than a tile."""
+    counts = [(i * 7) % (most + 1) if i % every == 0 else 0 for i in range(1100)]
+    counts[3] = most
+    test_grouped_product(counts, 72, 64, planes)
+
+
 @pytest.mark.parametrize("n,experts,identity,top,d,ff", [(1, 4, 0, 2, 40, 32), (1, 3, 2, 4, 256, 64), (2, 5, 1, 3, 64, 32), (9, 5, 3, 5, 64, 96), (130, 12, 4, 3, 48, 64)])
 def test_plain_gated_experts_and_identity_experts(n, experts, identity, top, d, ff):
     """Routing, both products in f32 arithmetic, and the residual sum that takes the identity experts and the shared expert in."""
