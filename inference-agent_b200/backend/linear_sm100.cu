@@ -391,7 +391,8 @@ linear_few_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_const
 // 28672 x 4096 603 us (807 before; 1595 TFLOP/s), by 4096 x 14336 322 us (376), by 10240 x 4096 210 us (312).
 constexpr int kPairStages = 6, kPairRows = 256, kPairGroups = 512;
 constexpr int kPairStageBytes = 2 * kBoxBytes;                       // W, and the activation rows of all planes
-constexpr int kPairSwapBytes = 2 * 2 * 2 * 16 * 32 * 4;              // halves of gate / up columns on their way: [buffer][warp pair][from][16 rows][32 outputs]
+constexpr int kPairThreads = 320;                                    // 8 warps of epilogue: with 4, gated products of short rows waited for them
+constexpr int kPairSwapBytes = 2 * 4 * 2 * 8 * 32 * 4;               // halves of gate / up columns on their way: [buffer][warp pair][from][8 rows][32 outputs]
 struct PairParams {
     GemmParams g;
     int rows, planes;     // rows of a tile at most (grouped: 256 / planes)
@@ -409,7 +410,7 @@ constexpr int kPairSmem = kPairOffGroups + kPairGroups * 16 + 1024;  // groups: 
 static_assert(sizeof(PairBars) <= 256 && kPairSmem <= 227 * 1024, "shared memory");
 
 template <bool kGrouped>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
 linear_pair_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_constant__ CUtensorMap map_lo,
                    const __grid_constant__ CUtensorMap map_w0, const __grid_constant__ CUtensorMap map_w1,
                    const __grid_constant__ CUtensorMap map_w2, const PairParams pp) {
@@ -426,7 +427,7 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_cons
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kPairStages; s++) { mbar_init(smem_u32(&bars->full[s]), 1); mbar_init(smem_u32(&bars->empty[s]), 1); }
-        for (int b = 0; b < 2; b++) { mbar_init(smem_u32(&bars->acc_full[b]), 1); mbar_init(smem_u32(&bars->acc_empty[b]), 8); }
+        for (int b = 0; b < 2; b++) { mbar_init(smem_u32(&bars->acc_full[b]), 1); mbar_init(smem_u32(&bars->acc_empty[b]), 16); }
         bars->abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -593,15 +594,16 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_cons
             }
         }
     } else if (warp_u >= 2) {
-        // ---------------- epilogue: one thread per output, 32 rows at a time ----------------
+        // ---------------- epilogue: one thread per output, two warps for the same outputs and every second run of rows ----------------
         const int lg = warp & 3;  // the tensor-memory lane group this warp may read
+        const int half = (warp - 2) >> 2, duo = 2 * half + (lg >> 1);  // duo: the warps of neighbouring outputs
         const bool split_k = p.n_split > 1 || p.to_partial;
         int j = 0;
         bool ok = true;
         for (int index = pair; index < n_items && ok; index += n_pairs, j++) {
             const Item t = item_at(index);
             ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars->acc_full[j & 1]), (uint32_t)((j >> 1) & 1), abort_flag, kWaitLimitNs)) != 0;
-            if (kGrouped && p.act == 2) ok = pair_all(1 + (lg >> 1), ok);  // they go on, or leave, together
+            if (kGrouped && p.act == 2) ok = pair_all(1 + duo, ok);  // they go on, or leave, together
             if (!ok) break;
             tc_fence_after();
             const uint32_t acc = tmem + (uint32_t)((j & 1) * kPairRows) + ((uint32_t)(lg * 32) << 16);
@@ -613,33 +615,33 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_cons
                 if (p.out_lo) p.out_lo[at] = __float2bfloat16_rn(x - __bfloat162float(h));
             };
             if (kGrouped && p.act == 2) {
-                // Runs of 32 gate outputs, each followed by the 32 up outputs that go with them: one warp's lanes and the next one's. Of 32
-                // rows each warp finishes 16: it hands the other half of its own values over.
+                // Runs of 32 gate outputs, each followed by the 32 up outputs that go with them: one warp's lanes and the next one's. Of 16
+                // rows each warp finishes 8: it hands the other half of its own values over.
                 const bool is_up = lg & 1;
                 const int half_out = n_out / 2, out_col = t.n0 / 2 + (lg >> 1) * 32 + lane;
-                for (int c = 0, buffer = 0; c < t.n_rows; c += 32, buffer ^= 1) {
-                    float v[32];
-                    tmem_ld32(acc + c, v);
+                for (int c = half * 16, buffer = 0; c < t.n_rows; c += 32, buffer ^= 1) {
+                    float v[16], x[8];
+                    tmem_ld16(acc + c, v);
                     tmem_wait_ld();
-                    float* const swap = reinterpret_cast<float*>(smem_al + kPairOffSwap) + ((buffer * 2 + (lg >> 1)) * 2) * 512;
+                    float* const swap = reinterpret_cast<float*>(smem_al + kPairOffSwap) + (buffer * 4 + duo) * 512;
 #pragma unroll
-                    for (int i = 0; i < 16; i++) swap[is_up * 512 + i * 32 + lane] = is_up ? v[i] : v[16 + i];
-                    asm volatile("bar.sync %0, 64;" ::"r"(1 + (lg >> 1)) : "memory");
+                    for (int i = 0; i < 8; i++) swap[is_up * 256 + i * 32 + lane] = is_up ? v[i] : v[8 + i];
+                    asm volatile("bar.sync %0, 64;" ::"r"(1 + duo) : "memory");
                     if (col >= t.col_end) continue;
+                    const int row = t.m0 + c + (is_up ? 8 : 0), n = t.m0 + t.n_rows - row;
 #pragma unroll
-                    for (int i = 0; i < 16; i++) {
-                        const int local = c + (is_up ? 16 : 0) + i;
-                        const float other = swap[!is_up * 512 + i * 32 + lane], gate = is_up ? other : v[i], up = is_up ? v[16 + i] : other;
-                        if (local < t.n_rows) {
-                            const int row = t.m0 + local;
-                            put_pair((size_t)row * half_out + out_col, gate / (1.0f + expf(-gate)) * up * (p.row_scale ? p.row_scale[row] : 1.0f));
-                        }
+                    for (int i = 0; i < 8; i++) {
+                        const float other = swap[!is_up * 256 + i * 32 + lane], gate = is_up ? other : v[i], up = is_up ? v[8 + i] : other;
+                        x[i] = gate / (1.0f + expf(-gate)) * up;
                     }
+#pragma unroll
+                    for (int i = 0; i < 8; i++)
+                        if (i < n) put_pair((size_t)(row + i) * half_out + out_col, p.row_scale ? x[i] * p.row_scale[row + i] : x[i]);
                 }
             } else {
                 float* const part = t.mat == 0 ? p.partial[0] : t.mat == 1 ? p.partial[1] : p.partial[2];
                 float* const dst = (split_k ? part + (size_t)t.split * p.n_tok * n_out : p.out) + col;
-                for (int c = 0; c < t.n_rows; c += 32) {
+                for (int c = half * 32; c < t.n_rows; c += 64) {
                     float v[32];
                     tmem_ld32(acc + c, v);
                     tmem_wait_ld();
@@ -947,7 +949,7 @@ cudaError_t launch_pair(const GemmParams& g, int rows, int planes, int box_rows,
     p.items = items;
     p.box_bytes = box_rows * kBK * 2;
     p.idesc = g.idesc | ((256u >> 4) << 24);
-    return launch_pdl(linear_pair_kernel<kGrouped>, dim3(2 * std::min(items, num_sms / 2)), dim3(kThreads), (size_t)kPairSmem, s, hi, lo, *w[0], *w[1], *w[2], p);
+    return launch_pdl(linear_pair_kernel<kGrouped>, dim3(2 * std::min(items, num_sms / 2)), dim3(kPairThreads), (size_t)kPairSmem, s, hi, lo, *w[0], *w[1], *w[2], p);
 }
 
 // Rows of a tile and k slices for n_tok rows against tiles_n tiles of 256 outputs: the least rounds of all pairs of CTAs times what one costs.
