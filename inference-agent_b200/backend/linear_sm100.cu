@@ -609,6 +609,14 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_cons
             const uint32_t acc = tmem + (uint32_t)((j & 1) * kPairRows) + ((uint32_t)(lg * 32) << 16);
             const int n_out = t.mat == 0 ? p.n_out[0] : t.mat == 1 ? p.n_out[1] : p.n_out[2];
             const int col = t.n0 + lg * 32 + lane;
+            // As soon as the last values are in registers. A release of the stores before it would wait for them at every item.
+            bool drained = false;
+            auto release = [&] {
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_cluster_relaxed(map_to_rank(smem_u32(&bars->acc_empty[j & 1]), 0));
+                drained = true;
+            };
             auto put_pair = [&](size_t at, float x) {
                 const __nv_bfloat16 h = __float2bfloat16_rn(x);
                 p.out_hi[at] = h;
@@ -623,6 +631,7 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_cons
                     float v[16], x[8];
                     tmem_ld16(acc + c, v);
                     tmem_wait_ld();
+                    if (c + 32 >= t.n_rows) release();
                     float* const swap = reinterpret_cast<float*>(smem_al + kPairOffSwap) + (buffer * 4 + duo) * 512;
 #pragma unroll
                     for (int i = 0; i < 8; i++) swap[is_up * 256 + i * 32 + lane] = is_up ? v[i] : v[8 + i];
@@ -645,8 +654,15 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_cons
                     float v[32];
                     tmem_ld32(acc + c, v);
                     tmem_wait_ld();
+                    if (c + 64 >= t.n_rows) release();
                     if (col >= t.col_end) continue;
                     const int n = t.n_rows - c;
+                    if (!kGrouped && n >= 32 && !p.out_half && (split_k || !p.accumulate)) {  // plain rows: no conditions in between
+                        float* d = dst + (size_t)(t.m0 + c) * n_out;
+#pragma unroll
+                        for (int i = 0; i < 32; i++, d += n_out) *d = v[i];
+                        continue;
+                    }
 #pragma unroll
                     for (int i = 0; i < 32; i++) {
                         if (i >= n) break;
@@ -667,9 +683,7 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_cons
                     }
                 }
             }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(map_to_rank(smem_u32(&bars->acc_empty[j & 1]), 0));
+            if (!drained) release();
         }
     }
 
