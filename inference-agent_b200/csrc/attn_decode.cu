@@ -27,6 +27,7 @@
 #include "attn_common.cuh"
 #include "ingot_internal.cuh"
 #include "attn_decode_params.cuh"
+#include "sm100_ptx.cuh"
 
 // This file is compiled twice. attn_decode_append.cu defines INGOT_DECODE_APPEND and includes it: the kernel then is
 // the single-token form that also does K1's work (RoPE on q and on the new k, the K/V row written to the cache by the
@@ -58,6 +59,8 @@ namespace {
 
 constexpr int kMaxDecodeWarps = 8;
 constexpr int kMaxParts = 64;
+constexpr int kClusterParts = 8;  // CTAs of a portable cluster
+constexpr int kClusterKeys = 8192;
 
 // Merges the splits of one (sequence, kv head): out = sum_s o_s 2^(m_s-M) / sum_s l_s 2^(m_s-M)
 // (the attn_combine formula, shaders/kernels.metal:502-516). Runs in one extra CTA per (kv head,
@@ -188,6 +191,8 @@ __device__ __forceinline__ void combine_splits(const DecodeParams& p, float* sme
 struct KRegs { uint4 k[8]; };  // [n-tile 0/1][i=0..3]: key (nt*8 + g), 16-byte chunk (4i + j)
 struct VRegs { uint4 v[8]; };  // [slot 0..3 -> keys 2j, 2j+1, 2j+8, 2j+9][chunk g / g+8]
 
+// kCluster: the splits of a range are the CTAs of a cluster, and its first CTA merges them in shared memory.
+template <bool kCluster>
 __global__ void __launch_bounds__(kMaxDecodeWarps * 32, 1) DECODE_KERNEL(const DECODE_PARAMS p) {
     extern __shared__ float smem[];
     // Programmatic dependent launch: let the next kernel in the stream start as soon as SM resources allow, and
@@ -198,15 +203,18 @@ __global__ void __launch_bounds__(kMaxDecodeWarps * 32, 1) DECODE_KERNEL(const D
         combine_splits(p, smem, blockIdx.y, blockIdx.z / p.n_seq, blockIdx.z % p.n_seq);
         return;
     }
+    if (kCluster) ingot_sm100::cluster_arrive();  // this CTA has started: its shared memory may be written
     if (p.pdl_mode == kPdlWaitFirst) asm volatile("griddepcontrol.wait;" ::: "memory");
 
     const int chunk = blockIdx.x, kvh = blockIdx.y, layer = blockIdx.z / p.n_seq, seq = blockIdx.z % p.n_seq;
     const __half* const kc = p.kc + (size_t)layer * p.cache_layer_stride;
     const __half* const vc = p.vc + (size_t)layer * p.cache_layer_stride;
     const int n_keys = load_seq_len(p, seq);
-    if (n_keys < 1) return;
-    const int n_chunks = (n_keys + p.chunk_keys - 1) / p.chunk_keys;
-    if (chunk >= n_chunks) return;
+    const int n_chunks = (max(n_keys, 0) + p.chunk_keys - 1) / p.chunk_keys;
+    if (chunk >= n_chunks) {  // no keys, or none for this split
+        if (kCluster) { ingot_sm100::cluster_wait(); ingot_sm100::cluster_sync(); }
+        return;
+    }
     const int k_begin = chunk * p.chunk_keys;
     const int k_end = min(n_keys, k_begin + p.chunk_keys);
     const int n_units = (k_end - k_begin + 15) >> 4;
@@ -436,6 +444,10 @@ __global__ void __launch_bounds__(kMaxDecodeWarps * 32, 1) DECODE_KERNEL(const D
     if (p.pdl_mode == kPdlEarlyLoads) asm volatile("griddepcontrol.wait;" ::: "memory");
 
     const bool single = n_chunks == 1;
+    // Cluster form: this split's sums go to the first CTA's shared memory, [split][G][128 + m, l], behind its own warps' states.
+    float* const gather = so + (size_t)n_warps * G * (kHeadDim + 2);
+    if (kCluster) ingot_sm100::cluster_wait();
+    const uint32_t gather0 = kCluster ? ingot_sm100::map_to_rank((uint32_t)__cvta_generic_to_shared(gather + (size_t)chunk * G * (kHeadDim + 2)), 0) : 0u;
     const size_t part_row0 = ((size_t)seq * p.n_parts_max + chunk) * p.n_head + (size_t)kvh * G;
     const size_t part0 = (size_t)layer * p.part_layer_stride, out0 = (size_t)layer * p.qo_layer_stride;
     for (int idx = threadIdx.x; idx < G * kHeadDim; idx += blockDim.x) {
@@ -451,12 +463,59 @@ __global__ void __launch_bounds__(kMaxDecodeWarps * 32, 1) DECODE_KERNEL(const D
         if (single) {
             const size_t e = out0 + ((size_t)seq * p.n_head + (size_t)kvh * G + gi) * kHeadDim + dim;
             if (INGOT_CHECK(e, 1, p.out_extent, p.status)) store_out(p.out, p.out_dtype, e, O / L);
+        } else if (kCluster) {
+            const uint32_t row = gather0 + gi * (kHeadDim + 2) * 4;
+            ingot_sm100::cluster_store(row + dim * 4, O);
+            if (dim == 0) { ingot_sm100::cluster_store(row + 512, M); ingot_sm100::cluster_store(row + 516, L); }
         } else if (INGOT_CHECK(part0 + (part_row0 + gi) * kPartStride, kPartStride, p.part_extent, p.status)) {
             float* row = p.part + part0 + (part_row0 + gi) * kPartStride;
             row[dim] = O;
             if (dim == 0) { row[128] = M; row[129] = L; }
         }
     }
+    if (!kCluster) return;
+    ingot_sm100::cluster_sync();
+    if (single || chunk > 0) return;
+    for (int idx = threadIdx.x; idx < G * kHeadDim; idx += blockDim.x) {  // the attn_combine formula again, over the splits
+        const int gi = idx >> 7, dim = idx & 127;
+        const float* row = gather + gi * (kHeadDim + 2);
+        const int step = G * (kHeadDim + 2);
+        float M = -INFINITY;
+        for (int c = 0; c < n_chunks; c++) M = fmaxf(M, row[c * step + 128]);
+        float L = 0.f, O = 0.f;
+        for (int c = 0; c < n_chunks; c++) {
+            const float wgt = exp2f(row[c * step + 128] - M);
+            L += row[c * step + 129] * wgt;
+            O += row[c * step + dim] * wgt;
+        }
+        const size_t e = out0 + ((size_t)seq * p.n_head + (size_t)kvh * G + gi) * kHeadDim + dim;
+        if (INGOT_CHECK(e, 1, p.out_extent, p.status)) store_out(p.out, p.out_dtype, e, O / L);
+    }
+}
+
+// The splits of a range as one cluster (grid.x = its size), or as CTAs of their own.
+template <typename P>
+int launch_splits(void (*kernel)(P), dim3 grid, int threads, size_t smem, bool cluster, cudaStream_t stream, const P& p) {
+    if (smem > 48 * 1024) INGOT_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    if (cluster) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        attr[cfg.numAttrs].val.clusterDim.x = grid.x;
+        attr[cfg.numAttrs].val.clusterDim.y = attr[cfg.numAttrs].val.clusterDim.z = 1;
+        cfg.numAttrs++;
+    }
+    if (ingot_use_pdl()) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    cfg.attrs = attr;
+    INGOT_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, p));
+    return INGOT_OK;
 }
 
 }  // namespace
@@ -476,6 +535,11 @@ int decode_warps_cfg() {
 // SMs idle. Measured on a B200, 28 layers x 4096 keys in one grid: 3.2 / 4.4 / 5.2 / 5.4 / 5.1 / 5.3 TB/s with
 // 128 / 256 / 512 / 768 / 1024 / 2048 keys per split; a 64-sequence paged batch (lengths 256..8192, 4 layers):
 // 5.4 / 5.7 / 5.9 / 6.1 TB/s with 512 / 768 / 1024 / 2048.
+//   * A single layer of one sequence up to 8192 keys (so few ranges that clusters of 8 find room for all): latency. CTAs of 8 warps, one per
+//     range up to 256 keys, else the CTAs of a cluster, whose first one merges: there is no merge launch and no partial in memory. Append and
+//     attention of 28 layers, 24 heads (B200, a graph): 1000 keys 272 -> 214 us, 400: 267 -> 212, 2000: 338 -> 253, 4096: 392 -> 327, 8192:
+//     489 -> 462; longer ranges want all SMs. Clusters for the jobs that fill the GPU cost more than their merge launch, since a
+//     split waits for its neighbours (28 layers at once, 4096 keys: 87 -> 99 us).
 //   * Up to 256 keys: one split (the CTA writes the output itself; a merge launch would cost more than it saves).
 //   * Jobs that do not fill the CTA slots of the GPU even with 512-key splits (a single layer of one sequence):
 //     fill every slot once with whole 16-key units per warp.
@@ -485,12 +549,18 @@ int decode_warps_cfg() {
 //     short last split of a range as a full one, as an earlier form of this rule did, picked 960 for 28 x 4096 keys:
 //     four rounds of 1024; 832 - five equal splits, four rounds of 896 - streams the same keys in 12 % less.)
 DecodePlan decode_plan(const ingot_kv* kv, int n_layers, int n_seq, int max_seq_len, int chunk_keys) {
-    const int n_warps = decode_warps_cfg();
+    int n_warps = decode_warps_cfg();
+    bool cluster = false;
     const int min_chunk = ((max_seq_len + kMaxParts - 1) / kMaxParts + 15) / 16 * 16;
     if (chunk_keys == 0) {
         const int slots = kv->num_sms * (8 / n_warps);
         const long long ranges = (long long)n_layers * n_seq * kv->n_head_kv;
-        if (max_seq_len <= 256) {
+        if (n_seq == 1 && ranges * kClusterParts <= kv->num_sms && max_seq_len <= kClusterKeys) {
+            n_warps = max_seq_len <= 64 ? decode_warps_cfg() : kMaxDecodeWarps;
+            const int per_part = ((max_seq_len + kClusterParts - 1) / kClusterParts + 15) / 16 * 16;
+            chunk_keys = max_seq_len <= 256 ? 256 : std::max(per_part, kMaxDecodeWarps * 16);
+            cluster = true;
+        } else if (max_seq_len <= 256) {
             chunk_keys = 256;  // one split per range: its CTA writes the output itself and no merge launch is needed
         } else if (ranges * ((max_seq_len + 511) / 512) <= slots) {
             const int per_range = (int)std::max<long long>(1, slots / ranges);
@@ -514,6 +584,8 @@ DecodePlan decode_plan(const ingot_kv* kv, int n_layers, int n_seq, int max_seq_
     DecodePlan plan;
     plan.chunk_keys = chunk_keys;
     plan.n_parts = (max_seq_len + chunk_keys - 1) / chunk_keys;
+    plan.n_warps = n_warps;
+    plan.cluster = cluster && plan.n_parts > 1;
     return plan;
 }
 int decode_slots(const ingot_kv* kv) { return kv->num_sms * (8 / decode_warps_cfg()); }
@@ -530,8 +602,8 @@ size_t decode_part_floats(int n_seq, int n_parts, int n_head) {
 int launch_attn_decode(ingot_kv* kv, int layer, int n_layers, const void* q, int q_dtype, void* out, int out_dtype, int n_head,
                        int n_seq, const int32_t* seq_lens, int max_seq_len, const int32_t* block_tables,
                        int max_blocks_per_seq, DecodePlan plan, float* part, int merge_only, int pdl_mode, cudaStream_t stream) {
-    if (merge_only && plan.n_parts <= 1) return INGOT_OK;
-    const int n_warps = decode_warps_cfg();
+    if (merge_only && (plan.n_parts <= 1 || plan.cluster)) return INGOT_OK;
+    const int n_warps = plan.n_warps;
     DecodeParams p;
     p.kc = kv->k + size_t(layer) * kv->layer_elems;
     p.vc = kv->v + size_t(layer) * kv->layer_elems;
@@ -554,10 +626,9 @@ int launch_attn_decode(ingot_kv* kv, int layer, int n_layers, const void* q, int
     const int threads = n_warps * 32;
     const size_t smem_split = (size_t)n_warps * p.group * (kHeadDim + 2);
     const size_t smem_merge = (size_t)2 * p.group * kMaxParts + (size_t)4 * std::max(threads, p.group * 32);
-    const size_t smem = std::max(smem_split, smem_merge) * sizeof(float);
+    const size_t smem = (plan.cluster ? smem_split + (size_t)plan.n_parts * p.group * (kHeadDim + 2) : std::max(smem_split, smem_merge)) * sizeof(float);
     const dim3 grid(merge_only ? 1 : plan.n_parts, kv->n_head_kv, (unsigned)(n_layers * n_seq));
-    INGOT_CUDA_TRY(ingot_launch_pdl(attn_decode_kernel, grid, dim3(threads), smem, stream, p));
-    return INGOT_OK;
+    return launch_splits(plan.cluster ? attn_decode_kernel<true> : attn_decode_kernel<false>, grid, threads, smem, plan.cluster, stream, p);
 }
 
 // ---- decode without any allocation ----------------------------------------------------------------
@@ -642,11 +713,11 @@ extern "C" int ingot_attn_decode_noalloc(const void* k_dev, const void* v_dev, i
     const size_t smem = max(smem_split, smem_merge) * sizeof(float);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     p.split_parts = n_parts;
-    attn_decode_kernel<<<dim3(n_parts, n_head_kv, 1), threads, smem, s>>>(p);
+    attn_decode_kernel<false><<<dim3(n_parts, n_head_kv, 1), threads, smem, s>>>(p);
     INGOT_CUDA_TRY(cudaGetLastError());
     if (n_parts > 1) {  // merge-only launch; stream order makes the partials visible
         p.split_parts = 0;
-        attn_decode_kernel<<<dim3(1, n_head_kv, 1), threads, smem, s>>>(p);
+        attn_decode_kernel<false><<<dim3(1, n_head_kv, 1), threads, smem, s>>>(p);
         INGOT_CUDA_TRY(cudaGetLastError());
     }
     return INGOT_OK;
@@ -660,7 +731,7 @@ extern "C" int ingot_attn_decode_noalloc(const void* k_dev, const void* v_dev, i
 int launch_attn_decode_append(ingot_kv* kv, int layer, const float* q, const float* k, const float* v, const float* inv_freq, void* out,
                               int out_dtype, int n_head, const int32_t* seq_lens, int max_seq_len, DecodePlan plan, float* part,
                               cudaStream_t stream) {
-    const int n_warps = decode_warps_cfg();
+    const int n_warps = plan.n_warps;
     DecodeAppendParams p;
     p.kc = kv->k + size_t(layer) * kv->layer_elems;
     p.vc = kv->v + size_t(layer) * kv->layer_elems;
@@ -686,9 +757,8 @@ int launch_attn_decode_append(ingot_kv* kv, int layer, const float* q, const flo
     const int threads = n_warps * 32;
     const size_t smem_split = (size_t)n_warps * p.group * (kHeadDim + 2);
     const size_t smem_merge = (size_t)2 * p.group * kMaxParts + (size_t)4 * std::max(threads, p.group * 32);
-    const size_t smem = std::max(smem_split, smem_merge) * sizeof(float);
+    const size_t smem = (plan.cluster ? smem_split + (size_t)plan.n_parts * p.group * (kHeadDim + 2) : std::max(smem_split, smem_merge)) * sizeof(float);
     const dim3 grid(plan.n_parts, kv->n_head_kv, 1);
-    INGOT_CUDA_TRY(ingot_launch_pdl(attn_decode_append_kernel, grid, dim3(threads), smem, stream, p));
-    return INGOT_OK;
+    return launch_splits(plan.cluster ? attn_decode_append_kernel<true> : attn_decode_append_kernel<false>, grid, threads, smem, plan.cluster, stream, p);
 }
 #endif

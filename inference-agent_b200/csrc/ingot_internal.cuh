@@ -157,7 +157,10 @@ int launch_rope_kv_append(ingot_kv* kv, int layer, const float* q, __half* q_out
                           int layer_count, cudaStream_t stream);
 int launch_kv_import_f16(ingot_kv* kv, int layer, const __half* k, const __half* v, int pos0, int n_tok,
                          const int32_t* block_table, cudaStream_t stream);
-struct DecodePlan { int chunk_keys, n_parts; };
+struct DecodePlan {
+    int chunk_keys, n_parts, n_warps;  // n_warps: per CTA
+    bool cluster;                      // the splits of a range share a cluster: no partials in memory, no merge launch
+};
 DecodePlan decode_plan(const ingot_kv* kv, int n_layers, int n_seq, int max_seq_len, int chunk_keys);
 int decode_slots(const ingot_kv* kv);
 int decode_warps_cfg();

@@ -249,3 +249,30 @@ def test_device_length_beyond_the_cache_is_clamped_and_flagged():
     torch.cuda.synchronize()
     assert kv.status() == 1
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("n_keys,bound", [(64, 64), (65, 65), (256, 256), (257, 257), (385, 385), (1025, 1025), (8192, 8192), (8193, 8193), (1, 4096), (130, 4096), (2000, 8192)])
+@pytest.mark.parametrize("n_head,paged", [(24, False), (64, True)])
+def test_decode_of_one_sequence_around_its_splits(n_keys, bound, n_head, paged):
+    """Splits that share a cluster: the first and the last key count of each form, splits without keys (the count is read from device memory,
+    the bound sizes the launch), the largest group of heads. Against float64."""
+    import torch
+    import ingot_b200 as ib
+    g = torch.Generator(device="cuda").manual_seed(n_keys + n_head)
+    pages = (bound + 15) // 16
+    kv = ib.KVCache(ib.KV_PAGED if paged else ib.KV_CONTIGUOUS, 1, 8, pages if paged else bound)
+    for which in "kv":
+        kv.layer_view(0, which).normal_(generator=g)
+    q = torch.randn(1, n_head, 128, device="cuda", generator=g).half()
+    table = torch.randperm(pages, device="cuda", generator=g).int()[None]
+    k, v = (kv.layer_view(0, w).double() for w in "kv")
+    if paged:
+        k, v = (x[table[0].long()].transpose(0, 1).reshape(8, -1, 128) for x in (k, v))
+    s = torch.einsum("hgd,hkd->hgk", q[0].double().view(8, -1, 128), k[:, :n_keys]) / 128 ** 0.5
+    want = torch.einsum("hgk,hkd->hgd", s.softmax(-1), v[:, :n_keys]).reshape(1, n_head, 128)
+    count = torch.tensor([n_keys], dtype=torch.int32, device="cuda")
+    out = ib.attn_decode(kv, 0, q, seq_lens=count, max_seq_len=bound, block_tables=table if paged else None)
+    torch.cuda.synchronize()
+    assert kv.status() == 0
+    # weights rounded to f16: 2^-11 of each term; terms of size 1, weights that sum to 1
+    assert (out.double() - want).abs().max().item() < 2.0 ** -11 * v.abs().max().item()
