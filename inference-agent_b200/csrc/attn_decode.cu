@@ -181,6 +181,10 @@ __device__ __forceinline__ void combine_splits(const DecodeParams& p, float* sme
         }
         const float inv = L > 0.f ? 1.0f / L : 0.f;
         const size_t e = out0 + ((size_t)seq * p.n_head + (size_t)kvh * G + gi) * kHeadDim + cl * 4;
+        if (p.out_dtype == INGOT_F32 && reinterpret_cast<uintptr_t>(p.c_out) % 16 == 0) {  // whole lines: the output may be in host memory
+            *reinterpret_cast<float4*>(static_cast<float*>(p.c_out) + e) = make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv);
+            continue;
+        }
         store_out(p.c_out, p.out_dtype, e + 0, acc.x * inv);
         store_out(p.c_out, p.out_dtype, e + 1, acc.y * inv);
         store_out(p.c_out, p.out_dtype, e + 2, acc.z * inv);
