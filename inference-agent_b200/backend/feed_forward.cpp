@@ -7,8 +7,16 @@ namespace {
 class GatedFeedForward : public FeedForward {
 public:
     GatedFeedForward(LayerOps& ops, const Json& c, const std::string& p) {
-        const Groups ff = flat(get_int(c, "ff")), d = flat(ops.width);
-        w_gu_ = ops.matrix(2 * ff.padded, d.padded, {Part{p + "gate", {ff.count(), d.count()}, ff, d, 0}, Part{p + "up", {ff.count(), d.count()}, ff, d, ff.padded}});
+        const Groups d = flat(ops.width), ff = {1, get_int(c, "ff"), round_up(get_int(c, "ff"), 32)};
+        // runs of 32 gate rows, each followed by the 32 up rows that go with them: what finishes a gate meets its up value
+        std::vector<Part> parts;
+        const int full = ff.size / 32, rest = ff.size % 32;
+        for (int up = 0; up < 2; up++) {
+            const std::string name = p + (up ? "up" : "gate");
+            if (full) parts.push_back(Part{name, {ff.count(), d.count()}, {full, 32, 64}, d, 32 * up});
+            if (rest) parts.push_back(Part{name, {ff.count(), d.count()}, {1, rest, rest}, d, 64 * full + 32 * up, 0, 32 * full});
+        }
+        w_gu_ = ops.matrix(2 * ff.padded, d.padded, parts);
         w_down_ = ops.matrix(p + "down", d, ff);
         ops.need(kGateUp, 2 * ff.padded);
         ops.need(kMid, ff.padded);

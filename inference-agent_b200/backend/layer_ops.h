@@ -62,7 +62,7 @@ cudaError_t ingot_linear_tc_run_f16(ingot_linear_ws* ws, void* out, int out_ld, 
                                     cudaStream_t s);
 cudaError_t ingot_linear_tc_finish_residual_norm_bf16(ingot_linear_ws* ws, float* x, const float* norm_w, float eps, int n_mean, int planes,
                                                       const float* pair_rows, const int32_t* row_of, int top, cudaStream_t s);
-cudaError_t ingot_linear_tc_finish_gated_bf16(ingot_linear_ws* ws, int act, int planes, cudaStream_t s);
+cudaError_t ingot_linear_tc_run_gated_bf16(ingot_linear_ws* ws, const void* w, int n_in, int n_out, int act, int planes, cudaStream_t s);
 }
 
 inline constexpr int kMinTcTokens = 2;  // from two tokens on, a 128-token tile that is mostly padding still only streams the weights once
@@ -465,7 +465,7 @@ public:
         project(s, x, w, buf(kConcat), 2 * n);
         norm_ready_ = Norm();
     }
-    // kMid (or the operand planes) = act(W_gate h) * (W_up h), h = norm(x); w holds the gate rows and then the up rows
+    // kMid (or the operand planes) = act(W_gate h) * (W_up h), h = norm(x); w holds runs of 32 gate rows, each followed by its up rows
     void gated_project(const StepCtx& s, const Matrix& w, const Norm& norm) {
         if (s.tc) prepare_norm(s, w, norm);
         else if (norm.apart() || !(s.st.n_tok == 1 && streams(w))) norm_rows(s, norm);
@@ -475,8 +475,7 @@ public:
     void gated_project_normed(const StepCtx& s, const Matrix& w, const Norm& norm) {
         const int ff = w.n_out / 2;
         if (s.tc) {
-            cuda_check(ingot_linear_tc_run_partial(ws, w.data, w.n_in, w.n_out, 0, stream), "gate / up");
-            cuda_check(ingot_linear_tc_finish_gated_bf16(ws, design.act, s.planes, stream), "gate");
+            cuda_check(ingot_linear_tc_run_gated_bf16(ws, w.data, w.n_in, w.n_out, design.act, s.planes, stream), "gate / up");
         } else if (s.st.n_tok == 1 && streams(w)) {
             cuda_check(ingot_support_gemv_bf16(buf(kMid), w.data, ff, w.n_in, norm.apart() ? buf(kNormed) : x, norm.apart() ? nullptr : norm.w, eps, width, 1, design.act, 0, stream), "gate / up");
         } else {

@@ -99,6 +99,9 @@ struct GemmParams {
     int to_partial;  // write the slice(s) to `partial` even when there is only one (a consumer kernel sums them)
 };
 
+__device__ __forceinline__ float silu_of(float g) { return g / (1.0f + expf(-g)); }
+__device__ __forceinline__ float gelu_of(float g) { return 0.5f * g * (1.0f + tanhf(0.7978845608028654f * (g + 0.044715f * g * g * g))); }  // the tanh form
+
 // ---- few rows ----------------------------------------------------------------------------------------------------------
 //
 // Products of up to kFewRows rows whose activations are a pair of planes: decoded tokens, short prompts, experts with a few rows each.
@@ -332,7 +335,7 @@ linear_few_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_const
                         for (int i = 0; i < 8; i++)
                             if (c + i < n_rows) {
                                 const int row = t.m0 + c + i;
-                                put_pair((size_t)row * half_out + out_col, v[i] / (1.0f + expf(-v[i])) * swap[(c + i) * 32 + lane] * (p.row_scale ? p.row_scale[row] : 1.0f));
+                                put_pair((size_t)row * half_out + out_col, silu_of(v[i]) * swap[(c + i) * 32 + lane] * (p.row_scale ? p.row_scale[row] : 1.0f));
                             }
                     }
                 }
@@ -603,7 +606,7 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_cons
         for (int index = pair; index < n_items && ok; index += n_pairs, j++) {
             const Item t = item_at(index);
             ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars->acc_full[j & 1]), (uint32_t)((j >> 1) & 1), abort_flag, kWaitLimitNs)) != 0;
-            if (kGrouped && p.act == 2) ok = pair_all(1 + duo, ok);  // they go on, or leave, together
+            if (p.act >= 2) ok = pair_all(1 + duo, ok);  // they go on, or leave, together
             if (!ok) break;
             tc_fence_after();
             const uint32_t acc = tmem + (uint32_t)((j & 1) * kPairRows) + ((uint32_t)(lg * 32) << 16);
@@ -622,7 +625,7 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_cons
                 p.out_hi[at] = h;
                 if (p.out_lo) p.out_lo[at] = __float2bfloat16_rn(x - __bfloat162float(h));
             };
-            if (kGrouped && p.act == 2) {
+            if (p.act >= 2) {
                 // Runs of 32 gate outputs, each followed by the 32 up outputs that go with them: one warp's lanes and the next one's. Of 16
                 // rows each warp finishes 8: it hands the other half of its own values over.
                 const bool is_up = lg & 1;
@@ -638,11 +641,15 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_cons
                     asm volatile("bar.sync %0, 64;" ::"r"(1 + duo) : "memory");
                     if (col >= t.col_end) continue;
                     const int row = t.m0 + c + (is_up ? 8 : 0), n = t.m0 + t.n_rows - row;
+                    auto gated = [&](auto act) {
 #pragma unroll
-                    for (int i = 0; i < 8; i++) {
-                        const float other = swap[!is_up * 256 + i * 32 + lane], gate = is_up ? other : v[i], up = is_up ? v[8 + i] : other;
-                        x[i] = gate / (1.0f + expf(-gate)) * up;
-                    }
+                        for (int i = 0; i < 8; i++) {
+                            const float other = swap[!is_up * 256 + i * 32 + lane], gate = is_up ? other : v[i], up = is_up ? v[8 + i] : other;
+                            x[i] = act(gate) * up;
+                        }
+                    };
+                    if (kGrouped || p.act == 2) gated([](float g) { return silu_of(g); });
+                    else gated([](float g) { return gelu_of(g); });
 #pragma unroll
                     for (int i = 0; i < 8; i++)
                         if (i < n) put_pair((size_t)(row + i) * half_out + out_col, p.row_scale ? x[i] * p.row_scale[row + i] : x[i]);
@@ -882,7 +889,8 @@ __global__ void finish_swiglu_kernel(__half* hi, __half* lo, const Slices gate, 
     store_split4<kActF16Pair>(hi, lo, i, f);
 }
 
-// One or two bf16 planes of act(gate) * up, where one product of width 2 n holds both: gate = columns 0..n-1, up = columns n..2n-1.
+// One or two bf16 planes of act(gate) * up, where one product of width 2 n holds both as runs of 32 gate columns, each followed by the 32
+// up columns that go with them.
 // act: 0 silu, 1 the tanh form of gelu. grid.y = row.
 template <int kAct>
 __global__ void finish_gated_kernel(__half* hi, __half* lo, const Slices in, int n, size_t slice, int act) {
@@ -892,13 +900,14 @@ __global__ void finish_gated_kernel(__half* hi, __half* lo, const Slices in, int
     if (i >= n) return;
     const size_t row = (size_t)blockIdx.y * 2 * n;
     const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-    const float4 g = sum_slices(in, row + i, slice, z), u = sum_slices(in, row + n + i, slice, z);
+    const int at = (i & ~31) * 2 + (i & 31);
+    const float4 g = sum_slices(in, row + at, slice, z), u = sum_slices(in, row + at + 32, slice, z);
     const float gv[4] = {g.x, g.y, g.z, g.w}, uv[4] = {u.x, u.y, u.z, u.w};
     float f[4];
 #pragma unroll
     for (int e = 0; e < 4; e++) {
         const float t = gv[e];
-        f[e] = (act == 0 ? t / (1.0f + expf(-t)) : 0.5f * t * (1.0f + tanhf(0.7978845608028654f * (t + 0.044715f * t * t * t)))) * uv[e];
+        f[e] = (act == 0 ? silu_of(t) : gelu_of(t)) * uv[e];
     }
     store_split4<kAct>(hi, lo, (size_t)blockIdx.y * n + i, f);
 }
@@ -1143,7 +1152,7 @@ cudaError_t ingot_linear_tc_prepare_norm_bf16(ingot_linear_ws* ws, const float* 
 // n_out / rows_per_block such blocks side by side.
 static cudaError_t launch_gemm(ingot_linear_ws* ws, float* out, const void* const* w, int n_in, const int* n_out, int count,
                                int accumulate, int first_slot, bool to_partial, bool append, cudaStream_t s, int rows_per_block = 0,
-                               __half* out_half = nullptr, int half_ld = 0, int half_block = 0) {
+                               __half* out_half = nullptr, int half_ld = 0, int half_block = 0, int gate = 0) {
     const int n_tok = ws->prepared_tok;
     if (rows_per_block > 0 && (count != 1 || n_out[0] % rows_per_block != 0 || rows_per_block % 4 != 0 || n_in % 8 != 0)) return cudaErrorInvalidValue;
     const int act_in = rows_per_block > 0 ? n_in * (n_out[0] / rows_per_block) : n_in;
@@ -1172,7 +1181,7 @@ static cudaError_t launch_gemm(ingot_linear_ws* ws, float* out, const void* cons
     const int k_steps = (n_in + kBK - 1) / kBK;
     // enough k slices to give every SM a CTA, at least 4 k-steps each, and no more than the slots hold
     if (to_partial && fit < 1) return cudaErrorInvalidValue;
-    const int most = out_half ? 1 : std::max(fit, 1);
+    const int most = out_half || gate ? 1 : std::max(fit, 1);
     const PairTiles t = pair_tiles(n_tok, tiles_n, ws->planes, k_steps, most, ws->num_sms);
     const int n_split = few ? std::max(1, std::min({ws->num_sms / tiles_n, k_steps / 4, most})) : t.n_split;
     // A batch of few tokens fetches only its own rows (whole 8-row swizzle groups). What else the boxes hold is multiplied along and never stored.
@@ -1183,6 +1192,8 @@ static cudaError_t launch_gemm(ingot_linear_ws* ws, float* out, const void* cons
     p.half_ld = half_ld;
     p.half_block = half_block;
     p.out = out; p.status = ws->status;
+    p.act = gate;
+    if (gate) p.out_hi = reinterpret_cast<__nv_bfloat16*>(ws->lo);
     p.n_tok = n_tok; p.k_steps = k_steps; p.n_split = n_split; p.accumulate = accumulate;
     p.to_partial = to_partial ? 1 : 0;
     p.idesc = kIdescF16 | (ws->bf16 ? kIdescBF16 : 0u);
@@ -1346,10 +1357,21 @@ cudaError_t ingot_linear_tc_finish_residual_norm_bf16(ingot_linear_ws* ws, float
     return norm_w ? set_prepared(ws, n, n_tok) : cudaGetLastError();
 }
 
-// The product in slot 0 (width 2 n: gate half, up half) becomes the bf16 operand act(gate) * up of the next product.
-cudaError_t ingot_linear_tc_finish_gated_bf16(ingot_linear_ws* ws, int act, int planes, cudaStream_t s) {
-    const int n = ws->slot_out[0] / 2, n_tok = ws->prepared_tok;
-    if (!ws->bf16 || n % 8 != 0 || !act_shape_ok(ws, n, n_tok)) return cudaErrorInvalidValue;
+// The bf16 operand act(gate) * up of the next product, from W whose rows are runs of 32 gate rows, each followed by the 32 up rows that go
+// with them (n_out: both). act: 0 silu, 1 the tanh form of gelu; planes: of the operand. With one plane in and out the accumulators
+// become the operand on their way out, in the plane that is not read (the lo plane; the two then change places): 4096 rows of 28672
+// wide results took 150 us more to write in f32 and to read again (B200). Otherwise, and where k slices fill the GPU, through slot 0.
+cudaError_t ingot_linear_tc_run_gated_bf16(ingot_linear_ws* ws, const void* w, int n_in, int n_out, int act, int planes, cudaStream_t s) {
+    const int n = n_out / 2, n_tok = ws->prepared_tok;
+    if (!ws->bf16 || n_out % 64 != 0 || !act_shape_ok(ws, n, n_tok)) return cudaErrorInvalidValue;
+    if (ws->planes == 1 && planes == 1 && pair_tiles(n_tok, (n_out + 255) / 256, 1, (n_in + kBK - 1) / kBK, 1 << 20, ws->num_sms).n_split == 1) {
+        const cudaError_t e = launch_gemm(ws, nullptr, &w, n_in, &n_out, 1, 0, 0, false, false, s, 0, nullptr, 0, 0, 2 + act);
+        if (e != cudaSuccess) return e;
+        std::swap(ws->hi, ws->lo);
+        return set_prepared(ws, n, n_tok);
+    }
+    const cudaError_t e = launch_gemm(ws, nullptr, &w, n_in, &n_out, 1, 0, 0, true, false, s);
+    if (e != cudaSuccess) return e;
     const dim3 grid((unsigned)((n / 4 + 255) / 256), n_tok);
     cudaError_t le = planes > 1
         ? launch_pdl(finish_gated_kernel<kActBF16Pair>, grid, dim3(256), 0, s, ws->hi, ws->lo, slices_of(ws, 0), n, (size_t)n_tok * 2 * n, act)

@@ -97,7 +97,8 @@ __global__ void gated_act_kernel(float* out, const float* in, int n, size_t tota
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total) return;
     const size_t r = i / n, c = i - r * n;
-    out[i] = gate_act(in[r * 2 * n + c], act) * in[r * 2 * n + n + c];
+    const size_t at = r * 2 * n + (c & ~size_t(31)) * 2 + (c & 31);  // runs of 32 gate values, each followed by their up values
+    out[i] = gate_act(in[at], act) * in[at + 32];
 }
 
 // gate[i] = silu(gate[i]) * up[i]      (src/cpu_backend.cpp:79, ops::silu src/ops.h:35)
@@ -387,8 +388,9 @@ __global__ void __launch_bounds__(StreamThreads<kFmt>::value) gemv_stream_kernel
 
     auto row_base = [&](int r, const char*& wa, const char*& wb, const __half*& da, const __half*& db) {
         if (kSwiGLU) {
-            wa = static_cast<const char*>(g.w[0]) + (size_t)r * row_bytes;
-            wb = static_cast<const char*>(g.w[1]) + (size_t)r * row_bytes;
+            const size_t row = kFmt == kFmtBF16 ? size_t(r & ~31) * 2 + (r & 31) : size_t(r);  // bf16: runs of 32 gate rows and 32 up rows
+            wa = static_cast<const char*>(g.w[0]) + row * row_bytes;
+            wb = static_cast<const char*>(g.w[1]) + row * row_bytes;
             da = FmtTraits<kFmt>::kPlain ? nullptr : g.d[0] + (size_t)r * row_scales;
             db = FmtTraits<kFmt>::kPlain ? nullptr : g.d[1] + (size_t)r * row_scales;
         } else {
@@ -761,7 +763,8 @@ cudaError_t ingot_support_gemv_group(float* const* outs, const void* const* ws, 
 cudaError_t ingot_support_gemv_bf16(float* out, const void* w, int n_out, int n_in, const float* x, const float* norm_w, float eps, int n_mean,
                                     int gated, int act, int accumulate, cudaStream_t s) {
     float* outs[2] = {out, out};
-    const void* ws[2] = {w, static_cast<const char*>(w) + (size_t)n_out * n_in * 2};
+    if (gated && n_out % 32 != 0) return cudaErrorInvalidValue;
+    const void* ws[2] = {w, static_cast<const char*>(w) + (gated ? (size_t)32 : (size_t)n_out) * n_in * 2};
     const int rows[2] = {n_out, n_out};
     return gemv_group(outs, ws, nullptr, kFmtBF16, rows, gated ? 2 : 1, gated, act, x, norm_w, eps, n_in, n_mean, accumulate, s);
 }
@@ -843,7 +846,7 @@ cudaError_t ingot_support_rmsnorm_rows(float* out, const float* x, const float* 
     return support_launch(rmsnorm_rows_kernel, dim3(n_rows), dim3(256), 0, s, out, x, w, rows_dev, n, n_mean, eps);
 }
 
-// out[r][i] = act(gate) * up with gate = in[r][i], up = in[r][n + i] (one product holds both halves); act: 0 silu, 1 gelu (tanh form)
+// out[r][i] = act(gate) * up; one product holds both, as runs of 32 gate values and 32 up values (n a multiple of 32); act: 0 silu, 1 gelu (tanh form)
 cudaError_t ingot_support_gated_act(float* out, const float* in, int n_rows, int n, int act, cudaStream_t s) {
     const size_t total = (size_t)n_rows * n;
     return support_launch(gated_act_kernel, dim3(unsigned((total + 255) / 256)), dim3(256), 0, s, out, in, n, total, act);

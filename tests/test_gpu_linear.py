@@ -324,3 +324,39 @@ def test_products_of_bf16_planes(n_tok, n_in, n_out, blocks, planes):
             assert (out.double() - 2 * want).abs().max().item() <= 2 * 5 * 2.0 ** -24 * n_in ** 0.5 * 8
     finally:
         lib.ingot_linear_ws_destroy(ws)
+
+
+@pytest.mark.parametrize("n_tok,n_in,ff,act,planes", [(2, 64, 32, 0, 2), (70, 2048, 96, 1, 1), (70, 264, 9504, 0, 1), (600, 512, 5024, 1, 1), (300, 72, 64, 1, 2)])
+def test_gated_products(n_tok, n_in, ff, act, planes):
+    """The gate in the epilogue (one plane, tiles enough), and through slices: the operand that is left, against float64."""
+    import torch
+    lib = _lib()
+    vp, ci = C.c_void_p, C.c_int
+    lib.ingot_linear_ws_create_bf16.argtypes = [C.POINTER(vp), ci, ci, ci]
+    lib.ingot_linear_tc_prepare_bf16.argtypes = [vp, vp, ci, ci, ci, ci, vp]
+    lib.ingot_linear_tc_run_gated_bf16.argtypes = [vp, vp, ci, ci, ci, ci, vp]
+    ws = vp()
+    assert lib.ingot_linear_ws_create_bf16(C.byref(ws), n_tok, max(n_in, ff), max(2 * ff, 256)) == 0
+    try:
+        g = torch.Generator(device="cuda").manual_seed(ff)
+        x = torch.randn(n_tok, n_in, device="cuda", generator=g)
+        gate, up = ((torch.randn(ff, n_in, device="cuda", generator=g) / n_in ** 0.5).bfloat16() for _ in range(2))
+        w = torch.stack([gate.view(-1, 32, n_in), up.view(-1, 32, n_in)], dim=1).reshape(2 * ff, n_in).contiguous()
+        hi = x.bfloat16()
+        seen = hi.double() + ((x - hi.float()).bfloat16().double() if planes > 1 else 0)
+        a, b = seen @ gate.double().T, seen @ up.double().T
+        want = (torch.nn.functional.silu(a) if act == 0 else torch.nn.functional.gelu(a, approximate="tanh")) * b
+        # the operand as the next product sees it: times the identity (exact in f32)
+        eye = torch.eye(ff, device="cuda").bfloat16()
+        out = torch.full((n_tok, ff), float("nan"), device="cuda")
+        st = vp(torch.cuda.current_stream().cuda_stream)
+        for _ in range(2):  # once more with the planes the other way round
+            assert lib.ingot_linear_tc_prepare_bf16(ws, x.data_ptr(), n_in, n_in, n_tok, planes, st) == 0
+            assert lib.ingot_linear_tc_run_gated_bf16(ws, w.data_ptr(), n_in, 2 * ff, act, planes, st) == 0
+            assert lib.ingot_linear_tc_run(ws, out.data_ptr(), eye.data_ptr(), ff, ff, 0, st) == 0
+            torch.cuda.synchronize()
+            assert lib.ingot_linear_ws_status(ws) == 0
+            # one bf16 rounding (two planes: 2^-17) of the value, and f32 sums of n_in terms
+            assert ((out.double() - want).abs() <= 2.0 ** (-8 if planes < 2 else -16) * want.abs() + 1e-4).all()
+    finally:
+        lib.ingot_linear_ws_destroy(ws)
