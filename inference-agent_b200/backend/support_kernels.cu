@@ -365,11 +365,12 @@ __device__ __forceinline__ float dot_load(const uint4& raw, const float4* x4, un
 // L2 traffic per launch. f16 rows need 80 registers per thread and fit 768 threads (24 warps, one CTA per SM);
 // the quantised formats need up to 122 and stay at 256 threads, two or three CTAs per SM (512-thread CTAs measured:
 // Q8_0 tg32 561 -> 536 tok/s, Q4_0 539 -> 544).
-template <int kFmt>
-struct StreamThreads { static constexpr int value = FmtTraits<kFmt>::kPlain ? 768 : 256; };
+// kLoads = 8 (plain formats): 512 threads with a row each, where that many rows there are at most (see gemv_group).
+template <int kFmt, int kLoads>
+struct StreamThreads { static constexpr int value = !FmtTraits<kFmt>::kPlain ? 256 : kLoads == 8 ? 512 : 768; };
 
 template <bool kNorm, bool kSwiGLU, int kLoads, int kFmt>
-__global__ void __launch_bounds__(StreamThreads<kFmt>::value) gemv_stream_kernel(const GemvGroup g, const float* x, const float* norm_w, float eps, int n_in,
+__global__ void __launch_bounds__(StreamThreads<kFmt, kLoads>::value) gemv_stream_kernel(const GemvGroup g, const float* x, const float* norm_w, float eps, int n_in,
                                                           int total_rows, int accumulate, int use_pdl, int n_mean, int act) {
     extern __shared__ float xs[];  // x', n_in floats
     __shared__ float red[25];
@@ -701,11 +702,20 @@ static cudaError_t gemv_group(float* const* outs, const void* const* ws, const v
     const size_t smem = (size_t)n_in * sizeof(float);
     // kLoads = 6 for short rows: with the current and the next step in flight the whole row is requested at once
     const bool short_rows = n_in / chunk <= 12;  // current and next step together cover the row
+    int dev = 0, num_sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return e;
+    // Long rows, no more than 16 per SM: warps of 512-thread CTAs take one each, with up to 4096 weights of it requested before the wait for
+    // the kernel before - the time such a launch has is mostly that kernel's. 2048 x 4096 7.4 -> 7.2 us, 2048 x 8192 11.6 -> 9.5 us inside a step (B200).
+    const bool row_each = plain && !short_rows && !swiglu && rows <= num_sms * 16;
     typedef void (*Kernel)(GemvGroup, const float*, const float*, float, int, int, int, int, int, int);
     auto pick = [&](auto fmt_tag) -> Kernel {
         constexpr int F = decltype(fmt_tag)::value;
         if constexpr (F == kFmtBF16)
             if (swiglu && !norm_w) return short_rows ? gemv_stream_kernel<false, true, 6, F> : gemv_stream_kernel<false, true, 4, F>;
+        if constexpr (FmtTraits<F>::kPlain)
+            if (row_each) return norm_w ? gemv_stream_kernel<true, false, 8, F> : gemv_stream_kernel<false, false, 8, F>;
         return short_rows ? (swiglu ? gemv_stream_kernel<true, true, 6, F> : norm_w ? gemv_stream_kernel<true, false, 6, F> : gemv_stream_kernel<false, false, 6, F>)
                           : (swiglu ? gemv_stream_kernel<true, true, 4, F> : norm_w ? gemv_stream_kernel<true, false, 4, F> : gemv_stream_kernel<false, false, 4, F>);
     };
@@ -717,12 +727,8 @@ static cudaError_t gemv_group(float* const* outs, const void* const* ws, const v
     // CTAs of one launch per SM. Fewer than fit leaves room for the next launch's CTAs, which then request
     // their first weights while this launch is still streaming (programmatic dependent launch).
     static const int ctas_per_sm_cap = [] { const char* c = getenv("INGOT_GEMV_CTAS_PER_SM"); return c ? atoi(c) : 0; }();
-    int dev = 0, num_sms = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e != cudaSuccess) return e;
     int occ = 0;
-    const int threads = plain ? StreamThreads<kFmtF16>::value : StreamThreads<kFmtQ8_0>::value, cta_warps = threads / 32;
+    const int threads = row_each ? StreamThreads<kFmtF16, 8>::value : plain ? StreamThreads<kFmtF16, 6>::value : StreamThreads<kFmtQ8_0, 6>::value, cta_warps = threads / 32;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, threads, smem);
     if (e != cudaSuccess) return e;
     if (occ < 1) occ = 1;
