@@ -365,7 +365,7 @@ __device__ __forceinline__ float dot_load(const uint4& raw, const float4* x4, un
 // L2 traffic per launch. f16 rows need 80 registers per thread and fit 768 threads (24 warps, one CTA per SM);
 // the quantised formats need up to 122 and stay at 256 threads, two or three CTAs per SM (512-thread CTAs measured:
 // Q8_0 tg32 561 -> 536 tok/s, Q4_0 539 -> 544).
-// kLoads = 8 (plain formats): 512 threads with a row each, where that many rows there are at most (see gemv_group).
+// kLoads = 8 (plain formats): 512 threads, for a few long rows per warp (see gemv_group).
 template <int kFmt, int kLoads>
 struct StreamThreads { static constexpr int value = !FmtTraits<kFmt>::kPlain ? 256 : kLoads == 8 ? 512 : 768; };
 
@@ -706,9 +706,11 @@ static cudaError_t gemv_group(float* const* outs, const void* const* ws, const v
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
-    // Long rows, no more than 16 per SM: warps of 512-thread CTAs take one each, with up to 4096 weights of it requested before the wait for
-    // the kernel before - the time such a launch has is mostly that kernel's. 2048 x 4096 7.4 -> 7.2 us, 2048 x 8192 11.6 -> 9.5 us inside a step (B200).
-    const bool row_each = plain && !short_rows && !swiglu && rows <= num_sms * 16;
+    // Long rows, one or two per warp of 512-thread CTAs (no more than the 768-thread ones would have): up to 4096 weights of a row are
+    // requested before the wait for the kernel before - the time such a launch has is mostly that kernel's. Inside a step (B200): 2048 x 4096
+    // 7.4 -> 7.2 us, 2048 x 8192 11.6 -> 9.5, 4096 x 8192 22.5 -> 18. With more rows per warp the 24 warps stream faster (32768 x 2048 27.5 against 32).
+    const int per_warp = (rows + num_sms * 16 - 1) / (num_sms * 16);
+    const bool row_each = plain && !short_rows && !swiglu && per_warp <= 2 && per_warp <= (rows + num_sms * 24 - 1) / (num_sms * 24);
     typedef void (*Kernel)(GemvGroup, const float*, const float*, float, int, int, int, int, int, int);
     auto pick = [&](auto fmt_tag) -> Kernel {
         constexpr int F = decltype(fmt_tag)::value;
