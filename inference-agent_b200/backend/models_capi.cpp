@@ -29,6 +29,16 @@ static int guarded(F&& f) {
     }
 }
 
+// Whether a kernel can write this place of host memory under its own address.
+static bool device_writes(float* host) {
+    cudaPointerAttributes at = {};
+    if (cudaPointerGetAttributes(&at, host) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return at.type == cudaMemoryTypeHost && at.devicePointer == host;
+}
+
 extern "C" {
 
 const char* ingot_models_last_error() { return g_models_error.c_str(); }
@@ -66,9 +76,8 @@ int ingot_model_step(ingot_model* m, int n, const int32_t* seq_ids, const int32_
             want += n_want[i];
             rows += size_t(n_want[i]);
         }
-        cudaPointerAttributes at = {};
-        const bool pinned = logits_out && cudaPointerGetAttributes(&at, logits_out) == cudaSuccess && at.type == cudaMemoryTypeHost && at.devicePointer == logits_out;
-        if (logits_out && !pinned) cudaGetLastError();
+        const size_t count = rows * size_t(m->backend->n_vocab());
+        const bool pinned = logits_out && count > 0 && device_writes(logits_out) && device_writes(logits_out + count - 1);
         if (pinned) m->backend->step_into(logits_out);
         const float* logits = m->backend->forward_step(e.data(), n, m->backend->n_vocab());
         if (logits_out && logits && logits != logits_out) std::copy(logits, logits + rows * size_t(m->backend->n_vocab()), logits_out);
