@@ -975,22 +975,27 @@ cudaError_t launch_pair(const GemmParams& g, int rows, int planes, int box_rows,
     return launch_pdl(linear_pair_kernel<kGrouped>, dim3(2 * std::min(items, num_sms / 2)), dim3(kPairThreads), (size_t)kPairSmem, s, hi, lo, *w[0], *w[1], *w[2], p);
 }
 
-// Rows of a tile and k slices for n_tok rows against tiles_n tiles of 256 outputs: the least rounds of all pairs of CTAs times what one costs.
+// k slices of a product of `tiles` blocks of 128 outputs by 128 rows: enough to give every SM a block, at least 4 k-steps each. The last bits of a
+// product depend on its slices, and what follows rounds them to 16 bits: the number depends on nothing but the product's size and the SMs,
+// so that other tiles or another kernel leave a model's results as they are.
+int k_slices(long long tiles, int k_steps, int most, int num_sms) {
+    return (int)std::max(1ll, std::min({num_sms / tiles, (long long)k_steps / 4, (long long)most}));
+}
+long long blocks_of(int n) { return (n + 127) / 128; }
+
+// Rows of a tile for n_tok rows against tiles_n tiles of 256 outputs in n_split slices: the least rounds of all pairs of CTAs times what one costs.
 // A k-step takes a pair as long as it takes to load it, about as 256 + rows (at 256 rows that is 512 cycles, what the MMAs take), and a
 // tile starts and ends for about four k-steps.
-struct PairTiles { int rows, row_tiles, n_split; };
-PairTiles pair_tiles(int n_tok, int tiles_n, int planes, int k_steps, int most_splits, int num_sms) {
+struct PairTiles { int rows, row_tiles; };
+PairTiles pair_tiles(int n_tok, int tiles_n, int planes, int k_steps, int n_split, int num_sms) {
     const int pairs = num_sms / 2;
     PairTiles best = {};
     long long least = 0;
     for (int rows = kPairRows / planes; rows >= 32; rows -= 32) {
-        PairTiles t;
-        t.rows = rows;
-        t.row_tiles = (n_tok + rows - 1) / rows;
-        const long long tiles = (long long)tiles_n * t.row_tiles;
-        t.n_split = (int)std::max(1ll, std::min({pairs / tiles, (long long)k_steps / 4, (long long)most_splits}));
-        const long long rounds = (tiles * t.n_split + pairs - 1) / pairs, cost = rounds * ((k_steps + t.n_split - 1) / t.n_split + 4) * (256 + rows * planes);
-        if (best.rows == 0 || cost < least) { best = t; least = cost; }
+        const int row_tiles = (n_tok + rows - 1) / rows;
+        const long long items = (long long)tiles_n * row_tiles * n_split, rounds = (items + pairs - 1) / pairs;
+        const long long cost = rounds * ((k_steps + n_split - 1) / n_split + 4) * (256 + rows * planes);
+        if (best.rows == 0 || cost < least) { best = {rows, row_tiles}; least = cost; }
     }
     return best;
 }
@@ -1168,9 +1173,11 @@ static cudaError_t launch_gemm(ingot_linear_ws* ws, float* out, const void* cons
     const bool few = ws->planes > 1 && n_tok <= kFewRows;  // linear_few_kernel
     const int tile = few ? 128 : 256;
     int tiles_n = 0, fit = 1 << 30;
+    long long blocks = 0;  // of 128 outputs
     for (int m = 0; m < count; m++) {
         if (!(maps[m] = map_of(ws, w[m], n_out[m], n_in, 128, ws->bf16))) return cudaErrorUnknown;
         tiles_n += rows_per_block > 0 ? n_out[m] / rows_per_block * ((rows_per_block + tile - 1) / tile) : (n_out[m] + tile - 1) / tile;
+        blocks += rows_per_block > 0 ? n_out[m] / rows_per_block * blocks_of(rows_per_block) : blocks_of(n_out[m]);
         p.tile_end[m] = tiles_n;
         p.n_out[m] = n_out[m];
         p.partial[m] = ws->partial + (size_t)(first_slot + m) * ws->partial_floats + (size_t)held * n_tok * n_out[m];
@@ -1179,11 +1186,9 @@ static cudaError_t launch_gemm(ingot_linear_ws* ws, float* out, const void* cons
     for (int m = count; m < 3; m++) { maps[m] = maps[count - 1]; p.tile_end[m] = tiles_n; p.n_out[m] = n_out[count - 1]; p.partial[m] = p.partial[count - 1]; }
     p.tiles_n = tiles_n;
     const int k_steps = (n_in + kBK - 1) / kBK;
-    // enough k slices to give every SM a CTA, at least 4 k-steps each, and no more than the slots hold
     if (to_partial && fit < 1) return cudaErrorInvalidValue;
-    const int most = out_half || gate ? 1 : std::max(fit, 1);
-    const PairTiles t = pair_tiles(n_tok, tiles_n, ws->planes, k_steps, most, ws->num_sms);
-    const int n_split = few ? std::max(1, std::min({ws->num_sms / tiles_n, k_steps / 4, most})) : t.n_split;
+    const int n_split = out_half || gate ? 1 : k_slices(blocks * blocks_of(n_tok), k_steps, fit, ws->num_sms);  // no more than the slots hold
+    const PairTiles t = pair_tiles(n_tok, tiles_n, ws->planes, k_steps, n_split, ws->num_sms);
     // A batch of few tokens fetches only its own rows (whole 8-row swizzle groups). What else the boxes hold is multiplied along and never stored.
     const int box = few ? (n_tok + 7) / 8 * 8 : t.rows / 2;
     const CUtensorMap *hi = map_of(ws, ws->hi, n_tok, act_in, box, ws->bf16), *lo = ws->planes > 1 ? map_of(ws, ws->lo, n_tok, act_in, box, ws->bf16) : hi;
@@ -1364,7 +1369,7 @@ cudaError_t ingot_linear_tc_finish_residual_norm_bf16(ingot_linear_ws* ws, float
 cudaError_t ingot_linear_tc_run_gated_bf16(ingot_linear_ws* ws, const void* w, int n_in, int n_out, int act, int planes, cudaStream_t s) {
     const int n = n_out / 2, n_tok = ws->prepared_tok;
     if (!ws->bf16 || n_out % 64 != 0 || !act_shape_ok(ws, n, n_tok)) return cudaErrorInvalidValue;
-    if (ws->planes == 1 && planes == 1 && pair_tiles(n_tok, (n_out + 255) / 256, 1, (n_in + kBK - 1) / kBK, 1 << 20, ws->num_sms).n_split == 1) {
+    if (ws->planes == 1 && planes == 1 && k_slices(blocks_of(n_out) * blocks_of(n_tok), (n_in + kBK - 1) / kBK, 1 << 20, ws->num_sms) == 1) {
         const cudaError_t e = launch_gemm(ws, nullptr, &w, n_in, &n_out, 1, 0, 0, false, false, s, 0, nullptr, 0, 0, 2 + act);
         if (e != cudaSuccess) return e;
         std::swap(ws->hi, ws->lo);

@@ -326,6 +326,50 @@ def test_products_of_bf16_planes(n_tok, n_in, n_out, blocks, planes):
         lib.ingot_linear_ws_destroy(ws)
 
 
+@pytest.mark.parametrize("n_tok,n_in,n_out,planes", [
+    (2048, 1000, 288, 1),  # 3 slices, the last one ragged
+    (1000, 832, 1024, 1),  # 2
+    (1000, 2048, 16, 1),   # 8, as many as there are four k-steps
+    (2047, 1344, 264, 2),
+    (33, 1000, 520, 2),    # few rows
+])
+def test_k_slices_follow_from_the_size_of_a_product(n_tok, n_in, n_out, planes):
+    """A product that does not fill the GPU with 128 x 128 blocks is the sum, in order, of as many k slices as give every SM a block: bit for bit
+    what products of those parts of the rows and weights add up to, whatever tiles a kernel works on."""
+    import torch
+    lib = _lib()
+    vp, ci = C.c_void_p, C.c_int
+    lib.ingot_linear_ws_create_bf16.argtypes = [C.POINTER(vp), ci, ci, ci]
+    lib.ingot_linear_tc_prepare_bf16.argtypes = [vp, vp, ci, ci, ci, ci, vp]
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    steps = -(-n_in // 64)
+    slices = min(sms // (-(-n_out // 128) * -(-n_tok // 128)), steps // 4)
+    assert slices > 1 and -(-steps // slices) < 8  # a part of up to 7 k-steps is not cut again
+    ws = vp()
+    assert lib.ingot_linear_ws_create_bf16(C.byref(ws), n_tok, n_in, n_out) == 0
+    try:
+        g = torch.Generator(device="cuda").manual_seed(n_tok)
+        x = torch.randn(n_tok, n_in, device="cuda", generator=g)
+        w = (torch.randn(n_out, n_in, device="cuda", generator=g) / n_in ** 0.5).bfloat16()
+        st = vp(torch.cuda.current_stream().cuda_stream)
+
+        def product(x, w):
+            x, w, out = x.contiguous(), w.contiguous(), torch.full((n_tok, n_out), float("nan"), device="cuda")
+            assert lib.ingot_linear_tc_prepare_bf16(ws, x.data_ptr(), x.shape[1], x.shape[1], n_tok, planes, st) == 0
+            assert lib.ingot_linear_tc_run(ws, out.data_ptr(), w.data_ptr(), x.shape[1], n_out, 0, st) == 0
+            torch.cuda.synchronize()
+            return out
+
+        whole, parts = product(x, w), torch.zeros(n_tok, n_out, device="cuda")
+        for i in range(slices):
+            k = slice(steps * i // slices * 64, min(steps * (i + 1) // slices * 64, n_in))
+            parts = parts + product(x[:, k], w[:, k])
+        assert lib.ingot_linear_ws_status(ws) == 0
+        assert torch.equal(whole, parts)
+    finally:
+        lib.ingot_linear_ws_destroy(ws)
+
+
 @pytest.mark.parametrize("n_tok,n_in,ff,act,planes", [(2, 64, 32, 0, 2), (70, 2048, 96, 1, 1), (70, 264, 9504, 0, 1), (600, 512, 5024, 1, 1), (300, 72, 64, 1, 2)])
 def test_gated_products(n_tok, n_in, ff, act, planes):
     """The gate in the epilogue (one plane, tiles enough), and through slices: the operand that is left, against float64."""
