@@ -123,7 +123,8 @@ int ingot_kv_import_f16(ingot_kv* kv, int layer, const void* k_f16_dev, const vo
  *   out_dev [n_seq][n_head][128]  out_dtype in {F32, F16}
  *   seq_lens_dev [n_seq] int32: keys 0..len-1 of each sequence are attended (len >= 1).
  *          NULL with n_seq == 1 means the single length max_seq_len.
- *   max_seq_len: host-side upper bound of every length (sizes the launch grid).
+ *   max_seq_len: host-side upper bound of every length (sizes the launch grid). A device length beyond what the grid covers is
+ *          clamped and raises bit 0 of the status word.
  *   block_tables_dev [n_seq][max_blocks_per_seq]: paged caches only.
  * chunk_keys: keys per split (multiple of 16), or 0 to let the library choose. */
 int ingot_attn_decode(ingot_kv* kv, int layer, const void* q_dev, int q_dtype, void* out_dev, int out_dtype,

@@ -236,6 +236,7 @@ __global__ void __launch_bounds__(kMaxDecodeWarps * 32, 1) DECODE_KERNEL(const D
     // per thread.
     __shared__ __align__(16) __half new_q[8 * kHeadDim];
     __shared__ __align__(16) __half new_kv[2 * kHeadDim];
+    const bool appends = p.seq_lens == nullptr || p.seq_lens[seq] == n_keys;  // of a count that was clamped the row is skipped, as by K1
     {
         const float fpos = float(n_keys - 1);
         for (int u = threadIdx.x; u < (G + 2) * 16; u += blockDim.x) {
@@ -280,7 +281,7 @@ __global__ void __launch_bounds__(kMaxDecodeWarps * 32, 1) DECODE_KERNEL(const D
                     const int c = 4 * i + j;
                     const uint4 val = *reinterpret_cast<const uint4*>(new_kv + c * 8);
                     r.k[nt * 4 + i] = val;
-                    if (nt * 8 + g == last) *reinterpret_cast<uint4*>(p.kc_w + (size_t)layer * p.cache_layer_stride + ub + (size_t)row * kHeadDim + c * 8) = val;
+                    if (nt * 8 + g == last && appends) *reinterpret_cast<uint4*>(p.kc_w + (size_t)layer * p.cache_layer_stride + ub + (size_t)row * kHeadDim + c * 8) = val;
                 }
                 continue;
             }
@@ -305,7 +306,7 @@ __global__ void __launch_bounds__(kMaxDecodeWarps * 32, 1) DECODE_KERNEL(const D
                     const int c = g + 8 * hgh;
                     const uint4 val = *reinterpret_cast<const uint4*>(new_kv + kHeadDim + c * 8);
                     r.v[s * 2 + hgh] = val;
-                    if (row_own == last) *reinterpret_cast<uint4*>(p.vc_w + (size_t)layer * p.cache_layer_stride + ub + (size_t)row * kHeadDim + c * 8) = val;
+                    if (row_own == last && appends) *reinterpret_cast<uint4*>(p.vc_w + (size_t)layer * p.cache_layer_stride + ub + (size_t)row * kHeadDim + c * 8) = val;
                 }
                 continue;
             }

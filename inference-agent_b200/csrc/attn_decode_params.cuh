@@ -34,11 +34,12 @@ struct DecodeParams {
 };
 enum : int { kPdlWaitFirst = 0, kPdlEarlyLoads = 1 };
 
-// Number of keys of sequence `seq`. Lengths that come from device memory cannot be checked on the host:
-// one that exceeds what the cache (or the block table) can hold is clamped and raises the status word.
+// Number of keys of sequence `seq`. Lengths that come from device memory cannot be checked on the host: one that exceeds
+// what the cache (or the block table) can hold, or the splits that were launched (sized by the caller's max_seq_len, as
+// are the partials and their place in shared memory), is clamped and raises the status word.
 __device__ __forceinline__ int load_seq_len(const DecodeParams& p, int seq) {
     int n = p.seq_lens ? p.seq_lens[seq] : p.len0;
-    const int bound = p.paged ? p.max_blocks_per_seq * kBlockTokens : p.capacity;
+    const int bound = min(p.paged ? p.max_blocks_per_seq * kBlockTokens : p.capacity, p.n_parts_max * p.chunk_keys);
     if (n > bound) {
         if (threadIdx.x == 0 && p.status) atomicOr(p.status, kDevErrPosRange);
         n = bound;

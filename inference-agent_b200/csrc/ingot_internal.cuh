@@ -23,7 +23,7 @@ constexpr int kHostPosSlots = 256;  // host-buffer calls that may be queued befo
 
 // Bits of the device status word (ingot_kv::status_dev).
 enum : int {
-    kDevErrPosRange = 1,      // K1: a position fell outside the cache; the row was skipped
+    kDevErrPosRange = 1,      // K1: a position fell outside the cache; the row was skipped. K3: a key count read from device memory was clamped
     kDevErrBlockRange = 2,    // a block-table entry fell outside the pool; the access was skipped
     kDevErrBarrierTimeout = 4,// a bounded wait expired; the kernel gave up cleanly
     kDevErrBounds = 8         // bounds-check build only: an offset fell outside its buffer; the access was skipped

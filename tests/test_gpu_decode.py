@@ -251,6 +251,35 @@ def test_device_length_beyond_the_cache_is_clamped_and_flagged():
     assert torch.equal(got, want)
 
 
+@pytest.mark.parametrize("bound,chunk,covered", [(200, 0, 256), (300, 128, 384), (1000, 128, 1024), (300, 0, 384)])
+def test_device_length_beyond_the_launched_splits_is_clamped_and_flagged(bound, chunk, covered):
+    """max_seq_len sizes the grid, the partials and the shared memory of the splits: a longer device length, though the cache could hold it, is cut
+    to what the splits cover - nothing is read behind them. The one-launch form does not append its row then."""
+    import torch
+    import ingot_b200 as ib
+    g = torch.Generator(device="cuda").manual_seed(bound)
+    kv = ib.KVCache(ib.KV_CONTIGUOUS, 1, HKV, 8192)
+    for which in "kv":
+        kv.layer_view(0, which).normal_(generator=g)
+    k, v = (kv.layer_view(0, w).clone() for w in "kv")
+    q = torch.randn(1, H, D, device="cuda", generator=g).half()
+    s = torch.einsum("hgd,hkd->hgk", q[0].double().view(HKV, -1, D), k[:, :covered].double()) / D ** 0.5
+    want = torch.einsum("hgk,hkd->hgd", s.softmax(-1), v[:, :covered].double()).reshape(1, H, D)
+    for count in (covered + 1, 5000, 8192):
+        n = torch.tensor([count], dtype=torch.int32, device="cuda")
+        out = ib.attn_decode(kv, 0, q, seq_lens=n, max_seq_len=bound, chunk_keys=chunk)
+        torch.cuda.synchronize()
+        assert kv.status() == 1
+        # weights rounded to f16: 2^-11 of each term; terms of size 1, weights that sum to 1
+        assert (out.double() - want).abs().max().item() < 2.0 ** -11 * v.abs().max().item()
+        if not chunk:
+            f = [torch.randn(h, D, device="cuda", generator=g) for h in (H, HKV, HKV)]
+            ib.rope_append_decode(kv, 0, *f, helpers.to_dev(helpers.inv_freq()), 0, key_count=n, max_seq_len=bound)
+            torch.cuda.synchronize()
+            assert kv.status() == 1
+            assert torch.equal(kv.layer_view(0, "k"), k) and torch.equal(kv.layer_view(0, "v"), v)
+
+
 @pytest.mark.parametrize("n_keys,bound", [(64, 64), (65, 65), (256, 256), (257, 257), (385, 385), (1025, 1025), (8192, 8192), (8193, 8193), (1, 4096), (130, 4096), (2000, 8192)])
 @pytest.mark.parametrize("n_head,paged", [(24, False), (64, True)])
 def test_decode_of_one_sequence_around_its_splits(n_keys, bound, n_head, paged):
