@@ -8,7 +8,7 @@ struct ingot_linear_ws;
 
 struct ingot_grouped_gemm {
     const void *a_hi, *a_lo;       // bf16 activation rows [n_rows][n_in], sorted by group; a_lo null: one plane
-    int n_rows, rows_per_group;    // rows_per_group: the most rows a group can have
+    int n_rows, rows_per_group;    // rows_per_group: the most rows a group can have (of a longer one the status word may tell instead of the result)
     const void* w;                 // bf16 [n_groups][n_out][n_in]
     int n_in, n_out, n_groups;     // lengths are multiples of 8
     const int32_t* group_start;    // device, [n_groups + 1]

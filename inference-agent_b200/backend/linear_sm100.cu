@@ -173,7 +173,8 @@ linear_few_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_const
                 const unsigned some = __ballot_sync(0xffffffffu, b > a);
                 if (b > a) {
                     int* e = group_list + 3 * (count + __popc(some & ((1u << lane) - 1)));
-                    e[0] = mine; e[1] = a; e[2] = b;
+                    e[0] = mine; e[1] = a; e[2] = min(b, a + fp.rows);  // what tensor memory and the exchange have room for
+                    if (b - a > fp.rows) atomicOr(p.status, 2);
                 }
                 count += __popc(some);
             }
@@ -1398,7 +1399,8 @@ cudaError_t ingot_linear_tc_finish_swiglu(ingot_linear_ws* ws, int slot_gate, in
 
 int* ingot_linear_ws_status_dev(ingot_linear_ws* ws) { return ws->status; }
 
-// The status word: non-zero after a bounded wait expired in some launch since the last call. Synchronises the device.
+// The status word: non-zero after a bounded wait expired (bit 0) or a group was longer than rows_per_group said (bit 1; its other rows are
+// left out) in some launch since the last call. Synchronises the device.
 int ingot_linear_ws_status(ingot_linear_ws* ws) {
     int v = 0;
     if (cudaMemcpy(&v, ws->status, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) return -1;

@@ -192,6 +192,41 @@ def test_grouped_product_of_many_groups(planes, every, most):
     test_grouped_product(counts, 72, 64, planes)
 
 
+@pytest.mark.parametrize("act", [0, 2])
+@pytest.mark.parametrize("said,counts", [(1, [9, 8, 0, 7]), (5, [3, 20, 8, 64]), (64, [65, 64, 130, 1])])
+def test_groups_longer_than_said_are_cut_and_reported(said, counts, act):
+    """A launch for few rows a group has no room for more: rows behind it are left out and the status word tells, and nothing else changes."""
+    import torch
+    L = M.lib()
+    L.ingot_linear_ws_create_bf16.argtypes = [C.POINTER(C.c_void_p), C.c_int, C.c_int, C.c_int]
+    L.ingot_linear_ws_status.argtypes = L.ingot_linear_ws_destroy.argtypes = [C.c_void_p]
+    L.ingot_grouped_tc_run.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p]
+    rng, n_in, n_out = np.random.default_rng(said), 136, 192
+    rows, start, room = sum(counts), np.concatenate([[0], np.cumsum(counts)]), (said + 7) // 8 * 8
+    hi = bf16(rng.standard_normal((rows, n_in)))
+    lo, w, sd = torch.zeros_like(hi), bf16(rng.standard_normal((len(counts), n_out, n_in)) / n_in ** 0.5), dev(start, np.int32)
+    want = torch.cat([hi[a:b].double() @ w[g].double().T for g, (a, b) in enumerate(zip(start[:-1], start[1:]))])
+    if act:
+        runs = want.view(rows, -1, 2, 32)
+        want = (torch.nn.functional.silu(runs[:, :, 0]) * runs[:, :, 1]).reshape(rows, -1)
+    ws = C.c_void_p()
+    assert L.ingot_linear_ws_create_bf16(C.byref(ws), 8, 8, 8) == 0
+    try:
+        out, (o_hi, o_lo) = torch.full(want.shape, np.nan, device="cuda"), (torch.full(want.shape, np.nan, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+        outs = (None, o_hi.data_ptr(), o_lo.data_ptr()) if act else (out.data_ptr(), None, None)
+        g = CGrouped(hi.data_ptr(), lo.data_ptr(), rows, said, w.data_ptr(), n_in, n_out, len(counts), sd.data_ptr(), None, act, *outs)
+        assert L.ingot_grouped_tc_run(ws, C.byref(g), None) == 0
+        torch.cuda.synchronize()
+        assert L.ingot_linear_ws_status(ws) == (2 if max(counts) > room else 0) and L.ingot_linear_ws_status(ws) == 0
+        got = (o_hi.double() + o_lo.double()) if act else out.double()
+        for a, b in zip(start[:-1], start[1:]):
+            cut = min(b, a + room)
+            assert (got[a:cut] - want[a:cut]).abs().max() < 1e-4 if cut > a else True
+            assert got[cut:b].isnan().all()
+    finally:
+        L.ingot_linear_ws_destroy(ws)
+
+
 @pytest.mark.parametrize("n,experts,identity,top,d,ff", [(1, 4, 0, 2, 40, 32), (1, 3, 2, 4, 256, 64), (2, 5, 1, 3, 64, 32), (9, 5, 3, 5, 64, 96), (130, 12, 4, 3, 48, 64)])
 def test_plain_gated_experts_and_identity_experts(n, experts, identity, top, d, ff):
     """Routing, both products in f32 arithmetic, and the residual sum that takes the identity experts and the shared expert in."""
