@@ -504,7 +504,7 @@ typedef struct ingot_moe_router {
 int ingot_moe_route_grouped(const ingot_moe_router* router, const float* logits_dev, int ld, int n_tok, int32_t* expert_of_dev, float* weight_of_dev,
                             int32_t* group_start_dev, int32_t* row_of_dev, int32_t* pair_of_dev, float* row_weight_dev, float* self_gain_dev,
                             float* shared_gain_dev, void* stream);
-/* The same without a router: table_dev [vocabulary][top] holds each token id's experts (0..n_expert-1, different ones in a row), tokens_dev
+/* The same without a router: table_dev [vocabulary][top] holds each token id's experts (0..n_expert-1; one that is named twice counts twice), tokens_dev
  * [n_tok] the ids; every pair weighs `weight`. expert_of and weight_of may be left unwritten. */
 int ingot_moe_route_table(const int32_t* table_dev, const int32_t* tokens_dev, int n_tok, int n_expert, int top, float weight, int32_t* expert_of_dev,
                           float* weight_of_dev, int32_t* group_start_dev, int32_t* row_of_dev, int32_t* pair_of_dev, float* row_weight_dev, void* stream);

@@ -163,7 +163,7 @@ private:
             ingot_check(ingot_moe_gather(in_hi, in_lo, h_hi, h_lo, pair_of_, rows, start_ + experts_, top_, d_, ops.stream));
             ingot_grouped_gemm g = {};
             g.n_rows = rows;
-            g.rows_per_group = s.st.n_tok;
+            g.rows_per_group = s.st.n_tok * repeats_;
             g.n_groups = experts_;
             g.group_start = start_;
             g.a_hi = in_hi; g.a_lo = in_lo; g.w = w_up_.data; g.n_in = d_; g.n_out = up_rows_;
@@ -185,6 +185,8 @@ private:
         memcpy(table.data(), t.data, table.size() * 4);
         for (int32_t e : table)
             if (e < 0 || e >= experts_) throw std::runtime_error("model: tensor " + name + " names an expert that does not exist");
+        for (auto row = table.begin(); row != table.end(); row += top_)
+            for (auto e = row; e != row + top_; ++e) repeats_ = std::max(repeats_, int(std::count(row, row + top_, *e)));
         table_ = static_cast<int32_t*>(ops.alloc(table.size() * 4));
         cuda_check(cudaMemcpy(table_, table.data(), table.size() * 4, cudaMemcpyHostToDevice), "cudaMemcpy");
     }
@@ -192,6 +194,7 @@ private:
     const bool gated_, by_table_;
     int32_t* table_ = nullptr;
     int experts_, top_, ff_, d_, up_rows_;
+    int repeats_ = 1;  // pairs that a token can have with one expert: a row of the table may name it more than once
     Matrix w_router_, w_up_, w_down_;
     std::unique_ptr<GatedFeedForward> shared_;
     ingot_moe_router route_ = {};

@@ -118,6 +118,21 @@ def test_reach_of_the_input_convolutions(tmp_path, taps, f32):
 
 
 @pytest.mark.parametrize("f32", [True, False])
+def test_experts_that_a_table_names_more_than_once(tmp_path, f32):
+    """Token ids whose rows name an expert twice or three times: it counts as often, for steps of few tokens and of many."""
+    cfg = G.config([G.gla(2, 24, 16, mlp=G.moe(4, 3, 32)), G.mamba2(3, 1, 16, 16)], vocab=50, width=40)
+    w = G.random_weights(cfg, 6)
+    w["l0.mlp.table"][::2] = 1
+    w["l0.mlp.table"][1::4, 2] = w["l0.mlp.table"][1::4, 0]
+    t = np.random.default_rng(3).integers(0, 50, 330).tolist()
+    want = H.reference_logits(cfg, w, t)
+    with open_model(tmp_path, cfg, w, f32=f32, max_tokens=384) as m:
+        for cuts in ([330], [20, 22, 60, 64, 100, 61, 1, 1, 1]):
+            assert H.error(feed(m, 0, t, cuts), want).max() < TOL[f32], cuts
+            m.release(0)
+
+
+@pytest.mark.parametrize("f32", [True, False])
 def test_strong_decays(tmp_path, f32):
     """Powers of the sigmoid that lose a state within a few tokens, or one token, beside rows that keep it."""
     cfg = G.config([G.gla(2, 24, 16, tau=0.5, mlp=G.moe(2, 1, 16)), G.mamba2(3, 1, 16, 16)], vocab=50, width=40)
