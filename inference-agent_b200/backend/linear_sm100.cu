@@ -346,6 +346,7 @@ linear_few_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_const
                 float* const dst = (split_k ? part + (size_t)t.split * p.n_tok * n_out : p.out) + col;
                 for (int c = 0; c < n_rows; c += 8) {
                     float v[8];
+                    __syncwarp();  // lanes past the last output have left the round before early; tensor memory is read by whole warps
                     read(c, v);
                     if (col >= t.col_end) continue;
 #pragma unroll
@@ -633,6 +634,7 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_cons
                 const int half_out = n_out / 2, out_col = t.n0 / 2 + (lg >> 1) * 32 + lane;
                 for (int c = half * 16, buffer = 0; c < t.n_rows; c += 32, buffer ^= 1) {
                     float v[16], x[8];
+                    __syncwarp();
                     tmem_ld16(acc + c, v);
                     tmem_wait_ld();
                     if (c + 32 >= t.n_rows) release();
@@ -660,6 +662,7 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_cons
                 float* const dst = (split_k ? part + (size_t)t.split * p.n_tok * n_out : p.out) + col;
                 for (int c = half * 32; c < t.n_rows; c += 64) {
                     float v[32];
+                    __syncwarp();  // as above: lanes past the last output
                     tmem_ld32(acc + c, v);
                     tmem_wait_ld();
                     if (c + 64 >= t.n_rows) release();
