@@ -498,10 +498,12 @@ __global__ void __launch_bounds__(kMaxDecodeWarps * 32, 1) DECODE_KERNEL(const D
     }
 }
 
-// The splits of a range as one cluster (grid.x = its size), or as CTAs of their own.
+// The splits of a range as one cluster (grid.x = its size), or as CTAs of their own. Static shared memory (2.5 KB of the append form) counts
+// towards the 48 KB that need no permission; every launch asks for the same, so that threads do not take it from one another.
+constexpr size_t kMostSplitSmem = (size_t)(kMaxDecodeWarps + kClusterParts) * 8 * (kHeadDim + 2) * sizeof(float);
 template <typename P>
 int launch_splits(void (*kernel)(P), dim3 grid, int threads, size_t smem, bool cluster, cudaStream_t stream, const P& p) {
-    if (smem > 48 * 1024) INGOT_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > 40 * 1024) INGOT_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMostSplitSmem));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(threads);

@@ -221,6 +221,36 @@ def test_rope_append_decode_equals_k1_then_k3(pos):
     helpers.assert_parity(one_dev.cpu().numpy()[None], want, "fused, key count from device memory")
 
 
+@pytest.mark.parametrize("n_head,n_head_kv,n_keys", [(28, 4, 640), (12, 2, 896), (28, 4, 513), (48, 8, 769)] +
+                         [(h, kvh, n) for h, kvh in ((12, 2), (28, 4), (16, 2), (48, 8), (5, 1)) for n in (512, 577, 769, 1024, 1100)])
+def test_rope_append_decode_of_other_groups(n_head, n_head_kv, n_keys):
+    """Groups of 5 to 8 heads around every number of splits that share a cluster: the shared memory of the one-launch form grows with both. The
+    first ones need just less than a launch may have without asking, were it not for the kernel's static part: they come before any that
+    asks for more. Against K1 + K3 bit for bit, and against float64."""
+    import torch
+    import ingot_b200 as ib
+    g = torch.Generator(device="cuda").manual_seed(n_head + n_keys)
+    caches = [ib.KVCache(ib.KV_CONTIGUOUS, 1, n_head_kv, n_keys) for _ in range(2)]
+    for which in "kv":
+        rows = caches[0].layer_view(0, which).normal_(generator=g)
+        caches[1].layer_view(0, which).copy_(rows)
+    q, k, v = (torch.randn(1, h, D, device="cuda", generator=g) for h in (n_head, n_head_kv, n_head_kv))
+    inv = helpers.to_dev(helpers.inv_freq())
+    one = ib.rope_append_decode(caches[0], 0, q[0], k[0], v[0], inv, n_keys - 1)
+    rotated = ib.rope_kv_append(caches[1], 0, q, k, v, inv, n_keys - 1)
+    two = ib.attn_decode(caches[1], 0, rotated, max_seq_len=n_keys)
+    torch.cuda.synchronize()
+    assert caches[0].status() == caches[1].status() == 0
+    ks, vs = (caches[0].layer_view(0, w).double() for w in "kv")
+    s = torch.einsum("hgd,hkd->hgk", rotated[0].double().view(n_head_kv, -1, D), ks) / D ** 0.5
+    want = torch.einsum("hgk,hkd->hgd", s.softmax(-1), vs).reshape(n_head, D)
+    # weights rounded to f16: 2^-11 of each term; terms of size 1, weights that sum to 1
+    assert (one.double() - want).abs().max().item() < 2.0 ** -11 * vs.abs().max().item()
+    assert torch.equal(one, two[0])
+    for which in "kv":
+        assert torch.equal(caches[0].layer_view(0, which), caches[1].layer_view(0, which))
+
+
 def test_empty_calls_are_no_ops():
     import ingot_b200 as ib
     lib = ib.lib()
