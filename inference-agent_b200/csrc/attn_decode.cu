@@ -195,6 +195,14 @@ __device__ __forceinline__ void combine_splits(const DecodeParams& p, float* sme
 struct KRegs { uint4 k[8]; };  // [n-tile 0/1][i=0..3]: key (nt*8 + g), 16-byte chunk (4i + j)
 struct VRegs { uint4 v[8]; };  // [slot 0..3 -> keys 2j, 2j+1, 2j+8, 2j+9][chunk g / g+8]
 
+// Keys of a split where the splits are the n_parts CTAs of a cluster: an equal share of the keys that there are (up to 256 of them go to
+// one CTA). The kernel works it out again from the count in device memory, which may be far below the bound that sized the cluster: 1000 keys under
+// a bound of 8192 go to eight CTAs and not to one.
+__host__ __device__ constexpr int cluster_share(int n_keys, int n_parts) {
+    const int share = ((n_keys + n_parts - 1) / n_parts + 15) / 16 * 16, least = kMaxDecodeWarps * 16;
+    return n_keys <= 256 ? 256 : share > least ? share : least;
+}
+
 // kCluster: the splits of a range are the CTAs of a cluster, and its first CTA merges them in shared memory.
 template <bool kCluster>
 __global__ void __launch_bounds__(kMaxDecodeWarps * 32, 1) DECODE_KERNEL(const DECODE_PARAMS p) {
@@ -214,13 +222,14 @@ __global__ void __launch_bounds__(kMaxDecodeWarps * 32, 1) DECODE_KERNEL(const D
     const __half* const kc = p.kc + (size_t)layer * p.cache_layer_stride;
     const __half* const vc = p.vc + (size_t)layer * p.cache_layer_stride;
     const int n_keys = load_seq_len(p, seq);
-    const int n_chunks = (max(n_keys, 0) + p.chunk_keys - 1) / p.chunk_keys;
+    const int chunk_keys = kCluster ? cluster_share(n_keys, p.n_parts_max) : p.chunk_keys;
+    const int n_chunks = (max(n_keys, 0) + chunk_keys - 1) / chunk_keys;
     if (chunk >= n_chunks) {  // no keys, or none for this split
         if (kCluster) { ingot_sm100::cluster_wait(); ingot_sm100::cluster_sync(); }
         return;
     }
-    const int k_begin = chunk * p.chunk_keys;
-    const int k_end = min(n_keys, k_begin + p.chunk_keys);
+    const int k_begin = chunk * chunk_keys;
+    const int k_end = min(n_keys, k_begin + chunk_keys);
     const int n_units = (k_end - k_begin + 15) >> 4;
 
     const int n_warps = blockDim.x >> 5;
@@ -564,8 +573,7 @@ DecodePlan decode_plan(const ingot_kv* kv, int n_layers, int n_seq, int max_seq_
         const long long ranges = (long long)n_layers * n_seq * kv->n_head_kv;
         if (n_seq == 1 && ranges * kClusterParts <= kv->num_sms && max_seq_len <= kClusterKeys) {
             n_warps = max_seq_len <= 64 ? decode_warps_cfg() : kMaxDecodeWarps;
-            const int per_part = ((max_seq_len + kClusterParts - 1) / kClusterParts + 15) / 16 * 16;
-            chunk_keys = max_seq_len <= 256 ? 256 : std::max(per_part, kMaxDecodeWarps * 16);
+            chunk_keys = cluster_share(max_seq_len, kClusterParts);
             cluster = true;
         } else if (max_seq_len <= 256) {
             chunk_keys = 256;  // one split per range: its CTA writes the output itself and no merge launch is needed

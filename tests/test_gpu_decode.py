@@ -251,6 +251,29 @@ def test_rope_append_decode_of_other_groups(n_head, n_head_kv, n_keys):
         assert torch.equal(caches[0].layer_view(0, which), caches[1].layer_view(0, which))
 
 
+@pytest.mark.parametrize("bound", [300, 4096, 8192])
+@pytest.mark.parametrize("n_keys", [1, 130, 257, 300, 400, 1000, 1040, 4095])
+def test_a_count_below_its_bound_is_split_as_if_it_were_the_bound(n_keys, bound):
+    """A replayed graph reads the key count from device memory, under a bound that holds for the whole conversation: its keys are shared out as for
+    a call that names the count (the same bits), not as the bound's would be."""
+    import torch
+    import ingot_b200 as ib
+    if n_keys > bound:
+        pytest.skip("beyond the bound")
+    g = torch.Generator(device="cuda").manual_seed(n_keys)
+    kv = ib.KVCache(ib.KV_CONTIGUOUS, 1, HKV, 8192)
+    for which in "kv":
+        kv.layer_view(0, which).normal_(generator=g)
+    q = torch.randn(1, H, D, device="cuda", generator=g).half()
+    want = ib.attn_decode(kv, 0, q, max_seq_len=n_keys)
+    got = ib.attn_decode(kv, 0, q, seq_lens=torch.tensor([n_keys], dtype=torch.int32, device="cuda"), max_seq_len=bound)
+    torch.cuda.synchronize()
+    assert kv.status() == 0
+    if n_keys > 64:  # below, a call that names the count takes smaller CTAs
+        assert torch.equal(got, want)
+    assert (got - want).abs().max().item() < 1e-5
+
+
 def test_empty_calls_are_no_ops():
     import ingot_b200 as ib
     lib = ib.lib()
