@@ -59,7 +59,6 @@ namespace {
 
 constexpr int kMaxDecodeWarps = 8;
 constexpr int kMaxParts = 64;
-constexpr int kClusterParts = 8;  // CTAs of a portable cluster
 constexpr int kClusterKeys = 8192;
 
 // Merges the splits of one (sequence, kv head): out = sum_s o_s 2^(m_s-M) / sum_s l_s 2^(m_s-M)
@@ -551,11 +550,12 @@ int decode_warps_cfg() {
 // SMs idle. Measured on a B200, 28 layers x 4096 keys in one grid: 3.2 / 4.4 / 5.2 / 5.4 / 5.1 / 5.3 TB/s with
 // 128 / 256 / 512 / 768 / 1024 / 2048 keys per split; a 64-sequence paged batch (lengths 256..8192, 4 layers):
 // 5.4 / 5.7 / 5.9 / 6.1 TB/s with 512 / 768 / 1024 / 2048.
-//   * A single layer of one sequence up to 8192 keys (so few ranges that clusters of 8 find room for all): latency. CTAs of 8 warps, one per
-//     range up to 256 keys, else the CTAs of a cluster, whose first one merges: there is no merge launch and no partial in memory. Append and
-//     attention of 28 layers, 24 heads (B200, a graph): 1000 keys 272 -> 214 us, 400: 267 -> 212, 2000: 338 -> 253, 4096: 392 -> 327, 8192:
-//     489 -> 462; longer ranges want all SMs. Clusters for the jobs that fill the GPU cost more than their merge launch, since a
-//     split waits for its neighbours (28 layers at once, 4096 keys: 87 -> 99 us).
+//   * A single layer of one sequence up to 8192 keys: latency. CTAs of 8 warps, one per range up to 256 keys, else the CTAs of a cluster, whose
+//     first one merges: there is no merge launch and no partial in memory. Append and attention of 28 layers, 24 heads (B200, a graph): 1000
+//     keys 272 -> 214 us, 400: 267 -> 212, 2000: 338 -> 253, 4096: 392 -> 327, 8192: 489 -> 462; with one KV head 8192: 759 -> 497; longer
+//     ranges want all SMs. Only where the device holds the clusters of all ranges at a time (15 of 8 CTAs here: a cluster lies within
+//     one of its groups of SMs): 15 KV heads 8192 keys 552 -> 503, but 16 584 -> 822. Clusters for the jobs that fill the GPU cost more than
+//     their merge launch, since a split waits for its neighbours (28 layers at once, 4096 keys: 87 -> 99 us).
 //   * Up to 256 keys: one split (the CTA writes the output itself; a merge launch would cost more than it saves).
 //   * Jobs that do not fill the CTA slots of the GPU even with 512-key splits (a single layer of one sequence):
 //     fill every slot once with whole 16-key units per warp.
@@ -571,9 +571,10 @@ DecodePlan decode_plan(const ingot_kv* kv, int n_layers, int n_seq, int max_seq_
     if (chunk_keys == 0) {
         const int slots = kv->num_sms * (8 / n_warps);
         const long long ranges = (long long)n_layers * n_seq * kv->n_head_kv;
-        if (n_seq == 1 && ranges * kClusterParts <= kv->num_sms && max_seq_len <= kClusterKeys) {
+        const int share = cluster_share(max_seq_len, kClusterParts), parts = (max_seq_len + share - 1) / share;
+        if (n_seq == 1 && ranges * kClusterParts <= kv->num_sms && max_seq_len <= kClusterKeys && (parts == 1 || ranges <= kv->cluster_room[parts])) {
             n_warps = max_seq_len <= 64 ? decode_warps_cfg() : kMaxDecodeWarps;
-            chunk_keys = cluster_share(max_seq_len, kClusterParts);
+            chunk_keys = share;
             cluster = true;
         } else if (max_seq_len <= 256) {
             chunk_keys = 256;  // one split per range: its CTA writes the output itself and no merge launch is needed
@@ -602,6 +603,26 @@ DecodePlan decode_plan(const ingot_kv* kv, int n_layers, int n_seq, int max_seq_
     plan.n_warps = n_warps;
     plan.cluster = cluster && plan.n_parts > 1;
     return plan;
+}
+// How many clusters of n CTAs the current device holds at a time, for n = 2..8; 0 where it cannot tell.
+void decode_cluster_room(int (&room)[kClusterParts + 1]) {
+    for (int n = 0; n <= kClusterParts; n++) {
+        cudaLaunchAttribute attr;
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = n;
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(n * 64);
+        cfg.blockDim = dim3(kMaxDecodeWarps * 32);
+        cfg.dynamicSmemBytes = 40 * 1024;  // what needs no permission; a CTA's registers leave no room for a second one in any case
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        room[n] = 0;
+        if (n >= 2 && cudaOccupancyMaxActiveClusters(&room[n], attn_decode_kernel<true>, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            room[n] = 0;
+        }
+    }
 }
 int decode_slots(const ingot_kv* kv) { return kv->num_sms * (8 / decode_warps_cfg()); }
 

@@ -45,9 +45,12 @@ __device__ __forceinline__ bool ingot_in_bounds(size_t first, size_t count, size
 #define INGOT_CHECK(first, count, extent, status) true
 #endif
 
+constexpr int kClusterParts = 8;  // CTAs of a portable cluster
+
 struct ingot_kv {
     int device = 0;
     int num_sms = 0;  // of `device`
+    int cluster_room[kClusterParts + 1] = {};  // how many clusters of decode CTAs it holds at a time, by their size
     int layout = INGOT_KV_CONTIGUOUS;
     int n_layer = 0, n_head_kv = 0, head_dim = kHeadDim;
     int capacity = 0;   // positions (contiguous) or blocks (paged)
@@ -162,6 +165,7 @@ struct DecodePlan {
     bool cluster;                      // the splits of a range share a cluster: no partials in memory, no merge launch
 };
 DecodePlan decode_plan(const ingot_kv* kv, int n_layers, int n_seq, int max_seq_len, int chunk_keys);
+void decode_cluster_room(int (&room)[kClusterParts + 1]);
 int decode_slots(const ingot_kv* kv);
 int decode_warps_cfg();
 int launch_attn_decode_append(ingot_kv* kv, int layer, const float* q, const float* k, const float* v, const float* inv_freq, void* out,

@@ -31,6 +31,7 @@ int ingot_kv_create(ingot_kv** out, int layout, int n_layer, int n_head_kv, int 
     if (e != cudaSuccess) { delete kv; return ingot_cuda_fail(e, "cudaGetDevice"); }
     e = cudaDeviceGetAttribute(&kv->num_sms, cudaDevAttrMultiProcessorCount, kv->device);
     if (e != cudaSuccess) { delete kv; return ingot_cuda_fail(e, "cudaDeviceGetAttribute"); }
+    decode_cluster_room(kv->cluster_room);
     kv->layout = layout;
     kv->n_layer = n_layer;
     kv->n_head_kv = n_head_kv;

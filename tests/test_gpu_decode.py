@@ -274,6 +274,23 @@ def test_a_count_below_its_bound_is_split_as_if_it_were_the_bound(n_keys, bound)
     assert (got - want).abs().max().item() < 1e-5
 
 
+@pytest.mark.parametrize("n_keys,chunk", [(1000, 64), (4096, 256), (8192, 512)])
+def test_ranges_whose_clusters_do_not_fit_at_a_time_are_split_separately(n_keys, chunk):
+    """18 clusters of 8 CTAs would need 144 of 148 SMs in whole clusters per group of SMs: such a layer takes separate splits, of the size that
+    fills the GPU once (the bits of a call that names it)."""
+    import torch
+    import ingot_b200 as ib
+    assert torch.cuda.get_device_properties(0).multi_processor_count == 148
+    g = torch.Generator(device="cuda").manual_seed(n_keys)
+    kv = ib.KVCache(ib.KV_CONTIGUOUS, 1, 18, n_keys)
+    for which in "kv":
+        kv.layer_view(0, which).normal_(generator=g)
+    q = torch.randn(1, 36, D, device="cuda", generator=g).half()
+    planned, named = (ib.attn_decode(kv, 0, q, max_seq_len=n_keys, chunk_keys=c) for c in (0, chunk))
+    torch.cuda.synchronize()
+    assert kv.status() == 0 and torch.equal(planned, named)
+
+
 def test_empty_calls_are_no_ops():
     import ingot_b200 as ib
     lib = ib.lib()
