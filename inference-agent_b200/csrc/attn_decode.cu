@@ -633,7 +633,7 @@ size_t decode_part_floats(int n_seq, int n_parts, int n_head) {
 // One launch of the decode kernel over `n_layers` consecutive layers starting at `layer`: either the split CTAs
 // (merge_only == 0; partials of split ranges into `part`, outputs of single-split ranges straight into `out`) or
 // one merge CTA per (kv head, layer, sequence) that turns the partials in `part` into `out` (merge_only != 0; a
-// no-op when the plan has a single split). q and out are [n_layers][n_seq][n_head][128], `part` holds n_layers
+// no-op when the plan has a single split, or a cluster, which leaves no partials). q and out are [n_layers][n_seq][n_head][128], `part` holds n_layers
 // blocks of decode_part_floats(). pdl_mode: kPdlWaitFirst or kPdlEarlyLoads (see DecodeParams).
 int launch_attn_decode(ingot_kv* kv, int layer, int n_layers, const void* q, int q_dtype, void* out, int out_dtype, int n_head,
                        int n_seq, const int32_t* seq_lens, int max_seq_len, const int32_t* block_tables,
@@ -763,7 +763,7 @@ extern "C" int ingot_attn_decode_noalloc(const void* k_dev, const void* v_dev, i
 #ifdef INGOT_DECODE_APPEND
 // One launch of the fused form for one token of one sequence on a contiguous cache: q/k/v are the f32 projections, the
 // key count (position + 1) comes from seq_lens (device) or max_seq_len. Splits and partials as in launch_attn_decode;
-// with more than one split the caller follows up with the plain kernel's merge-only launch.
+// with more than one split, and no cluster, the caller follows up with the plain kernel's merge-only launch.
 int launch_attn_decode_append(ingot_kv* kv, int layer, const float* q, const float* k, const float* v, const float* inv_freq, void* out,
                               int out_dtype, int n_head, const int32_t* seq_lens, int max_seq_len, DecodePlan plan, float* part,
                               cudaStream_t stream) {

@@ -230,17 +230,18 @@ int ingot_attn_decode_layers(ingot_kv* kv, int layer_begin, int layer_count, con
     // The layers are independent of one another, so their split CTAs share a grid: blockIdx.z runs over (layer,
     // sequence), there is no launch boundary between layers and the block scheduler refills an SM the moment a CTA
     // retires. A merge-only launch (chained with programmatic dependent launch, so its CTAs are resident and
-    // waiting when the split grid drains) then turns the split partials into the outputs. A single layer is the
-    // same two launches. Only the size of the split scratch bounds how many layers share a launch:
-    // INGOT_DECODE_SCRATCH_MB (default 256) caps it, and more layers than fit are done in groups.
+    // waiting when the split grid drains) then turns the split partials into the outputs. Splits that share a cluster
+    // (a single layer of one sequence, see decode_plan) merge there: one launch, no scratch. Only the size of the split scratch
+    // bounds how many layers share a launch: INGOT_DECODE_SCRATCH_MB (default 256) caps it, and more layers than fit are done in groups.
     const DecodePlan plan = decode_plan(kv, layer_count, n_seq, max_seq_len, chunk_keys);
     const size_t per_layer = decode_part_floats(n_seq, plan.n_parts, n_head);
     size_t cap_mb = 256;
     if (const char* e = getenv("INGOT_DECODE_SCRATCH_MB")) cap_mb = size_t(std::max(1, atoi(e)));
-    int group = plan.n_parts > 1 ? int(std::max<size_t>(1, std::min<size_t>(size_t(layer_count), (cap_mb << 20) / (per_layer * sizeof(float)))))
-                                 : layer_count;
+    const bool partials = plan.n_parts > 1 && !plan.cluster;
+    int group = partials ? int(std::max<size_t>(1, std::min<size_t>(size_t(layer_count), (cap_mb << 20) / (per_layer * sizeof(float)))))
+                         : layer_count;
     group = std::min(group, std::max(1, 65535 / n_seq));  // gridDim.z
-    if (plan.n_parts > 1) {
+    if (partials) {
         rc = ensure_decode_scratch(kv, per_layer * size_t(group));
         if (rc != INGOT_OK) return rc;
     }
@@ -261,7 +262,7 @@ int ingot_attn_decode_layers(ingot_kv* kv, int layer_begin, int layer_count, con
 }
 
 // K1 + K3 for one token of the one sequence of a contiguous cache, in one launch (plus the merge launch when the keys
-// are split): see attn_decode_append.cu.
+// are split and the splits do not share a cluster): see attn_decode_append.cu.
 int ingot_rope_append_decode(ingot_kv* kv, int layer, const float* q_dev, const float* k_dev, const float* v_dev,
                              const float* inv_freq_dev, void* out_dev, int out_dtype, int n_head, const int32_t* key_count_dev,
                              int pos, int max_seq_len, void* stream) {
@@ -282,7 +283,7 @@ int ingot_rope_append_decode(ingot_kv* kv, int layer, const float* q_dev, const 
     INGOT_REQUIRE(max_seq_len >= 1 && max_seq_len <= kv->capacity, "ingot_rope_append_decode: max_seq_len out of range");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const DecodePlan plan = decode_plan(kv, 1, 1, max_seq_len, 0);
-    if (plan.n_parts > 1) {
+    if (plan.n_parts > 1 && !plan.cluster) {
         const int rc = ensure_decode_scratch(kv, decode_part_floats(1, plan.n_parts, n_head));
         if (rc != INGOT_OK) return rc;
     }
@@ -290,7 +291,7 @@ int ingot_rope_append_decode(ingot_kv* kv, int layer, const float* q_dev, const 
                                        plan, kv->part, s);
     if (rc != INGOT_OK) return rc;
     return launch_attn_decode(kv, layer, 1, nullptr, INGOT_F16, out_dev, out_dtype, n_head, 1, key_count_dev, max_seq_len, nullptr, 0, plan,
-                              kv->part, 1, kPdlWaitFirst, s);  // a no-op with a single split
+                              kv->part, 1, kPdlWaitFirst, s);  // a no-op with a single split or a cluster
 }
 
 int ingot_attn_prefill(ingot_kv* kv, int layer, const void* q_dev, int q_dtype, void* out_dev, int out_dtype,

@@ -291,6 +291,36 @@ def test_ranges_whose_clusters_do_not_fit_at_a_time_are_split_separately(n_keys,
     assert kv.status() == 0 and torch.equal(planned, named)
 
 
+@pytest.mark.parametrize("fused", [False, True])
+def test_the_first_call_of_a_handle_may_be_captured_where_it_needs_no_scratch(fused):
+    """Splits that share a cluster leave nothing in memory: nothing is allocated, so that the very first call can be part of a capture."""
+    import torch
+    import ingot_b200 as ib
+    g = torch.Generator(device="cuda").manual_seed(8)
+    kv = ib.KVCache(ib.KV_CONTIGUOUS, 1, HKV, 1000)
+    for which in "kv":
+        kv.layer_view(0, which).normal_(generator=g)
+    q, k, v = (torch.randn(1, h, D, device="cuda", generator=g) for h in (H, HKV, HKV))
+    inv, out = helpers.to_dev(helpers.inv_freq()), torch.empty(1, H, D, device="cuda")
+    torch.cuda.synchronize()
+
+    def call():
+        if fused:
+            ib.rope_append_decode(kv, 0, q[0], k[0], v[0], inv, 999, out=out[0])
+        else:
+            ib.attn_decode(kv, 0, q, out=out, max_seq_len=1000)
+
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        call()
+    graph.replay()
+    torch.cuda.synchronize()
+    replayed = out.clone()
+    call()
+    torch.cuda.synchronize()
+    assert kv.status() == 0 and torch.equal(out, replayed)
+
+
 def test_empty_calls_are_no_ops():
     import ingot_b200 as ib
     lib = ib.lib()
