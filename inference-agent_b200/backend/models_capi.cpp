@@ -29,17 +29,9 @@ static int guarded(F&& f) {
     }
 }
 
-// Whether a kernel can write this place of host memory under its own address.
-static bool device_writes(float* host) {
-    cudaPointerAttributes at = {};
-    if (cudaPointerGetAttributes(&at, host) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    return at.type == cudaMemoryTypeHost && at.devicePointer == host;
-}
-
 extern "C" {
+
+void* ingot_device_view(const void* host, size_t bytes);  // csrc/status.cu: where kernels see memory that is pinned throughout, or null
 
 const char* ingot_models_last_error() { return g_models_error.c_str(); }
 
@@ -77,7 +69,7 @@ int ingot_model_step(ingot_model* m, int n, const int32_t* seq_ids, const int32_
             rows += size_t(n_want[i]);
         }
         const size_t count = rows * size_t(m->backend->n_vocab());
-        const bool pinned = logits_out && count > 0 && device_writes(logits_out) && device_writes(logits_out + count - 1);
+        const bool pinned = logits_out && count > 0 && ingot_device_view(logits_out, count * sizeof(float)) == logits_out;
         if (pinned) m->backend->step_into(logits_out);
         const float* logits = m->backend->forward_step(e.data(), n, m->backend->n_vocab());
         if (logits_out && logits && logits != logits_out) std::copy(logits, logits + rows * size_t(m->backend->n_vocab()), logits_out);

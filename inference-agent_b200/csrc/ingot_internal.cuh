@@ -153,6 +153,10 @@ inline cudaError_t ingot_launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 bl
 #define INGOT_PDL_TRIGGER() asm volatile("griddepcontrol.launch_dependents;" ::: "memory")
 #define INGOT_PDL_WAIT() asm volatile("griddepcontrol.wait;" ::: "memory")
 
+// Where kernels see `bytes` of host memory: null unless one pinned, mapped allocation (or registration) holds all of them. Two that lie apart
+// look the same from their ends, whatever is between them.
+extern "C" void* ingot_device_view(const void* host, size_t bytes);
+
 // Launchers implemented in the kernel files.
 int launch_rope_kv_append(ingot_kv* kv, int layer, const float* q, __half* q_out, const float* k, const float* v,
                           const float* inv_freq, int n_head, int pos0, int n_tok, const int32_t* positions,

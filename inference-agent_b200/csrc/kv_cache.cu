@@ -374,18 +374,6 @@ int ingot_gather_wait(ingot_kv* kv, void* counters_dev, int n_src, int timeout_m
     return launch_gather_wait(kv, counters_dev, n_src, timeout_ms, static_cast<cudaStream_t>(stream));
 }
 
-// Where kernels see host memory, if all of it is pinned and mapped (and aligned for 16-byte loads); else null.
-static void* device_view(const void* host, size_t bytes) {
-    cudaPointerAttributes first = {}, last = {};
-    if (reinterpret_cast<uintptr_t>(host) % 16 != 0 || cudaPointerGetAttributes(&first, host) != cudaSuccess ||
-        cudaPointerGetAttributes(&last, static_cast<const char*>(host) + bytes - 1) != cudaSuccess) {
-        cudaGetLastError();
-        return nullptr;
-    }
-    if (first.type != cudaMemoryTypeHost || last.type != cudaMemoryTypeHost || !first.devicePointer) return nullptr;
-    return static_cast<char*>(first.devicePointer) + bytes - 1 == last.devicePointer ? first.devicePointer : nullptr;
-}
-
 int ingot_attn_layers_host(ingot_kv* kv, int layer_begin, int layer_count, const float* q_host, const float* k_host,
                            const float* v_host, float* out_host, const float* inv_freq_dev, int n_head, int pos0,
                            int n_tok, void* stream) {
@@ -421,10 +409,10 @@ int ingot_attn_layers_host(ingot_kv* kv, int layer_begin, int layer_count, const
     if (n_tok == 1) {
         // A token's rows in pinned memory are read over PCIe by the kernel that rotates and appends them, and the results are written there by
         // the attention kernel: no copies, and none of the gaps between copy engine and SMs. 28 layers, 300 keys (B200): 58.8 -> 50.6 us.
-        float* const q_m = static_cast<float*>(device_view(q_host, L * q_elems * 4));
-        float* const k_m = static_cast<float*>(device_view(k_host, L * kv_elems * 4));
-        float* const v_m = static_cast<float*>(device_view(v_host, L * kv_elems * 4));
-        float* const o_m = static_cast<float*>(device_view(out_host, L * q_elems * 4));
+        auto view = [&](const float* host, size_t elems) {  // aligned for 16-byte loads
+            return reinterpret_cast<uintptr_t>(host) % 16 == 0 ? static_cast<float*>(ingot_device_view(host, L * elems * 4)) : nullptr;
+        };
+        float *const q_m = view(q_host, q_elems), *const k_m = view(k_host, kv_elems), *const v_m = view(v_host, kv_elems), *const o_m = view(out_host, q_elems);
         if (q_m && k_m && v_m && o_m) {
             const int rc = launch_rope_kv_append(kv, layer_begin, q_m, qh_d, k_m, v_m, inv_freq_dev, n_head, pos0, 1, nullptr, nullptr, nullptr, 0, layer_count, s);
             if (rc != INGOT_OK) return rc;

@@ -1,4 +1,6 @@
 // Error reporting and build information of the library, shared by every entry point.
+#include <cuda.h>
+
 #include <cstdlib>
 
 #include "ingot_internal.cuh"
@@ -17,7 +19,39 @@ bool ingot_use_pdl() {
     return v;
 }
 
+typedef CUresult (*PointerAttributesFn)(unsigned, CUpointer_attribute*, void**, CUdeviceptr);
+static PointerAttributesFn pointer_attributes_fn() {
+    static const PointerAttributesFn fn = [] {
+        void* sym = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        const bool ok = cudaGetDriverEntryPoint("cuPointerGetAttributes", &sym, cudaEnableDefault, &found) == cudaSuccess && found == cudaDriverEntryPointSuccess;
+        return reinterpret_cast<PointerAttributesFn>(ok ? sym : nullptr);
+    }();
+    return fn;
+}
+
 extern "C" {
+
+void* ingot_device_view(const void* host, size_t bytes) {
+    unsigned type = 0, managed = 0;
+    void* at = nullptr;
+    unsigned long long first = 0;
+    size_t size = 0;
+    CUpointer_attribute which[5] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_IS_MANAGED, CU_POINTER_ATTRIBUTE_DEVICE_POINTER, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                                    CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    void* into[5] = {&type, &managed, &at, &first, &size};
+    const PointerAttributesFn ask = pointer_attributes_fn();
+    // the driver answers for the thread's context, and the runtime binds one only when a call of its own needs it
+    static thread_local const bool bound = [] {
+        int device = 0;
+        const bool ok = cudaGetDevice(&device) == cudaSuccess && cudaSetDevice(device) == cudaSuccess;
+        if (!ok) cudaGetLastError();
+        return ok;
+    }();
+    if (!ask || !bound || ask(5, which, into, reinterpret_cast<CUdeviceptr>(host)) != CUDA_SUCCESS || type != CU_MEMORYTYPE_HOST || managed || !at) return nullptr;
+    const unsigned long long view = reinterpret_cast<unsigned long long>(at);
+    return view >= first && bytes <= size && view - first <= size - bytes ? at : nullptr;
+}
 
 const char* ingot_status_string(int status) {
     switch (status) {

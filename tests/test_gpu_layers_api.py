@@ -1,4 +1,6 @@
 """The multi-layer and host-buffer entry points (the calls bench.py times) against the CPU reference."""
+from concurrent.futures import ThreadPoolExecutor
+
 import numpy as np
 import pytest
 
@@ -99,6 +101,39 @@ def test_layers_host_matches_reference(n_tok, pos0):
     torch.cuda.synchronize()
     want1, _, _ = helpers.oracle_prefill(W.Prefill(q[1], k[1], v[1], pos0, True, ck[1] if pos0 else None, cv[1] if pos0 else None))
     helpers.assert_parity(oh1.numpy(), want1, "layer_host")
+
+
+@pytest.mark.parametrize("library", ["cuda", "models"])
+def test_only_memory_that_is_pinned_throughout_is_seen_in_place(library):
+    """Which host rows kernels read and write themselves: those within one pinned allocation or registration. Nothing is launched."""
+    import ctypes as C
+    import mmap
+    import torch
+    import ingot_b200 as ib
+    from ingot_b200 import models as M
+    torch.zeros(1, device="cuda")
+    view = (ib if library == "cuda" else M).lib().ingot_device_view
+    view.argtypes, view.restype = [C.c_void_p, C.c_size_t], C.c_void_p
+    page, rt = mmap.PAGESIZE, torch.cuda.cudart()
+    pinned = torch.empty(3 * page, dtype=torch.uint8, pin_memory=True)
+    at = pinned.data_ptr()
+    assert view(at, 3 * page) == at and view(at + 20, 2 * page) == at + 20
+    with ThreadPoolExecutor(1) as fresh:  # a thread that has made no call yet
+        assert fresh.submit(view, at, 3 * page).result() == at
+    pageable = np.zeros(page, np.uint8)
+    assert view(pageable.ctypes.data, 8) is None
+    assert view(torch.zeros(8, device="cuda").data_ptr(), 8) is None
+    area = mmap.mmap(-1, 4 * page)  # pages 0 and 2 pinned, 1 and 3 not
+    at = C.addressof(C.c_char.from_buffer(area))
+    try:
+        for k in (0, 2):
+            assert int(rt.cudaHostRegister(at + k * page, page, 0)) == 0
+        assert view(at, page) == at and view(at + 2 * page + 16, page - 16) == at + 2 * page + 16
+        assert view(at, page + 1) is None and view(at, 2 * page + 1) is None and view(at, 3 * page) is None
+        assert view(at + page, 16) is None and view(at + page - 8, 16) is None
+    finally:
+        for k in (0, 2):
+            rt.cudaHostUnregister(at + k * page)
 
 
 def test_layers_host_single_token_calls_in_a_row():
