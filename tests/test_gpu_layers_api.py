@@ -68,8 +68,23 @@ def test_decode_layers_in_a_cuda_graph():
         assert torch.equal(out, eager)
 
 
+# What a caller's rows q, k, v and the results may lie in. A single token's rows are read and written in place where all four are pinned and
+# aligned; every other combination is copied.
+MEMORY = {"pinned": ["pinned"] * 4, "pageable": ["pageable"] * 4, "offset": ["offset"] * 4, "mixed": ["pinned", "pageable", "pinned", "pinned"],
+          "results apart": ["pinned", "pinned", "pinned", "pageable"]}
+
+
+def _host(x, kind):
+    """A copy of x in host memory: pinned, ordinary, or pinned and 4 bytes past an aligned address."""
+    import torch
+    x = torch.as_tensor(np.ascontiguousarray(x))
+    room = torch.empty(x.numel() + 1, pin_memory=kind != "pageable")
+    return room[int(kind == "offset"):][:x.numel()].view(x.shape).copy_(x)
+
+
+@pytest.mark.parametrize("memory", MEMORY)
 @pytest.mark.parametrize("n_tok,pos0", [(1, 511), (1, 0), (40, 100)])
-def test_layers_host_matches_reference(n_tok, pos0):
+def test_layers_host_matches_reference(n_tok, pos0, memory):
     """Host buffers in and out (q/k/v projections -> attention rows), all layers in one call: RoPE + append
     + attention must equal the reference's per-token loop on every layer."""
     import torch
@@ -85,8 +100,7 @@ def test_layers_host_matches_reference(n_tok, pos0):
     q = rng.standard_normal((n_layers, n_tok, H, D), dtype=np.float32)
     k = rng.standard_normal((n_layers, n_tok, HKV, D), dtype=np.float32)
     v = rng.standard_normal((n_layers, n_tok, HKV, D), dtype=np.float32)
-    qh, kh, vh = (torch.from_numpy(x).pin_memory() for x in (q, k, v))
-    oh = torch.empty(n_layers, n_tok, H, D).pin_memory()
+    qh, kh, vh, oh = (_host(x, m) for x, m in zip((q, k, v, np.zeros_like(q)), MEMORY[memory]))
     inv = helpers.to_dev(helpers.inv_freq())
     ib.attn_layers_host(kv, 0, qh, kh, vh, oh, inv, pos0)
     torch.cuda.synchronize()
@@ -96,7 +110,7 @@ def test_layers_host_matches_reference(n_tok, pos0):
         want, _, _ = helpers.oracle_prefill(wl)
         helpers.assert_parity(oh[l].numpy(), want, f"layers_host n_tok={n_tok} pos0={pos0} layer {l}")
     # single-layer form writes the same rows
-    oh1 = torch.empty(n_tok, H, D).pin_memory()
+    oh1 = _host(np.zeros((n_tok, H, D), np.float32), MEMORY[memory][3])
     ib.attn_layer_host(kv, 1, qh[1], kh[1], vh[1], oh1, inv, pos0)
     torch.cuda.synchronize()
     want1, _, _ = helpers.oracle_prefill(W.Prefill(q[1], k[1], v[1], pos0, True, ck[1] if pos0 else None, cv[1] if pos0 else None))
@@ -136,13 +150,16 @@ def test_only_memory_that_is_pinned_throughout_is_seen_in_place(library):
             rt.cudaHostUnregister(at + k * page)
 
 
-def test_layers_host_single_token_calls_in_a_row():
-    """Five single-token calls at consecutive positions on one handle: the first runs eagerly, the second is
-    captured into a graph, the others replay it with a new position read from device memory. Token i must
-    see keys 0..pos0+i, exactly like row i of a five-token chunk in the reference."""
+@pytest.mark.parametrize("memory", ["pinned", "pageable", "offset", "mixed", "in turn"])
+def test_layers_host_single_token_calls_in_a_row(memory):
+    """Six single-token calls at consecutive positions on one handle. Rows that are copied: the first call runs eagerly, the second is
+    captured into a graph, the others replay it with a new position read from device memory; pinned rows are read and written in place,
+    without a graph; "in turn": both forms on the same handle. Token i must see keys 0..pos0+i, exactly like row i of a six-token chunk in the
+    reference."""
     import torch
     import ingot_b200 as ib
-    n_layers, pos0, n_calls = 3, 200, 5
+    n_layers, pos0, n_calls = 3, 200, 6
+    kinds = lambda i: MEMORY[("pageable", "pinned", "mixed")[i % 3] if memory == "in turn" else memory]
     rng = np.random.default_rng(321)
     kv = ib.KVCache(ib.KV_CONTIGUOUS, n_layers, HKV, 512)
     ck = [rng.standard_normal((pos0, HKV, D), dtype=np.float32).astype(np.float16) for _ in range(n_layers)]
@@ -158,8 +175,7 @@ def test_layers_host_single_token_calls_in_a_row():
     stream = torch.cuda.Stream()
     with torch.cuda.stream(stream):
         for i in range(n_calls):
-            qh, kh, vh = (torch.from_numpy(np.ascontiguousarray(x[:, i:i + 1])).pin_memory() for x in (q, k, v))
-            oh = torch.empty(n_layers, 1, H, D).pin_memory()
+            qh, kh, vh, oh = (_host(x[:, i:i + 1], m) for x, m in zip((q, k, v, np.zeros_like(q)), kinds(i)))
             ib.attn_layers_host(kv, 0, qh, kh, vh, oh, inv, pos0 + i)
             stream.synchronize()
             got[:, i] = oh.numpy()[:, 0]
@@ -168,8 +184,7 @@ def test_layers_host_single_token_calls_in_a_row():
         want, _, _ = helpers.oracle_prefill(W.Prefill(q[l], k[l], v[l], pos0, True, ck[l], cv[l]))
         helpers.assert_parity(got[l], want, f"single-token host calls, layer {l}")
     # going back to an earlier position overwrites that row and attends over fewer keys (positions may go backwards)
-    qh, kh, vh = (torch.from_numpy(np.ascontiguousarray(x[:, 1:2])).pin_memory() for x in (q, k, v))
-    oh = torch.empty(n_layers, 1, H, D).pin_memory()
+    qh, kh, vh, oh = (_host(x[:, 1:2], m) for x, m in zip((q, k, v, np.zeros_like(q)), kinds(0)))
     ib.attn_layers_host(kv, 0, qh, kh, vh, oh, inv, pos0 + 1)
     torch.cuda.synchronize()
     for l in range(n_layers):
