@@ -706,8 +706,8 @@ static cudaError_t gemv_group(float* const* outs, const void* const* ws, const v
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
-    // Long rows, one or two per warp of 512-thread CTAs (no more than the 768-thread ones would have): up to 4096 weights of a row are
-    // requested before the wait for the kernel before - the time such a launch has is mostly that kernel's. Inside a step (B200): 2048 x 4096
+    // Long rows, one or two per warp of 512-thread CTAs (no more than the 768-thread ones would have): 2048 weights of a row are requested
+    // before the wait for the kernel before (1024 by the 768-thread ones) and 2048 more as soon as x' is staged, and rows spread over more SMs. Inside a step (B200): 2048 x 4096
     // 7.4 -> 7.2 us, 2048 x 8192 11.6 -> 9.5, 4096 x 8192 22.5 -> 18. With more rows per warp the 24 warps stream faster (32768 x 2048 27.5 against 32).
     const int per_warp = (rows + num_sms * 16 - 1) / (num_sms * 16);
     const bool row_each = plain && !short_rows && !swiglu && per_warp <= 2 && per_warp <= (rows + num_sms * 24 - 1) / (num_sms * 24);
@@ -767,7 +767,8 @@ cudaError_t ingot_support_gemv_group(float* const* outs, const void* const* ws, 
 }
 
 // The same streaming kernel for one bf16 matrix [n_out][n_in] (n_in a multiple of 256): out (+)= W x', x' = rmsnorm(x) with the mean
-// over n_mean floats if norm_w is given, else x itself. gated: W holds a gate and an up half of n_out rows each, out = act(gate) * up.
+// over n_mean floats if norm_w is given, else x itself. gated: W holds runs of 32 gate rows, each followed by the 32 up rows that go with them
+// (n_out of each, a multiple of 32), out = act(gate) * up.
 cudaError_t ingot_support_gemv_bf16(float* out, const void* w, int n_out, int n_in, const float* x, const float* norm_w, float eps, int n_mean,
                                     int gated, int act, int accumulate, cudaStream_t s) {
     float* outs[2] = {out, out};

@@ -162,6 +162,35 @@ def test_gemv_group_matches_float64(mode, wtype):
             assert err <= 1e-5 * max(1.0, ref.abs().max().item()), err
 
 
+@pytest.mark.parametrize("n_in", [3072, 3328, 4096, 8192, 8448])
+@pytest.mark.parametrize("n_out", [1, 2367, 2368, 2369, 3552, 3553, 4736, 4737])
+@pytest.mark.parametrize("fmt,norm,accumulate", [("f16", True, 0), ("f16", False, 1), ("bf16", True, 1), ("bf16", False, 0)])
+def test_gemv_of_long_rows(fmt, norm, accumulate, n_out, n_in):
+    """The forms of the plain formats around the lines between them (148 SMs): rows of up to 12 chunks of 256 weights and longer ones, the last
+    step ragged; one and two rows per warp of 512 threads, and of 768. Norm folded in or not, added up or not. Against float64."""
+    import torch
+    lib = _lib()
+    vp, ci, cf = C.c_void_p, C.c_int, C.c_float
+    lib.ingot_support_gemv_group.argtypes = [C.POINTER(vp), C.POINTER(vp), C.POINTER(vp), ci, C.POINTER(ci), ci, ci, vp, vp, cf, ci, ci, vp]
+    lib.ingot_support_gemv_bf16.argtypes = [vp, vp, ci, ci, vp, vp, cf, ci, ci, ci, ci, vp]
+    g = torch.Generator(device="cuda").manual_seed(n_out + n_in)
+    x = torch.randn(n_in, device="cuda", generator=g) * 3
+    nw = 1 + 0.1 * torch.randn(n_in, device="cuda", generator=g)
+    w = (torch.randn(n_out, n_in, device="cuda", generator=g) * 0.02).to(torch.float16 if fmt == "f16" else torch.bfloat16)
+    out = torch.randn(n_out, device="cuda", generator=g)
+    h = x.double() * torch.rsqrt((x.double() ** 2).mean() + 1e-5) * nw.double() if norm else x.double()
+    want = w.double() @ h + (out.double() if accumulate else 0)
+    nw_p = nw.data_ptr() if norm else None
+    if fmt == "f16":
+        one = lambda t: (vp * 1)(t.data_ptr())
+        assert lib.ingot_support_gemv_group(one(out), one(w), None, 0, (ci * 1)(n_out), 1, 0, x.data_ptr(), nw_p, 1e-5, n_in, accumulate, None) == 0
+    else:
+        assert lib.ingot_support_gemv_bf16(out.data_ptr(), w.data_ptr(), n_out, n_in, x.data_ptr(), nw_p, 1e-5, n_in, 0, 0, accumulate, None) == 0
+    torch.cuda.synchronize()
+    # f32 sums of n_in terms of size 0.06 (0.02 with the norm): n_in / 32 to a lane, each sum within 2^-24 of partial sums of up to about 3 times the result
+    assert (out.double() - want).abs().max().item() <= 1e-5 * max(1.0, want.abs().max().item())
+
+
 def test_slice_consumers_match_float64():
     """Split-k products left as k slices and summed by their consumers: the grouped q/k/v sum, the residual add
     with the next RMS norm folded in, and the SwiGLU product, each checked through the projection that follows."""
