@@ -16,7 +16,7 @@ The same JSON line carries, as objects of their own:
   c4_batched     64-sequence paged decode, sequences sharded over the N ranks by length (strong scaling);
   c1_prefill128, c3_chunked   the two chunked-prefill configurations (N = 1 only: they are replicas).
 Every object has `parity` (max-abs and relative L2 error against the CPU reference on the tensors that were timed,
-computed outside the timed region), `roofline`, and where it applies `e2e` (host buffers, copies inside the timed
+computed outside the timed region), `roofline`, and where it applies `e2e` (host buffers, their transfers inside the timed
 region) and `clocks` (NVML, sampled while the timed region runs).
 
 Timing: W warm-up steps, then blocks of K steps, each block timed with CUDA events on the launching stream, repeated
@@ -388,10 +388,11 @@ def run_decode(args, rank, world):
         roofline["in_backend_gbs"] = round(bytes_step / N_LAYER / (us * 1e-6) / 1e9, 1)
 
     mark(world, "decode: parity and per-layer form done")
-    # End to end through the host-buffer C-ABI call: per layer q/k/v rows host->device, RoPE+append,
-    # decode at position 4095 (4096 keys), output device->host; one synchronisation per step.
+    # End to end through the host-buffer C-ABI call: per layer q/k/v rows out of pinned host memory, RoPE+append,
+    # decode at position 4095 (4096 keys), output into pinned host memory; one synchronisation per step. The kernels read and
+    # write the rows over PCIe themselves.
     inv = torch.from_numpy(inv_freq_table()).cuda()
-    # q, k and v rows sit in one pinned block (q of all layers, then k, then v): the call then needs one copy in.
+    # q, k and v rows sit in one pinned block (q of all layers, then k, then v)
     nq, nk = N_LAYER * H * D, N_LAYER * HKV * D
     blk = torch.randn(nq + 2 * nk).pin_memory()
     qh, kh, vh = blk[:nq].view(N_LAYER, 1, H, D), blk[nq:nq + nk].view(N_LAYER, 1, HKV, D), blk[nq + nk:].view(N_LAYER, 1, HKV, D)
@@ -404,7 +405,7 @@ def run_decode(args, rank, world):
     te = timed(step_e2e, args.steps, args.warmup, world, 0.0 if args.no_graph else min(0.25, MIN_TIMED_S))
     ms_e2e = te["ms"]
     e2e = {"value": round(world * bytes_step * args.steps / (ms_e2e * 1e-3) / 1e9, 1), "unit": "GB/s",
-           "h2d_bytes_per_step": int(N_LAYER * (H + 2 * HKV) * D * 4 + 8), "d2h_bytes_per_step": int(N_LAYER * H * D * 4),
+           "h2d_bytes_per_step": int(N_LAYER * (H + 2 * HKV) * D * 4), "d2h_bytes_per_step": int(N_LAYER * H * D * 4),
            "ms_per_step": round(ms_e2e / args.steps, 4), "gpu_launches_per_step": 3,
            "timed_region_s": te["timed_region_s"]}
     assert kv.status() == 0

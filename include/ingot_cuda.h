@@ -255,14 +255,17 @@ int ingot_lpt_assign(const int32_t* lens, int n_seq, int n_ranks, int32_t* rank_
  * copies q/k/v f32 rows host->device, runs K1 then K3 (n_tok == 1) or K2 (n_tok > 1) on a contiguous
  * cache at positions pos0..pos0+n_tok-1, copies the f32 output device->host. All on `stream`,
  * asynchronous: call ingot_stream_sync (or cudaStreamSynchronize) before reading out_host.
- * Host buffers should be pinned for the copies to overlap. inv_freq_dev is a device pointer. */
+ * Host buffers should be pinned for the copies to overlap. inv_freq_dev is a device pointer.
+ * A single token whose q, k, v and output rows are all pinned, mapped and 16-byte aligned takes no copies: kernels read and write
+ * the rows where they are. As with the copies, the input rows may change and the output rows hold the results once `stream` has been
+ * synchronised, not before. */
 int ingot_attn_layer_host(ingot_kv* kv, int layer, const float* q_host, const float* k_host, const float* v_host,
                           float* out_host, const float* inv_freq_dev, int n_head, int pos0, int n_tok,
                           void* stream);
 /* The same for `layer_count` consecutive layers starting at `layer_begin` in one call, as the
  * reference's attention microbenchmark drives its backend (every layer's attention for one step,
  * src/metal_backend.mm:594-649): host arrays are [layer_count][n_tok][heads][128], one slice per layer.
- * If k_host directly follows q_host and v_host directly follows k_host in memory, the three arrays travel in one copy. */
+ * If k_host directly follows q_host and v_host directly follows k_host in memory, rows that are copied travel in one copy. */
 int ingot_attn_layers_host(ingot_kv* kv, int layer_begin, int layer_count, const float* q_host, const float* k_host,
                            const float* v_host, float* out_host, const float* inv_freq_dev, int n_head, int pos0,
                            int n_tok, void* stream);

@@ -65,7 +65,7 @@ cudaError_t ingot_linear_tc_finish_residual_norm_bf16(ingot_linear_ws* ws, float
 cudaError_t ingot_linear_tc_run_gated_bf16(ingot_linear_ws* ws, const void* w, int n_in, int n_out, int act, int planes, cudaStream_t s);
 }
 
-inline constexpr int kMinTcTokens = 2;  // from two tokens on, a 128-token tile that is mostly padding still only streams the weights once
+inline constexpr int kMinTcTokens = 2;  // from two tokens on, a product on the tensor cores streams the weights once, whatever rows are padding
 
 // Up to this many tokens a product is bound by streaming the weights, so the activations go in as a hi + lo pair at no cost: a
 // decoded token's logits then hardly depend on whether it is alone (f32 activations) or in a batch.
