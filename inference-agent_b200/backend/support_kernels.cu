@@ -707,8 +707,8 @@ static cudaError_t gemv_group(float* const* outs, const void* const* ws, const v
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
     // Long rows, one or two per warp of 512-thread CTAs (no more than the 768-thread ones would have): 2048 weights of a row are requested
-    // before the wait for the kernel before (1024 by the 768-thread ones) and 2048 more as soon as x' is staged, and rows spread over more SMs. Inside a step (B200): 2048 x 4096
-    // 7.4 -> 7.2 us, 2048 x 8192 11.6 -> 9.5, 4096 x 8192 22.5 -> 18. With more rows per warp the 24 warps stream faster (32768 x 2048 27.5 against 32).
+    // before the wait for the kernel before (1024 by the 768-thread ones) and 2048 more as soon as x' is staged, and rows spread over more
+    // SMs. Inside a step (B200): 2048 x 4096 7.4 -> 7.2 us, 2048 x 8192 11.6 -> 9.5, 4096 x 8192 22.5 -> 18. With more rows per warp the 24 warps stream faster (32768 x 2048 27.5 against 32).
     const int per_warp = (rows + num_sms * 16 - 1) / (num_sms * 16);
     const bool row_each = plain && !short_rows && !swiglu && per_warp <= 2 && per_warp <= (rows + num_sms * 24 - 1) / (num_sms * 24);
     typedef void (*Kernel)(GemvGroup, const float*, const float*, float, int, int, int, int, int, int);
