@@ -64,6 +64,24 @@ def test_causal_conv(taps, channels, cut, act):
         assert np.abs(g - e).max() < 2e-5
 
 
+@pytest.mark.parametrize("taps", [2, 3, 4])
+@pytest.mark.parametrize("lens,channels", [([1000, 29], 2048), ([524, 523, 2], 2008), ([1025], 2048), ([3, 4, 5, 8, 9], 512)])
+def test_causal_conv_of_long_portions(lens, channels, taps):
+    """On both sides of the line between runs of 8 and of 4 tokens, remainders of either; four f32 products and sums per value."""
+    import torch
+    rng = np.random.default_rng(channels + taps)
+    w, xs = rng.standard_normal((channels, taps)), [rng.standard_normal((n, channels)) for n in lens]
+    want = np.concatenate([R.causal_conv(x, w, np.zeros(channels)) for x in xs])
+    st, n = Step(lens, [0] * len(lens), list(range(len(lens)))), sum(lens)
+    x, wd, state = dev(np.concatenate(xs)), dev(w), torch.full((len(lens), taps - 1, channels), float("nan"), device="cuda")
+    out = torch.full((n, channels), float("nan"), device="cuda")
+    o = act_out(out)
+    lib(lib().ingot_causal_conv(C.byref(st.c), x.data_ptr(), channels, None, wd.data_ptr(), None, taps, channels, 0, state.data_ptr(), C.byref(o), None))
+    assert np.abs(out.cpu().numpy() - want).max() < 2e-5
+    kept = np.stack([np.concatenate([np.zeros((taps, channels)), a])[-(taps - 1):] for a in xs])
+    assert np.array_equal(state.cpu().numpy(), kept.astype(np.float32))
+
+
 @pytest.mark.parametrize("exact", [0, 1])
 @pytest.mark.parametrize("cut", CUTS)
 @pytest.mark.parametrize("inner,n_state", [(96, 16), (40, 20), (8, 1), (72, 33), (24, 70), (36, 5)])
