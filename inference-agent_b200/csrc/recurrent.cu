@@ -88,7 +88,7 @@ __global__ void __launch_bounds__(128) causal_conv_kernel(const ConvParams p) {
 
 // The same for 2 to 4 taps and four channels per thread (channels and row lengths multiples of 4), a run of kRun tokens whose inputs are all
 // requested together. Bound by DRAM (large steps) or by the latency of one round trip (small ones). Against runs of 16 in four dependent rounds
-// of loads (B200, inside a prompt's step): 1000 tokens x 2048 channels 12.7 -> 5.0 us, 1024 x 4096 14.6 -> 8.8, 2048 x 4096 25 -> 19.5, 2048 x 8192
+// of loads (B200, inside a prompt's step): 1000 tokens x 2048 channels 12.8 -> 5.0 us, 2048 x 4096 25 -> 19.4, 2048 x 8192
 // 43 -> 39.5. Runs of 4 read 1.75 times what they write from L2, but give a short step four times the CTAs; which run a launch takes is
 // decided in ingot_causal_conv.
 template <int kTaps, int kRun>
