@@ -91,7 +91,7 @@ struct Sm100Params {
     int* ticket;
     int* status;
     int q_dtype, out_dtype;
-    int n_head, group;
+    int n_head, n_head_kv, group;
     int q_pos0, n_tok;
     const int32_t* block_table;  // paged cache: this sequence's block-table row (device), else null
     int capacity;             // paged: blocks in the pool
@@ -170,9 +170,9 @@ attn_prefill_sm100_kernel(const __grid_constant__ CUtensorMap map_k, const __gri
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int warp_u = __shfl_sync(0xffffffffu, warp, 0);  // the same number, known to the compiler as warp-uniform
     const int G = p.group;
-    const int kvh = blockIdx.y;
+    int tile256, kvh;
+    prompt_tile(p.n_head_kv, tile256, kvh);
     const int n_rows = p.n_tok * G;
-    const int tile256 = gridDim.x - 1 - blockIdx.x;  // heavier (later) tiles first
     const int row_base = tile256 * 2 * kTileRows;
     const int last_row = min(row_base + 2 * kTileRows, n_rows) - 1;
     const int n_kv = (p.q_pos0 + last_row / G + 1 + kTileKeys - 1) / kTileKeys;  // K/V tiles these rows need
@@ -245,7 +245,7 @@ attn_prefill_sm100_kernel(const __grid_constant__ CUtensorMap map_k, const __gri
                         atomicOr(p.status, kDevErrBlockRange);
                         blk = 0;
                     }
-                    const int z = blk * (int)gridDim.y + kvh;  // pool is [block][kv head][16][128]
+                    const int z = blk * p.n_head_kv + kvh;  // pool is [block][kv head][16][128]
                     tma_load_3d(dst + lane * (kBlockTokens * 128), map, 0, 0, z, full);
                     tma_load_3d(dst + kHalfBytes + lane * (kBlockTokens * 128), map, 64, 0, z, full);
                 }
@@ -515,7 +515,7 @@ attn_prefill_sm100_kernel(const __grid_constant__ CUtensorMap map_k, const __gri
         const bool partial = p.n_split > 1;
         float* part_row = nullptr;
         if (partial && valid) {
-            part_row = p.part + (((size_t)split * gridDim.y + kvh) * n_rows + R) * kPartStride;
+            part_row = p.part + (((size_t)split * p.n_head_kv + kvh) * n_rows + R) * kPartStride;
             if (n_it == 0) { m_ref = -INFINITY; l = 0.f; }
             part_row[128] = m_ref;
             part_row[129] = l;
@@ -539,7 +539,7 @@ attn_prefill_sm100_kernel(const __grid_constant__ CUtensorMap map_k, const __gri
             // a row of the partials, or (token, head) of the output; -1 past the end.
             const int my_dst = !valid ? -1 : partial ? R : tok * p.out_n_head + p.out_head0 + head;
             const size_t dst_row_bytes = partial ? (size_t)kPartStride * 4 : (size_t)kHeadDim * (f32_out ? 4 : 2);
-            unsigned char* dst0 = partial ? reinterpret_cast<unsigned char*>(p.part + ((size_t)split * gridDim.y + kvh) * n_rows * kPartStride)
+            unsigned char* dst0 = partial ? reinterpret_cast<unsigned char*>(p.part + ((size_t)split * p.n_head_kv + kvh) * n_rows * kPartStride)
                                           : static_cast<unsigned char*>(p.outs[0]);
             for (int ps = 0; ps < n_pass; ps++) {
                 if (ps) __syncwarp();
@@ -782,7 +782,7 @@ int launch_attn_prefill_sm100(ingot_kv* kv, int layer, const void* q, int q_dtyp
     p.src_index = src_index;
     p.ticket = signals ? kv->status_dev + 1 : nullptr;
     p.q_dtype = q_dtype; p.out_dtype = out_dtype;
-    p.n_head = n_head; p.group = n_head / kv->n_head_kv;
+    p.n_head = n_head; p.n_head_kv = kv->n_head_kv; p.group = n_head / kv->n_head_kv;
     p.q_pos0 = q_pos0; p.n_tok = n_tok;
     p.block_table = paged ? block_table : nullptr;
     p.capacity = kv->capacity;
@@ -823,7 +823,7 @@ int launch_attn_prefill_sm100(ingot_kv* kv, int layer, const void* q, int q_dtyp
         p.part = st->part;
         p.part_extent = st->part_floats;
     }
-    dim3 grid(row_tiles, kv->n_head_kv, n_split);
+    const dim3 grid = prompt_grid(row_tiles, kv->n_head_kv, n_split, kv->num_sms);
     INGOT_CUDA_TRY(ingot_launch_pdl(attn_prefill_sm100_kernel, grid, dim3(kThreads), size_t(kSmemBytes), stream, st->maps[size_t(layer) * 2],
                                     st->maps[size_t(layer) * 2 + 1], p));
     if (n_split > 1) {

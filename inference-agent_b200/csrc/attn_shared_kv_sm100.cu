@@ -82,10 +82,12 @@ shared_kv_sm100_kernel(const __grid_constant__ CUtensorMap map_rows, const __gri
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int warp_u = __shfl_sync(0xffffffffu, warp, 0);
 
-    const int seq = blockIdx.z, kvh = blockIdx.y, G = p.n_head / p.n_head_kv;
+    const int seq = blockIdx.z, G = p.n_head / p.n_head_kv;
+    int tile, kvh;
+    prompt_tile(p.n_head_kv, tile, kvh);
     const int pos0 = p.st.pos0[seq], n_rows = p.st.len[seq] * G;
     const size_t tok0 = p.st.row_start[seq];
-    const int row_base = ((int)gridDim.x - 1 - (int)blockIdx.x) * 2 * kTileRows;  // later rows see more keys, they go first
+    const int row_base = tile * 2 * kTileRows;
     if (row_base >= n_rows) {
         INGOT_PDL_WAIT();
         return;
@@ -450,7 +452,7 @@ int launch_shared_kv_sm100(ingot_skv* kv, int layer, const AttendParams& p, cuda
         kv->tmaps = std::move(maps);
     }
     const int group = p.n_head / p.n_head_kv;
-    const dim3 grid((unsigned)(((size_t)p.st.max_len * group + 2 * kTileRows - 1) / (2 * kTileRows)), p.n_head_kv, p.st.n_seq);
+    const dim3 grid = prompt_grid((unsigned)(((size_t)p.st.max_len * group + 2 * kTileRows - 1) / (2 * kTileRows)), p.n_head_kv, p.st.n_seq, kv->num_sms);
     INGOT_CUDA_TRY(ingot_launch_pdl(shared_kv_sm100_kernel, grid, dim3(kThreads), size_t(kSmemBytes), stream, kv->tmaps[layer], p));
     return INGOT_OK;
 }
