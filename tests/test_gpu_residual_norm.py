@@ -45,6 +45,33 @@ def test_every_term(n, count, centred):
     assert ((hi.float() + lo.float() - out).abs().max() <= 1e-4 * out.abs().max()).item()
 
 
+@pytest.mark.parametrize("rows", [64, 65, 593, 1200])
+@pytest.mark.parametrize("n", [2048, 4096])
+@pytest.mark.parametrize("kind", ["rms", "centred", "groups"])
+def test_many_rows(n, rows, kind):
+    """Rows of a prompt, on both sides of the line to the launch that keeps the weights, one or several rows per CTA; slices, gains, branch rows, and
+    without each of the norms. Bounds as in test_every_term."""
+    import torch
+    rng = np.random.default_rng(n + rows)
+    top, groups = 3, 4 if kind == "groups" else 1
+    x, product, branch = 4 + rng.standard_normal((rows, n)), rng.standard_normal((2, rows, n)), rng.standard_normal((40, n))
+    pairs = [(rng.standard_normal(n) + 1, rng.standard_normal(n) if kind == "centred" else None) for _ in range(2)]
+    gain, row_of = rng.random(rows), rng.integers(-1, 40, (rows, top))
+    norm = (lambda v, p: G.grouped_rms_norm(v, p[0], groups, EPS)) if groups > 1 else plain
+    y = product.sum(axis=0) * gain[:, None] + (branch[row_of] * (row_of >= 0)[:, :, None]).sum(axis=1)
+    for post, following, terms in ((True, True, True), (False, True, True), (True, False, True), (False, True, False)):
+        want = x + ((norm(y, pairs[0]) if post else y) if terms else 0)
+        xd, out = dev(x), torch.full((rows, n), float("nan"), device="cuda")
+        hi, lo = (torch.full((rows, n), float("nan"), device="cuda", dtype=torch.bfloat16) for _ in range(2))
+        given = dict(product=dev(product), gain=dev(gain), branch=dev(branch), row_of=dev(row_of, np.int32), top=top) if terms else {}
+        N.run(xd, EPS, n, post=pairs[0] if post else None, next_norm=pairs[1] if following else None, out=out, hi=hi, lo=lo, groups=groups, **given)
+        assert np.abs(xd.cpu().numpy() - want).max() < 2e-4
+        if following:
+            read = norm(want, pairs[1])
+            assert np.abs(out.cpu().numpy() - read).max() < 3e-4 * np.abs(read).max()
+            assert ((hi.float() + lo.float() - out).abs().max() <= 1e-4 * out.abs().max()).item()
+
+
 def test_a_norm_alone_of_chosen_rows():
     import torch
     rng = np.random.default_rng(0)
