@@ -172,8 +172,9 @@ public:
         if (n_vocab != n_vocab_) throw std::runtime_error("engine: vocabulary size mismatch");
         Step step = check(entries, n);
         reserve_pages(entries, n);
-        const StepCtx s = upload_step(entries, n, step);
         reserve_logits(step.n_want);
+        float* const logits = into ? into : logits_;
+        const StepCtx s = lay_out_step(entries, n, step, logits);
         // Steps of single decoded tokens are the same launches every time but for what the metadata says: captured once per
         // batch size and reach (Step::reach) and replayed. The first such step of a size runs eagerly.
         const bool replay = step.decode && !tap_ && use_graphs_;
@@ -197,14 +198,10 @@ public:
         } else {
             encode(s, step);
         }
-        cuda_check(cudaEventRecord(ev1_, ops_.stream), "cudaEventRecord");
-        const int ld = head_.n_out;
-        float* const logits = into ? into : logits_;
-        const int by_kernel = step.n_want <= kDeliveredRows ? step.n_want : 0;
-        if (step.n_want > by_kernel)
-            cuda_check(cudaMemcpy2DAsync(logits, size_t(n_vocab_) * 4, logits_dev_, size_t(ld) * 4, size_t(n_vocab_) * 4, size_t(step.n_want),
+        if (step.n_want > kDeliveredRows)
+            cuda_check(cudaMemcpy2DAsync(logits, size_t(n_vocab_) * 4, logits_dev_, size_t(head_.n_out) * 4, size_t(n_vocab_) * 4, size_t(step.n_want),
                                          cudaMemcpyDeviceToHost, ops_.stream), "D2H logits");
-        cuda_check(ingot_support_deliver(logits, logits_dev_, ld, n_vocab_, by_kernel, status_host_, status_words_.data(), int(status_words_.size()), ops_.stream), "logits and status");
+        cuda_check(cudaEventRecord(ev1_, ops_.stream), "cudaEventRecord");
         cuda_check(cudaStreamSynchronize(ops_.stream), "step");
         cudaEventElapsedTime(&last_ms_, ev0_, ev1_);
         for (size_t i = 0; i < status_words_.size(); i++)
@@ -270,6 +267,8 @@ private:
         const int32_t* tokens = nullptr;     // device
         const int32_t* bigrams = nullptr;    // device: rows of the bigram table
         int first_want = 0;           // host copy of want_rows[0]
+        size_t pieces = 0;            // of 16 bytes: the metadata
+        float* const* logits_at = nullptr;   // device: where the wanted rows go (pinned host memory)
     };
     struct Graph {
         int seen = 0;
@@ -329,7 +328,8 @@ private:
         return even;
     }
 
-    StepCtx upload_step(const StepEntry* asked, int n, Step& step) {
+    // The step's metadata, in pinned host memory (the step's first launch fetches it), and where each part of it will be on the device.
+    StepCtx lay_out_step(const StepEntry* asked, int n, Step& step, float* logits) {
         // Sequences run in ascending order of their portions, so that decoded tokens and short portions are the first rows and a
         // mixer can treat them apart from long ones.
         std::vector<int> order(static_cast<size_t>(n));
@@ -344,6 +344,9 @@ private:
         std::vector<int32_t>& m = meta_;
         m.clear();
         auto mark = [&] { while (m.size() % 4) m.push_back(0); return m.size(); };
+        const size_t o_logits = mark();
+        m.resize(m.size() + sizeof(logits) / sizeof(int32_t));
+        memcpy(m.data() + o_logits, &logits, sizeof(logits));
         const size_t o_tok = mark();
         for (int i = 0; i < n; i++) m.insert(m.end(), entries[i].tokens, entries[i].tokens + entries[i].n_tokens);
         const size_t o_bigram = mark();
@@ -437,7 +440,8 @@ private:
             cuda_check(cudaMallocHost(&meta_host_, meta_cap_ * 4), "cudaMallocHost(step metadata)");
         }
         memcpy(meta_host_, m.data(), m.size() * 4);
-        cuda_check(cudaMemcpyAsync(meta_dev_, meta_host_, m.size() * 4, cudaMemcpyHostToDevice, ops_.stream), "H2D step metadata");
+        step.pieces = m.size() / 4;
+        step.logits_at = reinterpret_cast<float* const*>(meta_dev_ + o_logits);
 
         StepCtx s;
         s.st.n_tok = step.n_tok;
@@ -537,8 +541,15 @@ private:
         graphs_.clear();
     }
 
-    // Every launch of a step, from the token ids to the logits of the wanted rows.
+    // Every launch of a step, from its metadata to the logits of the wanted rows in host memory.
     void encode(const StepCtx& s, const Step& step) {
+        cuda_check(ingot_support_fetch(meta_dev_, meta_host_, step.pieces, ops_.stream), "step metadata");
+        encode_layers(s, step);
+        const bool there = step.n_want > 0 && encode_logits(step);
+        cuda_check(ingot_support_deliver(step.logits_at, logits_dev_, head_.n_out, n_vocab_, there || step.n_want > kDeliveredRows ? 0 : step.n_want, status_host_, status_words_.data(),
+                                         int(status_words_.size()), ops_.stream), "logits and status");
+    }
+    void encode_layers(const StepCtx& s, const Step& step) {
         if (bigram_.data || x0_)
             cuda_check(ingot_support_embed_sum_bf16(ops_.x, x0_, embed_.data, n_vocab_, step.tokens, bigram_.data, bigram_buckets_ + 1, step.bigrams, embed_.n_in,
                                                     s.st.n_tok, embed_scale_, embed_status_, ops_.stream), "embedding rows");
@@ -563,13 +574,16 @@ private:
             }
             if (tap_) tap(s.st.n_tok);
         }
-        if (!step.n_want) return;
+    }
+    // Returns whether the rows are in host memory already.
+    bool encode_logits(const Step& step) {
         const int ld = embed_.n_in;
+        int there = 0;
         if (step.n_want == 1 && LayerOps::streams(head_) && !final_norm_.apart()) {
             cuda_check(ingot_support_gemv_bf16(logits_dev_, head_.data, head_.n_out, head_.n_in, ops_.x + size_t(step.first_want) * ld, final_norm_.w, ops_.eps,
                                                ops_.width, 0, 0, 0, ops_.stream), "logits");
             cap_logits(step);
-            return;
+            return false;
         }
         if (final_norm_.apart()) {
             ingot_residual_norm r = {};
@@ -589,11 +603,15 @@ private:
             cuda_check(ingot_support_gemv_bf16(logits_dev_, head_.data, head_.n_out, head_.n_in, ops_.buf(kNormed), nullptr, 0.f, ld, 0, 0, 0, ops_.stream), "logits");
         } else if (ops_.ws && step.n_want >= kMinTcTokens) {
             cuda_check(ingot_linear_tc_prepare_bf16(ops_.ws, ops_.buf(kNormed), ld, ld, step.n_want, step.n_want <= kPairTokens ? 2 : 1, ops_.stream), "final norm");
-            cuda_check(ingot_linear_tc_run(ops_.ws, logits_dev_, head_.data, head_.n_in, head_.n_out, 0, ops_.stream), "logits");
+            // whole rows as they are: the product may write them where they are wanted
+            const bool to_host = softcap_ <= 0 && head_.n_out == n_vocab_ && step.n_want <= kDeliveredRows;
+            if (to_host) cuda_check(ingot_linear_tc_run_to(ops_.ws, logits_dev_, step.logits_at, head_.data, head_.n_in, head_.n_out, &there, ops_.stream), "logits");
+            else cuda_check(ingot_linear_tc_run(ops_.ws, logits_dev_, head_.data, head_.n_in, head_.n_out, 0, ops_.stream), "logits");
         } else {
             cuda_check(ingot_support_linear_bf16(logits_dev_, head_.data, ops_.buf(kNormed), ld, ld, head_.n_out, 0, step.n_want, 0, ops_.stream), "logits");
         }
         cap_logits(step);
+        return there != 0;
     }
     void cap_logits(const Step& step) {
         if (softcap_ > 0) cuda_check(ingot_support_softcap(logits_dev_, size_t(step.n_want) * head_.n_out, softcap_, ops_.stream), "softcap");

@@ -34,7 +34,8 @@ cudaError_t ingot_support_embed_rows_bf16(float* out, const void* table, int n_i
 cudaError_t ingot_support_embed_sum_bf16(float* out, float* copy, const void* table, int n_rows_table, const int32_t* rows_dev, const void* table2,
                                          int n_rows_table2, const int32_t* rows2_dev, int n_in, int n_rows, float scale, int* status_dev, cudaStream_t s);
 cudaError_t ingot_support_concat_rows(float* f32, void* hi, void* lo, const float* a, const float* b, int n, int n_rows, cudaStream_t s);
-cudaError_t ingot_support_deliver(float* dst, const float* src, int src_ld, int n, int rows, int* status, int* const* words, int n_words, cudaStream_t s);
+cudaError_t ingot_support_deliver(float* const* dst_at, const float* src, int src_ld, int n, int rows, int* status, int* const* words, int n_words, cudaStream_t s);
+cudaError_t ingot_support_fetch(void* dst, const void* src, size_t n, cudaStream_t s);
 cudaError_t ingot_support_softcap(float* x, size_t n, float cap, cudaStream_t s);
 cudaError_t ingot_support_rmsnorm_rows(float* out, const float* x, const float* w, const int32_t* rows_dev, int n_rows, int n, int n_mean,
                                        float eps, cudaStream_t s);
@@ -54,6 +55,7 @@ cudaError_t ingot_linear_tc_prepare_bf16(ingot_linear_ws* ws, const float* x, in
 cudaError_t ingot_linear_tc_prepare_norm_bf16(ingot_linear_ws* ws, const float* x, const float* norm_w, float eps, int n_in, int n_mean, int n_tok,
                                               int planes, cudaStream_t s);
 cudaError_t ingot_linear_tc_run(ingot_linear_ws* ws, float* out, const void* w, int n_in, int n_out, int accumulate, cudaStream_t s);
+cudaError_t ingot_linear_tc_run_to(ingot_linear_ws* ws, float* out, float* const* out_at, const void* w, int n_in, int n_out, int* there, cudaStream_t s);
 cudaError_t ingot_linear_tc_run_blocks(ingot_linear_ws* ws, float* out, const void* w, int k_block, int n_out, int rows_per_block, cudaStream_t s);
 cudaError_t ingot_linear_tc_run_partial(ingot_linear_ws* ws, const void* w, int n_in, int n_out, int slot, cudaStream_t s);
 cudaError_t ingot_linear_tc_run_half(ingot_linear_ws* ws, void* out, int out_ld, int out_block, const void* w, int n_in, int n_out, int rows_per_block,

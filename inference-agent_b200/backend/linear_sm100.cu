@@ -81,6 +81,7 @@ static cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
 // the token tiles and the output tiles of all of them, tile_end[m] being the running total of tiles up to and including matrix m.
 struct GemmParams {
     float* out;           // [n_tok][n_out] (single matrix only)
+    float* const* out_at; // linear_few_kernel: where `out` stands instead, in device memory (null: out)
     float* partial[3];    // per matrix: [n_split][n_tok][n_out] when n_split > 1 or to_partial
     int* status;
     int n_tok, k_steps, n_split, accumulate;
@@ -293,6 +294,7 @@ linear_few_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_const
         const int lg = warp & 3;  // the tensor-memory lane group this warp may read
         float* const swap = reinterpret_cast<float*>(smem_al + fp.off_swap) + (lg >> 1) * fp.rows * 32;  // [row][32] of a gate / up pair of warps
         const bool split_k = p.n_split > 1 || p.to_partial;
+        float* const out = !kGrouped && p.out_at ? *p.out_at : p.out;
         int j = 0;
         bool ok = true;
         for (int index = blockIdx.x; index < n_items && ok; index += gridDim.x, j++) {
@@ -344,7 +346,7 @@ linear_few_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_const
                 asm volatile("bar.sync %0, 64;" ::"r"(1 + (lg >> 1)) : "memory");
             } else {
                 float* const part = t.mat == 0 ? p.partial[0] : t.mat == 1 ? p.partial[1] : p.partial[2];
-                float* const dst = (split_k ? part + (size_t)t.split * p.n_tok * n_out : p.out) + col;
+                float* const dst = (split_k ? part + (size_t)t.split * p.n_tok * n_out : out) + col;
                 for (int c = 0; c < n_rows; c += 8) {
                     float v[8];
                     __syncwarp();  // lanes past the last output have left the round before early; tensor memory is read by whole warps
@@ -1162,7 +1164,7 @@ cudaError_t ingot_linear_tc_prepare_norm_bf16(ingot_linear_ws* ws, const float* 
 // n_out / rows_per_block such blocks side by side.
 static cudaError_t launch_gemm(ingot_linear_ws* ws, float* out, const void* const* w, int n_in, const int* n_out, int count,
                                int accumulate, int first_slot, bool to_partial, bool append, cudaStream_t s, int rows_per_block = 0,
-                               __half* out_half = nullptr, int half_ld = 0, int half_block = 0, int gate = 0) {
+                               __half* out_half = nullptr, int half_ld = 0, int half_block = 0, int gate = 0, float* const* out_at = nullptr, int* there = nullptr) {
     const int n_tok = ws->prepared_tok;
     if (rows_per_block > 0 && (count != 1 || n_out[0] % rows_per_block != 0 || rows_per_block % 4 != 0 || n_in % 8 != 0)) return cudaErrorInvalidValue;
     const int act_in = rows_per_block > 0 ? n_in * (n_out[0] / rows_per_block) : n_in;
@@ -1202,6 +1204,10 @@ static cudaError_t launch_gemm(ingot_linear_ws* ws, float* out, const void* cons
     p.half_ld = half_ld;
     p.half_block = half_block;
     p.out = out; p.status = ws->status;
+    if (out_at && few && n_split == 1) {
+        p.out_at = out_at;
+        *there = 1;
+    }
     p.act = gate;
     if (gate) p.out_hi = reinterpret_cast<__nv_bfloat16*>(ws->lo);
     p.n_tok = n_tok; p.k_steps = k_steps; p.n_split = n_split; p.accumulate = accumulate;
@@ -1229,6 +1235,14 @@ static cudaError_t launch_gemm(ingot_linear_ws* ws, float* out, const void* cons
 // out [n_tok][n_out] (+)= prepared activations x W^T, W f16 [n_out][n_in] on the device.
 cudaError_t ingot_linear_tc_run(ingot_linear_ws* ws, float* out, const void* w, int n_in, int n_out, int accumulate, cudaStream_t s) {
     return launch_gemm(ws, out, &w, n_in, &n_out, 1, accumulate, 0, false, false, s);
+}
+
+// The same to *out_at (a pointer in device memory, pinned host memory behind it) where the product's own kernel can write there as it goes
+// (*there = 1): few rows and no k slices; else to out. 8 rows of 32768 logits then cross PCIe while the weights stream:
+// product and delivery 53 -> 40 us (2048 wide, B200).
+cudaError_t ingot_linear_tc_run_to(ingot_linear_ws* ws, float* out, float* const* out_at, const void* w, int n_in, int n_out, int* there, cudaStream_t s) {
+    *there = 0;
+    return launch_gemm(ws, out, &w, n_in, &n_out, 1, 0, 0, false, false, s, 0, nullptr, 0, 0, 0, out_at, there);
 }
 
 // Block-diagonal product: W [n_out][k_block], output rows of block b = row / rows_per_block times the prepared columns

@@ -25,7 +25,7 @@ public:
     virtual void tap_residuals(std::vector<float>* out) = 0;
     // Bytes of weights a step reads once (embedding table excluded), and device time of the last step in milliseconds.
     virtual size_t weight_bytes() const = 0;
-    virtual float last_step_ms() const = 0;
+    virtual float last_step_ms() const = 0;  // device time, from the metadata coming in to the results going out
     // The next step's logits go to `rows` (pinned host memory with room for them) instead of the backend's own; false: it cannot do that.
     virtual bool step_into(float* rows) { (void)rows; return false; }
 };
