@@ -48,6 +48,15 @@ __device__ __forceinline__ void store_out(void* out, int dtype, size_t e, float 
     else static_cast<__half*>(out)[e] = __float2half_rn(v);
 }
 
+// Two neighbouring elements, e even.
+__device__ __forceinline__ void store_out2(void* out, int dtype, size_t e, float a, float b) {
+    if (dtype == INGOT_F32 && reinterpret_cast<uintptr_t>(out) % 8 == 0) {
+        *reinterpret_cast<float2*>(static_cast<float*>(out) + e) = make_float2(a, b);
+    } else {
+        store_out(out, dtype, e, a);
+        store_out(out, dtype, e + 1, b);
+    }
+}
 
 // Full m16n8k16 f16 MMA with f32 accumulation: d += A * B.
 __device__ __forceinline__ void mma_16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
