@@ -215,10 +215,16 @@ __global__ void __launch_bounds__(kMaxDecodeWarps * 32, 1) DECODE_KERNEL(const D
         return;
     }
     if (kCluster) ingot_sm100::cluster_arrive();  // this CTA has started: its shared memory may be written
-    // A single layer waits for the launch that appends its newest row; the rows it will read are requested into L2 meanwhile. Nothing is read
-    // before the wait (whatever the kernels before may still write is fetched again from L2), and only where the place and the number of the rows come from the host.
-    if (kCluster && p.pdl_mode == kPdlWaitFirst && !p.paged && !p.seq_lens) {
-        const int seq = blockIdx.z % p.n_seq, n = load_seq_len(p, seq), share = cluster_share(n, p.n_parts_max);
+#ifdef INGOT_DECODE_APPEND
+    constexpr bool kAhead = true;
+#else
+    constexpr bool kAhead = kCluster;
+#endif
+    // A single layer waits for the launch that appends its newest row, the append form for its own rows; the others that it will read are
+    // requested into L2 meanwhile. Nothing is read before the wait (whatever the kernels before may still write is fetched again from L2), and
+    // only where the place and the number of the rows come from the host.
+    if (kAhead && p.pdl_mode == kPdlWaitFirst && !p.paged && !p.seq_lens) {
+        const int n = load_seq_len(p, blockIdx.z % p.n_seq), share = kCluster ? cluster_share(n, p.n_parts_max) : p.chunk_keys;
         const int first = blockIdx.x * share, lines = (min(n, first + share) - first) * 2;  // of 64 values
         const size_t at = (size_t)(blockIdx.z / p.n_seq) * p.cache_layer_stride + kv_row_offset_contig(p.capacity, blockIdx.y, first);
         for (int i = threadIdx.x; i < lines; i += blockDim.x) {
@@ -262,10 +268,10 @@ __global__ void __launch_bounds__(kMaxDecodeWarps * 32, 1) DECODE_KERNEL(const D
             const int h = u >> 4, c = u & 15;
             if (h < G)
                 *reinterpret_cast<uint4*>(new_q + h * kHeadDim + c * 8) =
-                    rope_pack8(p.q_f32 + ((size_t)kvh * G + h) * kHeadDim + c * 8, c * 4, fpos, p.inv_freq, true);
+                    rope_pack8(p.q_f32 + ((size_t)layer * p.n_head + (size_t)kvh * G + h) * kHeadDim + c * 8, c * 4, fpos, p.inv_freq, true);
             else
                 *reinterpret_cast<uint4*>(new_kv + (h - G) * kHeadDim + c * 8) =
-                    rope_pack8((h == G ? p.k_new : p.v_new) + (size_t)kvh * kHeadDim + c * 8, c * 4, fpos, p.inv_freq, h == G);
+                    rope_pack8((h == G ? p.k_new : p.v_new) + ((size_t)layer * p.n_head_kv + kvh) * kHeadDim + c * 8, c * 4, fpos, p.inv_freq, h == G);
         }
         __syncthreads();
     }
@@ -798,10 +804,10 @@ extern "C" int ingot_attn_decode_noalloc(const void* k_dev, const void* v_dev, i
 #endif  // !INGOT_DECODE_APPEND
 
 #ifdef INGOT_DECODE_APPEND
-// One launch of the fused form for one token of one sequence on a contiguous cache: q/k/v are the f32 projections, the
+// One launch of the fused form for one token of one sequence on a contiguous cache, n_layers layers with stacked inputs and outputs: q/k/v are the f32 projections, the
 // key count (position + 1) comes from seq_lens (device) or max_seq_len. Splits and partials as in launch_attn_decode;
 // with more than one split, and no cluster, the caller follows up with the plain kernel's merge-only launch.
-int launch_attn_decode_append(ingot_kv* kv, int layer, const float* q, const float* k, const float* v, const float* inv_freq, void* out,
+int launch_attn_decode_append(ingot_kv* kv, int layer, int n_layers, const float* q, const float* k, const float* v, const float* inv_freq, void* out,
                               int out_dtype, int n_head, const int32_t* seq_lens, int max_seq_len, DecodePlan plan, float* part,
                               cudaStream_t stream) {
     const int n_warps = plan.n_warps;
@@ -818,8 +824,8 @@ int launch_attn_decode_append(ingot_kv* kv, int layer, const float* q, const flo
     p.qo_layer_stride = (size_t)n_head * kHeadDim;
     p.part_layer_stride = decode_part_floats(1, plan.n_parts, n_head);
     p.cache_extent = kv->checked_cache_elems();
-    p.part_extent = p.part_layer_stride;
-    p.out_extent = p.qo_layer_stride;
+    p.part_extent = p.part_layer_stride * n_layers;
+    p.out_extent = p.qo_layer_stride * n_layers;
     p.q_dtype = INGOT_F32; p.out_dtype = out_dtype;
     p.n_head = n_head; p.n_head_kv = kv->n_head_kv; p.group = n_head / kv->n_head_kv;
     p.capacity = kv->capacity; p.paged = 0; p.max_blocks_per_seq = 0;
@@ -831,7 +837,7 @@ int launch_attn_decode_append(ingot_kv* kv, int layer, const float* q, const flo
     const size_t smem_split = (size_t)n_warps * p.group * (kHeadDim + 2);
     const size_t smem_merge = (size_t)2 * p.group * kMaxParts + (size_t)4 * std::max(threads, p.group * 32);
     const size_t smem = (plan.cluster ? smem_split + (size_t)plan.n_parts * p.group * (kHeadDim + 2) : std::max(smem_split, smem_merge)) * sizeof(float);
-    const dim3 grid(plan.n_parts, kv->n_head_kv, 1);
+    const dim3 grid(plan.n_parts, kv->n_head_kv, (unsigned)n_layers);
     return launch_splits(plan.cluster ? attn_decode_append_kernel<true> : attn_decode_append_kernel<false>, grid, threads, smem, plan.cluster, stream, p);
 }
 #endif

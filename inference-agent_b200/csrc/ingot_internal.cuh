@@ -172,7 +172,7 @@ DecodePlan decode_plan(const ingot_kv* kv, int n_layers, int n_seq, int max_seq_
 void decode_cluster_room(int (&room)[kClusterParts + 1]);
 int decode_slots(const ingot_kv* kv);
 int decode_warps_cfg();
-int launch_attn_decode_append(ingot_kv* kv, int layer, const float* q, const float* k, const float* v, const float* inv_freq, void* out,
+int launch_attn_decode_append(ingot_kv* kv, int layer, int n_layers, const float* q, const float* k, const float* v, const float* inv_freq, void* out,
                               int out_dtype, int n_head, const int32_t* seq_lens, int max_seq_len, DecodePlan plan, float* part,
                               cudaStream_t stream);
 size_t decode_part_floats(int n_seq, int n_parts, int n_head);

@@ -287,7 +287,7 @@ int ingot_rope_append_decode(ingot_kv* kv, int layer, const float* q_dev, const 
         const int rc = ensure_decode_scratch(kv, decode_part_floats(1, plan.n_parts, n_head));
         if (rc != INGOT_OK) return rc;
     }
-    int rc = launch_attn_decode_append(kv, layer, q_dev, k_dev, v_dev, inv_freq_dev, out_dev, out_dtype, n_head, key_count_dev, max_seq_len,
+    int rc = launch_attn_decode_append(kv, layer, 1, q_dev, k_dev, v_dev, inv_freq_dev, out_dev, out_dtype, n_head, key_count_dev, max_seq_len,
                                        plan, kv->part, s);
     if (rc != INGOT_OK) return rc;
     return launch_attn_decode(kv, layer, 1, nullptr, INGOT_F16, out_dev, out_dtype, n_head, 1, key_count_dev, max_seq_len, nullptr, 0, plan,
@@ -414,6 +414,11 @@ int ingot_attn_layers_host(ingot_kv* kv, int layer_begin, int layer_count, const
         };
         float *const q_m = view(q_host, q_elems), *const k_m = view(k_host, kv_elems), *const v_m = view(v_host, kv_elems), *const o_m = view(out_host, q_elems);
         if (q_m && k_m && v_m && o_m) {
+            // One split per range (every row crosses PCIe once): append and attention in one launch, the cached keys on their way to L2 while the
+            // rows arrive. 28 layers (B200): 300 keys 49.9 -> 43.8 us.
+            const DecodePlan plan = decode_plan(kv, layer_count, 1, pos0 + 1, 0);
+            if (plan.n_parts == 1 && n_head / kv->n_head_kv <= 8 && layer_count <= 65535)
+                return launch_attn_decode_append(kv, layer_begin, layer_count, q_m, k_m, v_m, inv_freq_dev, o_m, INGOT_F32, n_head, nullptr, pos0 + 1, plan, kv->part, s);
             const int rc = launch_rope_kv_append(kv, layer_begin, q_m, qh_d, k_m, v_m, inv_freq_dev, n_head, pos0, 1, nullptr, nullptr, nullptr, 0, layer_count, s);
             if (rc != INGOT_OK) return rc;
             return ingot_attn_decode_layers(kv, layer_begin, layer_count, qh_d, INGOT_F16, o_m, INGOT_F32, n_head, 1, nullptr, pos0 + 1, nullptr, 0, 0, s);
