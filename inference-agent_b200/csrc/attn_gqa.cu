@@ -155,7 +155,7 @@ __global__ void __launch_bounds__(kAppendThreads) gqa_append_kernel(const Append
 // are merged by a second launch. kMax: most columns of a key or a value; the loops over 16-column steps stop at the true sizes.
 // Waits for copies are bounded: a warp that gives up waits, again bounded, for those in flight and raises the status word.
 constexpr unsigned long long kWaitLimitNs = 2000000000ull;
-constexpr int kMaxRing = 3, kWarps = 4, kMaxSharePages = 1024, kMaxSplits = 64, kSplitKeysMin = 128;
+constexpr int kMaxRing = 3, kWarps = 4, kMaxSharePages = 1024, kMaxSplits = 64, kSplitKeysMin = 128, kMaxCluster = 8;
 constexpr int kSmemLimit = 227 * 1024;
 struct GqaSmem {
     int stride, page_bytes, blocks, bytes;  // stride: halves between rows, 16 bytes past the row so that ldmatrix has no bank conflicts
@@ -181,10 +181,14 @@ __device__ __forceinline__ float ex2(float x) {
     return y;
 }
 
-template <int kMax>
+// kCluster: the shares of a range of rows are the CTAs of a cluster, which merge in each other's shared memory, every CTA its part of the
+// result, instead of through a scratch and a second launch:
+// 8 sequences of about 250 keys, 16 / 4 heads 11.0 -> 8.3 us (B200, inside a decoding step).
+template <int kMax, bool kCluster>
 __global__ void __launch_bounds__(kWarps * 32) gqa_mma_kernel(const AttendParams p, int share_pages) {
     constexpr int kK = kMax / 16, kN = kMax / 8;
     extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ float s_ml[kCluster ? 16 : 1][2];
     __shared__ uint64_t s_full[kWarps][kMaxRing];
     __shared__ uint32_t s_abort;
     INGOT_PDL_TRIGGER();
@@ -372,7 +376,10 @@ __global__ void __launch_bounds__(kWarps * 32) gqa_mma_kernel(const AttendParams
             x = fmaf(f, v.x, x);
             y = fmaf(f, v.y, y);
         }
-        if (p.n_splits == 1) {
+        if (kCluster) {  // stays here: only this thread has read the place of warp 0
+            *reinterpret_cast<float2*>(so + r * dv + d) = make_float2(x, y);
+            if (d == 0) { s_ml[r][0] = m; s_ml[r][1] = l; }
+        } else if (p.n_splits == 1) {
             const float inv = 1.0f / l;
             p.out.store2(row, h * dv + d, x * inv * p.gate.at(row, h, dv, d), y * inv * p.gate.at(row, h, dv, d + 1));
         } else {
@@ -380,6 +387,42 @@ __global__ void __launch_bounds__(kWarps * 32) gqa_mma_kernel(const AttendParams
             *reinterpret_cast<float2*>(part + d) = make_float2(x, y);
             if (d == 0) { part[dv] = m; part[dv + 1] = l; }
         }
+    }
+    if (kCluster) {
+        cluster_sync();
+        // as gqa_merge_kernel does it
+        const uint32_t my_o = smem_u32(so), my_ml = smem_u32(&s_ml[0][0]);
+        for (int i = (split * kWarps * 32 + (int)threadIdx.x) * 2; i < rows_here * dv; i += p.n_splits * kWarps * 64) {
+            const int r = i / dv, d = i - r * dv, h = kvh * group + (row0 + r) % group;
+            const size_t row = tok0 + (row0 + r) / group;
+            const float sink = p.sink ? p.sink[h] * 1.44269504f : -INFINITY;
+            float ms[kMaxCluster], ls[kMaxCluster];
+            float2 vs[kMaxCluster];
+#pragma unroll
+            for (int s = 0; s < kMaxCluster; s++) {
+                if (s >= p.n_splits) break;
+                const float2 ml = cluster_load2(map_to_rank(my_ml + r * 8, s));
+                ms[s] = ml.x;
+                ls[s] = ml.y;
+                vs[s] = cluster_load2(map_to_rank(my_o + (r * dv + d) * 4, s));
+            }
+            float top = sink;
+#pragma unroll
+            for (int s = 0; s < kMaxCluster; s++)
+                if (s < p.n_splits) top = fmaxf(top, ms[s]);
+            float l = exp2f(sink - top), a = 0.f, b = 0.f;
+#pragma unroll
+            for (int s = 0; s < kMaxCluster; s++) {
+                if (s >= p.n_splits) break;
+                const float f = exp2f(ms[s] - top);
+                l = fmaf(f, ls[s], l);
+                a = fmaf(f, vs[s].x, a);
+                b = fmaf(f, vs[s].y, b);
+            }
+            const float inv = 1.0f / l;
+            p.out.store2(row, h * dv + d, a * inv * p.gate.at(row, h, dv, d), b * inv * p.gate.at(row, h, dv, d + 1));
+        }
+        cluster_sync();  // nobody leaves while its shares may still be read
     }
 }
 
@@ -439,6 +482,33 @@ int launch_mma(ingot_skv* kv, AttendParams p, cudaStream_t s) {
     p.n_splits = std::max(p.n_splits, (pages + kMaxSharePages - 1) / kMaxSharePages);
     if (p.n_splits > kMaxSplits) return launch_shared_kv_plain(p, INGOT_F16, s);
     const int share_pages = (pages + p.n_splits - 1) / p.n_splits, smem = GqaSmem(p.dim, p.out_dim, share_pages).bytes;
+    const int most = std::max(p.q_dim, p.out_dim);
+    const dim3 grid(row_tiles * p.n_splits, p.n_head_kv, p.st.n_seq);
+    // Clusters where the device holds those of all ranges at a time, so that none waits for a place where separate CTAs would find one.
+    if (p.n_splits > 1 && p.n_splits <= kMaxCluster) {
+        auto kernel = most <= 64 ? gqa_mma_kernel<64, true> : most <= 128 ? gqa_mma_kernel<128, true> : gqa_mma_kernel<256, true>;
+        INGOT_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, widest));
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = grid;
+        cfg.blockDim = dim3(kWarps * 32);
+        cfg.dynamicSmemBytes = size_t(smem);
+        cfg.stream = s;
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = unsigned(p.n_splits);
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int room = 0;
+        if (cudaOccupancyMaxActiveClusters(&room, kernel, &cfg) != cudaSuccess) { cudaGetLastError(); room = 0; }
+        if (ctas <= room) {
+            cfg.numAttrs = ingot_use_pdl() ? 2 : 1;
+            INGOT_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, p, share_pages));
+            return INGOT_OK;
+        }
+    }
     if (p.n_splits > 1) {
         const size_t need = (size_t)p.st.n_tok * p.n_head * p.n_splits * (p.out_dim + 2);
         if (need > kv->part_floats) {
@@ -450,10 +520,9 @@ int launch_mma(ingot_skv* kv, AttendParams p, cudaStream_t s) {
         }
         p.part = kv->part;
     }
-    const int most = std::max(p.q_dim, p.out_dim);
-    auto kernel = most <= 64 ? gqa_mma_kernel<64> : most <= 128 ? gqa_mma_kernel<128> : gqa_mma_kernel<256>;
+    auto kernel = most <= 64 ? gqa_mma_kernel<64, false> : most <= 128 ? gqa_mma_kernel<128, false> : gqa_mma_kernel<256, false>;
     INGOT_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, widest));
-    INGOT_CUDA_TRY(ingot_launch_pdl(kernel, dim3(row_tiles * p.n_splits, p.n_head_kv, p.st.n_seq), dim3(kWarps * 32), size_t(smem), s, p, share_pages));
+    INGOT_CUDA_TRY(ingot_launch_pdl(kernel, grid, dim3(kWarps * 32), size_t(smem), s, p, share_pages));
     if (p.n_splits > 1) INGOT_CUDA_TRY(ingot_launch_pdl(gqa_merge_kernel, dim3(p.n_head, p.st.max_len, p.st.n_seq), dim3(128), 0, s, p));
     return INGOT_OK;
 }
