@@ -148,6 +148,124 @@ __global__ void __launch_bounds__(kAppendThreads) gqa_append_kernel(const Append
     }
 }
 
+// The same for prompts with f16 rows and heads of 128: half a warp per head, eight values per lane, queries, keys and values alike. The kernel
+// above is bound by instructions there (0.53 to 0.68 of the issue slots, DRAM at 0.3): a load, a store, addresses and conditions per
+// four values. 4096 tokens, 32 / 8 heads inside a step (B200): 46-50 -> 40-44 us without norms, 63 -> 52 with.
+__global__ void __launch_bounds__(kAppendThreads) gqa_append128_kernel(const AppendParams p) {
+    constexpr int kDim = 128, kHalves = kAppendThreads / 16;
+    INGOT_PDL_TRIGGER();
+    __shared__ float red[2 * kAppendThreads / 32];
+    __shared__ __align__(16) float s_cos[kDim / 2], s_sin[kDim / 2];
+    const int tok = blockIdx.x, seq = p.st.row_seq[tok], warp = threadIdx.x >> 5, lane = threadIdx.x & 31, piece = threadIdx.x & 15;
+    const int pos = p.st.pos0[seq] + tok - p.st.row_start[seq];
+    const int rot = p.sh.rot_dims, H = p.sh.n_head, G = p.sh.n_head_kv;
+    if (threadIdx.x < rot / 2) {
+        double t = double(pos) * p.turns[threadIdx.x];
+        t -= rint(t);
+        float c, s;
+        sincospif(2.0f * float(t), &s, &c);
+        s_cos[threadIdx.x] = c * p.rot_gain;
+        s_sin[threadIdx.x] = s * p.rot_gain;
+    }
+    INGOT_PDL_WAIT();
+    const float* row = p.proj + (size_t)tok * p.proj_ld;
+    float inv_q = 1.f, inv_k = 1.f;
+    if (p.sh.norm == INGOT_QK_NORM_ALL) {
+        float sq = 0.f, sk = 0.f;
+        for (int i = threadIdx.x * 4; i < H * kDim; i += kAppendThreads * 4) sq = dot4(*reinterpret_cast<const float4*>(row + p.q_off + i), sq);
+        for (int i = threadIdx.x * 4; i < G * kDim; i += kAppendThreads * 4) sk = dot4(*reinterpret_cast<const float4*>(row + p.k_off + i), sk);
+        sq = warp_sum(sq);
+        sk = warp_sum(sk);
+        if (lane == 0) { red[warp] = sq; red[kAppendThreads / 32 + warp] = sk; }
+    }
+    __syncthreads();
+    if (p.sh.norm == INGOT_QK_NORM_ALL) {
+        float sq = 0.f, sk = 0.f;
+#pragma unroll
+        for (int w = 0; w < kAppendThreads / 32; w++) { sq += red[w]; sk += red[kAppendThreads / 32 + w]; }
+        inv_q = 1.0f / sqrtf(sq / float(H * p.sh.dim_count) + p.eps);
+        inv_k = 1.0f / sqrtf(sk / float(G * p.sh.dim_count) + p.eps);
+    }
+    const int blk = table_block(p.tables, p.first_page, p.max_blocks, p.n_blocks, seq, p.map.page(pos), p.status);
+    __half* const page = static_cast<__half*>(p.rows) + ((size_t)max(blk, 0) * G * kBlockTokens + p.map.slot(pos)) * (2 * kDim) + piece * 8;  // of KV head 0
+    const size_t head_stride = (size_t)kBlockTokens * 2 * kDim;
+    __half* const q_out = static_cast<__half*>(p.q_out) + (size_t)tok * H * kDim + piece * 8;
+    float cs[4], sn[4];  // of this lane's four pairs
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const bool on = piece * 8 + 2 * i < rot;
+        cs[i] = on ? s_cos[piece * 4 + i] : 1.f;
+        sn[i] = on ? s_sin[piece * 4 + i] : 0.f;
+    }
+    const float keep = 1.0f - p.mix;
+    const int units = H + 2 * G;
+#pragma unroll 3
+    for (int u0 = 0; u0 < units; u0 += kHalves) {
+        const int u = u0 + (threadIdx.x >> 4);
+        if (u0 + kHalves > units && __all_sync(0xffffffffu, u >= units)) break;
+        const bool live = u < units, is_q = u < H, is_v = u >= H + G;
+        const int h = is_q ? u : is_v ? u - H - G : u - H;
+        const float* src = row + (is_q ? p.q_off : is_v ? p.v_off : p.k_off) + h * kDim + piece * 8;
+        float v[8] = {};
+        if (live) {
+            const float4 a = reinterpret_cast<const float4*>(src)[0], b = reinterpret_cast<const float4*>(src)[1];
+            v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+        }
+        if (p.sh.norm != INGOT_QK_NORM_NONE) {  // the two halves of a warp may hold a key and a value: all lanes take part
+            float inv = is_q ? inv_q : inv_k;
+            const float* w = (is_q ? p.q_norm : p.k_norm) + (p.sh.norm == INGOT_QK_NORM_ALL ? h * kDim : 0) + piece * 8;
+            if (p.sh.norm == INGOT_QK_NORM_HEAD) {
+                float ss = dot4(make_float4(v[0], v[1], v[2], v[3]), dot4(make_float4(v[4], v[5], v[6], v[7]), 0.f));
+#pragma unroll
+                for (int o = 8; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+                inv = 1.0f / sqrtf(ss / float(p.sh.dim_count) + p.eps);
+            }
+            if (live && !is_v) {
+                const float4 a = reinterpret_cast<const float4*>(w)[0], b = reinterpret_cast<const float4*>(w)[1];
+                const float g[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+                for (int i = 0; i < 8; i++) v[i] *= inv * g[i];
+            }
+        }
+        if (!live) continue;
+        __half* dst = q_out + h * kDim;
+        if (is_v) {
+            if (p.first_values) {
+                float4* f = reinterpret_cast<float4*>(p.first_values + (size_t)tok * G * kDim + h * kDim + piece * 8);
+                if (p.store_first) {
+                    f[0] = make_float4(v[0], v[1], v[2], v[3]);
+                    f[1] = make_float4(v[4], v[5], v[6], v[7]);
+                } else {
+                    const float4 a = f[0], b = f[1];
+                    const float x[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+                    for (int i = 0; i < 8; i++) v[i] = fmaf(p.mix, x[i], keep * v[i]);
+                }
+            }
+        } else if (rot > 0) {
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const float x = v[2 * i], y = v[2 * i + 1];
+                if (piece * 8 + 2 * i < rot) {
+                    v[2 * i] = x * cs[i] - y * sn[i];
+                    v[2 * i + 1] = y * cs[i] + x * sn[i];
+                }
+            }
+        }
+        if (!is_q) {
+            if (blk < 0) continue;
+            dst = page + h * head_stride + (is_v ? kDim : 0);
+        }
+        uint32_t packed[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const __half2 h2 = __floats2half2_rn(clamp_half(v[2 * i]), clamp_half(v[2 * i + 1]));
+            packed[i] = *reinterpret_cast<const uint32_t*>(&h2);
+        }
+        *reinterpret_cast<uint4*>(dst) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+    }
+}
+
 // ---- decoded tokens and short portions: f16, m16n8k16 MMAs, the keys split over CTAs ---------------------------------------------------
 // A CTA serves 16 (token, head) rows of one KV head of one sequence over one share of the pages they see. Its four warps take every fourth
 // page each through a ring of bulk copies of their own - a lane fetches a slot's row, no barrier in the key loop - the block table of the
@@ -560,6 +678,12 @@ int ingot_gqa_append(ingot_skv* kv, int layer, const ingot_step* step, const flo
     AppendParams p = {*step, proj_dev, proj_ld, q_off, k_off, v_off, *shape, q_norm_dev, k_norm_dev, eps, turns_dev, rot_gain, first_values_dev, store_first, mix,
                       q_out_dev, static_cast<char*>(kv->rows) + kv->layer_elems * layer * esz, tables_dev, first_page_dev, max_blocks, kv->n_blocks, page_map(kv),
                       kv->status_dev};
+    auto aligned = [](const void* a) { return reinterpret_cast<uintptr_t>(a) % 16 == 0; };
+    if (step->n_tok > 64 && kv->dtype == INGOT_F16 && shape->dim == 128 && shape->vdim == 128 && aligned(q_out_dev) && aligned(proj_dev) && aligned(q_norm_dev) &&
+        aligned(k_norm_dev) && aligned(first_values_dev)) {
+        INGOT_CUDA_TRY(ingot_launch_pdl(gqa_append128_kernel, dim3(step->n_tok), dim3(kAppendThreads), 0, static_cast<cudaStream_t>(stream), p));
+        return INGOT_OK;
+    }
     auto kernel = kv->dtype == INGOT_F32 ? gqa_append_kernel<float> : gqa_append_kernel<__half>;
     // few tokens: a CTA per eight heads, so that no warp has several in a row
     const int heads = shape->n_head + shape->n_head_kv, parts = step->n_tok <= 64 ? std::min(8, (heads + 7) / 8) : 1;

@@ -161,6 +161,31 @@ def test_ragged_portions(name, dtype, impl):
         assert np.abs(y - want).max() < (2e-5 if dtype == F32 else 6e-3) * max(1.0, np.abs(want).max())
 
 
+@pytest.mark.parametrize("heads,kv", [(4, 1), (5, 5), (24, 8)])  # units of a token: below a round of the append's half warps, one with a rest, several
+@pytest.mark.parametrize("norm,rot,mix", [(None, 128, None), ("head", 0, 0.4), ("whole", 90, 0.7), ("head", 34, None)])
+def test_prompts_of_128_wide_heads(heads, kv, norm, rot, mix):
+    s = Shape(heads, kv, 128, 128, norm=norm, rot=rot, mix=mix)
+    rng = np.random.default_rng(heads)
+    w, seqs = Weights(s, 2), [sequence(s, n, rng) for n in (97, 40)]
+    got = run(s, seqs, [[64, 33], [1, 39]], w, F16, 0)
+    for x, y in zip(seqs, got):
+        want = reference(s, x, w)
+        assert np.abs(y - want).max() < 6e-3 * max(1.0, np.abs(want).max())
+
+
+@pytest.mark.parametrize("keys", [129, 256, 700, 1024, 1500])
+@pytest.mark.parametrize("gate,sink", [(None, True), ("element", False), ("head", True)])
+def test_key_shares_that_merge_in_a_cluster(keys, gate, sink):
+    """Two to eight shares, the last of them short; sequences that need fewer than the longest one."""
+    s = Shape(6, 2, 64, 48, gate=gate, sink=sink)
+    rng = np.random.default_rng(keys)
+    w, seqs = Weights(s, 4), [sequence(s, n, rng) for n in (keys + 2, 20)]
+    got = run(s, seqs, [[keys, 1, 1], [18, 1, 1]], w, F16, 2)
+    for x, y in zip(seqs, got):
+        want = reference(s, x, w)
+        assert np.abs(y - want).max() < 6e-3 * max(1.0, np.abs(want).max())
+
+
 @pytest.mark.parametrize("decoded", [False, True])
 @pytest.mark.parametrize("dtype,impl", [(F32, 1), (F16, 2), (F16, 3)])
 @pytest.mark.parametrize("window", [0, 1, 16, 17, 40, 128, 129])
