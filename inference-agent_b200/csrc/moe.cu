@@ -218,17 +218,29 @@ __global__ void __launch_bounds__(256) moe_table_kernel(const int32_t* table, co
     weight_of[i] = weight;
 }
 
-// bf16 planes of the rows: row r is its token's row. n_rows (device, may be null): how many of the launch's rows there are.
-__global__ void __launch_bounds__(128) moe_gather_kernel(uint4* hi, uint4* lo, const uint4* src_hi, const uint4* src_lo, const int32_t* pair_of, int top, int n8,
-                                                         const int32_t* n_rows) {
+// bf16 planes of the rows: row r is its token's row. n_rows_dev (may be null): how many of the n_rows there are. A warp per row, eight 16-byte pieces
+// per lane in flight: 8000 rows of 2048 9.4 -> 7.4 us against a CTA per row (B200, inside a step).
+__global__ void __launch_bounds__(256) moe_gather_kernel(uint4* hi, uint4* lo, const uint4* src_hi, const uint4* src_lo, const int32_t* pair_of, int top, int n8, int n_rows,
+                                                         const int32_t* n_rows_dev) {
+    constexpr int kPieces = 8;
     INGOT_PDL_TRIGGER();
     INGOT_PDL_WAIT();
-    if (n_rows && (int)blockIdx.x >= *n_rows) return;
-    const size_t r = blockIdx.x, t = size_t(pair_of[r] / top);
-    for (int i = threadIdx.x; i < n8; i += 128) {
-        hi[r * n8 + i] = src_hi[t * n8 + i];
-        if (lo) lo[r * n8 + i] = src_lo[t * n8 + i];
-    }
+    const int r = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (r >= n_rows || (n_rows_dev && r >= *n_rows_dev)) return;
+    const size_t to = (size_t)r * n8, from = size_t(pair_of[r] / top) * n8;
+    auto copy = [&](uint4* dst, const uint4* src) {
+        for (int i = lane; i < n8; i += 32 * kPieces) {
+            uint4 v[kPieces];
+#pragma unroll
+            for (int k = 0; k < kPieces; k++)
+                if (i + 32 * k < n8) v[k] = src[from + i + 32 * k];
+#pragma unroll
+            for (int k = 0; k < kPieces; k++)
+                if (i + 32 * k < n8) dst[to + i + 32 * k] = v[k];
+        }
+    };
+    copy(hi, src_hi);
+    if (lo) copy(lo, src_lo);
 }
 
 // Plain products: out[row][o] = act(row_weight * W_e[o] . x[source(row)]), f32 arithmetic on bf16 weights. A warp owns one output of
@@ -465,8 +477,8 @@ int ingot_moe_gather(void* hi_dev, void* lo_dev, const void* src_hi_dev, const v
                      int n, void* stream) {
     INGOT_REQUIRE(hi_dev && src_hi_dev && pair_of_dev && (!lo_dev || src_lo_dev), "ingot_moe_gather: null argument");
     INGOT_REQUIRE(n_rows >= 1 && top >= 1 && n >= 8 && n % 8 == 0, "ingot_moe_gather: bad sizes");
-    INGOT_CUDA_TRY(ingot_launch_pdl(moe_gather_kernel, dim3(n_rows), dim3(128), 0, static_cast<cudaStream_t>(stream), static_cast<uint4*>(hi_dev), static_cast<uint4*>(lo_dev),
-                                    static_cast<const uint4*>(src_hi_dev), static_cast<const uint4*>(src_lo_dev), pair_of_dev, top, n / 8, n_rows_dev));
+    INGOT_CUDA_TRY(ingot_launch_pdl(moe_gather_kernel, dim3((n_rows + 7) / 8), dim3(256), 0, static_cast<cudaStream_t>(stream), static_cast<uint4*>(hi_dev), static_cast<uint4*>(lo_dev),
+                                    static_cast<const uint4*>(src_hi_dev), static_cast<const uint4*>(src_lo_dev), pair_of_dev, top, n / 8, n_rows, n_rows_dev));
     return INGOT_OK;
 }
 
