@@ -39,7 +39,7 @@ public:
         w_o_ = ops.matrix(p + "o", flat(d), in);
         conv_state_ = ops.state(size_t(taps_ - 1) * ip_);
         state_ = ops.state(size_t(ip_) * np_);
-        plan_ = ops.scan_plan(ip_ * 2, size_t(ip_) * (np_ + 1));
+        plan_ = ops.scan_plan(ip_ * 2, size_t(ip_) * (np_ + 1), !ops.opt.f32 && states_ <= 32 ? ip_ : 0);
         ops.need(kProj, 2 * ip_);
         ops.need(kConv, ip_);
         ops.need(kStateIn, rank_p_ + 2 * np_);

@@ -395,6 +395,214 @@ __global__ void __launch_bounds__(128) selective_scan_kernel(const ScanParams p)
     }
 }
 
+// ---- selective scan of long chunks: the output pass as a stream --------------------------------------------------------
+// The tile kernel above does its phases one after the other (stage, step sizes, tokens, gates), so that one chunk per sequence left it waiting
+// between them (2048 tokens, 8192 channels: 799 us). Here one half of a CTA does nothing but the recurrence and the other everything around it; a chunk as long as
+// the sequence keeps the units busy, and the passes that find the chunks' start states fall away. kLanes lanes share a channel, each with kS
+// of its states; kNch channels per CTA.
+//   helpers   request tiles of 16 tokens three ahead (cp.async, a ring of kStreamSlots), turn dt into softplus(dt + bias) and dt x, and
+//             write (y + D x) silu(z) of the tile before last
+//   scanners  walk the tokens of the tile that is ready and leave y
+// Hand-over by named barriers: kBarReady + parity (helpers arrive, scanners wait), kBarDone + parity (the reverse).
+// What bounds it: instruction issue and shared memory next to the 2^x. 64 channels of 16 states take 165 cycles a token; 80 are the 2^x of scan,
+// softplus and gates at 16 per clock, about 85 the instructions, 110 the shared-memory cycles. A single warp of scanners per scheduler with
+// twice the channels does not overlap them (it issues in order), four with half the states each fetch B and C twice as often (195 us below).
+// All passes inside a prompt's step, against chunks (B200): 2048 tokens x 8192 channels 223 -> 179 us, 300 x 8192 46 -> 29, 1024 x 4096 65 -> 61, 250 x 4096
+// 33 -> 18, four sequences of 190 to 300 67 -> 49. Error against 64 bits, 2048 tokens: 8.6e-7 -> 2.8e-7 of the result (chunks of 240 before).
+constexpr int kStreamSlots = 6, kStreamHelpers = 256, kStreamFrom = 64;  // portions of more than kStreamFrom tokens
+enum : int { kBarHelpers = 1, kBarReady = 2, kBarDone = 4 };  // + parity
+__device__ __forceinline__ void bar_arrive(int id, int n) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory"); }
+__device__ __forceinline__ void bar_wait(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
+// floats of a ring slot: x, dt, z, dt x, y of n_ch channels, B and C of np states
+__host__ __device__ constexpr int stream_slot_floats(int n_ch, int np) { return kScanTile * (5 * n_ch + 2 * np); }
+
+template <int kS, int kLanes, int kNch>
+__global__ void __launch_bounds__(kNch * kLanes + kStreamHelpers) selective_scan_stream_kernel(const ScanParams p) {
+    extern __shared__ __align__(16) float smem[];
+    static_assert(kLanes == 4 || kLanes == 8, "exchanges below");
+    constexpr int kScanners = kNch * kLanes, kAll = kScanners + kStreamHelpers, kNp = kS * kLanes, kCh4 = kNch / 4, kNp4 = kNp / 4;
+    constexpr int kSlot = stream_slot_floats(kNch, kNp), kDt = kScanTile * kNch, kZ = 2 * kDt, kDtx = 3 * kDt, kY = 4 * kDt, kB = 5 * kDt, kC = kB + kScanTile * kNp;
+    INGOT_PDL_TRIGGER();
+    INGOT_PDL_WAIT();
+    const int chunk = blockIdx.y;
+    const int seq = p.chunk_seq[chunk], t0 = p.chunk_t0[chunk], len = p.chunk_len[chunk];
+    const bool first = t0 == 0, last = t0 + len == p.st.len[seq];
+    const int c_base = blockIdx.x * kNch, n_tiles = (len + kScanTile - 1) / kScanTile;
+    const size_t row0 = (size_t)p.st.row_start[seq] + t0;
+
+    if (threadIdx.x >= kScanners) {
+        // ---------------- helpers ----------------
+        const int tid = threadIdx.x - kScanners;
+        auto stage = [&](int tile) {
+            if (tile < n_tiles) {
+                float* s = smem + tile % kStreamSlots * kSlot;
+                const int t_base = tile * kScanTile;
+#pragma unroll
+                for (int i = tid; i < kScanTile * kCh4; i += kStreamHelpers) {
+                    const int t = i / kCh4, q = (i - t * kCh4) * 4;
+                    const bool on = t_base + t < len && c_base + q < p.inner;
+                    const size_t row = row0 + min(t_base + t, len - 1);
+                    const int cc = min(c_base + q, p.inner - 4);
+                    cp_async16(s + t * kNch + q, p.x + row * p.x_ld + cc, on);
+                    cp_async16(s + kDt + t * kNch + q, p.dt + row * p.dt_ld + cc, on);
+                    cp_async16(s + kZ + t * kNch + q, p.z + row * p.z_ld + cc, on);
+                }
+#pragma unroll
+                for (int i = kStreamHelpers - 1 - tid; i < kScanTile * kNp4; i += kStreamHelpers) {
+                    const int t = i / kNp4, q = (i - t * kNp4) * 4;
+                    const bool on = t_base + t < len;
+                    const size_t row = row0 + min(t_base + t, len - 1);
+                    cp_async16(s + kB + t * kNp + q, p.bc + row * p.bc_ld + p.b_off + q, on);
+                    cp_async16(s + kC + t * kNp + q, p.bc + row * p.bc_ld + p.c_off + q, on);
+                }
+            }
+            cp_async_commit();  // a group per tile, also past the end, so that the count of those in flight stays the same
+        };
+        const int my_q = tid % kCh4 * 4;  // the four channels this thread prepares and writes
+        const bool my_live = c_base + my_q < p.inner;
+        const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 my_bias = my_live ? *reinterpret_cast<const float4*>(p.dt_bias + c_base + my_q) : zero4;
+        const float4 my_d = my_live ? *reinterpret_cast<const float4*>(p.d + c_base + my_q) : zero4;
+        auto finish = [&](int tile) {  // y of a tile is there
+            const float* s = smem + tile % kStreamSlots * kSlot;
+            const int n_t = min(kScanTile, len - tile * kScanTile);
+            if (!my_live) return;
+#pragma unroll
+            for (int i = tid; i < kScanTile * kCh4; i += kStreamHelpers) {
+                if (i >= n_t * kCh4) break;
+                const float4 xv = reinterpret_cast<const float4*>(s)[i], yv = reinterpret_cast<const float4*>(s + kY)[i], zv = reinterpret_cast<const float4*>(s + kZ)[i];
+                p.out.store4(row0 + tile * kScanTile + i / kCh4, c_base + my_q,
+                             make_float4(fmaf(my_d.x, xv.x, yv.x) * fast_silu(zv.x), fmaf(my_d.y, xv.y, yv.y) * fast_silu(zv.y),
+                                         fmaf(my_d.z, xv.z, yv.z) * fast_silu(zv.z), fmaf(my_d.w, xv.w, yv.w) * fast_silu(zv.w)));
+            }
+        };
+        stage(0);
+        stage(1);
+        stage(2);
+        for (int tile = 0; tile < n_tiles; tile++) {
+            if (tile >= 2) bar_wait(kBarDone + (tile & 1), kAll);  // tile - 2
+            cp_async_wait<2>();  // all but the next two tiles'
+            bar_wait(kBarHelpers, kStreamHelpers);  // every helper's copies have landed; every helper has finished tile - 3, whose slot tile + 3 takes
+            stage(tile + 3);
+            float* s = smem + tile % kStreamSlots * kSlot;
+#pragma unroll
+            for (int i = tid; i < kScanTile * kCh4; i += kStreamHelpers) {
+                const float4 raw = reinterpret_cast<const float4*>(s + kDt)[i], xv = reinterpret_cast<const float4*>(s)[i];
+                const float4 dt = make_float4(fast_softplus(raw.x + my_bias.x), fast_softplus(raw.y + my_bias.y), fast_softplus(raw.z + my_bias.z), fast_softplus(raw.w + my_bias.w));
+                reinterpret_cast<float4*>(s + kDt)[i] = dt;
+                reinterpret_cast<float4*>(s + kDtx)[i] = make_float4(dt.x * xv.x, dt.y * xv.y, dt.z * xv.z, dt.w * xv.w);
+            }
+            bar_arrive(kBarReady + (tile & 1), kAll);
+            if (tile >= 2) finish(tile - 2);
+        }
+        for (int tile = max(0, n_tiles - 2); tile < n_tiles; tile++) {
+            bar_wait(kBarDone + (tile & 1), kAll);
+            finish(tile);
+        }
+        cp_async_wait<0>();
+        return;
+    }
+
+    // ---------------- scanners ----------------
+    const int ch = threadIdx.x / kLanes, part = threadIdx.x % kLanes, c = c_base + ch;
+    const bool live = c < p.inner;
+    f32x2 a[kS / 2], s[kS / 2], local[kS / 2], begin[kS / 2];
+    const size_t sidx = (size_t)(live ? c : 0) * kNp + part * kS;
+    const size_t slot_base = (size_t)p.st.slot[seq] * p.inner * kNp;
+    {
+        // start state: as in the tile kernel
+        const float* from = nullptr;
+        if (!(first && last)) from = p.part + (size_t)chunk * p.inner * kNp + sidx;
+        else if (p.st.pos0[seq] > 0) from = p.state + slot_base + sidx;
+#pragma unroll
+        for (int i = 0; i < kS / 2; i++) {
+            a[i] = live ? *reinterpret_cast<const f32x2*>(p.a2 + sidx + 2 * i) : 0;
+            s[i] = live && from ? *reinterpret_cast<const f32x2*>(from + 2 * i) : 0;
+        }
+    }
+    // Four tokens at a time: what they need is requested while the four before them are computed, and before those store their y (the
+    // compiler must keep loads behind stores that might be to the same place). A channel's four y end up one per lane, or per two lanes.
+    struct Four {
+        float dt[4], dtx[4];
+        f32x2 b[4][kS / 2], c[4][kS / 2];
+    };
+    const bool high = part & (kLanes / 2), odd = part & (kLanes / 4);
+    const int my_token = (high ? 2 : 0) + (odd ? 1 : 0);
+    for (int tile = 0; tile < n_tiles; tile++) {
+        bar_wait(kBarReady + (tile & 1), kAll);
+        float* const base = smem + tile % kStreamSlots * kSlot;
+        const float *sdt = base + kDt + ch, *sdtx = base + kDtx + ch, *sb = base + kB + part * kS, *sc = base + kC + part * kS;
+        float* const sy = base + kY + ch + my_token * kNch;
+        auto load = [&](int t0, Four& f) {
+#pragma unroll
+            for (int t = 0; t < 4; t++) {
+                f.dt[t] = sdt[(t0 + t) * kNch];
+                f.dtx[t] = sdtx[(t0 + t) * kNch];
+                load_pairs<kS>(sb + (t0 + t) * kNp, f.b[t]);
+                load_pairs<kS>(sc + (t0 + t) * kNp, f.c[t]);
+            }
+        };
+        float sum_dt = 0.f;
+        // n: tokens of the four that count (a warp-uniform number; the state does not move at the others)
+        auto four = [&](int t0, const Four& f, int n) {
+            float y[4];
+#pragma unroll
+            for (int t = 0; t < 4; t++) {
+                if (t < n) sum_dt += f.dt[t];
+                const f32x2 dt2 = pair(f.dt[t], f.dt[t]), dtx2 = pair(f.dtx[t], f.dtx[t]);
+                f32x2 y2 = 0;
+#pragma unroll
+                for (int i = 0; i < kS / 2; i++) {
+                    const float2 x = unpair(mul2(dt2, a[i]));
+                    const f32x2 e = pair(ex2f(x.x), ex2f(x.y)), in = mul2(dtx2, f.b[t][i]), moved = fma2(e, s[i], in), from_zero = fma2(e, local[i], in);
+                    if (t < n) { s[i] = moved; local[i] = from_zero; }
+                    y2 = fma2(s[i], f.c[t][i], y2);
+                }
+                const float2 yv = unpair(y2);
+                y[t] = yv.x + yv.y;
+            }
+            // the upper half of the lanes takes tokens 2 and 3 over, then every second quarter the odd one of each two
+            const float even = (high ? y[2] : y[0]) + __shfl_xor_sync(0xffffffffu, high ? y[0] : y[2], kLanes / 2);
+            const float next = (high ? y[3] : y[1]) + __shfl_xor_sync(0xffffffffu, high ? y[1] : y[3], kLanes / 2);
+            float v = (odd ? next : even) + __shfl_xor_sync(0xffffffffu, odd ? even : next, kLanes / 4);
+            if (kLanes == 8) v += __shfl_xor_sync(0xffffffffu, v, 1);
+            if (kLanes == 4 || !(part & 1)) sy[t0 * kNch] = v;
+        };
+        // The unit's 2^x is good to about 2^-22, and a state that hardly decays would collect that at every token. So a tile's end state is what its
+        // tokens add up to from zero, and the state it began with times one decay over all of its tokens.
+#pragma unroll
+        for (int i = 0; i < kS / 2; i++) {
+            begin[i] = s[i];
+            local[i] = 0;
+        }
+        const int n_t = min(kScanTile, len - tile * kScanTile);
+        Four f[2];
+        load(0, f[0]);
+        if (n_t == kScanTile) {
+#pragma unroll
+            for (int t = 0; t < kScanTile; t += 4) {
+                if (t + 4 < kScanTile) load(t + 4, f[(t >> 2) + 1 & 1]);
+                four(t, f[t >> 2 & 1], 4);
+            }
+        } else {  // places of tokens past the end hold zeros
+            for (int t = 0; t < n_t; t += 4) {
+                four(t, f[0], n_t - t);
+                if (t + 4 < n_t) load(t + 4, f[0]);
+            }
+        }
+        bar_arrive(kBarDone + (tile & 1), kAll);
+#pragma unroll
+        for (int i = 0; i < kS / 2; i++) {
+            const float2 x = unpair(mul2(pair(sum_dt, sum_dt), a[i]));
+            s[i] = fma2(pair(ex2f(x.x), ex2f(x.y)), begin[i], local[i]);
+        }
+    }
+    if (live && last) {
+#pragma unroll
+        for (int i = 0; i < kS / 2; i++) *reinterpret_cast<f32x2*>(p.state + slot_base + sidx + 2 * i) = s[i];
+    }
+}
+
 // Pass 2: end states -> start states, sequence by sequence. The first chunk ran from the slot, so its end state is exact.
 __global__ void __launch_bounds__(256) selective_scan_link_kernel(const ScanParams p) {
     INGOT_PDL_TRIGGER();
@@ -523,6 +731,12 @@ __global__ void __launch_bounds__(128) gated_lru_link_kernel(const LruParams p) 
     }
 }
 
+constexpr size_t kHalfSm = 116 * 1024;  // shared memory of which an SM has less than twice
+bool one_per_sm(long long ctas) {
+    int dev = 0, num_sms = 0;
+    return cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && ctas <= num_sms;
+}
+
 int scan_lanes_log2(int n_state) {
     int l = 2;  // 4 lanes per channel up to 32 states, then as many as keep 8 states per lane
     while ((8 << l) < n_state) l++;
@@ -610,6 +824,27 @@ int ingot_selective_scan(const ingot_step* step, const ingot_scan_plan* plan, co
     if (multi) {
         INGOT_CUDA_TRY(ingot_launch_pdl(k_end, grid, dim3(128), smem, s, p));
         INGOT_CUDA_TRY(ingot_launch_pdl(selective_scan_link_kernel, dim3(unsigned(((size_t)inner * n_pad + 255) / 256), step->n_seq), dim3(256), 0, s, p));
+    }
+    // The output pass of long chunks as a stream; the tile kernel for the exact form, more than 32 states, and chunks too short to fill a ring.
+    if (!exact && lg == 2 && step->max_len > kStreamFrom) {
+        // 64 channels per CTA, or 32 with more lanes each where that would leave SMs without a CTA
+        const bool wide = (long long)((inner + 63) / 64) * plan->n_chunks >= 96;
+        const int ch = wide ? 64 : 32;
+        Kernel k_stream = nullptr;
+        int lanes = 4;
+        switch (per_lane) {
+            case 2: k_stream = wide ? selective_scan_stream_kernel<2, 4, 64> : selective_scan_stream_kernel<2, 4, 32>; break;
+            case 4: k_stream = wide ? selective_scan_stream_kernel<4, 4, 64> : selective_scan_stream_kernel<2, 8, 32>; lanes = wide ? 4 : 8; break;
+            case 6: k_stream = wide ? selective_scan_stream_kernel<6, 4, 64> : selective_scan_stream_kernel<6, 4, 32>; break;
+            case 8: k_stream = wide ? selective_scan_stream_kernel<8, 4, 64> : selective_scan_stream_kernel<4, 8, 32>; lanes = wide ? 4 : 8; break;
+        }
+        const int ctas = (inner + ch - 1) / ch;
+        // One CTA per SM where there are enough SMs: launched while the kernel before still holds some, two would share the first ones that come
+        // free and take twice as long beside idle ones.
+        const size_t need = size_t(kStreamSlots) * stream_slot_floats(ch, n_pad) * sizeof(float), bytes = one_per_sm((long long)ctas * plan->n_chunks) ? std::max(need, kHalfSm) : need;
+        INGOT_CUDA_TRY(cudaFuncSetAttribute(k_stream, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
+        INGOT_CUDA_TRY(ingot_launch_pdl(k_stream, dim3(ctas, plan->n_chunks), dim3(ch * lanes + kStreamHelpers), bytes, s, p));
+        return INGOT_OK;
     }
     INGOT_CUDA_TRY(ingot_launch_pdl(k_out, grid, dim3(128), smem, s, p));
     return INGOT_OK;

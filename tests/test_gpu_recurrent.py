@@ -166,6 +166,38 @@ def test_gated_lru(width, block, cut, exact):
         assert np.abs(g - e).max() < 2e-5
 
 
+@pytest.mark.parametrize("inner,n_state", [(96, 16), (100, 8), (68, 24), (36, 32), (6144, 3), (6148, 16), (6144, 20), (6144, 32)])
+@pytest.mark.parametrize("lens,run", [([65, 64, 3], 10 ** 9), ([160, 81], 10 ** 9), ([131], 48)])
+def test_selective_scan_of_long_chunks(inner, n_state, lens, run):
+    """The scan as a stream: both widths of a CTA and every number of states per lane, tiles with a rest, chunks that go on from one another, a second
+    portion from the first one's state."""
+    import torch
+    rng = np.random.default_rng(inner + n_state)
+    pad, n = lib().ingot_scan_state_pad(n_state), len(lens)
+    A = -np.exp(rng.uniform(-3, 2, (inner, n_state)))
+    D, bias = rng.standard_normal(inner), rng.uniform(-4, -1, inner)
+    total = [2 * m for m in lens]
+    x, raw, z = ([rng.standard_normal((m, inner)) for m in total] for _ in range(3))
+    B, Cm = ([rng.standard_normal((m, n_state)) for m in total] for _ in range(2))
+    want = [R.selective_scan(x[i], R.softplus(raw[i] + bias), A, B[i], Cm[i], D) * R.silu(z[i]) for i in range(n)]
+    a2 = np.zeros((inner, pad))
+    a2[:, :n_state] = A * np.log2(np.e)
+    a2d, dd, bd = dev(a2), dev(D), dev(bias)
+    state = torch.full((n, inner, pad), float("nan"), device="cuda")
+    for begin in (0, 1):
+        st = Step(lens, [begin * m for m in lens], list(range(n)))
+        take = lambda a: np.concatenate([a[i][begin * m:(begin + 1) * m] for i, m in enumerate(lens)])
+        bc = np.zeros((st.n_tok, 2 * pad))
+        bc[:, :n_state], bc[:, pad:pad + n_state] = take(B), take(Cm)
+        xd, td, zd, bcd = dev(take(x)), dev(take(raw)), dev(take(z)), dev(bc)
+        out = torch.full((st.n_tok, inner), float("nan"), device="cuda")
+        o, pl = act_out(out), plan(lens, run, inner * (pad + 1))
+        lib(lib().ingot_selective_scan(C.byref(st.c), C.byref(pl.c), xd.data_ptr(), inner, td.data_ptr(), inner, bd.data_ptr(), bcd.data_ptr(), 2 * pad, 0, pad, zd.data_ptr(), inner,
+                                       a2d.data_ptr(), dd.data_ptr(), state.data_ptr(), inner, n_state, 0, C.byref(o), None))
+        w = take(want)
+        assert np.abs(out.cpu().numpy() - w).max() < 3e-5 * max(1.0, np.abs(w).max())
+
+
 def test_long_memory_does_not_drift():
     """A channel that hardly decays, fed one token at a time: the exact forms stay within rounding of float64."""
     import torch
