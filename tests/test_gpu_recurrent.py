@@ -198,6 +198,31 @@ def test_selective_scan_of_long_chunks(inner, n_state, lens, run):
         assert np.abs(out.cpu().numpy() - w).max() < 3e-5 * max(1.0, np.abs(w).max())
 
 
+@pytest.mark.parametrize("width,block", [(32, 32), (100, 20), (257, 257)])
+@pytest.mark.parametrize("lens", [[65, 64, 1], [128, 127, 129], [300]])
+def test_gated_lru_of_whole_sequences(width, block, lens):
+    """The unit as a stream: tiles and the warps' shares of them with a rest, channels past a CTA's, a second portion from the first one's state."""
+    import torch
+    rng = np.random.default_rng(width)
+    n, total = len(lens), [2 * m for m in lens]
+    br, bi, yb = (rng.standard_normal(width) for _ in range(3))
+    lam = rng.uniform(-6, 1, width)
+    u, gr, gi, y = ([rng.standard_normal((m, width)) for m in total] for _ in range(4))
+    want = [0.75 * R.gated_lru_scan(u[i], R.sigmoid(gr[i] + br), R.sigmoid(gi[i] + bi), lam) * R.gelu_tanh(y[i] + yb) for i in range(n)]
+    dv = [dev(v) for v in (br, bi, R.softplus(lam), yb)]
+    state = torch.full((n, width), float("nan"), device="cuda")
+    for begin in (0, 1):
+        st = Step(lens, [begin * m for m in lens], list(range(n)))
+        take = lambda a: np.concatenate([a[i][begin * m:(begin + 1) * m] for i, m in enumerate(lens)])
+        g = np.stack([take(gr).reshape(st.n_tok, -1, block), take(gi).reshape(st.n_tok, -1, block)], axis=2).reshape(st.n_tok, 2 * width)
+        ud, gd, yd = dev(take(u)), dev(g), dev(take(y))
+        out = torch.full((st.n_tok, width), float("nan"), device="cuda")
+        o, pl = act_out(out), plan(lens, 10 ** 9, 2 * width)
+        lib(lib().ingot_gated_lru(C.byref(st.c), C.byref(pl.c), ud.data_ptr(), width, gd.data_ptr(), 2 * width, block, dv[0].data_ptr(), dv[1].data_ptr(), dv[2].data_ptr(),
+                                  yd.data_ptr(), width, dv[3].data_ptr(), state.data_ptr(), width, 0.75, 0, C.byref(o), None))
+        assert np.abs(out.cpu().numpy() - take(want)).max() < 2e-5
+
+
 def test_long_memory_does_not_drift():
     """A channel that hardly decays, fed one token at a time: the exact forms stay within rounding of float64."""
     import torch
