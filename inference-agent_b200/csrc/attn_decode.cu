@@ -61,6 +61,21 @@ constexpr int kMaxDecodeWarps = 8;
 constexpr int kMaxParts = 64;
 constexpr int kClusterKeys = 8192;
 
+// Four neighbouring values of a merged row.
+__device__ __forceinline__ void store_merged(const DecodeParams& p, size_t e, float4 acc, float L) {
+    const float inv = L > 0.f ? 1.0f / L : 0.f;
+    if (p.out_dtype == INGOT_F32 && reinterpret_cast<uintptr_t>(p.c_out) % 16 == 0) {  // whole lines: the output may be in host memory
+        *reinterpret_cast<float4*>(static_cast<float*>(p.c_out) + e) = make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv);
+        return;
+    }
+    store_out(p.c_out, p.out_dtype, e + 0, acc.x * inv);
+    store_out(p.c_out, p.out_dtype, e + 1, acc.y * inv);
+    store_out(p.c_out, p.out_dtype, e + 2, acc.z * inv);
+    store_out(p.c_out, p.out_dtype, e + 3, acc.w * inv);
+}
+
+constexpr int kFewParts = 8;
+
 // Merges the splits of one (sequence, kv head): out = sum_s o_s 2^(m_s-M) / sum_s l_s 2^(m_s-M)
 // (the attn_combine formula, shaders/kernels.metal:502-516). Runs in one extra CTA per (kv head,
 // sequence) of the launch that FOLLOWS the one that wrote the partials (or of a merge-only launch):
@@ -90,6 +105,34 @@ __device__ __forceinline__ void combine_splits(const DecodeParams& p, float* sme
         !INGOT_CHECK(out0 + ((size_t)seq * p.n_head + (size_t)kvh * G) * kHeadDim, (size_t)G * kHeadDim, p.out_extent, p.status))
         return;
     const float* base = p.c_part + part0 + (((size_t)seq * p.n_parts_max) * p.n_head + (size_t)kvh * G) * kPartStride;
+    if (n_chunks <= kFewParts) {
+        // Few splits: a thread holds four columns of all of them, one round trip and no exchange: 28 layers of
+        // 4096 keys 84.8 -> 82.7 us, 64 paged sequences 203.8 -> 200.5 (B200).
+        for (int pr = threadIdx.x; pr < G * 32; pr += blockDim.x) {
+            const int gi = pr >> 5, cl = pr & 31;
+            const float* row = base + (size_t)gi * kPartStride;
+            float2 ml[kFewParts];
+            float4 o[kFewParts];
+#pragma unroll
+            for (int c = 0; c < kFewParts; c++) {
+                const bool on = c < n_chunks;
+                ml[c] = on ? __ldcg(reinterpret_cast<const float2*>(row + c * step + 128)) : make_float2(-INFINITY, 0.f);
+                o[c] = on ? __ldcg(reinterpret_cast<const float4*>(row + c * step + cl * 4)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+            float M = ml[0].x, L = 0.f;
+#pragma unroll
+            for (int c = 1; c < kFewParts; c++) M = fmaxf(M, ml[c].x);
+            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int c = 0; c < kFewParts; c++) {
+                const float w = exp2f(ml[c].x - M);
+                L += ml[c].y * w;
+                acc.x += o[c].x * w; acc.y += o[c].y * w; acc.z += o[c].z * w; acc.w += o[c].w * w;
+            }
+            store_merged(p, out0 + ((size_t)seq * p.n_head + (size_t)kvh * G + gi) * kHeadDim + cl * 4, acc, L);
+        }
+        return;
+    }
     const float* my_rows = base + (size_t)gi_t * kPartStride + col * 4;
 
     float* mg_m = smem;                       // [G][kMaxParts] split maxima, then weights
@@ -178,16 +221,7 @@ __device__ __forceinline__ void combine_splits(const DecodeParams& p, float* sme
             const float4 x = reinterpret_cast<const float4*>(mg_acc)[sl_i * pairs + pr];
             acc.x += x.x; acc.y += x.y; acc.z += x.z; acc.w += x.w;
         }
-        const float inv = L > 0.f ? 1.0f / L : 0.f;
-        const size_t e = out0 + ((size_t)seq * p.n_head + (size_t)kvh * G + gi) * kHeadDim + cl * 4;
-        if (p.out_dtype == INGOT_F32 && reinterpret_cast<uintptr_t>(p.c_out) % 16 == 0) {  // whole lines: the output may be in host memory
-            *reinterpret_cast<float4*>(static_cast<float*>(p.c_out) + e) = make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv);
-            continue;
-        }
-        store_out(p.c_out, p.out_dtype, e + 0, acc.x * inv);
-        store_out(p.c_out, p.out_dtype, e + 1, acc.y * inv);
-        store_out(p.c_out, p.out_dtype, e + 2, acc.z * inv);
-        store_out(p.c_out, p.out_dtype, e + 3, acc.w * inv);
+        store_merged(p, out0 + ((size_t)seq * p.n_head + (size_t)kvh * G + gi) * kHeadDim + cl * 4, acc, L);
     }
 }
 

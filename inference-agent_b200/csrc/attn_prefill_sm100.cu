@@ -75,7 +75,7 @@ struct Bars {
     uint32_t abort_flag;
 };
 
-constexpr int kMaxOutputs = 8;
+constexpr int kMaxOutputs = 8, kMaxPrefillSplits = 8;
 
 struct Sm100Params {
     const void* q;
@@ -645,15 +645,26 @@ __global__ void __launch_bounds__(256) prefill_merge_kernel(const float* __restr
     const int kvh = int(w / n_rows), R = int(w % n_rows);
     const size_t split_stride = (size_t)n_kvh * n_rows * kPartStride;
     const float* row = part + ((size_t)kvh * n_rows + R) * kPartStride;
+    float2 ml[kMaxPrefillSplits];  // all of them requested together: 512 tokens onto 3584 44.9 -> 41.8 us with append and attention (B200)
+    float4 o[kMaxPrefillSplits];
+#pragma unroll
+    for (int s = 0; s < kMaxPrefillSplits; s++) {
+        if (s >= n_split) break;
+        ml[s] = *reinterpret_cast<const float2*>(row + s * split_stride + 128);
+        o[s] = *reinterpret_cast<const float4*>(row + s * split_stride + lane * 4);
+    }
     float M = -INFINITY;
-    for (int s = 0; s < n_split; s++) M = fmaxf(M, row[s * split_stride + 128]);
+#pragma unroll
+    for (int s = 0; s < kMaxPrefillSplits; s++)
+        if (s < n_split) M = fmaxf(M, ml[s].x);
     float L = 0.f;
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int s = 0; s < n_split; s++) {
-        const float wgt = ex2(row[s * split_stride + 128] - M);  // an empty partial has m = -inf: weight 0
-        L += row[s * split_stride + 129] * wgt;
-        const float4 o = *reinterpret_cast<const float4*>(row + s * split_stride + lane * 4);
-        acc.x += o.x * wgt; acc.y += o.y * wgt; acc.z += o.z * wgt; acc.w += o.w * wgt;
+#pragma unroll
+    for (int s = 0; s < kMaxPrefillSplits; s++) {
+        if (s >= n_split) break;
+        const float wgt = ex2(ml[s].x - M);  // an empty partial has m = -inf: weight 0
+        L += ml[s].y * wgt;
+        acc.x += o[s].x * wgt; acc.y += o[s].y * wgt; acc.z += o[s].z * wgt; acc.w += o[s].w * wgt;
     }
     const float inv = 1.0f / L;
     const size_t e = ((size_t)(R / G) * out_n_head + out_head0 + kvh * G + R % G) * kHeadDim + lane * 4;
@@ -806,7 +817,7 @@ int launch_attn_prefill_sm100(ingot_kv* kv, int layer, const void* q, int q_dtyp
     const int row_ctas = int(row_tiles) * kv->n_head_kv;
     const int kv_tiles_last = (q_pos0 + n_tok + kTileKeys - 1) / kTileKeys;
     int n_split = 1;
-    if (n_outs == 1 && !signals && row_ctas * 2 <= kv->num_sms) n_split = std::max(1, std::min({kv->num_sms / row_ctas, 8, kv_tiles_last / 2}));
+    if (n_outs == 1 && !signals && row_ctas * 2 <= kv->num_sms) n_split = std::max(1, std::min({kv->num_sms / row_ctas, kMaxPrefillSplits, kv_tiles_last / 2}));
     p.n_split = n_split;
     p.part = nullptr;
     if (n_split > 1) {
