@@ -395,7 +395,7 @@ __global__ void __launch_bounds__(128) selective_scan_kernel(const ScanParams p)
     }
 }
 
-// ---- selective scan of long chunks: the output pass as a stream --------------------------------------------------------
+// ---- selective scan of whole sequences, as a stream --------------------------------------------------------------------
 // The tile kernel above does its phases one after the other (stage, step sizes, tokens, gates), so that one chunk per sequence left it waiting
 // between them (2048 tokens, 8192 channels: 799 us). Here one half of a CTA does nothing but the recurrence and the other everything around it; a chunk as long as
 // the sequence keeps the units busy, and the passes that find the chunks' start states fall away. kLanes lanes share a channel, each with kS
@@ -424,11 +424,9 @@ __global__ void __launch_bounds__(kNch * kLanes + kStreamHelpers) selective_scan
     constexpr int kSlot = stream_slot_floats(kNch, kNp), kDt = kScanTile * kNch, kZ = 2 * kDt, kDtx = 3 * kDt, kY = 4 * kDt, kB = 5 * kDt, kC = kB + kScanTile * kNp;
     INGOT_PDL_TRIGGER();
     INGOT_PDL_WAIT();
-    const int chunk = blockIdx.y;
-    const int seq = p.chunk_seq[chunk], t0 = p.chunk_t0[chunk], len = p.chunk_len[chunk];
-    const bool first = t0 == 0, last = t0 + len == p.st.len[seq];
+    const int chunk = blockIdx.y, seq = p.chunk_seq[chunk], len = p.chunk_len[chunk];
     const int c_base = blockIdx.x * kNch, n_tiles = (len + kScanTile - 1) / kScanTile;
-    const size_t row0 = (size_t)p.st.row_start[seq] + t0;
+    const size_t row0 = (size_t)p.st.row_start[seq];
 
     if (threadIdx.x >= kScanners) {
         // ---------------- helpers ----------------
@@ -510,10 +508,7 @@ __global__ void __launch_bounds__(kNch * kLanes + kStreamHelpers) selective_scan
     const size_t sidx = (size_t)(live ? c : 0) * kNp + part * kS;
     const size_t slot_base = (size_t)p.st.slot[seq] * p.inner * kNp;
     {
-        // start state: as in the tile kernel
-        const float* from = nullptr;
-        if (!(first && last)) from = p.part + (size_t)chunk * p.inner * kNp + sidx;
-        else if (p.st.pos0[seq] > 0) from = p.state + slot_base + sidx;
+        const float* from = p.st.pos0[seq] > 0 ? p.state + slot_base + sidx : nullptr;
 #pragma unroll
         for (int i = 0; i < kS / 2; i++) {
             a[i] = live ? *reinterpret_cast<const f32x2*>(p.a2 + sidx + 2 * i) : 0;
@@ -597,7 +592,7 @@ __global__ void __launch_bounds__(kNch * kLanes + kStreamHelpers) selective_scan
             s[i] = fma2(pair(ex2f(x.x), ex2f(x.y)), begin[i], local[i]);
         }
     }
-    if (live && last) {
+    if (live) {
 #pragma unroll
         for (int i = 0; i < kS / 2; i++) *reinterpret_cast<f32x2*>(p.state + slot_base + sidx + 2 * i) = s[i];
     }
@@ -704,7 +699,7 @@ __global__ void __launch_bounds__(128) gated_lru_kernel(const LruParams p) {
     }
 }
 
-// The output pass of long chunks in one go: a warp takes 8 tokens of a tile of 128 for 32 channels, computes their decays and inputs once, and
+// Whole sequences in one go: a warp takes 8 tokens of a tile of 128 for 32 channels, computes their decays and inputs once, and
 // keeps them. It runs them from zero, the warps hand each other end states and decays, and every warp runs its tokens again from where
 // they start: two multiply-adds per token instead of the sigmoids, exponentials and loads of a pass of its own, so that chunks as long as
 // the sequence need no pass for their start states. The next tile's rows are requested before the current tile's states.
@@ -720,14 +715,12 @@ __global__ void __launch_bounds__(kLruWarps * 32) gated_lru_stream_kernel(const 
     const float br = p.br[c], bi = p.bi[c], k = -8.0f * p.sp[c], yb = p.y_bias[c];
     INGOT_PDL_WAIT();
     const int chunk = blockIdx.y;
-    const int seq = p.chunk_seq[chunk], t0 = p.chunk_t0[chunk], len = p.chunk_len[chunk];
-    const bool first = t0 == 0, last = t0 + len == p.st.len[seq];
-    const size_t row0 = (size_t)p.st.row_start[seq] + t0;
+    const int seq = p.chunk_seq[chunk], len = p.chunk_len[chunk];
+    const size_t row0 = (size_t)p.st.row_start[seq];
     const int gcol = (c / p.block) * 2 * p.block + c % p.block;
     float* slot = p.state + (size_t)p.st.slot[seq] * p.width + c;
     float s = 0.f;  // at the start of the tile, the same in every warp
-    if (!(first && last)) s = p.part[(size_t)chunk * p.width + c];
-    else if (p.st.pos0[seq] > 0) s = *slot;
+    if (p.st.pos0[seq] > 0) s = *slot;
     const float* u = p.u + row0 * p.u_ld + c;
     const float* g = p.gates + row0 * p.gates_ld + gcol;
     const float* y = p.y + row0 * p.y_ld + c;
@@ -774,7 +767,7 @@ __global__ void __launch_bounds__(kLruWarps * 32) gated_lru_stream_kernel(const 
             if (i < n && on) p.out.store(row0 + tb + i, c, p.out_scale * mine * out[i]);
         }
     }
-    if (on && last && warp == 0) *slot = s;
+    if (on && warp == 0) *slot = s;
 }
 
 __global__ void __launch_bounds__(128) gated_lru_link_kernel(const LruParams p) {
@@ -899,8 +892,8 @@ int ingot_selective_scan(const ingot_step* step, const ingot_scan_plan* plan, co
         INGOT_CUDA_TRY(ingot_launch_pdl(k_end, grid, dim3(128), smem, s, p));
         INGOT_CUDA_TRY(ingot_launch_pdl(selective_scan_link_kernel, dim3(unsigned(((size_t)inner * n_pad + 255) / 256), step->n_seq), dim3(256), 0, s, p));
     }
-    // The output pass of long chunks as a stream; the tile kernel for the exact form, more than 32 states, and chunks too short to fill a ring.
-    if (!exact && lg == 2 && step->max_len > kStreamFrom) {
+    // Whole sequences as a stream; the tile kernel for the exact form, more than 32 states, chunks, and steps too short to fill a ring.
+    if (!exact && lg == 2 && !multi && step->max_len > kStreamFrom) {
         // 64 channels per CTA, or 32 with more lanes each where that would leave SMs without a CTA
         const bool wide = (long long)((inner + 63) / 64) * plan->n_chunks >= 96;
         const int ch = wide ? 64 : 32;
