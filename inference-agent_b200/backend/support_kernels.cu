@@ -428,6 +428,13 @@ __global__ void __launch_bounds__(StreamThreads<kFmt, kLoads>::value) gemv_strea
     int r = gw, st = 0;
     bool have = r < total_rows;
     if (have) issue(cur_a, cur_b, cs_a, cs_b, r, 0);  // before the wait below: weights do not depend on the preceding kernel
+    // A row per warp: the second step too, while the small kernels before a product hardly touch memory. 2048 x 4096 inside a step 6.9 -> 4.8 us
+    // (B200). Warps of the other forms go through several rows; with two steps out that early they took longer (8192 x 2048 8.8 -> 10.6 us).
+    bool asked = false;
+    if (kLoads == 8 && have && steps > 1) {
+        issue(nxt_a, nxt_b, ns_a, ns_b, r, 1);
+        asked = true;
+    }
 
     if (use_pdl) asm volatile("griddepcontrol.wait;" ::: "memory");
     float ss = 0.f;
@@ -459,7 +466,8 @@ __global__ void __launch_bounds__(StreamThreads<kFmt, kLoads>::value) gemv_strea
         int r2 = r, st2 = st + 1;
         if (st2 == steps) { st2 = 0; r2 = r + W; }
         const bool have2 = r2 < total_rows;
-        if (have2) issue(nxt_a, nxt_b, ns_a, ns_b, r2, st2);
+        if (have2 && !asked) issue(nxt_a, nxt_b, ns_a, ns_b, r2, st2);
+        asked = false;
 #pragma unroll
         for (int h = 0; h < kPer; h++) {
             const int c = st * kPer + h;

@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(256) linear_scan_link_kernel(const LinearParam
     auto at = [&](int k) { return reinterpret_cast<float4*>(part + k * stride); };
     float4 s = p.st.pos0[seq] > 0 ? *reinterpret_cast<const float4*>(p.state + p.slot_at(seq, h) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
     const int n = k1 - k0 - 1;  // chunks that leave an end state
-    constexpr int kAhead = 4;   // of which so many are requested together
+    constexpr int kAhead = 16;  // of which so many are requested together
     for (int kb = 0; kb < n; kb += kAhead) {
         float4 e[kAhead];
         float f[kAhead];
