@@ -606,7 +606,9 @@ __global__ void deliver_kernel(float* const* dst_at, const float* src, int src_l
 // The beginning of a step: its metadata, from pinned host memory, read by the SMs, so that a captured step holds all its work and is one call.
 // With the delivery also inside the graph, and the logits of several rows written by their product, decoding steps of models with
 // four layers take (B200, wall clock of the step call) 202.5 -> 196.5 us with one sequence, 349 -> 328 with eight, 586 -> 580 with four and experts.
-// Nothing starts before this is over: the kernels of a step read their metadata ahead of the wait for the kernel before them.
+// The launch that follows must be an ordinary one (ingot_support_embed_rows_bf16 and ingot_support_embed_sum_bf16 are): later kernels of a step read the
+// metadata ahead of their wait for the kernel before them. Without an early trigger here a programmatic launch would still start only when these CTAs
+// are through, but what they wrote is certain to be seen after a griddepcontrol.wait alone.
 __global__ void __launch_bounds__(256) fetch_kernel(uint4* dst, const uint4* src, int n) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -630,11 +632,10 @@ __global__ void embed_rows_kernel(float* out, const W* __restrict__ table, int n
 }
 
 // The same of a bf16 table whose rows are whole 16-byte pieces, eight values per load: a prompt's rows are bound by writing them, a single
-// row by one trip to memory instead of one per 256 values (8 rows of 2048 inside a decoding step 5.8 -> 2.3 us, B200).
+// row by one trip to memory instead of one per 256 values. An ordinary launch: see fetch_kernel.
 __global__ void __launch_bounds__(256) embed_rows8_kernel(float* out, const __nv_bfloat16* __restrict__ table, int n_in, int n_rows_table, const int32_t* __restrict__ rows,
                                                           int* status, float scale) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
     const int row = rows[blockIdx.x];
     const bool ok = row >= 0 && row < n_rows_table;
     if (!ok && threadIdx.x == 0 && status) atomicOr(status, 1);
@@ -885,9 +886,9 @@ cudaError_t ingot_support_linear_bf16(float* out, const void* w, const float* x,
 cudaError_t ingot_support_embed_rows_bf16(float* out, const void* table, int n_in, int n_rows_table, const int32_t* rows_dev, int n_rows,
                                           float scale, int* status_dev, cudaStream_t s) {
     if (n_rows < 1 || n_in < 1) return cudaErrorInvalidValue;
-    if (n_in % 8 == 0 && (reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(table)) % 16 == 0)
-        return support_launch(embed_rows8_kernel, dim3(n_rows), dim3(256), 0, s, out, static_cast<const __nv_bfloat16*>(table), n_in, n_rows_table, rows_dev, status_dev, scale);
-    embed_rows_kernel<__nv_bfloat16><<<n_rows, 256, 0, s>>>(out, static_cast<const __nv_bfloat16*>(table), n_in, n_rows_table, rows_dev, status_dev, scale);
+    const bool pieces = n_in % 8 == 0 && (reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(table)) % 16 == 0;
+    auto kernel = pieces ? embed_rows8_kernel : embed_rows_kernel<__nv_bfloat16>;
+    kernel<<<n_rows, 256, 0, s>>>(out, static_cast<const __nv_bfloat16*>(table), n_in, n_rows_table, rows_dev, status_dev, scale);
     return cudaGetLastError();
 }
 
