@@ -372,7 +372,7 @@ struct StreamThreads { static constexpr int value = !FmtTraits<kFmt>::kPlain ? 2
 template <bool kNorm, bool kSwiGLU, int kLoads, int kFmt>
 __global__ void __launch_bounds__(StreamThreads<kFmt, kLoads>::value) gemv_stream_kernel(const GemvGroup g, const float* x, const float* norm_w, float eps, int n_in,
                                                           int total_rows, int accumulate, int use_pdl, int n_mean, int act) {
-    extern __shared__ float xs[];  // x', n_in floats
+    extern __shared__ __align__(16) float xs[];  // x', n_in floats
     __shared__ float red[25];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // Rows go round-robin over all warps of the grid, warp-major (warp w of CTA b is number w * gridDim.x + b): when the

@@ -239,7 +239,7 @@ __host__ __device__ constexpr int cluster_share(int n_keys, int n_parts) {
 // kCluster: the splits of a range are the CTAs of a cluster, and its first CTA merges them in shared memory.
 template <bool kCluster>
 __global__ void __launch_bounds__(kMaxDecodeWarps * 32, 1) DECODE_KERNEL(const DECODE_PARAMS p) {
-    extern __shared__ float smem[];
+    extern __shared__ __align__(16) float smem[];
     // Programmatic dependent launch: let the next kernel in the stream start as soon as SM resources allow, and
     // wait for the kernel before this one according to p.pdl_mode (see DecodeParams).
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -306,7 +306,7 @@ template <int kMax, bool kCluster>
 __global__ void __launch_bounds__(kWarps * 32) gqa_mma_kernel(const AttendParams p, int share_pages) {
     constexpr int kK = kMax / 16, kN = kMax / 8;
     extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ float s_ml[kCluster ? 16 : 1][2];
+    __shared__ float2 s_ml[kCluster ? 16 : 1];  // of each row: maximum, sum
     __shared__ uint64_t s_full[kWarps][kMaxRing];
     __shared__ uint32_t s_abort;
     INGOT_PDL_TRIGGER();
@@ -496,7 +496,7 @@ __global__ void __launch_bounds__(kWarps * 32) gqa_mma_kernel(const AttendParams
         }
         if (kCluster) {  // stays here: only this thread has read the place of warp 0
             *reinterpret_cast<float2*>(so + r * dv + d) = make_float2(x, y);
-            if (d == 0) { s_ml[r][0] = m; s_ml[r][1] = l; }
+            if (d == 0) s_ml[r] = make_float2(m, l);
         } else if (p.n_splits == 1) {
             const float inv = 1.0f / l;
             p.out.store2(row, h * dv + d, x * inv * p.gate.at(row, h, dv, d), y * inv * p.gate.at(row, h, dv, d + 1));
@@ -509,7 +509,7 @@ __global__ void __launch_bounds__(kWarps * 32) gqa_mma_kernel(const AttendParams
     if (kCluster) {
         cluster_sync();
         // as gqa_merge_kernel does it
-        const uint32_t my_o = smem_u32(so), my_ml = smem_u32(&s_ml[0][0]);
+        const uint32_t my_o = smem_u32(so), my_ml = smem_u32(s_ml);
         for (int i = (split * kWarps * 32 + (int)threadIdx.x) * 2; i < rows_here * dv; i += p.n_splits * kWarps * 64) {
             const int r = i / dv, d = i - r * dv, h = kvh * group + (row0 + r) % group;
             const size_t row = tok0 + (row0 + r) / group;
