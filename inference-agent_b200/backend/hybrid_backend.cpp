@@ -314,11 +314,6 @@ private:
             }
     }
 
-    // A streamed scan takes time by the tokens of the longest sequence, chunks by tokens times channels: whole sequences from this many
-    // channels on (times the sequences of the longest one's length that the step holds). 4096 channels, one sequence (B200): 250 tokens 33 us in
-    // chunks, 18 whole, 1024: 65 and 61, 4000: 223 and 217-224; with 2048 channels chunks would take half of that and whole sequences as long.
-    static constexpr int kStreamChannels = 3072;
-
     // INGOT_SCAN_THREADS: threads per SM the chunks of a recurrence aim for (tuning).
     // Length of the time chunks of a recurrence one token-chunk of which occupies `threads` threads: as few chunks as fill the GPU.
     // Longer ones if the sequences' ends would make it more chunks than that (a second round of CTAs).
@@ -381,9 +376,9 @@ private:
         lens_sorted_.assign(m.begin() + long(o_len), m.begin() + long(o_len) + n);
         step.first_want = step.n_want ? m[o_want] : 0;
         struct PlanAt { size_t seq, t0, len, first; int n_chunks, max_chunks; };
-        auto plan = [&](int threads, int streamed) {
+        auto plan = [&](int threads) {
             PlanAt p = {};
-            const int L = streamed > 0 && (long long)step.max_len * kStreamChannels <= (long long)step.n_tok * streamed ? step.max_len : chunk_tokens(entries, step.n_tok, threads);
+            const int L = chunk_tokens(entries, step.n_tok, threads);
             std::vector<int32_t> seq, t0, len, first;
             for (int i = 0; i < n; i++) {
                 first.push_back(int32_t(seq.size()));
@@ -403,7 +398,7 @@ private:
             return p;
         };
         std::vector<PlanAt> plans;
-        for (const auto& request : ops_.plans()) plans.push_back(plan(request.threads, request.streamed));
+        for (const auto& request : ops_.plans()) plans.push_back(plan(request.threads));
         struct TableAt { size_t first, table, key0, key_pos; };
         std::vector<TableAt> table_at;
         for (auto& g : ops_.caches) {

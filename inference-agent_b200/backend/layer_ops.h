@@ -552,16 +552,15 @@ public:
         return g;
     }
     // Time chunks for a recurrence: threads that one chunk occupies (they size the chunks of a step), floats of scratch that it needs. The
-    // number of the plan in StepCtx::plans; mixers of equal threads share one. streamed: channels of a selective scan whose output pass
-    // runs as a stream (0: none), so that sequences may stay whole.
-    struct PlanRequest { int threads; size_t scratch; int streamed; };
-    size_t scan_plan(int threads, size_t scratch, int streamed = 0) {
+    // number of the plan in StepCtx::plans; mixers of equal threads share one.
+    struct PlanRequest { int threads; size_t scratch; };
+    size_t scan_plan(int threads, size_t scratch) {
         for (size_t i = 0; i < plans_.size(); i++)
-            if (plans_[i].threads == threads && plans_[i].streamed == streamed) {
+            if (plans_[i].threads == threads) {
                 plans_[i].scratch = std::max(plans_[i].scratch, scratch);
                 return i;
             }
-        plans_.push_back({threads, scratch, streamed});
+        plans_.push_back({threads, scratch});
         return plans_.size() - 1;
     }
     const std::vector<PlanRequest>& plans() const { return plans_; }

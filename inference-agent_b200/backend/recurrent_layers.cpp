@@ -39,7 +39,7 @@ public:
         w_o_ = ops.matrix(p + "o", flat(d), in);
         conv_state_ = ops.state(size_t(taps_ - 1) * ip_);
         state_ = ops.state(size_t(ip_) * np_);
-        plan_ = ops.scan_plan(ip_ * 2, size_t(ip_) * (np_ + 1), !ops.opt.f32 && states_ <= 32 ? ip_ : 0);
+        plan_ = ops.scan_plan(ip_ * 2, size_t(ip_) * (np_ + 1));
         ops.need(kProj, 2 * ip_);
         ops.need(kConv, ip_);
         ops.need(kStateIn, rank_p_ + 2 * np_);
@@ -130,7 +130,7 @@ public:
         w_o_ = ops.matrix(in.padded, mix_ld_, {Part{L + "o", {d, q.count()}, in, heads_out, 0, 0}, Part{R + "o", {d, width_}, in, w, 0, attn_cols_}});
         conv_state_ = ops.state(size_t(taps_ - 1) * wp_);
         state_ = ops.state(size_t(wp_));
-        plan_ = ops.scan_plan(wp_, 2 * size_t(wp_), ops.opt.f32 ? 0 : wp_);
+        plan_ = ops.scan_plan(wp_, 2 * size_t(wp_));
         ops.need(kProj, proj_ld_);
         ops.need(kConv, wp_);
         ops.need(kGates, 2 * wp_);

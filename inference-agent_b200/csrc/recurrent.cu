@@ -13,6 +13,8 @@
 //   pass 2  one thread per state element walks a sequence's chunks in order and turns end states into start states;
 //   pass 3  every chunk runs again from its start state and writes the outputs; the last chunk writes the slot.
 // A sequence that is a single chunk (every decoded token) takes pass 3 alone, straight from and to its slot.
+// Where the sequences themselves fill the GPU one launch does all three (the stream kernels), to the same bits: which launches a call takes is
+// a matter of time alone.
 //
 // Decays. A slow channel multiplies its state by a = exp(x), x near 0, at every token, so an error of a that is always of
 // the same sign adds up over the memory of the channel (the 2^x unit is good to about 2^-22). Where that matters - the gated
@@ -395,51 +397,64 @@ __global__ void __launch_bounds__(128) selective_scan_kernel(const ScanParams p)
     }
 }
 
-// ---- selective scan of whole sequences, as a stream --------------------------------------------------------------------
-// The tile kernel above does its phases one after the other (stage, step sizes, tokens, gates), so that one chunk per sequence left it waiting
-// between them (2048 tokens, 8192 channels: 799 us). Here one half of a CTA does nothing but the recurrence and the other everything around it; a chunk as long as
-// the sequence keeps the units busy, and the passes that find the chunks' start states fall away. kLanes lanes share a channel, each with kS
-// of its states; kNch channels per CTA.
-//   helpers   request tiles of 16 tokens three ahead (cp.async, a ring of kStreamSlots), turn dt into softplus(dt + bias) and dt x, and
+// ---- selective scan as a stream --------------------------------------------------------------------------------------
+// The three passes in one, to the same bits: a CTA walks a sequence's chunks one after the other. The tile kernel above does its phases one after the other
+// (stage, step sizes, tokens, gates) and waits between them, so a single chunk per sequence would leave the GPU idle (2048 tokens, 8192 channels: 433 us). Here one
+// half of a CTA does nothing but the recurrence and the other everything around it. Four lanes share a channel, each with kS of its states; kNch channels per CTA.
+//   helpers   request tiles of 16 tokens of a chunk three ahead (cp.async, a ring of kStreamSlots), turn dt into softplus(dt + bias) and dt x, and
 //             write (y + D x) silu(z) of the tile before last
-//   scanners  walk the tokens of the tile that is ready and leave y
+//   scanners  walk the tokens of the tile that is ready and leave y. Beside the state they keep what the chunk adds up to from zero, and its sum of dt:
+//             the next chunk begins with what pass 2 makes of those
 // Hand-over by named barriers: kBarReady + parity (helpers arrive, scanners wait), kBarDone + parity (the reverse).
 // What bounds it: instruction issue and shared memory next to the 2^x. 64 channels of 16 states take 165 cycles a token; 80 are the 2^x of scan,
-// softplus and gates at 16 per clock, about 85 the instructions, 110 the shared-memory cycles. A single warp of scanners per scheduler with
-// twice the channels does not overlap them (it issues in order), four with half the states each fetch B and C twice as often (195 us below).
-// All passes inside a prompt's step, against chunks (B200): 2048 tokens x 8192 channels 223 -> 179 us, 300 x 8192 46 -> 29, 1024 x 4096 65 -> 61, 250 x 4096
-// 33 -> 18, four sequences of 190 to 300 67 -> 49. Error against 64 bits, 2048 tokens: 8.6e-7 -> 2.8e-7 of the result (chunks of 240 before).
-constexpr int kStreamSlots = 6, kStreamHelpers = 256, kStreamFrom = 64;  // portions of more than kStreamFrom tokens
+// softplus and gates at 16 per clock, about 85 the instructions, 110 the shared-memory cycles. Eight lanes a channel with half the states each fetch B and C
+// twice as often (64 channels: 195 us below; 32: 59 us per 1000 tokens of 4096 channels, 55 with four), and sum y in another order than the tile kernel.
+// Against the passes over chunks (B200, calls replayed as a graph): 2048 tokens x 8192 channels 228 -> 178 us, 300 x 8192 44 -> 29, 1000 x 4096 63 -> 56,
+// 300 x 4096 32 -> 19.
+constexpr int kStreamSlots = 6, kStreamHelpers = 256;
 enum : int { kBarHelpers = 1, kBarReady = 2, kBarDone = 4 };  // + parity
 __device__ __forceinline__ void bar_arrive(int id, int n) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory"); }
 __device__ __forceinline__ void bar_wait(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
 // floats of a ring slot: x, dt, z, dt x, y of n_ch channels, B and C of np states
 __host__ __device__ constexpr int stream_slot_floats(int n_ch, int np) { return kScanTile * (5 * n_ch + 2 * np); }
 
-template <int kS, int kLanes, int kNch>
-__global__ void __launch_bounds__(kNch * kLanes + kStreamHelpers) selective_scan_stream_kernel(const ScanParams p) {
+// A channel's states lie in four lanes as in the tile kernel, so that its y is summed in the same order.
+template <int kS, int kNch>
+__global__ void __launch_bounds__(kNch * 4 + kStreamHelpers) selective_scan_stream_kernel(const ScanParams p) {
     extern __shared__ __align__(16) float smem[];
-    static_assert(kLanes == 4 || kLanes == 8, "exchanges below");
-    constexpr int kScanners = kNch * kLanes, kAll = kScanners + kStreamHelpers, kNp = kS * kLanes, kCh4 = kNch / 4, kNp4 = kNp / 4;
+    struct Tile { int t, n; bool links; };  // first token and number of tokens (0: past the end); another chunk begins behind it
+    __shared__ Tile s_tile[kStreamSlots];
+    constexpr int kLanes = 4, kScanners = kNch * kLanes, kAll = kScanners + kStreamHelpers, kNp = kS * kLanes, kCh4 = kNch / 4, kNp4 = kNp / 4;
     constexpr int kSlot = stream_slot_floats(kNch, kNp), kDt = kScanTile * kNch, kZ = 2 * kDt, kDtx = 3 * kDt, kY = 4 * kDt, kB = 5 * kDt, kC = kB + kScanTile * kNp;
     INGOT_PDL_TRIGGER();
     INGOT_PDL_WAIT();
-    const int chunk = blockIdx.y, seq = p.chunk_seq[chunk], len = p.chunk_len[chunk];
-    const int c_base = blockIdx.x * kNch, n_tiles = (len + kScanTile - 1) / kScanTile;
+    const int seq = blockIdx.y, k0 = p.seq_chunk0[seq], k1 = p.seq_chunk0[seq + 1];
+    if (k0 == k1) return;
+    const int c_base = blockIdx.x * kNch, seq_len = p.st.len[seq];
     const size_t row0 = (size_t)p.st.row_start[seq];
 
     if (threadIdx.x >= kScanners) {
         // ---------------- helpers ----------------
         const int tid = threadIdx.x - kScanners;
+        // of the tile that is staged next; the length of the chunk after its own is requested a chunk ahead
+        int chunk = k0, at = 0, left = min(p.chunk_len[k0], seq_len), next_len = k0 + 1 < k1 ? p.chunk_len[k0 + 1] : 0;
+        auto next_chunk = [&] {
+            while (left == 0 && chunk + 1 < k1) {
+                left = min(next_len, seq_len - at);
+                next_len = ++chunk + 1 < k1 ? p.chunk_len[chunk + 1] : 0;
+            }
+        };
+        next_chunk();
         auto stage = [&](int tile) {
-            if (tile < n_tiles) {
+            const int n = min(kScanTile, left);
+            if (tid == 0) s_tile[tile % kStreamSlots] = Tile{at, n, n == left && chunk + 1 < k1};
+            if (n > 0) {
                 float* s = smem + tile % kStreamSlots * kSlot;
-                const int t_base = tile * kScanTile;
 #pragma unroll
                 for (int i = tid; i < kScanTile * kCh4; i += kStreamHelpers) {
                     const int t = i / kCh4, q = (i - t * kCh4) * 4;
-                    const bool on = t_base + t < len && c_base + q < p.inner;
-                    const size_t row = row0 + min(t_base + t, len - 1);
+                    const bool on = t < n && c_base + q < p.inner;
+                    const size_t row = row0 + at + min(t, n - 1);
                     const int cc = min(c_base + q, p.inner - 4);
                     cp_async16(s + t * kNch + q, p.x + row * p.x_ld + cc, on);
                     cp_async16(s + kDt + t * kNch + q, p.dt + row * p.dt_ld + cc, on);
@@ -448,11 +463,14 @@ __global__ void __launch_bounds__(kNch * kLanes + kStreamHelpers) selective_scan
 #pragma unroll
                 for (int i = kStreamHelpers - 1 - tid; i < kScanTile * kNp4; i += kStreamHelpers) {
                     const int t = i / kNp4, q = (i - t * kNp4) * 4;
-                    const bool on = t_base + t < len;
-                    const size_t row = row0 + min(t_base + t, len - 1);
+                    const bool on = t < n;
+                    const size_t row = row0 + at + min(t, n - 1);
                     cp_async16(s + kB + t * kNp + q, p.bc + row * p.bc_ld + p.b_off + q, on);
                     cp_async16(s + kC + t * kNp + q, p.bc + row * p.bc_ld + p.c_off + q, on);
                 }
+                at += n;
+                left -= n;
+                next_chunk();
             }
             cp_async_commit();  // a group per tile, also past the end, so that the count of those in flight stays the same
         };
@@ -463,13 +481,13 @@ __global__ void __launch_bounds__(kNch * kLanes + kStreamHelpers) selective_scan
         const float4 my_d = my_live ? *reinterpret_cast<const float4*>(p.d + c_base + my_q) : zero4;
         auto finish = [&](int tile) {  // y of a tile is there
             const float* s = smem + tile % kStreamSlots * kSlot;
-            const int n_t = min(kScanTile, len - tile * kScanTile);
+            const Tile of = s_tile[tile % kStreamSlots];
             if (!my_live) return;
 #pragma unroll
             for (int i = tid; i < kScanTile * kCh4; i += kStreamHelpers) {
-                if (i >= n_t * kCh4) break;
+                if (i >= of.n * kCh4) break;
                 const float4 xv = reinterpret_cast<const float4*>(s)[i], yv = reinterpret_cast<const float4*>(s + kY)[i], zv = reinterpret_cast<const float4*>(s + kZ)[i];
-                p.out.store4(row0 + tile * kScanTile + i / kCh4, c_base + my_q,
+                p.out.store4(row0 + of.t + i / kCh4, c_base + my_q,
                              make_float4(fmaf(my_d.x, xv.x, yv.x) * fast_silu(zv.x), fmaf(my_d.y, xv.y, yv.y) * fast_silu(zv.y),
                                          fmaf(my_d.z, xv.z, yv.z) * fast_silu(zv.z), fmaf(my_d.w, xv.w, yv.w) * fast_silu(zv.w)));
             }
@@ -477,25 +495,29 @@ __global__ void __launch_bounds__(kNch * kLanes + kStreamHelpers) selective_scan
         stage(0);
         stage(1);
         stage(2);
-        for (int tile = 0; tile < n_tiles; tile++) {
+        int tile = 0;
+        for (bool more = true; more; tile++) {  // once past the end, which the scanners learn of in the same way
             if (tile >= 2) bar_wait(kBarDone + (tile & 1), kAll);  // tile - 2
             cp_async_wait<2>();  // all but the next two tiles'
             bar_wait(kBarHelpers, kStreamHelpers);  // every helper's copies have landed; every helper has finished tile - 3, whose slot tile + 3 takes
             stage(tile + 3);
-            float* s = smem + tile % kStreamSlots * kSlot;
+            more = s_tile[tile % kStreamSlots].n > 0;
+            if (more) {
+                float* s = smem + tile % kStreamSlots * kSlot;
 #pragma unroll
-            for (int i = tid; i < kScanTile * kCh4; i += kStreamHelpers) {
-                const float4 raw = reinterpret_cast<const float4*>(s + kDt)[i], xv = reinterpret_cast<const float4*>(s)[i];
-                const float4 dt = make_float4(fast_softplus(raw.x + my_bias.x), fast_softplus(raw.y + my_bias.y), fast_softplus(raw.z + my_bias.z), fast_softplus(raw.w + my_bias.w));
-                reinterpret_cast<float4*>(s + kDt)[i] = dt;
-                reinterpret_cast<float4*>(s + kDtx)[i] = make_float4(dt.x * xv.x, dt.y * xv.y, dt.z * xv.z, dt.w * xv.w);
+                for (int i = tid; i < kScanTile * kCh4; i += kStreamHelpers) {
+                    const float4 raw = reinterpret_cast<const float4*>(s + kDt)[i], xv = reinterpret_cast<const float4*>(s)[i];
+                    const float4 dt = make_float4(fast_softplus(raw.x + my_bias.x), fast_softplus(raw.y + my_bias.y), fast_softplus(raw.z + my_bias.z), fast_softplus(raw.w + my_bias.w));
+                    reinterpret_cast<float4*>(s + kDt)[i] = dt;
+                    reinterpret_cast<float4*>(s + kDtx)[i] = make_float4(dt.x * xv.x, dt.y * xv.y, dt.z * xv.z, dt.w * xv.w);
+                }
             }
             bar_arrive(kBarReady + (tile & 1), kAll);
             if (tile >= 2) finish(tile - 2);
         }
-        for (int tile = max(0, n_tiles - 2); tile < n_tiles; tile++) {
+        if (tile >= 2) {  // tile - 1 was the one past the end
             bar_wait(kBarDone + (tile & 1), kAll);
-            finish(tile);
+            finish(tile - 2);
         }
         cp_async_wait<0>();
         return;
@@ -504,6 +526,7 @@ __global__ void __launch_bounds__(kNch * kLanes + kStreamHelpers) selective_scan
     // ---------------- scanners ----------------
     const int ch = threadIdx.x / kLanes, part = threadIdx.x % kLanes, c = c_base + ch;
     const bool live = c < p.inner;
+    // the state; what the chunk adds up to from zero, and the state it began with
     f32x2 a[kS / 2], s[kS / 2], local[kS / 2], begin[kS / 2];
     const size_t sidx = (size_t)(live ? c : 0) * kNp + part * kS;
     const size_t slot_base = (size_t)p.st.slot[seq] * p.inner * kNp;
@@ -513,18 +536,23 @@ __global__ void __launch_bounds__(kNch * kLanes + kStreamHelpers) selective_scan
         for (int i = 0; i < kS / 2; i++) {
             a[i] = live ? *reinterpret_cast<const f32x2*>(p.a2 + sidx + 2 * i) : 0;
             s[i] = live && from ? *reinterpret_cast<const f32x2*>(from + 2 * i) : 0;
+            local[i] = begin[i] = 0;
         }
     }
     // Four tokens at a time: what they need is requested while the four before them are computed, and before those store their y (the
-    // compiler must keep loads behind stores that might be to the same place). A channel's four y end up one per lane, or per two lanes.
+    // compiler must keep loads behind stores that might be to the same place). A channel's four y end up one per lane.
     struct Four {
         float dt[4], dtx[4];
         f32x2 b[4][kS / 2], c[4][kS / 2];
     };
-    const bool high = part & (kLanes / 2), odd = part & (kLanes / 4);
+    const bool high = part & 2, odd = part & 1;
     const int my_token = (high ? 2 : 0) + (odd ? 1 : 0);
-    for (int tile = 0; tile < n_tiles; tile++) {
+    float sum_dt = 0.f;  // of the chunk
+    bool first = true;   // the sequence's first chunk runs from the slot: its end state is the next one's start
+    for (int tile = 0;; tile++) {
         bar_wait(kBarReady + (tile & 1), kAll);
+        const Tile of = s_tile[tile % kStreamSlots];
+        if (of.n == 0) break;
         float* const base = smem + tile % kStreamSlots * kSlot;
         const float *sdt = base + kDt + ch, *sdtx = base + kDtx + ch, *sb = base + kB + part * kS, *sc = base + kC + part * kS;
         float* const sy = base + kY + ch + my_token * kNch;
@@ -537,7 +565,6 @@ __global__ void __launch_bounds__(kNch * kLanes + kStreamHelpers) selective_scan
                 load_pairs<kS>(sc + (t0 + t) * kNp, f.c[t]);
             }
         };
-        float sum_dt = 0.f;
         // n: tokens of the four that count (a warp-uniform number; the state does not move at the others)
         auto four = [&](int t0, const Four& f, int n) {
             float y[4];
@@ -556,40 +583,38 @@ __global__ void __launch_bounds__(kNch * kLanes + kStreamHelpers) selective_scan
                 const float2 yv = unpair(y2);
                 y[t] = yv.x + yv.y;
             }
-            // the upper half of the lanes takes tokens 2 and 3 over, then every second quarter the odd one of each two
-            const float even = (high ? y[2] : y[0]) + __shfl_xor_sync(0xffffffffu, high ? y[0] : y[2], kLanes / 2);
-            const float next = (high ? y[3] : y[1]) + __shfl_xor_sync(0xffffffffu, high ? y[1] : y[3], kLanes / 2);
-            float v = (odd ? next : even) + __shfl_xor_sync(0xffffffffu, odd ? even : next, kLanes / 4);
-            if (kLanes == 8) v += __shfl_xor_sync(0xffffffffu, v, 1);
-            if (kLanes == 4 || !(part & 1)) sy[t0 * kNch] = v;
+            // the upper half of the lanes takes tokens 2 and 3 over, then every second lane the odd one of each two
+            const float even = (high ? y[2] : y[0]) + __shfl_xor_sync(0xffffffffu, high ? y[0] : y[2], 2);
+            const float next = (high ? y[3] : y[1]) + __shfl_xor_sync(0xffffffffu, high ? y[1] : y[3], 2);
+            sy[t0 * kNch] = (odd ? next : even) + __shfl_xor_sync(0xffffffffu, odd ? even : next, 1);
         };
-        // The unit's 2^x is good to about 2^-22, and a state that hardly decays would collect that at every token. So a tile's end state is what its
-        // tokens add up to from zero, and the state it began with times one decay over all of its tokens.
-#pragma unroll
-        for (int i = 0; i < kS / 2; i++) {
-            begin[i] = s[i];
-            local[i] = 0;
-        }
-        const int n_t = min(kScanTile, len - tile * kScanTile);
         Four f[2];
         load(0, f[0]);
-        if (n_t == kScanTile) {
+        if (of.n == kScanTile) {
 #pragma unroll
             for (int t = 0; t < kScanTile; t += 4) {
                 if (t + 4 < kScanTile) load(t + 4, f[(t >> 2) + 1 & 1]);
                 four(t, f[t >> 2 & 1], 4);
             }
         } else {  // places of tokens past the end hold zeros
-            for (int t = 0; t < n_t; t += 4) {
-                four(t, f[0], n_t - t);
-                if (t + 4 < n_t) load(t + 4, f[0]);
+            for (int t = 0; t < of.n; t += 4) {
+                four(t, f[0], of.n - t);
+                if (t + 4 < of.n) load(t + 4, f[0]);
             }
         }
         bar_arrive(kBarDone + (tile & 1), kAll);
+        if (of.links) {
 #pragma unroll
-        for (int i = 0; i < kS / 2; i++) {
-            const float2 x = unpair(mul2(pair(sum_dt, sum_dt), a[i]));
-            s[i] = fma2(pair(ex2f(x.x), ex2f(x.y)), begin[i], local[i]);
+            for (int i = 0; i < kS / 2; i++) {
+                if (!first) {
+                    const float2 x = unpair(mul2(pair(sum_dt, sum_dt), a[i]));
+                    s[i] = fma2(pair(ex2f(x.x), ex2f(x.y)), begin[i], local[i]);
+                }
+                begin[i] = s[i];
+                local[i] = 0;
+            }
+            first = false;
+            sum_dt = 0.f;
         }
     }
     if (live) {
@@ -699,28 +724,28 @@ __global__ void __launch_bounds__(128) gated_lru_kernel(const LruParams p) {
     }
 }
 
-// Whole sequences in one go: a warp takes 8 tokens of a tile of 128 for 32 channels, computes their decays and inputs once, and
-// keeps them. It runs them from zero, the warps hand each other end states and decays, and every warp runs its tokens again from where
-// they start: two multiply-adds per token instead of the sigmoids, exponentials and loads of a pass of its own, so that chunks as long as
-// the sequence need no pass for their start states. The next tile's rows are requested before the current tile's states.
-// All passes inside a prompt's step, against chunks (B200): 2048 tokens x 4096 channels 107 -> 75 us, 300 x 4096 34 -> 13, four sequences of 190 to 300 x 2048
-// 40 -> 22. Bound by instructions (expm1, sigmoids, square root: about 190 per value). Only whole sequences: as the last pass of chunks it is slower than the
-// kernel above (1024 x 2048: 65 against 20 us). Error against 64 bits, 2048 tokens: 1.36e-7 -> 1.17e-7.
-constexpr int kLruRun = 8, kLruWarps = 16, kLruFrom = 64;  // portions of more than kLruFrom tokens
+// The three passes in one, to the same bits: a CTA walks 32 channels of a sequence. A warp takes 8 tokens of a tile of 128, computes their decays, inputs and gates and
+// keeps them; the recurrence itself - two dependent operations a token - goes from warp to warp through shared memory, while the others compute. Beside the state
+// the warps hand on what the chunk adds up to from zero, its sum of log a and the state that it began with: the next chunk begins with what the link pass makes of
+// those. The next tile's rows are requested before the current tile's states.
+// Bound by instructions (expm1, sigmoids, square root: about 190 per value), which the passes spend twice on every value, and by the way from warp to
+// warp (about 420 cycles). Against the passes over chunks (B200, calls replayed as a graph): 2048 tokens x 4096 channels 95 -> 57 us, 1000 x 4096 47 -> 30,
+// 300 x 4096 28 -> 15, 2048 x 8192 179 -> 111.
+constexpr int kLruRun = 8, kLruWarps = 16;
 __global__ void __launch_bounds__(kLruWarps * 32) gated_lru_stream_kernel(const LruParams p) {
-    __shared__ float s_end[2][kLruWarps][32], s_move[2][kLruWarps][32];
+    __shared__ float4 s_hand[kLruWarps][32];  // to the warp after this one: state, from zero, sum of log a, begin
     INGOT_PDL_TRIGGER();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c = min(blockIdx.x * 32 + lane, p.width - 1);
     const bool on = blockIdx.x * 32 + lane < p.width;
     const float br = p.br[c], bi = p.bi[c], k = -8.0f * p.sp[c], yb = p.y_bias[c];
     INGOT_PDL_WAIT();
-    const int chunk = blockIdx.y;
-    const int seq = p.chunk_seq[chunk], len = p.chunk_len[chunk];
+    const int seq = blockIdx.y, k0 = p.seq_chunk0[seq], k1 = p.seq_chunk0[seq + 1];
+    if (k0 == k1) return;
+    const int len = min(p.chunk_t0[k1 - 1] + p.chunk_len[k1 - 1], p.st.len[seq]);
+    if (len < 1) return;
     const size_t row0 = (size_t)p.st.row_start[seq];
     const int gcol = (c / p.block) * 2 * p.block + c % p.block;
     float* slot = p.state + (size_t)p.st.slot[seq] * p.width + c;
-    float s = 0.f;  // at the start of the tile, the same in every warp
-    if (p.st.pos0[seq] > 0) s = *slot;
     const float* u = p.u + row0 * p.u_ld + c;
     const float* g = p.gates + row0 * p.gates_ld + gcol;
     const float* y = p.y + row0 * p.y_ld + c;
@@ -736,38 +761,70 @@ __global__ void __launch_bounds__(kLruWarps * 32) gated_lru_stream_kernel(const 
         }
     };
     const int n_tiles = (len + kLruWarps * kLruRun - 1) / (kLruWarps * kLruRun);
+    const int second = k0 + 1 < k1 ? p.chunk_t0[k0 + 1] : -1;
+    int chunk = k0 + 1;  // chunks before it begin before this warp's tokens
     fetch(0);
     for (int tile = 0; tile < n_tiles; tile++) {
         const int tb = (tile * kLruWarps + warp) * kLruRun, n = len - tb;  // tokens of this warp that there are, maybe none
-        float e[kLruRun], b[kLruRun], out[kLruRun], sum = 0.f;
+        unsigned begins = 0;  // bit i: a chunk begins with token i
+        for (;;) {
+            const int t0 = chunk + lane < k1 ? p.chunk_t0[chunk + lane] - tb : kLruRun, before = __popc(__ballot_sync(0xffffffffu, t0 < 0));
+            begins = __reduce_or_sync(0xffffffffu, t0 >= 0 && t0 < kLruRun ? 1u << t0 : 0u);
+            if (before <= 32 - kLruRun) break;  // the others may hold all that begin here
+            chunk += before;
+        }
+        float log_a[kLruRun], e[kLruRun], b[kLruRun], out[kLruRun];
 #pragma unroll
         for (int i = 0; i < kLruRun; i++) {
-            const float log_a = i < n ? k * fast_sigmoid(gr[i] + br) : 0.f;
-            e[i] = expm1f(log_a);  // a - 1; 1 - a^2 = -e (2 + e)
-            b[i] = i < n ? sqrtf(-e[i] * (2.0f + e[i])) * (fast_sigmoid(gi[i] + bi) * uv[i]) : 0.f;
+            log_a[i] = k * fast_sigmoid(gr[i] + br);
+            e[i] = expm1f(log_a[i]);  // a - 1; 1 - a^2 = -e (2 + e)
+            b[i] = sqrtf(-e[i] * (2.0f + e[i])) * (fast_sigmoid(gi[i] + bi) * uv[i]);
             out[i] = fast_gelu_tanh(yv[i] + yb);
-            sum += log_a;
+            // computed here, not behind the wait below, where the compiler would put it to save registers: the other warps would wait for it in turn (4.5 times the time)
+            asm volatile("" : "+f"(log_a[i]), "+f"(e[i]), "+f"(b[i]), "+f"(out[i]));
         }
         if (tile + 1 < n_tiles) fetch(tile + 1);
-        float end = 0.f;
+        float4 h;  // state, from zero, sum of log a, begin
+        if (tile == 0 && warp == 0) {
+            h = make_float4(p.st.pos0[seq] > 0 ? *slot : 0.f, 0.f, 0.f, 0.f);
+        } else {
+            bar_wait(warp, 64);
+            h = s_hand[warp][lane];
+        }
+        float s[kLruRun];
+        auto token = [&](int i) {
+            h.x += fmaf(e[i], h.x, b[i]);
+            h.y += fmaf(e[i], h.y, b[i]);
+            h.z += log_a[i];
+            s[i] = h.x;
+        };
+        auto link = [&](int i) {  // a chunk begins with token i; the first chunk ran from the slot: its end is the second one's start
+            if (tb + i != second) h.x = fmaf(expf(h.z), h.w, h.y);
+            h.w = h.x;
+            h.y = h.z = 0.f;
+        };
+        if (begins & 1) link(0);
+        if (begins < 2 && n >= kLruRun) {  // warp-uniform: no conditions on the way
 #pragma unroll
-        for (int i = 0; i < kLruRun; i++) end += fmaf(e[i], end, b[i]);
-        s_end[tile & 1][warp][lane] = end;
-        s_move[tile & 1][warp][lane] = expm1f(sum);
-        __syncthreads();
-        float mine = s;
+            for (int i = 0; i < kLruRun; i++) token(i);
+        } else {
 #pragma unroll
-        for (int w = 0; w < kLruWarps; w++) {
-            if (w == warp) mine = s;
-            s += fmaf(s_move[tile & 1][w][lane], s, s_end[tile & 1][w][lane]);
+            for (int i = 0; i < kLruRun; i++) {
+                if (i > 0 && begins >> i & 1) link(i);
+                if (i < n) token(i);
+            }
+        }
+        if (tile + 1 < n_tiles || warp + 1 < kLruWarps) {
+            const int to = (warp + 1) % kLruWarps;
+            s_hand[to][lane] = h;
+            bar_arrive(to, 64);
+        } else if (on) {
+            *slot = h.x;
         }
 #pragma unroll
-        for (int i = 0; i < kLruRun; i++) {
-            mine += fmaf(e[i], mine, b[i]);
-            if (i < n && on) p.out.store(row0 + tb + i, c, p.out_scale * mine * out[i]);
-        }
+        for (int i = 0; i < kLruRun; i++)
+            if (i < n && on) p.out.store(row0 + tb + i, c, p.out_scale * s[i] * out[i]);
     }
-    if (on && warp == 0) *slot = s;
 }
 
 __global__ void __launch_bounds__(128) gated_lru_link_kernel(const LruParams p) {
@@ -802,6 +859,11 @@ constexpr size_t kHalfSm = 116 * 1024;  // shared memory of which an SM has less
 bool one_per_sm(long long ctas) {
     int dev = 0, num_sms = 0;
     return cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && ctas <= num_sms;
+}
+
+constexpr int kStreamFrom = 64, kStreamChannels = 3072;  // portions of more tokens; channels, times the sequences of the longest one's length that the step holds
+bool streams(const ingot_step* step, int channels) {
+    return step->max_len > kStreamFrom && (long long)step->max_len * kStreamChannels <= (long long)step->n_tok * channels;
 }
 
 int scan_lanes_log2(int n_state) {
@@ -888,30 +950,31 @@ int ingot_selective_scan(const ingot_step* step, const ingot_scan_plan* plan, co
         INGOT_CUDA_TRY(cudaFuncSetAttribute(k_end, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
         INGOT_CUDA_TRY(cudaFuncSetAttribute(k_out, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
     }
-    if (multi) {
-        INGOT_CUDA_TRY(ingot_launch_pdl(k_end, grid, dim3(128), smem, s, p));
-        INGOT_CUDA_TRY(ingot_launch_pdl(selective_scan_link_kernel, dim3(unsigned(((size_t)inner * n_pad + 255) / 256), step->n_seq), dim3(256), 0, s, p));
-    }
-    // Whole sequences as a stream; the tile kernel for the exact form, more than 32 states, chunks, and steps too short to fill a ring.
-    if (!exact && lg == 2 && !multi && step->max_len > kStreamFrom) {
-        // 64 channels per CTA, or 32 with more lanes each where that would leave SMs without a CTA
-        const bool wide = (long long)((inner + 63) / 64) * plan->n_chunks >= 96;
+    // As a stream; the tile kernel for the exact form, more than 32 states, steps too short to fill a ring, and channels too few for the GPU: a stream takes
+    // time by the tokens of the longest sequence, chunks by tokens times channels. 4096 channels, one sequence (B200): 250 tokens 33 us in chunks,
+    // 18 as a stream, 1024: 65 and 61, 4000: 223 and 217-224.
+    if (!exact && lg == 2 && streams(step, inner)) {
+        // 64 channels per CTA, or 32 where that would leave SMs without a CTA
+        const bool wide = (long long)((inner + 63) / 64) * step->n_seq >= 96;
         const int ch = wide ? 64 : 32;
         Kernel k_stream = nullptr;
-        int lanes = 4;
         switch (per_lane) {
-            case 2: k_stream = wide ? selective_scan_stream_kernel<2, 4, 64> : selective_scan_stream_kernel<2, 4, 32>; break;
-            case 4: k_stream = wide ? selective_scan_stream_kernel<4, 4, 64> : selective_scan_stream_kernel<2, 8, 32>; lanes = wide ? 4 : 8; break;
-            case 6: k_stream = wide ? selective_scan_stream_kernel<6, 4, 64> : selective_scan_stream_kernel<6, 4, 32>; break;
-            case 8: k_stream = wide ? selective_scan_stream_kernel<8, 4, 64> : selective_scan_stream_kernel<4, 8, 32>; lanes = wide ? 4 : 8; break;
+            case 2: k_stream = wide ? selective_scan_stream_kernel<2, 64> : selective_scan_stream_kernel<2, 32>; break;
+            case 4: k_stream = wide ? selective_scan_stream_kernel<4, 64> : selective_scan_stream_kernel<4, 32>; break;
+            case 6: k_stream = wide ? selective_scan_stream_kernel<6, 64> : selective_scan_stream_kernel<6, 32>; break;
+            case 8: k_stream = wide ? selective_scan_stream_kernel<8, 64> : selective_scan_stream_kernel<8, 32>; break;
         }
         const int ctas = (inner + ch - 1) / ch;
         // One CTA per SM where there are enough SMs: launched while the kernel before still holds some, two would share the first ones that come
         // free and take twice as long beside idle ones.
-        const size_t need = size_t(kStreamSlots) * stream_slot_floats(ch, n_pad) * sizeof(float), bytes = one_per_sm((long long)ctas * plan->n_chunks) ? std::max(need, kHalfSm) : need;
+        const size_t need = size_t(kStreamSlots) * stream_slot_floats(ch, n_pad) * sizeof(float), bytes = one_per_sm((long long)ctas * step->n_seq) ? std::max(need, kHalfSm) : need;
         INGOT_CUDA_TRY(cudaFuncSetAttribute(k_stream, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
-        INGOT_CUDA_TRY(ingot_launch_pdl(k_stream, dim3(ctas, plan->n_chunks), dim3(ch * lanes + kStreamHelpers), bytes, s, p));
+        INGOT_CUDA_TRY(ingot_launch_pdl(k_stream, dim3(ctas, step->n_seq), dim3(ch * 4 + kStreamHelpers), bytes, s, p));
         return INGOT_OK;
+    }
+    if (multi) {
+        INGOT_CUDA_TRY(ingot_launch_pdl(k_end, grid, dim3(128), smem, s, p));
+        INGOT_CUDA_TRY(ingot_launch_pdl(selective_scan_link_kernel, dim3(unsigned(((size_t)inner * n_pad + 255) / 256), step->n_seq), dim3(256), 0, s, p));
     }
     INGOT_CUDA_TRY(ingot_launch_pdl(k_out, grid, dim3(128), smem, s, p));
     return INGOT_OK;
@@ -931,16 +994,16 @@ int ingot_gated_lru(const ingot_step* step, const ingot_scan_plan* plan, const f
                    plan->scratch_dev ? plan->scratch_dev + (size_t)plan->n_chunks * width : nullptr, width, out_scale, act_out(out)};
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const dim3 grid((width + 127) / 128, plan->n_chunks);
+    if (!exact && streams(step, width)) {
+        const int ctas = (width + 31) / 32;
+        const size_t bytes = one_per_sm((long long)ctas * step->n_seq) ? kHalfSm : 0;  // as above
+        INGOT_CUDA_TRY(cudaFuncSetAttribute(gated_lru_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kHalfSm)));
+        INGOT_CUDA_TRY(ingot_launch_pdl(gated_lru_stream_kernel, dim3(ctas, step->n_seq), dim3(kLruWarps * 32), bytes, s, p));
+        return INGOT_OK;
+    }
     if (multi) {
         INGOT_CUDA_TRY(ingot_launch_pdl(exact ? gated_lru_kernel<false, true> : gated_lru_kernel<false, false>, grid, dim3(128), 0, s, p));
         INGOT_CUDA_TRY(ingot_launch_pdl(gated_lru_link_kernel, dim3((width + 127) / 128, step->n_seq), dim3(128), 0, s, p));
-    }
-    if (!exact && !multi && step->max_len > kLruFrom) {
-        const int ctas = (width + 31) / 32;
-        const size_t bytes = one_per_sm((long long)ctas * plan->n_chunks) ? kHalfSm : 0;  // as above
-        INGOT_CUDA_TRY(cudaFuncSetAttribute(gated_lru_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kHalfSm)));
-        INGOT_CUDA_TRY(ingot_launch_pdl(gated_lru_stream_kernel, dim3(ctas, plan->n_chunks), dim3(kLruWarps * 32), bytes, s, p));
-        return INGOT_OK;
     }
     INGOT_CUDA_TRY(ingot_launch_pdl(exact ? gated_lru_kernel<true, true> : gated_lru_kernel<true, false>, grid, dim3(128), 0, s, p));
     return INGOT_OK;
