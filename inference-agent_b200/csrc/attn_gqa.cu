@@ -215,10 +215,14 @@ __global__ void __launch_bounds__(kAppendThreads) gqa_append128_kernel(const App
             float inv = is_q ? inv_q : inv_k;
             const float* w = (is_q ? p.q_norm : p.k_norm) + (p.sh.norm == INGOT_QK_NORM_ALL ? h * kDim : 0) + piece * 8;
             if (p.sh.norm == INGOT_QK_NORM_HEAD) {
-                float ss = dot4(make_float4(v[0], v[1], v[2], v[3]), dot4(make_float4(v[4], v[5], v[6], v[7]), 0.f));
+                // the order in which the warp above adds its lanes' four values each: the same bits whichever kernel a step takes
+                float ss = dot4(make_float4(v[0], v[1], v[2], v[3]), 0.f), st = dot4(make_float4(v[4], v[5], v[6], v[7]), 0.f);
 #pragma unroll
-                for (int o = 8; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-                inv = 1.0f / sqrtf(ss / float(p.sh.dim_count) + p.eps);
+                for (int o = 8; o > 0; o >>= 1) {
+                    ss += __shfl_xor_sync(0xffffffffu, ss, o);
+                    st += __shfl_xor_sync(0xffffffffu, st, o);
+                }
+                inv = 1.0f / sqrtf((ss + st) / float(p.sh.dim_count) + p.eps);
             }
             if (live && !is_v) {
                 const float4 a = reinterpret_cast<const float4*>(w)[0], b = reinterpret_cast<const float4*>(w)[1];
@@ -247,8 +251,8 @@ __global__ void __launch_bounds__(kAppendThreads) gqa_append128_kernel(const App
             for (int i = 0; i < 4; i++) {
                 const float x = v[2 * i], y = v[2 * i + 1];
                 if (piece * 8 + 2 * i < rot) {
-                    v[2 * i] = x * cs[i] - y * sn[i];
-                    v[2 * i + 1] = y * cs[i] + x * sn[i];
+                    v[2 * i] = fmaf(x, cs[i], -__fmul_rn(y, sn[i]));  // spelled out as the compiler has it above
+                    v[2 * i + 1] = fmaf(y, cs[i], __fmul_rn(x, sn[i]));
                 }
             }
         }
