@@ -375,17 +375,18 @@ private:
             for (int t = 0; t < asked[i].n_tokens; t++) rows_asked_.push_back(m[o_start + size_t(place[size_t(i)])] + t);
         lens_sorted_.assign(m.begin() + long(o_len), m.begin() + long(o_len) + n);
         step.first_want = step.n_want ? m[o_want] : 0;
-        struct PlanAt { size_t seq, t0, len, first; int n_chunks, max_chunks; };
-        auto plan = [&](int threads) {
+        struct PlanAt { int seq0, seq1; size_t seq, t0, len, first; int n_chunks, max_chunks; };  // of sequences seq0 .. seq1 - 1
+        auto plan = [&](int seq0, int seq1, int chunk) {
             PlanAt p = {};
-            const int L = chunk_tokens(entries, step.n_tok, threads);
+            p.seq0 = seq0;
+            p.seq1 = seq1;
             std::vector<int32_t> seq, t0, len, first;
-            for (int i = 0; i < n; i++) {
+            for (int i = seq0; i < seq1; i++) {
                 first.push_back(int32_t(seq.size()));
-                for (int t = 0; t < entries[i].n_tokens; t += L) {
-                    seq.push_back(i);
+                for (int t = 0; t < entries[i].n_tokens; t += chunk) {
+                    seq.push_back(i - seq0);
                     t0.push_back(t);
-                    len.push_back(std::min(L, entries[i].n_tokens - t));
+                    len.push_back(std::min(chunk, entries[i].n_tokens - t));
                 }
                 p.max_chunks = std::max(p.max_chunks, int(seq.size()) - first.back());
             }
@@ -397,8 +398,17 @@ private:
             p.first = mark(); m.insert(m.end(), first.begin(), first.end());
             return p;
         };
-        std::vector<PlanAt> plans;
-        for (const auto& request : ops_.plans()) plans.push_back(plan(request.threads));
+        std::vector<std::vector<PlanAt>> plans;
+        for (const auto& r : ops_.plans()) {
+            const int chunk = chunk_tokens(entries, step.n_tok, r.threads);  // of the whole step, however it is cut: results do not depend on that
+            auto load = [&](int a, int b) {
+                const int longest = b > a ? lens_sorted_[size_t(b) - 1] : 0;
+                return ingot_scan::Load{std::accumulate(lens_sorted_.begin() + a, lens_sorted_.begin() + b, 0ll), longest, b - a, (longest + chunk - 1) / chunk};
+            };
+            const int cut = r.kind == ingot_scan::Kind::none ? 0 : int(std::upper_bound(lens_sorted_.begin(), lens_sorted_.end(), ingot_scan::kShort) - lens_sorted_.begin());
+            if (cut > 0 && ingot_scan::apart(r.kind, load(0, n), load(0, cut), load(cut, n), r.channels, r.states, num_sms_)) plans.push_back({plan(0, cut, chunk), plan(cut, n, chunk)});
+            else plans.push_back({plan(0, n, chunk)});
+        }
         struct TableAt { size_t first, table, key0, key_pos; };
         std::vector<TableAt> table_at;
         for (auto& g : ops_.caches) {
@@ -458,7 +468,8 @@ private:
         step.want_rows = meta_dev_ + o_want;
         size_t floats = 0;  // one scratch for all: mixers run one after the other
         for (size_t i = 0; i < plans.size(); i++)
-            if (plans[i].max_chunks > 1) floats = std::max(floats, ops_.plans()[i].scratch * size_t(plans[i].n_chunks));
+            for (const PlanAt& at : plans[i])
+                if (at.max_chunks > 1) floats = std::max(floats, ops_.plans()[i].scratch * size_t(at.n_chunks));
         if (floats > scan_cap_) {
             drop_graphs();
             cuda_check(cudaStreamSynchronize(ops_.stream), "scratch");
@@ -468,17 +479,24 @@ private:
             cuda_check(cudaMalloc(&scan_scratch_dev_, floats * 4), "cudaMalloc(scan scratch)");
             scan_cap_ = floats;
         }
-        for (const PlanAt& at : plans) {
-            ingot_scan_plan p = {};
-            p.n_chunks = at.n_chunks;
-            p.max_chunks = at.max_chunks;
-            p.chunk_seq = meta_dev_ + at.seq;
-            p.chunk_t0 = meta_dev_ + at.t0;
-            p.chunk_len = meta_dev_ + at.len;
-            p.seq_chunk0 = meta_dev_ + at.first;
-            p.scratch_dev = scan_scratch_dev_;
-            p.scratch_floats = scan_cap_;
-            s.plans.push_back(p);
+        for (const auto& parts : plans) {
+            s.plans.emplace_back();
+            for (const PlanAt& at : parts) {
+                StepCtx::ScanPart p = {s.st, {}};
+                p.st.n_tok = std::accumulate(lens_sorted_.begin() + at.seq0, lens_sorted_.begin() + at.seq1, 0);
+                p.st.n_seq = at.seq1 - at.seq0;
+                p.st.max_len = lens_sorted_[size_t(at.seq1) - 1];
+                for (const int32_t** a : {&p.st.row_start, &p.st.len, &p.st.pos0, &p.st.slot}) *a += at.seq0;
+                p.plan.n_chunks = at.n_chunks;
+                p.plan.max_chunks = at.max_chunks;
+                p.plan.chunk_seq = meta_dev_ + at.seq;
+                p.plan.chunk_t0 = meta_dev_ + at.t0;
+                p.plan.chunk_len = meta_dev_ + at.len;
+                p.plan.seq_chunk0 = meta_dev_ + at.first;
+                p.plan.scratch_dev = scan_scratch_dev_;
+                p.plan.scratch_floats = scan_cap_;
+                s.plans.back().push_back(p);
+            }
         }
         for (size_t i = 0; i < ops_.caches.size(); i++) {
             ops_.caches[i]->first_page = meta_dev_ + table_at[i].first;

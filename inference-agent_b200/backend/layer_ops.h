@@ -16,6 +16,7 @@
 #include <cmath>
 #include <cstring>
 #include <memory>
+#include <numeric>
 #include <string>
 #include <utility>
 #include <vector>
@@ -27,6 +28,7 @@
 #include "model_registry.h"
 #include "residual_norm.h"
 #include "weight_streamer.h"
+#include "../csrc/scan_routes.h"
 
 extern "C" {
 cudaError_t ingot_support_embed_rows_bf16(float* out, const void* table, int n_in, int n_rows_table, const int32_t* rows_dev, int n_rows,
@@ -164,7 +166,9 @@ enum Buf { kProj, kConv, kStateIn, kDt, kGates, kMix, kGateUp, kMid, kNormed, kQ
 // The step as the launches see it.
 struct StepCtx {
     ingot_step st = {};
-    std::vector<ingot_scan_plan> plans;  // time chunks, by LayerOps::scan_plan
+    // Time chunks, by LayerOps::scan_plan: one part for all sequences of the step, or one for the short ones and one for the others.
+    struct ScanPart { ingot_step st; ingot_scan_plan plan; };
+    std::vector<std::vector<ScanPart>> plans;
     const int32_t* lens = nullptr;  // host copy of st.len; sequences come in ascending order of it
     const int32_t* tokens = nullptr;  // device: the token id of each row
     bool tc = false;  // products on the tensor cores (16-bit form, more than one token)
@@ -552,15 +556,16 @@ public:
         return g;
     }
     // Time chunks for a recurrence: threads that one chunk occupies (they size the chunks of a step), floats of scratch that it needs. The
-    // number of the plan in StepCtx::plans; mixers of equal threads share one.
-    struct PlanRequest { int threads; size_t scratch; };
-    size_t scan_plan(int threads, size_t scratch) {
+    // number of the plan in StepCtx::plans; equal mixers share one. kind: of the recurrences over channels in 16-bit form (scan_routes.h), whose
+    // short sequences may go in a call of their own, with their channels and states per channel; Kind::none for the others.
+    struct PlanRequest { int threads; size_t scratch; ingot_scan::Kind kind; int channels, states; };
+    size_t scan_plan(int threads, size_t scratch, ingot_scan::Kind kind = ingot_scan::Kind::none, int channels = 0, int states = 0) {
         for (size_t i = 0; i < plans_.size(); i++)
-            if (plans_[i].threads == threads) {
+            if (plans_[i].threads == threads && plans_[i].kind == kind && plans_[i].channels == channels && plans_[i].states == states) {
                 plans_[i].scratch = std::max(plans_[i].scratch, scratch);
                 return i;
             }
-        plans_.push_back({threads, scratch});
+        plans_.push_back({threads, scratch, kind, channels, states});
         return plans_.size() - 1;
     }
     const std::vector<PlanRequest>& plans() const { return plans_; }

@@ -39,7 +39,7 @@ public:
         w_o_ = ops.matrix(p + "o", flat(d), in);
         conv_state_ = ops.state(size_t(taps_ - 1) * ip_);
         state_ = ops.state(size_t(ip_) * np_);
-        plan_ = ops.scan_plan(ip_ * 2, size_t(ip_) * (np_ + 1));
+        plan_ = ops.scan_plan(ip_ * 2, size_t(ip_) * (np_ + 1), !ops.opt.f32 && states_ <= 32 ? ingot_scan::Kind::selective : ingot_scan::Kind::none, ip_, np_);
         ops.need(kProj, 2 * ip_);
         ops.need(kConv, ip_);
         ops.need(kStateIn, rank_p_ + 2 * np_);
@@ -56,8 +56,9 @@ public:
         ops.project(s, dbc, w_x_, xc, ip_);
         ops.project_rows(s, dt, w_dt_, dbc, ld_bc, 2);
         const ingot_act_out y = ops.operand(s, ops.buf(kMix), ip_, false);
-        ingot_check(ingot_selective_scan(&s.st, &s.plans[plan_], xc, ip_, dt, ip_, dt_b_, dbc, ld_bc, rank_p_, rank_p_ + np_, xz + ip_, 2 * ip_, a2_, d_,
-                                         ops.at_pass(state_, size_t(ip_) * np_), ip_, states_, ops.opt.f32 ? 1 : 0, &y, ops.stream));
+        for (const auto& part : s.plans[plan_])
+            ingot_check(ingot_selective_scan(&part.st, &part.plan, xc, ip_, dt, ip_, dt_b_, dbc, ld_bc, rank_p_, rank_p_ + np_, xz + ip_, 2 * ip_, a2_, d_,
+                                             ops.at_pass(state_, size_t(ip_) * np_), ip_, states_, ops.opt.f32 ? 1 : 0, &y, ops.stream));
         ops.operand_ready(s, ip_);
         ops.project_residual(s, w_o_, ops.buf(kMix), n);
     }
@@ -130,7 +131,7 @@ public:
         w_o_ = ops.matrix(in.padded, mix_ld_, {Part{L + "o", {d, q.count()}, in, heads_out, 0, 0}, Part{R + "o", {d, width_}, in, w, 0, attn_cols_}});
         conv_state_ = ops.state(size_t(taps_ - 1) * wp_);
         state_ = ops.state(size_t(wp_));
-        plan_ = ops.scan_plan(wp_, 2 * size_t(wp_));
+        plan_ = ops.scan_plan(wp_, 2 * size_t(wp_), ops.opt.f32 ? ingot_scan::Kind::none : ingot_scan::Kind::gated, wp_, 1);
         ops.need(kProj, proj_ld_);
         ops.need(kConv, wp_);
         ops.need(kGates, 2 * wp_);
@@ -155,8 +156,9 @@ public:
         if (right.f32) right.f32 += attn_cols_;
         if (right.hi) right.hi = static_cast<char*>(right.hi) + size_t(attn_cols_) * 2;
         if (right.lo) right.lo = static_cast<char*>(right.lo) + size_t(attn_cols_) * 2;
-        ingot_check(ingot_gated_lru(&s.st, &s.plans[plan_], u, wp_, gates, 2 * wp_, block_, r_b_, i_b_, softplus_lam_, proj + y_off_, proj_ld_, y_b_, ops.at_pass(state_, size_t(wp_)), wp_,
-                                    right_scale_, ops.opt.f32 ? 1 : 0, &right, ops.stream));
+        for (const auto& part : s.plans[plan_])
+            ingot_check(ingot_gated_lru(&part.st, &part.plan, u, wp_, gates, 2 * wp_, block_, r_b_, i_b_, softplus_lam_, proj + y_off_, proj_ld_, y_b_, ops.at_pass(state_, size_t(wp_)), wp_,
+                                        right_scale_, ops.opt.f32 ? 1 : 0, &right, ops.stream));
         ops.operand_ready(s, mix_ld_);
         ops.project_residual(s, w_o_, mix, n);
     }
@@ -193,7 +195,7 @@ public:
         in.n_head = heads_;
         in.n_state = np();
         in.n_value = vp();
-        ingot_check(ingot_linear_scan(&s.st, &s.plans[plan_], &in, ops.at_pass(state_, floats()), y, width(), s.lens[0], f32_ ? 1 : 0, ops.stream));
+        ingot_check(ingot_linear_scan(&s.st, &s.plans[plan_][0].plan, &in, ops.at_pass(state_, floats()), y, width(), s.lens[0], f32_ ? 1 : 0, ops.stream));
         norm.x = y;
         norm.x_ld = width();
         norm.heads = heads_;

@@ -13,13 +13,13 @@
 //   pass 2  one thread per state element walks a sequence's chunks in order and turns end states into start states;
 //   pass 3  every chunk runs again from its start state and writes the outputs; the last chunk writes the slot.
 // A sequence that is a single chunk (every decoded token) takes pass 3 alone, straight from and to its slot.
-// Where the sequences themselves fill the GPU one launch does all three (the stream kernels), to the same bits: which launches a call takes is
-// a matter of time alone.
+// One launch may do all three (the stream kernels), to the same bits: which launches a call takes is a matter of time alone (scan_routes.h).
 //
 // Decays. A slow channel multiplies its state by a = exp(x), x near 0, at every token, so an error of a that is always of
 // the same sign adds up over the memory of the channel (the 2^x unit is good to about 2^-22). Where that matters - the gated
 // unit, and the selective scan in its exact form - the state moves by S + S expm1(x), whose error is relative to 1 - a.
 #include "recurrent_common.cuh"
+#include "scan_routes.h"
 
 namespace {
 
@@ -188,6 +188,7 @@ struct ScanParams {
     float* part_sum;     // [chunk][inner] sum of dt
     int inner, n_pad, lanes_log2;
     ActOut out;
+    bool whole;          // grid.y: sequences
 };
 // Pairs of f32 in one 64-bit register: two multiply-adds per instruction.
 typedef unsigned long long f32x2;
@@ -235,9 +236,10 @@ __global__ void __launch_bounds__(128) selective_scan_kernel(const ScanParams p)
     INGOT_PDL_TRIGGER();
     INGOT_PDL_WAIT();
     const int chunk = blockIdx.y;
-    const int seq = p.chunk_seq[chunk], t0 = p.chunk_t0[chunk], len = p.chunk_len[chunk];
+    const bool whole = kOutput && p.whole;  // sequences as they are instead of chunks
+    const int seq = whole ? chunk : p.chunk_seq[chunk], t0 = whole ? 0 : p.chunk_t0[chunk], len = whole ? p.st.len[seq] : p.chunk_len[chunk];
     const bool first = t0 == 0, last = t0 + len == p.st.len[seq];
-    if (!kOutput && last) return;  // nothing follows a sequence's last chunk
+    if ((!kOutput && last) || (whole && len < 1)) return;  // nothing follows a sequence's last chunk
     const int lg = kLg >= 0 ? kLg : p.lanes_log2;
     const int lanes = 1 << lg, n_ch = 256 >> lg;
     const int ch = threadIdx.x >> lg, part = threadIdx.x & (lanes - 1);
@@ -428,7 +430,7 @@ __global__ void __launch_bounds__(kNch * 4 + kStreamHelpers) selective_scan_stre
     constexpr int kSlot = stream_slot_floats(kNch, kNp), kDt = kScanTile * kNch, kZ = 2 * kDt, kDtx = 3 * kDt, kY = 4 * kDt, kB = 5 * kDt, kC = kB + kScanTile * kNp;
     INGOT_PDL_TRIGGER();
     INGOT_PDL_WAIT();
-    const int seq = blockIdx.y, k0 = p.seq_chunk0[seq], k1 = p.seq_chunk0[seq + 1];
+    const int seq = gridDim.y - 1 - blockIdx.y, k0 = p.seq_chunk0[seq], k1 = p.seq_chunk0[seq + 1];  // the last first: steps hold their sequences in ascending order of tokens
     if (k0 == k1) return;
     const int c_base = blockIdx.x * kNch, seq_len = p.st.len[seq];
     const size_t row0 = (size_t)p.st.row_start[seq];
@@ -674,15 +676,17 @@ struct LruParams {
     int width;
     float out_scale;
     ActOut out;
+    bool whole;  // grid.y: sequences
 };
 template <bool kOutput, bool kExact>
 __global__ void __launch_bounds__(128) gated_lru_kernel(const LruParams p) {
     INGOT_PDL_TRIGGER();
     INGOT_PDL_WAIT();
     const int chunk = blockIdx.y, c = blockIdx.x * 128 + threadIdx.x;
-    const int seq = p.chunk_seq[chunk], t0 = p.chunk_t0[chunk], len = p.chunk_len[chunk];
+    const bool whole = kOutput && p.whole;
+    const int seq = whole ? chunk : p.chunk_seq[chunk], t0 = whole ? 0 : p.chunk_t0[chunk], len = whole ? p.st.len[seq] : p.chunk_len[chunk];
     const bool first = t0 == 0, last = t0 + len == p.st.len[seq];
-    if ((!kOutput && last) || c >= p.width) return;
+    if ((!kOutput && last) || (whole && len < 1) || c >= p.width) return;
     const size_t row0 = (size_t)p.st.row_start[seq] + t0;
     const int gcol = (c / p.block) * 2 * p.block + c % p.block;
     const float br = p.br[c], bi = p.bi[c], k = -8.0f * p.sp[c], yb = kOutput ? p.y_bias[c] : 0.f;
@@ -739,10 +743,10 @@ __global__ void __launch_bounds__(kLruWarps * 32) gated_lru_stream_kernel(const 
     const bool on = blockIdx.x * 32 + lane < p.width;
     const float br = p.br[c], bi = p.bi[c], k = -8.0f * p.sp[c], yb = p.y_bias[c];
     INGOT_PDL_WAIT();
-    const int seq = blockIdx.y, k0 = p.seq_chunk0[seq], k1 = p.seq_chunk0[seq + 1];
+    const int seq = gridDim.y - 1 - blockIdx.y, k0 = p.seq_chunk0[seq], k1 = p.seq_chunk0[seq + 1];  // as above
     if (k0 == k1) return;
     const int len = min(p.chunk_t0[k1 - 1] + p.chunk_len[k1 - 1], p.st.len[seq]);
-    if (len < 1) return;
+    if (warp * kLruRun >= len) return;  // no tokens for this warp
     const size_t row0 = (size_t)p.st.row_start[seq];
     const int gcol = (c / p.block) * 2 * p.block + c % p.block;
     float* slot = p.state + (size_t)p.st.slot[seq] * p.width + c;
@@ -760,12 +764,11 @@ __global__ void __launch_bounds__(kLruWarps * 32) gated_lru_stream_kernel(const 
             yv[i] = y[t * p.y_ld];
         }
     };
-    const int n_tiles = (len + kLruWarps * kLruRun - 1) / (kLruWarps * kLruRun);
     const int second = k0 + 1 < k1 ? p.chunk_t0[k0 + 1] : -1;
     int chunk = k0 + 1;  // chunks before it begin before this warp's tokens
     fetch(0);
-    for (int tile = 0; tile < n_tiles; tile++) {
-        const int tb = (tile * kLruWarps + warp) * kLruRun, n = len - tb;  // tokens of this warp that there are, maybe none
+    for (int tile = 0; (tile * kLruWarps + warp) * kLruRun < len; tile++) {
+        const int tb = (tile * kLruWarps + warp) * kLruRun, n = len - tb;  // tokens from here on
         unsigned begins = 0;  // bit i: a chunk begins with token i
         for (;;) {
             const int t0 = chunk + lane < k1 ? p.chunk_t0[chunk + lane] - tb : kLruRun, before = __popc(__ballot_sync(0xffffffffu, t0 < 0));
@@ -783,7 +786,7 @@ __global__ void __launch_bounds__(kLruWarps * 32) gated_lru_stream_kernel(const 
             // computed here, not behind the wait below, where the compiler would put it to save registers: the other warps would wait for it in turn (4.5 times the time)
             asm volatile("" : "+f"(log_a[i]), "+f"(e[i]), "+f"(b[i]), "+f"(out[i]));
         }
-        if (tile + 1 < n_tiles) fetch(tile + 1);
+        if (n > kLruWarps * kLruRun) fetch(tile + 1);
         float4 h;  // state, from zero, sum of log a, begin
         if (tile == 0 && warp == 0) {
             h = make_float4(p.st.pos0[seq] > 0 ? *slot : 0.f, 0.f, 0.f, 0.f);
@@ -814,7 +817,7 @@ __global__ void __launch_bounds__(kLruWarps * 32) gated_lru_stream_kernel(const 
                 if (i < n) token(i);
             }
         }
-        if (tile + 1 < n_tiles || warp + 1 < kLruWarps) {
+        if (n > kLruRun) {
             const int to = (warp + 1) % kLruWarps;
             s_hand[to][lane] = h;
             bar_arrive(to, 64);
@@ -856,14 +859,14 @@ __global__ void __launch_bounds__(128) gated_lru_link_kernel(const LruParams p) 
 }
 
 constexpr size_t kHalfSm = 116 * 1024;  // shared memory of which an SM has less than twice
-bool one_per_sm(long long ctas) {
+int sm_count() {
     int dev = 0, num_sms = 0;
-    return cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && ctas <= num_sms;
+    return cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess ? num_sms : 0;
 }
-
-constexpr int kStreamFrom = 64, kStreamChannels = 3072;  // portions of more tokens; channels, times the sequences of the longest one's length that the step holds
-bool streams(const ingot_step* step, int channels) {
-    return step->max_len > kStreamFrom && (long long)step->max_len * kStreamChannels <= (long long)step->n_tok * channels;
+// A call of single tokens (every decoded step) has one form.
+ingot_scan::Form form_of(ingot_scan::Kind kind, const ingot_step* step, const ingot_scan_plan* plan, int channels, int states, int num_sms) {
+    if (step->max_len == 1 || num_sms < 1) return ingot_scan::Form::chunks;
+    return ingot_scan::choose(kind, {step->n_tok, step->max_len, step->n_seq, plan->max_chunks}, channels, states, num_sms).form;
 }
 
 int scan_lanes_log2(int n_state) {
@@ -926,7 +929,7 @@ int ingot_selective_scan(const ingot_step* step, const ingot_scan_plan* plan, co
     ScanParams p = {*step, plan->chunk_seq, plan->chunk_t0, plan->chunk_len, plan->seq_chunk0, plan->n_chunks,
                     x_dev, x_ld, dt_dev, dt_ld, dt_bias_dev, bc_dev, bc_ld, b_off, c_off, z_dev, z_ld, a_log2e_dev, d_dev,
                     state_dev, plan->scratch_dev, plan->scratch_dev ? plan->scratch_dev + (size_t)plan->n_chunks * inner * n_pad : nullptr,
-                    inner, n_pad, lg, act_out(out)};
+                    inner, n_pad, lg, act_out(out), false};
     const size_t smem = (size_t)kScanTile * (2 * (3 * n_ch + 2 * n_pad) + 2 * n_ch) * sizeof(float);
     typedef void (*Kernel)(ScanParams);
     Kernel k_end, k_out;
@@ -950,13 +953,12 @@ int ingot_selective_scan(const ingot_step* step, const ingot_scan_plan* plan, co
         INGOT_CUDA_TRY(cudaFuncSetAttribute(k_end, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
         INGOT_CUDA_TRY(cudaFuncSetAttribute(k_out, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
     }
-    // As a stream; the tile kernel for the exact form, more than 32 states, steps too short to fill a ring, and channels too few for the GPU: a stream takes
-    // time by the tokens of the longest sequence, chunks by tokens times channels. 4096 channels, one sequence (B200): 250 tokens 33 us in chunks,
-    // 18 as a stream, 1024: 65 and 61, 4000: 223 and 217-224.
-    if (!exact && lg == 2 && streams(step, inner)) {
-        // 64 channels per CTA, or 32 where that would leave SMs without a CTA
-        const bool wide = (long long)((inner + 63) / 64) * step->n_seq >= 96;
-        const int ch = wide ? 64 : 32;
+    // More than 32 states and the exact form: the plan's chunks.
+    const int num_sms = !exact && lg == 2 ? sm_count() : 0;
+    const ingot_scan::Form form = form_of(ingot_scan::Kind::selective, step, plan, inner, n_pad, num_sms);
+    if (form == ingot_scan::Form::stream) {
+        const int ch = ingot_scan::stream_channels({step->n_tok, step->max_len, step->n_seq, plan->max_chunks}, inner, num_sms);
+        const bool wide = ch == 64;
         Kernel k_stream = nullptr;
         switch (per_lane) {
             case 2: k_stream = wide ? selective_scan_stream_kernel<2, 64> : selective_scan_stream_kernel<2, 32>; break;
@@ -967,9 +969,14 @@ int ingot_selective_scan(const ingot_step* step, const ingot_scan_plan* plan, co
         const int ctas = (inner + ch - 1) / ch;
         // One CTA per SM where there are enough SMs: launched while the kernel before still holds some, two would share the first ones that come
         // free and take twice as long beside idle ones.
-        const size_t need = size_t(kStreamSlots) * stream_slot_floats(ch, n_pad) * sizeof(float), bytes = one_per_sm((long long)ctas * step->n_seq) ? std::max(need, kHalfSm) : need;
+        const size_t need = size_t(kStreamSlots) * stream_slot_floats(ch, n_pad) * sizeof(float), bytes = (long long)ctas * step->n_seq <= num_sms ? std::max(need, kHalfSm) : need;
         INGOT_CUDA_TRY(cudaFuncSetAttribute(k_stream, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
         INGOT_CUDA_TRY(ingot_launch_pdl(k_stream, dim3(ctas, step->n_seq), dim3(ch * 4 + kStreamHelpers), bytes, s, p));
+        return INGOT_OK;
+    }
+    if (form == ingot_scan::Form::tile && multi) {
+        p.whole = true;
+        INGOT_CUDA_TRY(ingot_launch_pdl(k_out, dim3(grid.x, step->n_seq), dim3(128), smem, s, p));
         return INGOT_OK;
     }
     if (multi) {
@@ -991,14 +998,21 @@ int ingot_gated_lru(const ingot_step* step, const ingot_scan_plan* plan, const f
     INGOT_REQUIRE(!multi || (plan->scratch_dev && plan->scratch_floats >= (size_t)plan->n_chunks * width * 2), "ingot_gated_lru: scratch too small");
     LruParams p = {*step, plan->chunk_seq, plan->chunk_t0, plan->chunk_len, plan->seq_chunk0, plan->n_chunks, u_dev, u_ld, gates_dev, gates_ld,
                    block, r_bias_dev, i_bias_dev, softplus_lam_dev, y_dev, y_ld, y_bias_dev, state_dev, plan->scratch_dev,
-                   plan->scratch_dev ? plan->scratch_dev + (size_t)plan->n_chunks * width : nullptr, width, out_scale, act_out(out)};
+                   plan->scratch_dev ? plan->scratch_dev + (size_t)plan->n_chunks * width : nullptr, width, out_scale, act_out(out), false};
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const dim3 grid((width + 127) / 128, plan->n_chunks);
-    if (!exact && streams(step, width)) {
+    const int num_sms = exact ? 0 : sm_count();
+    const ingot_scan::Form form = form_of(ingot_scan::Kind::gated, step, plan, width, 1, num_sms);
+    if (form == ingot_scan::Form::stream) {
         const int ctas = (width + 31) / 32;
-        const size_t bytes = one_per_sm((long long)ctas * step->n_seq) ? kHalfSm : 0;  // as above
+        const size_t bytes = (long long)ctas * step->n_seq <= num_sms ? kHalfSm : 0;  // as above
         INGOT_CUDA_TRY(cudaFuncSetAttribute(gated_lru_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kHalfSm)));
         INGOT_CUDA_TRY(ingot_launch_pdl(gated_lru_stream_kernel, dim3(ctas, step->n_seq), dim3(kLruWarps * 32), bytes, s, p));
+        return INGOT_OK;
+    }
+    if (form == ingot_scan::Form::tile && multi) {
+        p.whole = true;
+        INGOT_CUDA_TRY(ingot_launch_pdl(gated_lru_kernel<true, false>, dim3(grid.x, step->n_seq), dim3(128), 0, s, p));
         return INGOT_OK;
     }
     if (multi) {
