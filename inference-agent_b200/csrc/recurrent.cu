@@ -93,7 +93,8 @@ __global__ void __launch_bounds__(128) causal_conv_kernel(const ConvParams p) {
 // of loads (B200, inside a prompt's step): 1000 tokens x 2048 channels 12.8 -> 5.0 us, 2048 x 4096 25 -> 19.4, 2048 x 8192
 // 43 -> 39.5. Runs of 4 read 1.75 times what they write from L2, but give a short step four times the CTAs; which run a launch takes is
 // decided in ingot_causal_conv.
-template <int kTaps, int kRun>
+// kPacked: grid.y holds the runs of all sequences one after the other, instead of those of the longest one for every sequence (grid.z).
+template <int kTaps, int kRun, bool kPacked>
 __global__ void __launch_bounds__(128) causal_conv4_kernel(const ConvParams p) {
     static_assert(kRun >= kMaxConvTaps4 - 1, "a run replaces its history");
     INGOT_PDL_TRIGGER();
@@ -121,7 +122,30 @@ __global__ void __launch_bounds__(128) causal_conv4_kernel(const ConvParams p) {
         }
     }
     INGOT_PDL_WAIT();
-    const int seq = blockIdx.z, len = p.st.len[seq], t0 = blockIdx.y * kRun;
+    int seq = blockIdx.z, run = blockIdx.y;
+    if (kPacked) {  // every warp finds the sequence by the runs before it
+        const int lane = threadIdx.x & 31;
+        seq = -1;
+        for (int s0 = 0; s0 < p.st.n_seq; s0 += 32) {
+            const int own = s0 + lane < p.st.n_seq ? (p.st.len[s0 + lane] + kRun - 1) / kRun : 0;
+            int upto = own;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, upto, o);
+                if (lane >= o) upto += v;
+            }
+            const unsigned past = __ballot_sync(0xffffffffu, upto > run);
+            if (past) {
+                const int at = __ffs(past) - 1;
+                seq = s0 + at;
+                run -= __shfl_sync(0xffffffffu, upto - own, at);
+                break;
+            }
+            run -= __shfl_sync(0xffffffffu, upto, 31);
+        }
+        if (seq < 0) return;
+    }
+    const int len = p.st.len[seq], t0 = run * kRun;
     if (!on || t0 >= len) return;
     const int pos0 = p.st.pos0[seq];
     const size_t row0 = p.st.row_start[seq];
@@ -890,18 +914,30 @@ int ingot_causal_conv(const ingot_step* step, const float* in_dev, int in_ld, co
                       void* stream) {
     INGOT_REQUIRE(step_ok(step) && in_dev && w_dev && state_dev && out, "ingot_causal_conv: null argument or empty step");
     INGOT_REQUIRE(channels >= 1 && taps >= 1 && taps <= kMaxTaps, "ingot_causal_conv: between 1 and 16 taps");
-    ConvParams p = {*step, in_dev, in_ld, in_bias_dev, w_dev, bias_dev, taps, channels, silu, state_dev, act_out(out)};
-    const bool four = taps >= 2 && taps <= kMaxConvTaps4 && step->max_len <= 4 * 65535 && channels % 4 == 0 && in_ld % 4 == 0 && out->ld % 4 == 0;
-    // Four-channel form: runs of 8 tokens where that still is a CTA of 128 threads for every place on the GPU (about 65536 threads at the registers
-    // a run of 8 takes), else of 4.
-    const bool full = (long long)step->n_tok * (channels / 4) >= 8ll * 65536;
-    const int run = !four ? kConvRun : full ? 8 : 4;
-    const dim3 grid(four ? (channels + 511) / 512 : (channels + 127) / 128, (step->max_len + run - 1) / run, step->n_seq);
     INGOT_REQUIRE((step->max_len + kConvRun - 1) / kConvRun <= 65535, "ingot_causal_conv: too many tokens of one sequence in one step");
+    const bool four = taps >= 2 && taps <= kMaxConvTaps4 && channels % 4 == 0 && in_ld % 4 == 0 && out->ld % 4 == 0;
+    // Four-channel form: runs of 8 tokens where that still is a CTA of 128 threads for every place on the GPU (about 65536 threads at the registers
+    // a run of 8 takes), else of 4. A grid of the longest sequence's runs for every sequence is mostly empty CTAs where one prompt is beside many short portions:
+    // 63 decoded tokens beside a prompt of 2048 of 8192 channels took 343 us with runs of 8 (169 with runs of 16, as they were), and 34 with the runs of
+    // all sequences packed; of 2048 channels 86, 49 and 9. Finding one's sequence costs about a microsecond; past kPackedSeqs sequences runs of 16 bound the number of empty CTAs instead.
+    constexpr int kPackedSeqs = 1024;
+    auto rows = [&](int run) { return ((long long)step->max_len + run - 1) / run; };
+    int run = !four ? kConvRun : (long long)step->n_tok * (channels / 4) >= 8ll * 65536 ? 8 : 4;
+    const long long runs = (long long)step->n_tok / run + step->n_seq;  // at most, of all sequences
+    const bool sparse = four && rows(run) * step->n_seq > 2 * runs, packed = sparse && step->n_seq <= kPackedSeqs && runs <= 65535;
+    if (four && !packed) {
+        if (sparse) run = kConvRun;
+        while (rows(run) > 65535) run *= 2;  // 16 at most
+    }
+    const ConvParams p = {*step, in_dev, in_ld, in_bias_dev, w_dev, bias_dev, taps, channels, silu, state_dev, act_out(out)};
+    const dim3 grid(four ? (channels + 511) / 512 : (channels + 127) / 128, unsigned(packed ? runs : rows(run)), packed ? 1u : unsigned(step->n_seq));
     auto pick = [&](auto two, auto three, auto any) { return taps == 2 ? two : taps == 3 ? three : any; };
-    auto kernel = !four ? taps == 4 ? causal_conv_kernel<4> : taps < 2 || taps > 4 ? causal_conv_kernel<0> : pick(causal_conv_kernel<2>, causal_conv_kernel<3>, causal_conv_kernel<4>)
-                  : full ? pick(causal_conv4_kernel<2, 8>, causal_conv4_kernel<3, 8>, causal_conv4_kernel<4, 8>)
-                         : pick(causal_conv4_kernel<2, 4>, causal_conv4_kernel<3, 4>, causal_conv4_kernel<4, 4>);
+    auto kernel = !four      ? taps == 4 ? causal_conv_kernel<4> : taps < 2 || taps > 4 ? causal_conv_kernel<0> : pick(causal_conv_kernel<2>, causal_conv_kernel<3>, causal_conv_kernel<4>)
+                  : packed   ? run == 4 ? pick(causal_conv4_kernel<2, 4, true>, causal_conv4_kernel<3, 4, true>, causal_conv4_kernel<4, 4, true>)
+                                        : pick(causal_conv4_kernel<2, 8, true>, causal_conv4_kernel<3, 8, true>, causal_conv4_kernel<4, 8, true>)
+                  : run == 4 ? pick(causal_conv4_kernel<2, 4, false>, causal_conv4_kernel<3, 4, false>, causal_conv4_kernel<4, 4, false>)
+                  : run == 8 ? pick(causal_conv4_kernel<2, 8, false>, causal_conv4_kernel<3, 8, false>, causal_conv4_kernel<4, 8, false>)
+                             : pick(causal_conv4_kernel<2, 16, false>, causal_conv4_kernel<3, 16, false>, causal_conv4_kernel<4, 16, false>);
     INGOT_CUDA_TRY(ingot_launch_pdl(kernel, grid, dim3(128), 0, static_cast<cudaStream_t>(stream), p));
     return INGOT_OK;
 }
