@@ -3,6 +3,7 @@
 #pragma once
 
 #include "ingot_internal.cuh"
+#include "prompt_order.h"
 
 __device__ __forceinline__ uint4 ld_stream16(const void* p) {
     uint4 r;
@@ -67,11 +68,8 @@ __device__ __forceinline__ void mma_16816(float (&d)[4], uint32_t a0, uint32_t a
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// Which row tile and KV head a CTA of a prompt's attention takes. Later tiles may see more keys and go first. Up to two tiles per SM and head
-// the heads go side by side (grid.x = tiles x heads), so that the longest CTAs of all heads start first: with head after head the
-// last heads' long CTAs began when the SMs were about to run dry (4096 tokens, 32 / 8 heads: SMs busy 0.80 of the launch; inside a prompt's step
-// 207-241 -> 180-213 us per layer, 2048 tokens with chunks of their own, 8 KV heads: 69 -> 51; B200).
-// With more tiles each head's own tail is short, and one head after the other keeps the keys in use in L2.
+// Which row tile and KV head a CTA of a prompt's attention takes: later tiles may see more keys and go first, the heads side by side (grid.x = tiles x
+// heads) or one after the other (prompt_order.h).
 __device__ __forceinline__ void prompt_tile(int n_head_kv, int& tile, int& kvh) {
     if (gridDim.y == 1) {
         const int n = (int)gridDim.x / n_head_kv, t = (int)blockIdx.x / n_head_kv;
@@ -82,8 +80,8 @@ __device__ __forceinline__ void prompt_tile(int n_head_kv, int& tile, int& kvh) 
         kvh = blockIdx.y;
     }
 }
-inline dim3 prompt_grid(unsigned tiles, int n_head_kv, int z, int num_sms) {
-    return tiles <= 2u * unsigned(num_sms) ? dim3(tiles * unsigned(n_head_kv), 1, unsigned(z)) : dim3(tiles, unsigned(n_head_kv), unsigned(z));
+inline dim3 prompt_grid(unsigned tiles, int n_head_kv, int z, int num_sms, size_t key_bytes) {
+    return heads_side_by_side(tiles, num_sms, key_bytes) ? dim3(tiles * unsigned(n_head_kv), 1, unsigned(z)) : dim3(tiles, unsigned(n_head_kv), unsigned(z));
 }
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }

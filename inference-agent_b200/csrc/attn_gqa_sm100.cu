@@ -446,7 +446,7 @@ int launch_gqa_sm100(ingot_skv* kv, int layer, const AttendParams& p, cudaStream
         kv->tmaps = std::move(maps);
     }
     const int group = p.n_head / p.n_head_kv;
-    const dim3 grid = prompt_grid((unsigned)(((size_t)p.st.max_len * group + 2 * kTileRows - 1) / (2 * kTileRows)), p.n_head_kv, p.st.n_seq, kv->num_sms);
+    const dim3 grid = prompt_grid((unsigned)(((size_t)p.st.max_len * group + 2 * kTileRows - 1) / (2 * kTileRows)), p.n_head_kv, p.st.n_seq, kv->num_sms, prompt_key_bytes(p));
     INGOT_CUDA_TRY(ingot_launch_pdl(gqa_sm100_kernel, grid, dim3(kThreads), size_t(kSmemBytes), stream, kv->tmaps[layer], p));
     return INGOT_OK;
 }

@@ -834,7 +834,7 @@ int launch_attn_prefill_sm100(ingot_kv* kv, int layer, const void* q, int q_dtyp
         p.part = st->part;
         p.part_extent = st->part_floats;
     }
-    const dim3 grid = prompt_grid(row_tiles, kv->n_head_kv, n_split, kv->num_sms);
+    const dim3 grid = prompt_grid(row_tiles, kv->n_head_kv, n_split, kv->num_sms, size_t(q_pos0 + n_tok) * kv->n_head_kv * kHeadDim * 2 * sizeof(__half));
     INGOT_CUDA_TRY(ingot_launch_pdl(attn_prefill_sm100_kernel, grid, dim3(kThreads), size_t(kSmemBytes), stream, st->maps[size_t(layer) * 2],
                                     st->maps[size_t(layer) * 2 + 1], p));
     if (n_split > 1) {

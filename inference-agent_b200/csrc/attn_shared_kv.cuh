@@ -111,6 +111,12 @@ struct AttendParams {
     OutGate gate = {};
 };
 
+// Bytes of the rows that a sequence's tiles see at a time: all that the tables hold, or a window or chunk of them.
+inline size_t prompt_key_bytes(const AttendParams& p) {
+    const size_t held = size_t(p.max_blocks) * kBlockTokens, span = size_t(p.map.window > 0 ? p.map.window : p.map.chunk);
+    return (span > 0 && span < held ? span : held) * p.n_head_kv * p.dim * sizeof(__half);
+}
+
 // The plain kernel (f32 arithmetic, any row length up to 1024, window, chunk and sink); dtype of rows and queries.
 int launch_shared_kv_plain(const AttendParams& p, int dtype, cudaStream_t stream);
 
