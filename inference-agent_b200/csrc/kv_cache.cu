@@ -415,9 +415,12 @@ int ingot_attn_layers_host(ingot_kv* kv, int layer_begin, int layer_count, const
         float *const q_m = view(q_host, q_elems), *const k_m = view(k_host, kv_elems), *const v_m = view(v_host, kv_elems), *const o_m = view(out_host, q_elems);
         if (q_m && k_m && v_m && o_m) {
             // One split per range (every row crosses PCIe once): append and attention in one launch, the cached keys on their way to L2 while the
-            // rows arrive. 28 layers (B200): 300 keys 49.9 -> 43.8 us.
+            // rows arrive. 28 layers (B200): 300 keys 49.9 -> 43.8 us. A CTA reads its heads' queries before it writes their results, so these may lie where
+            // the queries do, but not over rows that other CTAs still have to read.
+            auto apart = [&](const float* rows, size_t elems) { return o_m + L * q_elems <= rows || rows + L * elems <= o_m; };
+            const bool joins = apart(k_m, kv_elems) && apart(v_m, kv_elems) && (o_m == q_m || apart(q_m, q_elems));
             const DecodePlan plan = decode_plan(kv, layer_count, 1, pos0 + 1, 0);
-            if (plan.n_parts == 1 && n_head / kv->n_head_kv <= 8 && layer_count <= 65535)
+            if (joins && plan.n_parts == 1 && n_head / kv->n_head_kv <= 8 && layer_count <= 65535)
                 return launch_attn_decode_append(kv, layer_begin, layer_count, q_m, k_m, v_m, inv_freq_dev, o_m, INGOT_F32, n_head, nullptr, pos0 + 1, plan, kv->part, s);
             const int rc = launch_rope_kv_append(kv, layer_begin, q_m, qh_d, k_m, v_m, inv_freq_dev, n_head, pos0, 1, nullptr, nullptr, nullptr, 0, layer_count, s);
             if (rc != INGOT_OK) return rc;
