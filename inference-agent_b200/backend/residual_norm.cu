@@ -482,7 +482,8 @@ cudaError_t launch_rows(const ingot_residual_norm& r, int groups, cudaStream_t s
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
-    auto kernel = groups > 1 ? residual_rows_kernel<kThreads, kGroups> : r.post.b || r.next.b ? residual_rows_kernel<kThreads, kCentred> : residual_rows_kernel<kThreads, kRms>;
+    const bool centred = (r.post.w && r.post.b) || (r.next.w && r.next.b);  // a bias without a weight is no norm's
+    auto kernel = groups > 1 ? residual_rows_kernel<kThreads, kGroups> : centred ? residual_rows_kernel<kThreads, kCentred> : residual_rows_kernel<kThreads, kRms>;
     if ((e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, RowsSmem<kThreads>::kBytes)) != cudaSuccess) return e;
     const int slots = num_sms * (512 / kThreads), rounds = (r.n_rows + slots - 1) / slots;
     return ingot_launch_pdl(kernel, dim3((r.n_rows + rounds - 1) / rounds), dim3(kThreads), RowsSmem<kThreads>::kBytes, s, r, 1.0f / float(r.n_mean));
