@@ -28,7 +28,7 @@ def test_nothing_starts_before_the_metadata_is_there(table_kind):
     """Captured only, as a step's first two launches: the second one hangs on the fetch by an ordinary edge."""
     import torch
     L = M.lib()
-    n = 60 if table_kind == "odd rows" else 64
+    n = 62 if table_kind == "odd rows" else 64
     host, meta = torch.zeros(64, dtype=torch.int32, pin_memory=True), torch.empty(64, dtype=torch.int32, device="cuda")
     table, out = torch.zeros(8, n, dtype=torch.bfloat16, device="cuda"), torch.empty(4, n, device="cuda")
     words = torch.zeros(1, dtype=torch.int32, device="cuda")
