@@ -756,7 +756,7 @@ __global__ void __launch_bounds__(128) gated_lru_kernel(const LruParams p) {
 // keeps them; the recurrence itself - two dependent operations a token - goes from warp to warp through shared memory, while the others compute. Beside the state
 // the warps hand on what the chunk adds up to from zero, its sum of log a and the state that it began with: the next chunk begins with what the link pass makes of
 // those. The next tile's rows are requested before the current tile's states.
-// Bound by instructions (expm1, sigmoids, square root: about 190 per value), which the passes spend twice on every value, and by the way from warp to
+// Bound by instructions (expm1, sigmoids, square root: about 130 per value), which the passes spend twice on every value, and by the way from warp to
 // warp (about 420 cycles). Against the passes over chunks (B200, calls replayed as a graph): 2048 tokens x 4096 channels 95 -> 57 us, 1000 x 4096 47 -> 30,
 // 300 x 4096 28 -> 15, 2048 x 8192 179 -> 111.
 constexpr int kLruRun = 8, kLruWarps = 16;
