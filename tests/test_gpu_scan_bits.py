@@ -1,5 +1,6 @@
 """Streams of recurrences over channels (csrc/recurrent.cu) do the arithmetic of the passes over chunks in their order: a sequence that is alone in its step
-(chunks: too few channels for a stream) and 33 times the same (streams) leave the same bits, outputs and states, over two portions; a sequence that is one chunk has those of its tokens one after the other."""
+(chunks: too few channels for a stream) and many times the same (streams) leave the same bits, outputs and states, over two portions; a sequence that is one
+chunk has those of its tokens one after the other. test_scan_routes.py checks that the two take different launches."""
 import ctypes as C
 
 import numpy as np
@@ -8,9 +9,10 @@ import pytest
 from hybrid_step import Step, act_out, dev, lib, plan
 
 pytestmark = pytest.mark.gpu
-COPIES = 33
-# (tokens, tokens of a chunk): whole; chunks of whole tiles and of others; more chunks than lanes; chunks of single tokens
-CUTS = [(131, 10 ** 9), (131, 48), (300, 32), (265, 41), (1111, 32), (70, 1), (129, 16)]
+# (tokens, tokens of a chunk): more chunks than lanes, chunks of whole tiles and of others, of single tokens, two
+CUTS = [(1111, 32), (600, 48), (523, 41), (450, 16), (441, 1), (700, 129), (500, 260)]
+SCANS = [(128, 3, 36), (124, 16, 36), (120, 20, 36), (128, 32, 36), (192, 3, 49), (192, 16, 49), (188, 24, 49), (192, 31, 49)]  # channels, states, copies: 32 and 64 channels per CTA
+UNITS = [(128, 32, 36), (99, 33, 36)]  # channels, block, copies
 
 
 def token_by_token(run, n):
@@ -23,20 +25,20 @@ def token_by_token(run, n):
     assert np.array_equal(out[0].view(np.int32), np.concatenate(parts).view(np.int32)) and np.array_equal(left.view(np.int32), state.view(np.int32))
 
 
-def both(run, portions):
+def both(run, copies):
     """run(copies, portion, state or None) -> (outputs [copies, n, channels], state [copies, ...])."""
     one = many = None
-    for portion in range(portions):
+    for portion in (0, 1):
         a, one = run(1, portion, one)
-        b, many = run(COPIES, portion, many)
+        b, many = run(copies, portion, many)
         for x, y in ((a, b), (one, many)):
             assert np.isfinite(x).all()
             assert all(np.array_equal(x[0].view(np.int32), v.view(np.int32)) for v in y)
 
 
-@pytest.mark.parametrize("inner,n_state", [(36, 3), (92, 16), (64, 20), (96, 32), (200, 3), (200, 16), (196, 24), (192, 31)])
+@pytest.mark.parametrize("inner,n_state,copies", SCANS)
 @pytest.mark.parametrize("n,chunk", CUTS)
-def test_selective_scan(n, chunk, inner, n_state):
+def test_selective_scan(n, chunk, inner, n_state, copies):
     """Both widths of a CTA and every number of states per lane; decays from nearly none to fast ones."""
     import torch
     rng = np.random.default_rng(n + inner)
@@ -59,13 +61,13 @@ def test_selective_scan(n, chunk, inner, n_state):
         torch.cuda.synchronize()
         return out.cpu().numpy().reshape(copies, m, inner), state.cpu().numpy()
 
-    both(run, 2)
+    both(run, copies)
     token_by_token(run, n)
 
 
-@pytest.mark.parametrize("width,block", [(32, 32), (90, 18), (257, 257)])
+@pytest.mark.parametrize("width,block,copies", UNITS)
 @pytest.mark.parametrize("n,chunk", CUTS)
-def test_gated_lru(n, chunk, width, block):
+def test_gated_lru(n, chunk, width, block, copies):
     import torch
     rng = np.random.default_rng(n + width)
     dv = [dev(v) for v in (rng.standard_normal(width), rng.standard_normal(width), np.log1p(np.exp(rng.uniform(-6, 1, width))), rng.standard_normal(width))]
@@ -84,5 +86,5 @@ def test_gated_lru(n, chunk, width, block):
         torch.cuda.synchronize()
         return out.cpu().numpy().reshape(copies, m, width), state.cpu().numpy()
 
-    both(run, 2)
+    both(run, copies)
     token_by_token(run, n)

@@ -65,14 +65,32 @@ def chunk_tokens(lens, threads, sms=148, per_sm=1024):
     return even
 
 
-def test_ways_that_were_measured(tmp_path):
+@pytest.fixture(scope="module")
+def ways(tmp_path_factory):
+    """[(kind, channels, states, chunk, [(tokens, sequences), ...])] -> what such steps do."""
     cxx = shutil.which("g++")
     if not cxx:
         pytest.skip("no g++")
-    exe = str(tmp_path / "routes")
+    exe = str(tmp_path_factory.mktemp("routes") / "routes")
     subprocess.run([cxx, "-std=c++17", "-O1", "-Wall", "-Wextra", "-Werror", "-fsanitize=address,undefined", "-I", os.path.join(ROOT, "inference-agent_b200", "csrc"),
                     os.path.join(ROOT, "tests", "native", "scan_routes.cpp"), "-o", exe], check=True, timeout=120)
-    lines = "".join(f"{kind} {channels} {16 if kind == 'scan' else 1} 148 {chunk_tokens(lens, channels * (2 if kind == 'scan' else 1))} "
-                    + " ".join(f"{n} {count}" for n, count in lens) + "\n" for kind, channels, lens, _ in MEASURED)
-    got = subprocess.run([exe], input=lines, capture_output=True, text=True, check=True, timeout=60).stdout.split()
+
+    def of(steps):
+        lines = "".join(f"{kind} {channels} {states} 148 {chunk} " + " ".join(f"{n} {count}" for n, count in lens) + "\n" for kind, channels, states, chunk, lens in steps)
+        return subprocess.run([exe], input=lines, capture_output=True, text=True, check=True, timeout=60).stdout.split()
+    return of
+
+
+def test_ways_that_were_measured(ways):
+    got = ways([(kind, channels, 16 if kind == "scan" else 1, chunk_tokens(lens, channels * (2 if kind == "scan" else 1)), lens) for kind, channels, lens, _ in MEASURED])
     assert [(m[:3], m[3], g) for m, g in zip(MEASURED, got) if m[3] != g] == [] and len(got) == len(MEASURED)
+
+
+def test_shapes_of_the_comparison_of_bits(ways):
+    """test_gpu_scan_bits.py compares chunks with streams."""
+    import test_gpu_scan_bits as B
+    for kind, shapes in (("scan", [(c, B.lib().ingot_scan_state_pad(n), m) for c, n, m in B.SCANS]), ("gated", [(c, 1, m) for c, _, m in B.UNITS])):
+        steps = [(kind, c, states, chunk, [(n, m)]) for c, states, copies in shapes for n, chunk in B.CUTS for m in (1, copies)]
+        got = ways(steps)
+        wrong = [(s, g) for s, g, want in zip(steps, got, ["chunks", "stream"] * len(steps)) if g != want and (g, want, s[3]) != ("tile", "chunks", 260)]
+        assert wrong == [], wrong
